@@ -19,6 +19,9 @@ HERE = Path(__file__).resolve().parent
 SOURCES = ["tx_api.cu", "tx_pack.cu", "tx_gemv.cu", "tx_prefill.cu", "tx_aux.cu", "tx_encode.cu"]
 LIBRARY = HERE / "libtexelator_b200.so"
 STAMP = HERE / ".build_stamp"
+BINDING_SOURCE = HERE / "tx_torch.cpp"
+BINDING = HERE / "_tx_torch.so"          # CPython module: the operator call without Python in between
+BINDING_STAMP = HERE / ".binding_stamp"
 
 
 def source_digest() -> str:
@@ -56,6 +59,30 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     return LIBRARY
 
 
+def build_binding(force: bool = False, verbose: bool = False) -> Path:
+    """The CPython module ``_tx_torch`` (host code only; g++ against the installed torch's headers)."""
+    import sysconfig
+
+    import torch
+    digest = hashlib.sha256(BINDING_SOURCE.read_bytes() + torch.__version__.encode() + sys.version.encode()).hexdigest()
+    if not force and BINDING.exists() and BINDING_STAMP.exists() and BINDING_STAMP.read_text().strip() == digest:
+        return BINDING
+    root = Path(torch.__file__).resolve().parent
+    cuda = Path(nvcc_path()).resolve().parent.parent
+    include = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include", sysconfig.get_paths()["include"], cuda / "include"]
+    command = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+               *[f"-I{path}" for path in include], str(BINDING_SOURCE), "-o", str(BINDING), f"-L{root / 'lib'}", f"-Wl,-rpath,{root / 'lib'}",
+               "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python"]
+    result = subprocess.run(command, capture_output=True, text=True)
+    if verbose or result.returncode:
+        sys.stderr.write(result.stdout + result.stderr)
+    if result.returncode:
+        raise RuntimeError(f"g++ failed with exit code {result.returncode} on {BINDING_SOURCE.name}")
+    BINDING_STAMP.write_text(digest + "\n")
+    return BINDING
+
+
 if __name__ == "__main__":
+    build_binding(force="--force" in sys.argv, verbose="--verbose" in sys.argv)
     path = build(force="--force" in sys.argv, verbose="--verbose" in sys.argv)
     print(path, os.path.getsize(path), "bytes")

@@ -6,7 +6,8 @@ Mirrors ``texelator/runtime.py`` of the reference (``extension()`` :27-63,
 :242-263, ``free`` :266-274) with the same names, argument meaning and error
 behaviour, but the object returned by ``extension()`` drives the sm_100a C-ABI
 library ``texelator_b200/cuda/libtexelator_b200.so`` through ctypes instead of a
-pybind11 torch extension.  PyTorch is used for device memory and streams only.
+pybind11 torch extension; the operator call itself (``linear``, ``linear_out``) goes through the small
+CPython module ``cuda/_tx_torch.so``.  PyTorch is used for device memory and streams only.
 
 There is no CPU fallback: if the CUDA library is missing and cannot be built,
 ``extension()`` raises.
@@ -27,6 +28,7 @@ from .adapters import resolve_parent
 
 PACKAGE_ROOT = Path(__file__).resolve().parent
 LIBRARY_PATH = PACKAGE_ROOT / "cuda" / "libtexelator_b200.so"
+BINDING_PATH = PACKAGE_ROOT / "cuda" / "_tx_torch.so"
 _EXTENSION = None
 PREFILL_THRESHOLD = int(os.environ.get("TEXELATOR_PREFILL_THRESHOLD", "16"))
 PREFILL_TILE_ROWS = int(os.environ.get("TEXELATOR_PREFILL_TILE_ROWS", "1024"))
@@ -92,13 +94,35 @@ def load_library(path: Path | None = None) -> ctypes.CDLL:
     return library
 
 
+def load_binding(path: Path | None = None):
+    """Import the CPython module of the operator call (raises if it does not fit the installed torch)."""
+    from importlib.machinery import ExtensionFileLoader
+    from importlib.util import module_from_spec, spec_from_file_location
+    location = str(path or BINDING_PATH)
+    spec = spec_from_file_location("_tx_torch", location, loader=ExtensionFileLoader("_tx_torch", location))
+    module = module_from_spec(spec)
+    spec.loader.exec_module(module)
+    return module
+
+
 class _Extension:
     """The module-like object the reference gets from ``extension()``
-    (texelator/cuda/extension.cpp:27-48): same function names and semantics."""
+    (texelator/cuda/extension.cpp:27-48): same function names and semantics.
 
-    def __init__(self, library: ctypes.CDLL):
-        self._lib = library
+    ``linear(handle, x)`` returns ``[..., M]`` in the input's type; ``linear_out(handle, x, y)`` writes into a
+    caller-provided output (static buffers for CUDA graphs).  Both are functions of the native binding."""
+
+    def __init__(self, library: ctypes.CDLL, binding):
+        self._lib, self._binding = library, binding
         self._shapes: dict[int, tuple[int, int, int]] = {}   # handle -> (M, K, device)
+        address = lambda function: ctypes.cast(function, ctypes.c_void_p).value
+        binding.bind(address(library.tx_linear), address(library.tx_last_error))
+        self.linear, self.linear_out = binding.linear, binding.linear_out
+
+    def _remember(self, handle: int, m: int, k: int, device: int) -> int:
+        self._shapes[handle] = (m, k, device)
+        self._binding.remember(handle, m, k, device)
+        return handle
 
     # -- helpers -------------------------------------------------------------
     def _check(self, status: int) -> None:
@@ -126,9 +150,7 @@ class _Extension:
         handle = _u64(0)
         self._check(self._lib.tx_pack_encoded(blocks.data_ptr(), blocks.numel(), scales.data_ptr(), m,
                                               bias_ptr, bias_dtype, device, ctypes.byref(handle)))
-        k = 16 * (blocks.numel() // (8 * m))
-        self._shapes[handle.value] = (m, k, device)
-        return handle.value
+        return self._remember(handle.value, m, 16 * (blocks.numel() // (8 * m)), device)
 
     def pack_encoded_device(self, blocks: torch.Tensor, scales: torch.Tensor, bias: torch.Tensor | None = None) -> int:
         """``pack_encoded`` for blocks/scales that already live on the current CUDA device (an
@@ -144,8 +166,7 @@ class _Extension:
         handle = _u64(0)
         self._check(self._lib.tx_pack_encoded(blocks.data_ptr(), blocks.numel(), scales.data_ptr(), m,
                                               bias_ptr, bias_dtype, device, ctypes.byref(handle)))
-        self._shapes[handle.value] = (m, 16 * (blocks.numel() // (8 * m)), device)
-        return handle.value
+        return self._remember(handle.value, m, 16 * (blocks.numel() // (8 * m)), device)
 
     def pack_encoded_shard(self, blocks: torch.Tensor, scales: torch.Tensor, m: int, k: int,
                            rows: tuple[int, int], kblocks: tuple[int, int],
@@ -162,8 +183,7 @@ class _Extension:
         self._check(self._lib.tx_pack_encoded_shard(blocks.data_ptr(), blocks.numel(), scales.data_ptr(), m, k,
                                                     rows[0], rows[1], kblocks[0], kblocks[1], bias_ptr, bias_dtype,
                                                     device, ctypes.byref(handle)))
-        self._shapes[handle.value] = (rows[1] - rows[0], 16 * (kblocks[1] - kblocks[0]), device)
-        return handle.value
+        return self._remember(handle.value, rows[1] - rows[0], 16 * (kblocks[1] - kblocks[0]), device)
 
     @staticmethod
     def _bias_argument(bias, m, device):
@@ -187,27 +207,6 @@ class _Extension:
         if x.size(-1) != k or x.get_device() != device:
             raise RuntimeError("input shape/device mismatch")
         return m, k, device, x.numel() // k
-
-    @staticmethod
-    def _dtype_flag(x: torch.Tensor) -> int:
-        return DTYPE_BF16 if x.dtype == torch.bfloat16 else DTYPE_F16
-
-    def linear(self, handle: int, x: torch.Tensor) -> torch.Tensor:
-        m, k, device, tokens = self._activation(handle, x)
-        y = torch.empty(x.shape[:-1] + (m,), dtype=x.dtype, device=x.device)
-        if tokens:
-            self._check(self._lib.tx_linear(handle, x.data_ptr(), y.data_ptr(), tokens, self._dtype_flag(x),
-                                            torch.cuda.current_stream(device).cuda_stream))
-        return y
-
-    def linear_out(self, handle: int, x: torch.Tensor, y: torch.Tensor) -> torch.Tensor:
-        """``linear`` into a caller-provided output (static buffers for CUDA graphs)."""
-        m, k, device, tokens = self._activation(handle, x)
-        if y.numel() != tokens * m or y.dtype != x.dtype or not y.is_contiguous() or y.device != x.device:
-            raise RuntimeError("input shape/device mismatch")
-        self._check(self._lib.tx_linear(handle, x.data_ptr(), y.data_ptr(), tokens, self._dtype_flag(x),
-                                        torch.cuda.current_stream(device).cuda_stream))
-        return y
 
     def linear_static_scratch(self, handle: int, x: torch.Tensor) -> torch.Tensor:
         """``linear`` for a small token group through the entry point that allocates nothing on the
@@ -278,6 +277,7 @@ class _Extension:
 
     def free(self, handle: int) -> None:
         self._shapes.pop(handle, None)
+        self._binding.forget(handle)
         self._check(self._lib.tx_free(handle))
 
     def palette_probe(self) -> torch.Tensor:
@@ -487,15 +487,17 @@ def extension(verbose: bool = False):
     ``TEXELATOR_DISABLE_JIT`` forbids the nvcc build."""
     global _EXTENSION
     if _EXTENSION is None:
-        if not LIBRARY_PATH.exists():
+        if not (LIBRARY_PATH.exists() and BINDING_PATH.exists()):
             if os.environ.get("TEXELATOR_DISABLE_JIT", "").upper() in {"1", "ON", "YES", "TRUE"}:
                 raise RuntimeError(
                     "the prebuilt Texelator CUDA library is unavailable and JIT compilation is disabled")
-            from .cuda.build import build
-            build(verbose=verbose)
+            from .cuda.build import build, build_binding
+            if not LIBRARY_PATH.exists():
+                build(verbose=verbose)
+            build_binding(verbose=verbose)
         try:
-            _EXTENSION = _Extension(load_library())
-        except (OSError, AttributeError) as error:
+            _EXTENSION = _Extension(load_library(), load_binding())
+        except (OSError, AttributeError, ImportError) as error:
             raise RuntimeError(f"the Texelator CUDA library could not be loaded: {error}") from error
     return _EXTENSION
 
@@ -514,12 +516,13 @@ class TexelatorLinear(nn.Module):
         self.bias = bias
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        ext = extension()
-        x = x.contiguous()
+        linear = (_EXTENSION or extension()).linear
+        if not x.is_contiguous():
+            x = x.contiguous()
         if len(self.handles) == 1:
-            y = ext.linear(self.handles[0], x)
+            y = linear(self.handles[0], x)
         else:
-            y = torch.cat([ext.linear(handle, x) for handle in self.handles], dim=-1)
+            y = torch.cat([linear(handle, x) for handle in self.handles], dim=-1)
         return y if self.bias is None else y + self.bias
 
 
