@@ -454,6 +454,16 @@ static TileShape backend_shape(int backend) {
   }
 }
 
+// Handles that were packed without a tuned backend.  Short prompts are paced by the producers, so the narrowest tile that
+// holds all tokens wins; from 192 tokens on, 192-token tiles unless the 256-token ones need fewer token blocks per SM.
+int prefill_choose_backend(const Handle *h, int tokens) {
+  if (tokens <= 64) return 8;
+  if (tokens <= 128) return 7;
+  const int blocks = (h->M + 127) / 128;
+  const auto waves = [&](int bn) { return (long(blocks) * ((tokens + bn - 1) / bn) + 147) / 148 * bn; };
+  return waves(192) < waves(256) ? 9 : 5;
+}
+
 bool prefill_tile_eligible(const Handle *h, int backend, int tokens) {
   return backend_shape(backend).mt != 0 && tokens >= 1 && h->K % 16 == 0 && encode_tiled_entry() != nullptr;
 }
