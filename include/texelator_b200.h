@@ -204,6 +204,8 @@ int tx_kernel_status(int device, int clear);
  *   add_rmsnorm      : h += delta (delta may be null); y = rmsnorm(h) * weight, per token row
  *   rope_append      : rotate q and k of one token in place (rotate-half), append k and v to the
  *                      caches [kv_heads, max_len, head_dim] at *position (device int64)
+ *   rope_append_prompt : the same for `tokens` rows of qkv at positions first, first + 1, ... (head_dim a
+ *                      multiple of 16)
  *   attention_decode : one query per head over cache positions 0..*position, grouped-query; `scratch`
  *                      holds q_heads * ceil(max_len/128) * (head_dim+2) floats; head_dim must be 128
  *   attention_step   : rope_append + attention_decode of one token in one call (q is rotated on the
@@ -259,6 +261,8 @@ int tx_aux_peer_best_token(const float *local_score, const void *local_token, lo
                            int world, void *epoch_word, void *next_token, void *stream);
 int tx_aux_rope_append(void *qkv, const float *cos_table, const float *sin_table, const void *position, void *k_cache,
                        void *v_cache, int q_heads, int kv_heads, int head_dim, int max_len, void *stream);
+int tx_aux_rope_append_prompt(void *qkv, const float *cos_table, const float *sin_table, int first, int tokens, void *k_cache,
+                              void *v_cache, int q_heads, int kv_heads, int head_dim, int max_len, void *stream);
 int tx_aux_attention_decode(const void *qkv, const void *k_cache, const void *v_cache, const void *position, float *scratch,
                             void *out, int q_heads, int kv_heads, int head_dim, int max_len, float scale, void *stream);
 int tx_aux_attention_step(const void *qkv, const float *cos_table, const float *sin_table, const void *position, void *k_cache,

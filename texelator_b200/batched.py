@@ -115,23 +115,28 @@ class BatchedBC4Decoder(BC4Decoder):
         """Run one sequence's prompt from position 0 (the linears take the tensor-core path from the prefill
         threshold on), fill its cache rows, set its position; returns the final hidden states ``[T, hidden]``."""
         tokens = ids.numel()
-        index = torch.arange(tokens, device=self.device)
-        cos, sin = self.cos[:tokens], self.sin[:tokens]
         k_all, v_all = self.k_cache, self.v_cache
         self.k_cache, self.v_cache = k_all[:, sequence], v_all[:, sequence]       # views: _layer indexes [layer]
         try:
-            def attend(layer, q):
-                k = self.k_cache[layer][:, :tokens].unsqueeze(0)
-                v = self.v_cache[layer][:, :tokens].unsqueeze(0)
-                return F.scaled_dot_product_attention(q, k, v, is_causal=True, enable_gqa=True)
-
             h = self.embed.index_select(0, ids.to(self.device).reshape(-1))
-            for layer in range(self.config.layers):
-                h = self._layer(layer, h, cos, sin, index, attend, dense)
+            if tokens and self._prompt_kernels(dense):
+                h = self._prompt_stack(h)
+            else:
+                index = torch.arange(tokens, device=self.device)
+                cos, sin = self.cos[:tokens], self.sin[:tokens]
+
+                def attend(layer, q):
+                    k = self.k_cache[layer][:, :tokens].unsqueeze(0)
+                    v = self.v_cache[layer][:, :tokens].unsqueeze(0)
+                    return F.scaled_dot_product_attention(q, k, v, is_causal=True, enable_gqa=True)
+
+                for layer in range(self.config.layers):
+                    h = self._layer(layer, h, cos, sin, index, attend, dense)
+                h = _rmsnorm(h, self.final_norm, self.config.rms_eps)
         finally:
             self.k_cache, self.v_cache = k_all, v_all
         self.pos[sequence] = tokens
-        return _rmsnorm(h, self.final_norm, self.config.rms_eps)
+        return h
 
     @torch.no_grad()
     def fill_context(self, sequence: int, first: int, last: int, seed: int = 0) -> None:

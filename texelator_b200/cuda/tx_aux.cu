@@ -558,6 +558,49 @@ __global__ void __launch_bounds__(64) rope_append_kernel(__nv_bfloat16 *__restri
   }
 }
 
+// The same for the tokens of a prompt: positions first, first + 1, ...; qkv [tokens, q_rows + 2 kv_rows], q and k
+// rotated in place, k and v appended to the caches.  Bound by memory (every value is read once and written at most
+// twice): a thread owns eight dimensions of both halves of one head, so all accesses are 16 bytes and a warp
+// covers four heads of a token.
+__global__ void __launch_bounds__(256) rope_append_prompt_kernel(__nv_bfloat16 *__restrict__ qkv, const float *__restrict__ cos_table,
+                                                                 const float *__restrict__ sin_table, int first, int tokens,
+                                                                 __nv_bfloat16 *__restrict__ k_cache, __nv_bfloat16 *__restrict__ v_cache,
+                                                                 int q_heads, int kv_heads, int head_dim, int max_len) {
+  grid_launch_dependents();
+  grid_dependency_wait();
+  const int half = head_dim / 2, per_head = half / 8, heads = q_heads + 2 * kv_heads;
+  const size_t total = size_t(tokens) * heads * per_head;
+  for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += size_t(gridDim.x) * blockDim.x) {
+    const int part = int(i % per_head), head = int(i / per_head % heads), token = int(i / (size_t(per_head) * heads));
+    const int pos = first + token;
+    uint4 *lo = reinterpret_cast<uint4 *>(qkv + (size_t(token) * heads + head) * head_dim + part * 8);
+    uint4 *hi = reinterpret_cast<uint4 *>(qkv + (size_t(token) * heads + head) * head_dim + half + part * 8);
+    uint4 a = __ldcg(lo), b = __ldcg(hi);
+    if (head < q_heads + kv_heads) {
+      const float4 *ct = reinterpret_cast<const float4 *>(cos_table + size_t(pos) * half + part * 8);
+      const float4 *st = reinterpret_cast<const float4 *>(sin_table + size_t(pos) * half + part * 8);
+      const float4 c4[2] = {ct[0], ct[1]}, s4[2] = {st[0], st[1]};
+      const float *c = reinterpret_cast<const float *>(c4), *s = reinterpret_cast<const float *>(s4);
+      __nv_bfloat162 *pa = reinterpret_cast<__nv_bfloat162 *>(&a), *pb = reinterpret_cast<__nv_bfloat162 *>(&b);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 x1 = __bfloat1622float2(pa[e]), x2 = __bfloat1622float2(pb[e]);
+        pa[e] = __floats2bfloat162_rn(x1.x * c[2 * e] - x2.x * s[2 * e], x1.y * c[2 * e + 1] - x2.y * s[2 * e + 1]);
+        pb[e] = __floats2bfloat162_rn(x2.x * c[2 * e] + x1.x * s[2 * e], x2.y * c[2 * e + 1] + x1.y * s[2 * e + 1]);
+      }
+      *lo = a;
+      *hi = b;
+    }
+    if (head >= q_heads) {
+      const bool key = head < q_heads + kv_heads;
+      __nv_bfloat16 *cache = key ? k_cache : v_cache;
+      __nv_bfloat16 *dst = cache + (size_t(head - q_heads - (key ? 0 : kv_heads)) * max_len + pos) * head_dim + part * 8;
+      *reinterpret_cast<uint4 *>(dst) = a;
+      *reinterpret_cast<uint4 *>(dst + half) = b;
+    }
+  }
+}
+
 // Single-query attention over cache positions [0, pos], split along the sequence: CTA (split, kv head)
 // handles kKeys keys for the G query heads of its group.  Scores: one warp per key, lanes across the
 // head dimension (coalesced 256-byte key rows, q in registers).  Values: one thread per head dimension
@@ -1559,6 +1602,21 @@ int tx_aux_rope_append(void *qkv, const float *cos_table, const float *sin_table
                      static_cast<__nv_bfloat16 *>(qkv), cos_table, sin_table, static_cast<const long long *>(position),
                      static_cast<__nv_bfloat16 *>(k_cache), static_cast<__nv_bfloat16 *>(v_cache), q_heads, kv_heads,
                      head_dim, max_len));
+  count_launch();
+  TX_CUDA(cudaGetLastError());
+  return TX_OK;
+}
+
+int tx_aux_rope_append_prompt(void *qkv, const float *cos_table, const float *sin_table, int first, int tokens, void *k_cache,
+                              void *v_cache, int q_heads, int kv_heads, int head_dim, int max_len, void *stream) {
+  if (!qkv || !cos_table || !sin_table || !k_cache || !v_cache || q_heads < 1 || kv_heads < 1 || head_dim < 16 || head_dim % 16)
+    return fail(TX_EINVAL, "tx_aux_rope_append_prompt: head_dim must be a multiple of 16 and no pointer null");
+  if (tokens < 1 || first < 0 || max_len - first < tokens) return fail(TX_EINVAL, "tx_aux_rope_append_prompt: positions must lie inside the cache");
+  const size_t total = size_t(tokens) * (q_heads + 2 * kv_heads) * (head_dim / 16);
+  const int grid = int(std::min<size_t>((total + 255) / 256, 148 * 8));
+  TX_CUDA(launch_pdl(rope_append_prompt_kernel, dim3(grid), dim3(256), 0, static_cast<cudaStream_t>(stream),
+                     static_cast<__nv_bfloat16 *>(qkv), cos_table, sin_table, first, tokens, static_cast<__nv_bfloat16 *>(k_cache),
+                     static_cast<__nv_bfloat16 *>(v_cache), q_heads, kv_heads, head_dim, max_len));
   count_launch();
   TX_CUDA(cudaGetLastError());
   return TX_OK;

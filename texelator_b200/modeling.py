@@ -335,22 +335,58 @@ class BC4Decoder:
         act = (F.silu(gu[:, :, 0].float()) * gu[:, :, 1].float()).to(h.dtype).reshape(tokens, self.i_loc)
         return h + self._reduce(self._linear(self.h_down[layer], act, dense))
 
+    def _prompt_kernels(self, dense) -> bool:
+        """Whether a prompt can run on the library's row kernels instead of PyTorch ops between the linears."""
+        c = self.config
+        return not dense and c.head_dim % 16 == 0 and c.head_dim <= 256 and c.hidden % 8 == 0 and c.hidden <= 16384 and self.i_loc % 8 == 0
+
+    def _prompt_stack(self, h):
+        """All layers and the final norm over the prompt rows ``h [T, hidden]`` (overwritten): nine launches a layer with the
+        rounding points of ``_layer``.  Written with PyTorch ops the same layer is 58 launches that move the gate/up rows
+        (the widest of the layer) seven times in fp32; the host could not keep the GPU busy with them and they
+        cost more than half of what the linears did."""
+        c, ext = self.config, self.ext
+        tokens = h.shape[0]
+        q_heads, kv_heads = c.q_heads // self.world, c.kv_heads // self.world
+        make = lambda columns: torch.empty(tokens, columns, dtype=torch.bfloat16, device=self.device)
+        x, qkv, gate_up, act, out = make(c.hidden), make(self.q_loc + 2 * self.kv_loc), make(2 * self.i_loc), make(self.i_loc), make(c.hidden)
+        q = qkv[:, :self.q_loc].view(tokens, q_heads, c.head_dim).transpose(0, 1).unsqueeze(0)
+        delta = None
+        for layer in range(c.layers):
+            ext.add_rmsnorm(h, delta, self.norm1[layer], x, c.rms_eps)
+            ext.linear_out(self.h_qkv[layer], x, qkv)
+            k_cache, v_cache = self.k_cache[layer], self.v_cache[layer]
+            ext.rope_append_prompt(qkv, self.cos, self.sin, 0, k_cache, v_cache, q_heads, kv_heads, c.head_dim)
+            attended = F.scaled_dot_product_attention(q, k_cache[:, :tokens].unsqueeze(0), v_cache[:, :tokens].unsqueeze(0),
+                                                      is_causal=True, enable_gqa=True)
+            attended = attended.squeeze(0).transpose(0, 1).reshape(tokens, self.q_loc).contiguous()
+            delta = self._reduce(ext.linear_out(self.h_o[layer], attended, out))
+            ext.add_rmsnorm(h, delta, self.norm2[layer], x, c.rms_eps)
+            ext.linear_out(self.h_gu[layer], x, gate_up)
+            ext.silu_mul_pairs(gate_up, act)
+            delta = self._reduce(ext.linear_out(self.h_down[layer], act, out))
+        ext.add_rmsnorm(h, delta, self.final_norm, x, c.rms_eps)
+        return x
+
     @torch.no_grad()
     def prefill(self, ids: torch.Tensor, dense: bool = False) -> torch.Tensor:
         """Run a prompt from position 0, fill the KV cache, return the final hidden states ``[T, hidden]``."""
         tokens = ids.numel()
-        index = torch.arange(tokens, device=self.device)
-        cos, sin = self.cos[:tokens], self.sin[:tokens]
-
-        def attend(layer, q):
-            k = self.k_cache[layer][:, :tokens].unsqueeze(0)
-            v = self.v_cache[layer][:, :tokens].unsqueeze(0)
-            return F.scaled_dot_product_attention(q, k, v, is_causal=True, enable_gqa=True)
-
         h = self.embed.index_select(0, ids.to(self.device).reshape(-1))
-        for layer in range(self.config.layers):
-            h = self._layer(layer, h, cos, sin, index, attend, dense)
-        h = _rmsnorm(h, self.final_norm, self.config.rms_eps)
+        if tokens and self._prompt_kernels(dense):
+            h = self._prompt_stack(h)
+        else:
+            index = torch.arange(tokens, device=self.device)
+            cos, sin = self.cos[:tokens], self.sin[:tokens]
+
+            def attend(layer, q):
+                k = self.k_cache[layer][:, :tokens].unsqueeze(0)
+                v = self.v_cache[layer][:, :tokens].unsqueeze(0)
+                return F.scaled_dot_product_attention(q, k, v, is_causal=True, enable_gqa=True)
+
+            for layer in range(self.config.layers):
+                h = self._layer(layer, h, cos, sin, index, attend, dense)
+            h = _rmsnorm(h, self.final_norm, self.config.rms_eps)
         self.pos.fill_(tokens)
         self.mask.zero_()
         self.mask[..., :tokens] = True

@@ -67,6 +67,7 @@ C_API = {
     "tx_kernel_status": (_i32, [_i32, _i32]),
     "tx_aux_add_rmsnorm": (_i32, [_vp, _vp, _vp, _vp, _i32, _i32, ctypes.c_float, _vp]),
     "tx_aux_rope_append": (_i32, [_vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp]),
+    "tx_aux_rope_append_prompt": (_i32, [_vp, _vp, _vp, _i32, _i32, _vp, _vp, _i32, _i32, _i32, _i32, _vp]),
     "tx_aux_attention_decode": (_i32, [_vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, ctypes.c_float, _vp]),
     "tx_aux_allreduce_add_rmsnorm": (_i32, [_vp, _vp, _vp, _vp, _i32, ctypes.c_float, _vp, _vp, _i32, _i32, _vp, _vp]),
     "tx_aux_attention_step": (_i32, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, ctypes.c_float, _vp]),
@@ -344,6 +345,12 @@ class _Extension:
         self._check(self._lib.tx_aux_rope_append(qkv.data_ptr(), cos.data_ptr(), sin.data_ptr(), position.data_ptr(),
                                                  k_cache.data_ptr(), v_cache.data_ptr(), q_heads, kv_heads, head_dim,
                                                  k_cache.shape[1], self._stream(qkv)))
+
+    def rope_append_prompt(self, qkv, cos, sin, first: int, k_cache, v_cache, q_heads: int, kv_heads: int, head_dim: int) -> None:
+        """``rope_append`` for all rows of ``qkv [tokens, ...]`` at positions ``first, first + 1, ...``."""
+        self._check(self._lib.tx_aux_rope_append_prompt(qkv.data_ptr(), cos.data_ptr(), sin.data_ptr(), int(first), qkv.shape[0],
+                                                        k_cache.data_ptr(), v_cache.data_ptr(), q_heads, kv_heads, head_dim,
+                                                        k_cache.shape[1], self._stream(qkv)))
 
     def attention_decode(self, qkv, k_cache, v_cache, position, scratch, out, q_heads: int, kv_heads: int, head_dim: int) -> None:
         self._check(self._lib.tx_aux_attention_decode(qkv.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), position.data_ptr(),
