@@ -42,3 +42,58 @@ def test_native_call_checks_and_keywords(ext, lut):
     ext.free(h)
     with pytest.raises(RuntimeError, match="null Texelator handle"):
         ext.linear(h, x)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("tokens", [16, 64, 65, 128, 129, 400])
+def test_untuned_handle_matches_oracle(ext, lut, tokens, dtype):
+    m, k = 200, 656
+    blocks, scales, gen = _encoded(m, k, tokens, lut)
+    h = ext.pack_encoded(torch.from_numpy(blocks).reshape(-1), torch.from_numpy(scales))
+    x = torch.randn(tokens, k, generator=gen).cuda().to(dtype)
+    y = ext.linear(h, x).float().cpu().numpy()
+    xs = x.float().cpu().numpy()
+    ref = O.linear_bf16(xs, blocks, scales, lut) if dtype == torch.bfloat16 else O.linear_f16(xs, blocks, scales, lut)
+    # weights are not rounded to the activations' type here: 2^-9 (2^-12) per weight and output at most, in quadrature
+    assert O.rel_rms(y, ref) <= (1e-2 if dtype == torch.bfloat16 else 2e-3)
+    assert ext.handle_info(h)[4] == 0
+    ext.free(h)
+
+
+@pytest.mark.parametrize("tokens,first,q_heads,kv_heads,head_dim", [(1, 0, 4, 2, 128), (37, 5, 5, 1, 64), (130, 0, 16, 2, 128), (3, 61, 2, 2, 16)])
+def test_rope_append_prompt(ext, tokens, first, q_heads, kv_heads, head_dim):
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    max_len, half = first + tokens + 3, head_dim // 2
+    qkv = torch.randn(tokens, (q_heads + 2 * kv_heads) * head_dim, device="cuda", generator=gen).bfloat16()
+    angle = torch.rand(max_len, half, device="cuda", generator=gen) * 6.28
+    cos, sin = angle.cos(), angle.sin()
+    k_cache = torch.full((kv_heads, max_len, head_dim), 7.0, device="cuda", dtype=torch.bfloat16)
+    v_cache = k_cache.clone()
+    rows = qkv.float().view(tokens, -1, head_dim)
+    c, s = cos[first:first + tokens, None], sin[first:first + tokens, None]
+    x1, x2 = rows[..., :half], rows[..., half:]
+    rotated = torch.cat([x1 * c - x2 * s, x2 * c + x1 * s], -1).bfloat16()
+    expected_v = qkv.view(tokens, -1, head_dim)[:, q_heads + kv_heads:].clone()
+    ext.rope_append_prompt(qkv, cos, sin, first, k_cache, v_cache, q_heads, kv_heads, head_dim)
+    got = qkv.view(tokens, -1, head_dim)
+    # one bf16 rounding (2^-8 of the value at most between neighbours) of fp32 sums that may be contracted
+    close = lambda a, b: torch.allclose(a.float(), b.float(), rtol=2 ** -7, atol=1e-5)
+    assert close(got[:, :q_heads + kv_heads], rotated[:, :q_heads + kv_heads])
+    assert torch.equal(got[:, q_heads + kv_heads:], expected_v)
+    assert torch.equal(k_cache[:, first:first + tokens], got[:, q_heads:q_heads + kv_heads].transpose(0, 1))
+    assert torch.equal(v_cache[:, first:first + tokens], expected_v.transpose(0, 1))
+    assert bool((k_cache[:, :first] == 7).all()) and bool((v_cache[:, first + tokens:] == 7).all())
+    with pytest.raises(RuntimeError, match="inside the cache"):
+        ext.rope_append_prompt(qkv, cos, sin, max_len, k_cache, v_cache, q_heads, kv_heads, head_dim)
+
+
+@pytest.mark.parametrize("m,k", [(1, 16), (5, 528), (3, 1040), (130, 3168), (9, 2064)])
+def test_encoder_ragged_rows_match_restatement(ext, lut, m, k):
+    gen = torch.Generator().manual_seed(m + k)
+    w = torch.randn(m, k, generator=gen) * torch.exp(4 * torch.randn(m, 1, generator=gen))
+    w[w.abs() < 0.3 * w.abs().mean()] = 0
+    hdiag = torch.exp(torch.randn(k, generator=gen))
+    blocks, scales = ext.encode(w.cuda(), hdiag.cuda(), torch.from_numpy(lut).cuda())
+    want_blocks, want_scales = O.encode_linear(w, hdiag, lut)
+    assert np.array_equal(scales.cpu().numpy(), want_scales)
+    assert np.array_equal(blocks.cpu().numpy(), want_blocks.reshape(-1))
