@@ -97,3 +97,32 @@ def test_encoder_ragged_rows_match_restatement(ext, lut, m, k):
     want_blocks, want_scales = O.encode_linear(w, hdiag, lut)
     assert np.array_equal(scales.cpu().numpy(), want_scales)
     assert np.array_equal(blocks.cpu().numpy(), want_blocks.reshape(-1))
+
+
+@pytest.mark.parametrize("hardware", [False, True])
+@pytest.mark.parametrize("tokens", [1, 9, 128])
+def test_low_mode_entries_one_by_one(ext, lut, tokens, hardware):
+    """Random endpoints, most blocks in the low mode, every selector; unit activations read single weights back."""
+    rng = np.random.default_rng(tokens)
+    m, k = 512, 128
+    ends = rng.integers(-127, 128, (2, m, k // 16))
+    low = rng.random((m, k // 16)) < 0.8
+    e0, e1 = np.where(low, ends.min(0), ends.max(0)).astype(np.int8), np.where(low, ends.max(0), ends.min(0)).astype(np.int8)
+    e1[:8] = e0[:8]
+    blocks = O.pack_blocks(e0, e1, rng.integers(0, 8, (m, k // 16, 16)).astype(np.uint8))
+    table = O.hardware_palette() if hardware else lut
+    want = O.dequant_palette(blocks, m, table).reshape(m, k).astype(np.float64)
+    h = ext.pack_encoded(torch.from_numpy(blocks).reshape(-1), torch.ones(m))
+    ext.set_palette(h, 1 if hardware else 0)
+    got = np.empty((m, k))
+    for first in range(0, k, tokens):
+        x = torch.zeros(tokens, k, dtype=torch.float16)
+        columns = [c % k for c in range(first, first + tokens)]
+        x[torch.arange(tokens), torch.tensor(columns)] = 1
+        got[:, columns] = ext.linear(h, x.cuda()).float().cpu().numpy().T
+    ext.free(h)
+    # a low-mode weight: fp16 numerator (2^-11 of it, or half a subnormal step 2^-25 * 65536 / 889), then the fp16 output (2^-11);
+    # under the texture palette the high mode rounds its two step sizes to fp16 as well (2^-10 of the steps' sum, at most 2, and
+    # 3e-5 of the endpoints' widening)
+    bound = np.abs(want) * 2.0 ** -10 + 3e-6 + (0 if not hardware else 2.0 ** -9 + 6e-5) * ~np.repeat(e0 <= e1, 16, 1)
+    assert (np.abs(got - want) <= bound).all()

@@ -18,7 +18,7 @@
 // never rounded to bf16: the result is the un-rounded BC4 linear, which differs from the
 // reference's bf16(pal*scale) arithmetic by that rounding only (rel-RMS about 1e-3).
 // Blocks in the low palette mode (e0 <= e1) are rare; units that contain one are flagged at pack
-// time and take a warp-uniform slow path with per-weight arithmetic.
+// time and look their weights up instead (tx_decode.cuh).
 //
 // The warps of a CTA combine their fp32 partial tiles through shared memory in warp order, so
 // results are deterministic; the only waits in this file are CTA barriers.
@@ -359,8 +359,8 @@ gemv_tile_kernel(const GemvParams p) {
           else { decode_duo_second(q, aq); decode_duo_second(r, ar); }
         }
         if (LOWMODE && __any_sync(0xffffffffu, flag != 0)) {   // rare, warp-uniform: redo the low-mode blocks
-          if (duo_block_is_low(q, sub)) decode_block_slow(q, sub, aq, p.palette & 0xff);
-          if (duo_block_is_low(r, sub)) decode_block_slow(r, sub, ar, p.palette & 0xff);
+          if (duo_block_is_low(q, sub)) decode_block_low(q, sub, aq, p.palette & 0xff);
+          if (duo_block_is_low(r, sub)) decode_block_low(r, sub, ar, p.palette & 0xff);
         }
         if (NT == 1) {
           // One token tile: lanes whose token does not exist skip the load (their MMA columns are never

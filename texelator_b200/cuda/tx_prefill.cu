@@ -317,7 +317,7 @@ prefill_umma_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap x
               } else {
                 if (sub == 0) decode_duo_first(u, packed); else decode_duo_second(u, packed);
               }
-              if (cflag[m] && duo_block_is_low(u, sub)) decode_block_slow(u, sub, packed, p.palette);
+              if (cflag[m] && duo_block_is_low(u, sub)) decode_block_low(u, sub, packed, p.palette);
               // block kb of the stage -> K chunks 2kb, 2kb+1; row = (m*8 + tile_warp)*16 + half*8 + g
               const int kb = (kSubs == 2 ? 0 : sub * 4) + t;
               uint8_t *dst = stage + (2 * kb) * Cfg::a_lbo + ((m * kTileWarps + tile_warp) * 2 + half) * kASbo + g * 16;
