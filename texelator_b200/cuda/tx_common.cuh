@@ -300,19 +300,33 @@ __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddep
 
 bool pdl_enabled();
 
+// `ctas` consecutive CTAs along x form a cluster (1: none)
 template <typename... KernelArgs, typename... Args>
-cudaError_t launch_pdl(void (*kernel)(KernelArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+cudaError_t launch_pdl_cluster(void (*kernel)(KernelArgs...), int ctas, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
   cudaLaunchConfig_t config{};
   config.gridDim = grid;
   config.blockDim = block;
   config.dynamicSmemBytes = smem;
   config.stream = stream;
-  cudaLaunchAttribute attribute{};
-  attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attribute.val.programmaticStreamSerializationAllowed = 1;
-  config.attrs = &attribute;
-  config.numAttrs = pdl_enabled() ? 1 : 0;
+  cudaLaunchAttribute attributes[2]{};
+  int count = 0;
+  if (pdl_enabled()) {
+    attributes[count].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attributes[count++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (ctas > 1) {
+    attributes[count].id = cudaLaunchAttributeClusterDimension;
+    attributes[count].val.clusterDim.x = unsigned(ctas);
+    attributes[count].val.clusterDim.y = attributes[count].val.clusterDim.z = 1;
+    ++count;
+  }
+  config.attrs = attributes;
+  config.numAttrs = count;
   return cudaLaunchKernelEx(&config, kernel, KernelArgs(args)...);
+}
+template <typename... KernelArgs, typename... Args>
+cudaError_t launch_pdl(void (*kernel)(KernelArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+  return launch_pdl_cluster(kernel, 1, grid, block, smem, stream, args...);
 }
 
 // launchers implemented in the other translation units

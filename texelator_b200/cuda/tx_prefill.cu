@@ -7,13 +7,13 @@
 //
 //   pre-pass   one small kernel rescales the activations per token by an exact power of two and stores
 //              them as fp16 (the decode GEMV's staging) in the chunk-major order of the B operand;
-//   warps 0-15 producers: 128-bit loads of the tiled BC4 payload (one 8-row half of a 16-row tile per
-//              warp), decode in registers exactly like the decode GEMV (masked index fields + HFMA2 ->
-//              exact numerators n * 2^-16, n = 7*e0 + g*(e1-e0), as fp16) and store the A tile into shared
-//              memory in the canonical K-major core-matrix layout (no swizzle);
-//   warp 16    one lane issues the TMA load of the staged X tile (BN tokens x BK columns) per stage
+//   warps 0-15 producers: 128-bit loads of the tiled BC4 payload, decode in registers exactly like the decode GEMV
+//              (masked index fields + HFMA2 -> exact numerators n * 2^-16, n = 7*e0 + g*(e1-e0), as fp16) and
+//              tcgen05.st of the A stage into TMEM: the payload's lane order is the 16x256b fragment order, so
+//              nothing is shuffled and shared memory holds the activations alone;
+//   warp 16    one lane issues the TMA load of the staged X tile (128 columns) per stage
 //              through a 3-D tensor map whose rows are 512 contiguous bytes (no multicast);
-//   warp 17    allocates TMEM, and one lane issues MT * BK/16 tcgen05.mma kind::f16 (M=128, N=BN, K=16)
+//   warp 17    allocates TMEM and issues eight tcgen05.mma kind::f16 (A from TMEM, M=128 or a pair's 256, N=BN, K=16)
 //              per stage, committing to the stage's "empty" barrier;
 //   warps 0-15 epilogue: tcgen05.ld of the fp32 accumulators, * scale_m * 2^s * 65536/889, + bias, one bf16
 //              rounding, store.
@@ -41,41 +41,37 @@
 
 namespace tx {
 
-constexpr int kMmaM = 128;               // rows of one tcgen05.mma (TMEM lanes)
-constexpr int kASbo = 128;               // byte stride between 8-row groups of the A tile
-// Sixteen producer warps, one 8-row half of a 16-row tile each, all on every pipeline stage.  Measured and not
-// adopted: two groups of eight warps taking alternate stages with a whole tile per warp (same speed at 32 and
-// 128 tokens, 2-4 % slower at 512), a four-unit register look-ahead (same / 10 % slower), a 128 x 32 tile with a
-// five-stage ring against the 128 x 64 tile with four stages at 32 tokens (same).
-constexpr int kProducerWarps = 16;              // 8: one 16-row tile per warp; 16: one 8-row half of a tile per warp
-constexpr int kTileWarps = 8;                   // 16-row tiles of one 128-row accumulator
-constexpr int kGroups = 1;                      // groups of producer warps that take alternate units
-constexpr int kHalvesPerWarp = 16 * kGroups / kProducerWarps;
+constexpr int kMmaM = 128;               // rows of a CTA's accumulator (TMEM lanes)
+// Sixteen producer warps: warp w reaches the TMEM lanes of quarter w & 3 only, holds one of that quarter's two 16-row
+// tiles and decodes whole 128-column units of it on alternate pipeline stages.
+constexpr int kProducerWarps = 16;
+constexpr int kGroups = 2;                      // groups of producer warps that take alternate units
+constexpr int kLook = 2;                        // units of its row a producer warp keeps in flight as register loads
 constexpr int kTmaWarp = kProducerWarps, kMmaWarp = kProducerWarps + 1;
 constexpr int kPrefillThreads = (kProducerWarps + 2) * 32;   // producer/epilogue warps + TMA warp + MMA warp
-static_assert(kProducerWarps == 8 || kProducerWarps == 16, "producer warps split tiles whole or by halves");
 constexpr unsigned kSpinLimit = 1u << 22;
+constexpr int kBK = 128;                        // columns per pipeline stage: one unit of the payload
+constexpr int kChunks = kBK / 8;                // 16-byte K chunks of the activation tile per stage
+constexpr int kAColumns = kBK / 2;              // TMEM columns of one A stage (two fp16 per 32-bit column)
 
-// One tile shape: MT x 128 output rows (MT accumulators side by side in TMEM), BN tokens, BK columns
-// per pipeline stage.  Per FLOP the X tile is re-read 1/(128*MT) times, so tall tiles relieve L2; the
-// BC4 side costs a quarter of a byte per weight either way.
-template <int MT, int BN, int BK> struct TileConfig {
-  static constexpr int rows = MT * kMmaM;
-  static constexpr int chunks = BK / 8;                       // 16-byte K chunks per stage
-  static constexpr int a_lbo = MT * 16 * kASbo + 16;          // chunk stride (+16: conflict-free stores)
-  static constexpr int a_stage = chunks * a_lbo;
-  static constexpr int b_lbo = BN * 16;
-  static constexpr int b_stage = chunks * b_lbo;
-  static constexpr int fixed = 1024 + 16 /*alignment*/ + 256 /*barriers*/;
-  static constexpr int fit = (220 * 1024 - fixed) / (a_stage + b_stage);
-  static constexpr int stages = fit > 4 ? 4 : fit;
-  static constexpr size_t smem = fixed + size_t(stages) * (a_stage + b_stage);
-  static constexpr int used_columns = MT * BN;
-  // allocations are powers of two (a 192-token tile takes 256 columns)
-  static constexpr int tmem_columns = used_columns <= 32 ? 32 : used_columns <= 64 ? 64 : used_columns <= 128 ? 128 : used_columns <= 256 ? 256 : 512;
+// One tile shape: CTAS x 128 output rows x BN tokens.  The accumulator takes BN columns of every CTA's TMEM, the ring of
+// decoded A stages the columns behind it; shared memory holds the activations alone, and with CTAS = 2 each CTA keeps
+// half of the tokens (the tensor cores of a pair read both halves).
+template <int CTAS, int BN> struct TileConfig {
+  static constexpr int rows = CTAS * kMmaM;
+  static constexpr int tokens = BN / CTAS;                    // tokens this CTA stages
+  static constexpr int b_lbo = tokens * 16;
+  static constexpr int b_stage = kChunks * b_lbo;
+  static constexpr int fixed = 1024 /*alignment*/ + 256 /*barriers*/;
+  static constexpr int fit_smem = (220 * 1024 - fixed) / b_stage, fit_tmem = (512 - BN) / kAColumns;
+  static constexpr int fit = fit_smem < fit_tmem ? fit_smem : fit_tmem;
+  static constexpr int stages = fit > 6 ? 6 : fit;
+  static constexpr size_t smem = fixed + size_t(stages) * b_stage;
+  static constexpr int tmem_columns = 512;
   static_assert(stages >= 2, "tile does not fit two pipeline stages");
-  static_assert(BN % 32 == 0, "the activation box is made of 32-token runs");
-  static_assert(used_columns <= 512 && BN % 16 == 0 && BN <= 256, "accumulators must fit 512 TMEM columns; N is a multiple of 16 up to 256");
+  static_assert(BN + stages * kAColumns <= tmem_columns, "accumulator and A stages must fit TMEM");
+  static_assert(tokens % 32 == 0 && BN % 32 == 0 && BN <= 256, "the activation box is made of 32-token runs; N is at most 256");
+  static_assert(stages * b_stage >= BN * kMmaM * 2, "the output tile is staged where the activations were");
 };
 
 struct PrefillParams {
@@ -96,25 +92,41 @@ struct PrefillParams {
 __device__ __forceinline__ void mbar_init(unsigned bar, unsigned count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
+// arrival on the barrier at this shared-memory offset of the CTA `rank` of the cluster, releasing at cluster scope
+__device__ __forceinline__ void mbar_arrive_at(unsigned bar, unsigned rank) {
+  asm volatile(
+      "{\n\t.reg .b32 remote;\n\t"
+      "mapa.shared::cluster.u32 remote, %0, %1;\n\t"
+      "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [remote];\n\t}" ::"r"(bar), "r"(rank) : "memory");
+}
 __device__ __forceinline__ void mbar_arrive(unsigned bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void mbar_expect_tx(unsigned bar, unsigned bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
+template <bool CLUSTER = false>   // whether the arrivals it acquires come from another CTA of the cluster too
 __device__ __forceinline__ bool mbar_try_wait(unsigned bar, unsigned parity) {
   unsigned done;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+  if (CLUSTER)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done) : "r"(bar), "r"(parity) : "memory");
   return done != 0;
 }
 // Bounded wait; returns false (after recording `code`) when the limit is reached or the CTA aborted.
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, volatile int *abort_flag, int *status, int code) {
   for (unsigned spin = 0; spin < kSpinLimit; ++spin) {
-    if (mbar_try_wait(bar, parity)) return true;
+    if (mbar_try_wait<CLUSTER>(bar, parity)) return true;
     if (*abort_flag) return false;
   }
   atomicCAS(status, 0, code);
@@ -126,16 +138,47 @@ __device__ __forceinline__ void tma_load_3d(unsigned dst, const CUtensorMap *map
       "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
       ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2) : "memory");
 }
-__device__ __forceinline__ void umma_bf16(unsigned tmem_d, unsigned long long adesc, unsigned long long bdesc,
-                                          unsigned idesc, unsigned accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
+// one lane of a converged warp; the compiler keeps what it guards on the uniform datapath, which tcgen05.mma wants
+__device__ __forceinline__ bool elect_one() {
+  unsigned elected;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(elected));
+  return elected != 0;
 }
+// D[tmem] (+)= A[tmem] * B[smem]: M = CTAS * 128, fp16 operands, fp32 accumulation
+template <int CTAS>
+__device__ __forceinline__ void umma_f16(unsigned tmem_d, unsigned tmem_a, unsigned long long bdesc, unsigned idesc, unsigned accumulate) {
+  if (CTAS == 1)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+}
+// arrives at the barrier (of both CTAs of a pair) when the MMAs issued so far are complete
+template <int CTAS>
 __device__ __forceinline__ void umma_commit(unsigned bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+  if (CTAS == 1)
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+  else
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                 ::"r"(bar), "h"((unsigned short)3) : "memory");
+}
+// Sixteen TMEM lanes x 32 columns in the fragment order of mma.sync: registers 4j, 4j+1 of lane (g, t) are columns
+// 8j + 2t, 8j + 2t + 1 of TMEM lane g, registers 4j+2, 4j+3 those of lane g + 8.
+__device__ __forceinline__ void tmem_store_fragments(unsigned taddr, const unsigned (&q)[8], const unsigned (&r)[8]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+      ::"r"(taddr), "r"(q[0]), "r"(q[1]), "r"(r[0]), "r"(r[1]), "r"(q[2]), "r"(q[3]), "r"(r[2]), "r"(r[3]),
+        "r"(q[4]), "r"(q[5]), "r"(r[4]), "r"(r[5]), "r"(q[6]), "r"(q[7]), "r"(r[6]), "r"(r[7]) : "memory");
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void tmem_load32(unsigned taddr, unsigned (&r)[32]) {
   asm volatile(
@@ -163,6 +206,10 @@ __device__ __forceinline__ unsigned long long smem_desc(unsigned addr, unsigned 
 // was a TMA row of its own and the load, not the tensor pipe, set the pace of the wide tiles.
 // One CTA of 1024 threads stages eight tokens: four warps find the scaling of each token, then all
 // threads convert and write 128-byte runs (eight tokens of one chunk).
+//
+// Order of K.  A producer lane (g, t) holds whole 16-column blocks, and TMEM wants from it four K elements of every
+// 16-element MMA step, so the K elements are numbered the way the lanes hold them: element 4t + i of step j of a
+// 64-column half unit is column 16t + 4j + i.  The activations are written in that order here.
 constexpr int kStageThreads = 1024;
 __global__ void __launch_bounds__(kStageThreads) stage_activations_kernel(const __nv_bfloat16 *__restrict__ x, __half *__restrict__ out,
                                                                           float *__restrict__ xmul, int K, int KP, int tokens,
@@ -190,46 +237,60 @@ __global__ void __launch_bounds__(kStageThreads) stage_activations_kernel(const 
   if (half_in) inverse = 1.f;   // fp16 activations (x then points to fp16) are the operand as they are
   if (threadIdx.x < 8 && tok < tokens && blockIdx.y == 0) xmul[tok] = inverse * kNumeratorScale;
   uint4 *dst = reinterpret_cast<uint4 *>(out);
-  const uint4 *src = reinterpret_cast<const uint4 *>(x + size_t(tok < tokens ? tok : 0) * K);
+  const __nv_bfloat16 *src = x + size_t(tok < tokens ? tok : 0) * K;
   // few tokens give few CTAs: blockIdx.y cuts the conversion (not the scan above) into column slices
   const int per_slice = (padded + int(gridDim.y) - 1) / int(gridDim.y);
   const int slice_end = min(padded, (int(blockIdx.y) + 1) * per_slice);
-  for (int chunk = int(blockIdx.y) * per_slice + (threadIdx.x >> 3); chunk < slice_end; chunk += kStageThreads / 8)
-    dst[size_t(chunk) * padded_tokens + tok] =
-        (tok < tokens && chunk < chunks) ? (half_in ? src[chunk] : convert_chunk(src[chunk], mult)) : make_uint4(0, 0, 0, 0);
+  for (int chunk = int(blockIdx.y) * per_slice + (threadIdx.x >> 3); chunk < slice_end; chunk += kStageThreads / 8) {
+    // chunk 2j + c of a half unit: columns 16(2c) + 4j .. + 3 and 16(2c + 1) + 4j .. + 3
+    const int column = (chunk >> 3) * 64 + (chunk & 1) * 32 + ((chunk >> 1) & 3) * 4;
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (tok < tokens) {
+      if (column < K) {
+        const uint2 low = *reinterpret_cast<const uint2 *>(src + column);
+        v.x = low.x;
+        v.y = low.y;
+      }
+      if (column + 16 < K) {
+        const uint2 high = *reinterpret_cast<const uint2 *>(src + column + 16);
+        v.z = high.x;
+        v.w = high.y;
+      }
+      if (!half_in) v = convert_chunk(v, mult);
+    }
+    dst[size_t(chunk) * padded_tokens + tok] = v;
+  }
 }
 
-template <int MT, int BN, int BK>
+template <int CTAS, int BN, bool GENERIC>
 __global__ void __launch_bounds__(kPrefillThreads, 1)
 prefill_umma_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap x_map) {
-  using Cfg = TileConfig<MT, BN, BK>;
+  using Cfg = TileConfig<CTAS, BN>;
   constexpr int S = Cfg::stages;
-  constexpr int kSubs = 128 / BK;            // pipeline stages per 128-column unit of the payload (1 or 2)
   extern __shared__ uint8_t smem_raw[];
   const unsigned sbase = unsigned(__cvta_generic_to_shared(smem_raw));
-  const unsigned bars_s = (sbase + 15) & ~15u;          // barriers + small state (256 bytes)
+  const unsigned b_s = (sbase + 1023) & ~1023u;          // activation stages, then barriers + small state (256 bytes)
+  const unsigned bars_s = b_s + S * Cfg::b_stage;
   uint8_t *bars_g = smem_raw + (bars_s - sbase);
-  const unsigned full_a = bars_s, full_b = bars_s + 8 * S, empty = bars_s + 16 * S, accum = bars_s + 24 * S;
+  const unsigned full = bars_s, empty = bars_s + 8 * S, accum = bars_s + 16 * S;
   volatile int *abort_flag = reinterpret_cast<volatile int *>(bars_g + 200);
   unsigned *tmem_slot = reinterpret_cast<unsigned *>(bars_g + 208);
-  const unsigned tiles_s = (bars_s + 256 + 1023) & ~1023u;   // A stages then B stages, 1 KiB aligned
-  uint8_t *tiles_g = smem_raw + (tiles_s - sbase);
-  const unsigned a_s = tiles_s, b_s = tiles_s + S * Cfg::a_stage;
 
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+  const unsigned rank = CTAS == 2 ? blockIdx.x & 1 : 0;  // the pair is cut from blockIdx.x; rank 0 issues its MMAs
   // Launched with programmatic stream serialisation behind the staging kernel: everything up to the first read
   // of the staged activations (the TMA lane) or of the token multipliers (the epilogue) touches only the
   // immutable payload and this CTA's own memory and may run while the staging kernel is still at work.
   grid_launch_dependents();
-  // this CTA's range of 128-column units (the whole row unless the launch cuts K)
+  // this CTA's range of 128-column units (the whole row unless the launch cuts K); one unit is one pipeline stage
   const int u0 = int(blockIdx.z) * p.KI / int(gridDim.z), u1 = (int(blockIdx.z) + 1) * p.KI / int(gridDim.z);
-  const int KT = (u1 - u0) * kSubs;                      // pipeline stages over this range
-  const int row0 = blockIdx.x * Cfg::rows, tok0 = blockIdx.y * BN;
+  const int KT = u1 - u0;
+  const int row0 = blockIdx.x * kMmaM, tok0 = blockIdx.y * BN;
 
   if (tid == 0) {
     for (int s = 0; s < S; ++s) {
-      mbar_init(full_a + 8 * s, kProducerWarps / kGroups);
-      mbar_init(full_b + 8 * s, 1);
+      // the producer warps and the TMA lane of a stage; on the issuing CTA of a pair also one arrival for the other CTA's half
+      mbar_init(full + 8 * s, kProducerWarps / kGroups + 1 + (CTAS == 2 && rank == 0 ? 1 : 0));
       mbar_init(empty + 8 * s, 1);
     }
     mbar_init(accum, 1);
@@ -237,184 +298,221 @@ prefill_umma_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap x
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == kMmaWarp) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(bars_s + 208), "r"(unsigned(Cfg::tmem_columns)) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    if (CTAS == 1) {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(bars_s + 208), "r"(unsigned(Cfg::tmem_columns)) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(bars_s + 208), "r"(unsigned(Cfg::tmem_columns)) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if (CTAS == 2) cluster_sync();                         // the other CTA's barriers exist
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const unsigned tmem_base = *tmem_slot;
 
   if (warp < kProducerWarps) {
-    // ---------------- producers: BC4 -> fp16 A tile; warp w owns 16-row tiles w, w+8, ... of the CTA ----------------
-    const int g = lane >> 2, t = lane & 3;
-    const int tile_warp = warp % kTileWarps;
-    const int group = kGroups > 1 ? warp / kTileWarps : 0, half0 = kGroups > 1 ? 0 : warp / kTileWarps;   // half0 is 0 with eight producers
-    const uint4 *src[MT];
-    const uint8_t *fl[MT];
-    bool live[MT];
-#pragma unroll
-    for (int m = 0; m < MT; ++m) {
-      const int rt = blockIdx.x * (Cfg::rows / 16) + m * kTileWarps + tile_warp;
-      live[m] = rt < p.MT;
-      src[m] = p.tiles + (size_t(live[m] ? rt : 0) * p.KI) * 64 + half0 * 32 + lane;
-      fl[m] = p.flags + size_t(live[m] ? rt : 0) * p.KI;
-    }
-    // kLook units of every tile in flight per warp as register loads.  One is enough: four measured the same at
-    // 32 tokens (the pace there is set by the stage hand-over, not by DRAM latency) and 10 % slower at 512 tokens
-    constexpr int kLook = 1;
-    uint4 q[kLook][MT][kHalvesPerWarp];
-    unsigned flag[kLook][MT];
-#pragma unroll
-    for (int slot = 0; slot < kLook; ++slot)
-#pragma unroll
-      for (int m = 0; m < MT; ++m) {
-        if (u0 + group + slot * kGroups < u1) {
-#pragma unroll
-          for (int h = 0; h < kHalvesPerWarp; ++h) q[slot][m][h] = ldg_stream(src[m] + size_t(u0 + group + slot * kGroups) * 64 + h * 32);
-          flag[slot][m] = fl[m][u0 + group + slot * kGroups];
-        }
+    // ---------------- producers: BC4 -> fp16 A stage in TMEM ----------------
+    const int quarter = warp & 3, pair = (warp >> 2) & 1, group = warp >> 3;
+    const int rt = blockIdx.x * (kMmaM / 16) + quarter * 2 + pair;
+    // (row tiles past the end of the matrix decode tile 0 again: their accumulator rows are never stored)
+    const uint4 *src = p.tiles + size_t(rt < p.MT ? rt : 0) * p.KI * 64 + lane;
+    const uint8_t *flags = p.flags + size_t(rt < p.MT ? rt : 0) * p.KI;
+    const unsigned a_lane = tmem_base + (unsigned(quarter * 32 + pair * 16) << 16) + BN;
+    uint4 pend[kLook][2];
+    unsigned flag[kLook];
+    auto fetch = [&](int slot, int unit) {
+      if (unit < u1) {
+        pend[slot][0] = ldg_stream(src + size_t(unit) * 64);
+        pend[slot][1] = ldg_stream(src + size_t(unit) * 64 + 32);
+        if (GENERIC) flag[slot] = flags[unit];
       }
+    };
+#pragma unroll
+    for (int slot = 0; slot < kLook; ++slot) fetch(slot, u0 + group + slot * kGroups);
+    int s = group % S;
+    unsigned parity = 1;                                 // of the stage's previous release; a fresh barrier passes
     bool ok = true;
     for (int base = u0 + group; base < u1 && ok; base += kLook * kGroups) {
 #pragma unroll
-     for (int slot = 0; slot < kLook; ++slot) {
-      const int unit = base + slot * kGroups;
-      if (unit >= u1 || !ok) break;                      // warp-uniform
-      uint4 cq[MT][kHalvesPerWarp];
-      unsigned cflag[MT];
+      for (int slot = 0; slot < kLook; ++slot) {
+        const int unit = base + slot * kGroups;
+        if (unit >= u1 || !ok) break;                    // warp-uniform
+        const uint4 q = pend[slot][0], r = pend[slot][1];   // duos of rows g and g + 8
+        const bool low = GENERIC && flag[slot];          // warp-uniform: the unit's flag
+        fetch(slot, unit + kLook * kGroups);
+        // Decode before waiting for the stage: a warp takes a few hundred cycles over a unit, and the time from a
+        // stage's release to its next use is what sets the pace.
+        unsigned a[2][2][8];                             // [block column][row g / g + 8]: exact numerators n * 2^-16 as fp16x2
 #pragma unroll
-      for (int m = 0; m < MT; ++m) {
-        cflag[m] = flag[slot][m];
-#pragma unroll
-        for (int h = 0; h < kHalvesPerWarp; ++h) cq[m][h] = q[slot][m][h];
-        if (unit + kLook * kGroups < u1) {               // refill the slot with this warp's next unit
-#pragma unroll
-          for (int h = 0; h < kHalvesPerWarp; ++h) q[slot][m][h] = ldg_stream(src[m] + size_t(unit + kLook * kGroups) * 64 + h * 32);
-          flag[slot][m] = fl[m][unit + kLook * kGroups];
-        }
-      }
-#pragma unroll
-      for (int part = 0; part < kSubs; ++part) {
-        const int kt = (unit - u0) * kSubs + part, s = kt % S;
-        if (kt >= S && !mbar_wait(empty + 8 * s, ((kt / S) - 1) & 1, abort_flag, p.status, 1)) {
-          ok = false;
-          break;
-        }
-        uint8_t *stage = tiles_g + s * Cfg::a_stage;
-#pragma unroll
-        for (int m = 0; m < MT; ++m) {
-#pragma unroll
-          for (int h = 0; h < kHalvesPerWarp; ++h) {
-            const uint4 u = cq[m][h];
-            const int half = half0 + h;
-#pragma unroll
-            for (int sub = 0; sub < 2; ++sub) {
-              if (kSubs == 2 && sub != part) continue;   // 64-column stages take one block column of the unit each
-              unsigned packed[8];                                   // exact numerators n * 2^-16 as fp16x2
-              if (p.palette == TX_PALETTE_HARDWARE) {               // uniform
-                if (sub == 0) decode_duo_first<true>(u, packed); else decode_duo_second<true>(u, packed);
-              } else {
-                if (sub == 0) decode_duo_first(u, packed); else decode_duo_second(u, packed);
-              }
-              if (cflag[m] && duo_block_is_low(u, sub)) decode_block_low(u, sub, packed, p.palette);
-              // block kb of the stage -> K chunks 2kb, 2kb+1; row = (m*8 + tile_warp)*16 + half*8 + g
-              const int kb = (kSubs == 2 ? 0 : sub * 4) + t;
-              uint8_t *dst = stage + (2 * kb) * Cfg::a_lbo + ((m * kTileWarps + tile_warp) * 2 + half) * kASbo + g * 16;
-              // (row tiles past the end of the matrix decode tile 0 again: their accumulator rows are never stored)
-              *reinterpret_cast<uint4 *>(dst) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-              *reinterpret_cast<uint4 *>(dst + Cfg::a_lbo) = make_uint4(packed[4], packed[5], packed[6], packed[7]);
-            }
+        for (int h = 0; h < 2; ++h) {
+          const uint4 duo = h == 0 ? q : r;
+          if (GENERIC && p.palette == TX_PALETTE_HARDWARE) {   // uniform
+            decode_duo_first<true>(duo, a[0][h]);
+            decode_duo_second<true>(duo, a[1][h]);
+          } else {
+            decode_duo_first(duo, a[0][h]);
+            decode_duo_second(duo, a[1][h]);
+          }
+          if (low) {
+            if (duo_block_is_low(duo, 0)) decode_block_low(duo, 0, a[0][h], p.palette);
+            if (duo_block_is_low(duo, 1)) decode_block_low(duo, 1, a[1][h], p.palette);
           }
         }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic-proxy stores -> tensor core
-        __syncwarp();
-        if (lane == 0) mbar_arrive(full_a + 8 * s);
-      }
-     }
-    }
-  } else if (warp == kTmaWarp) {
-    // ---------------- TMA: staged X tile [BN tokens x BK columns] per stage ----------------
-    if (lane == 0) {
-      grid_dependency_wait();              // the staged activations are complete
-      int issued = 0;
-      for (int kt = 0; kt < KT; ++kt) {
-        const int s = kt % S;
-        if (kt >= S && !mbar_wait(empty + 8 * s, ((kt / S) - 1) & 1, abort_flag, p.status, 2)) break;
-        mbar_expect_tx(full_b + 8 * s, Cfg::b_stage);
-        tma_load_3d(b_s + s * Cfg::b_stage, &x_map, full_b + 8 * s, 0, tok0 / 32, (u0 * kSubs + kt) * Cfg::chunks);
-        issued = kt + 1;
-      }
-      if (*abort_flag) {
-        // wait (bounded) for copies that were issued but never consumed, so none lands after exit
-        for (int kt = issued > S ? issued - S : 0; kt < issued; ++kt)
-          for (unsigned spin = 0; spin < (1u << 20) && !mbar_try_wait(full_b + 8 * (kt % S), (kt / S) & 1); ++spin) {}
-      }
-    }
-  } else {
-    // ---------------- MMA issue ----------------
-    if (lane == 0) {
-      // D = f32 (bits 4-5 = 1), A = B = f16 (format 0), both K-major, N at bit 17, M at bit 24
-      const unsigned idesc = (1u << 4) | (unsigned(BN >> 3) << 17) | (unsigned(kMmaM >> 4) << 24);
-      bool ok = true;
-      for (int kt = 0; kt < KT && ok; ++kt) {
-        const int s = kt % S;
-        const unsigned parity = (kt / S) & 1;
-        ok = mbar_wait(full_a + 8 * s, parity, abort_flag, p.status, 3) && mbar_wait(full_b + 8 * s, parity, abort_flag, p.status, 4);
+        ok = __all_sync(0xffffffffu, mbar_wait(empty + 8 * s, parity, abort_flag, p.status, 1));
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-        for (int m = 0; m < MT; ++m)
-#pragma unroll
-          for (int j = 0; j < BK / 16; ++j) {
-            const unsigned long long adesc = smem_desc(a_s + s * Cfg::a_stage + m * 16 * kASbo + j * 2 * Cfg::a_lbo, Cfg::a_lbo, kASbo);
-            const unsigned long long bdesc = smem_desc(b_s + s * Cfg::b_stage + j * 2 * Cfg::b_lbo, Cfg::b_lbo, 128);
-            umma_bf16(tmem_base + unsigned(m * BN), adesc, bdesc, idesc, (kt | j) ? 1u : 0u);
-          }
-        umma_commit(empty + 8 * s);        // frees the stage when these MMAs have read it
+        tmem_store_fragments(a_lane + unsigned(s * kAColumns), a[0][0], a[0][1]);
+        tmem_store_fragments(a_lane + unsigned(s * kAColumns + kAColumns / 2), a[1][0], a[1][1]);
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(full + 8 * s);
+        s += kGroups;
+        if (s >= S) {
+          s -= S;
+          parity ^= 1;
+        }
       }
-      if (ok) umma_commit(accum);          // accumulators complete
+    }
+  } else if (warp == kTmaWarp) {
+    // ---------------- TMA: this CTA's tokens of the staged X tile, 128 columns per stage ----------------
+    if (lane == 0) {
+      grid_dependency_wait();              // the staged activations are complete
+      int issued = 0, s = 0;
+      unsigned parity = 1;
+      for (int kt = 0; kt < KT; ++kt) {
+        if (!mbar_wait(empty + 8 * s, parity, abort_flag, p.status, 2)) break;
+        mbar_expect_tx(full + 8 * s, Cfg::b_stage);
+        tma_load_3d(b_s + s * Cfg::b_stage, &x_map, full + 8 * s, 0, (tok0 + int(rank) * Cfg::tokens) / 32, (u0 + kt) * kChunks);
+        issued = kt + 1;
+        if (++s == S) {
+          s = 0;
+          parity ^= 1;
+        }
+      }
+      if (*abort_flag) {
+        // give copies that were issued but never consumed time (bounded) to land before the CTA exits
+        for (int kt = issued > S ? issued - S : 0; kt < issued; ++kt)
+          for (unsigned spin = 0; spin < (1u << 16) && !mbar_try_wait(full + 8 * (kt % S), (kt / S) & 1); ++spin) {}
+      }
+    }
+  } else if (rank == 0) {
+    // ---------------- MMA issue ----------------
+    // One instruction stream feeds the tensor core, and what it spends on a stage beyond the MMAs' own time leaves the core
+    // idle.  A single lane in a divergent branch, with two barriers a stage and descriptors built on the spot, spent
+    // 1240 cycles on a stage whatever the tile (a 256-token stage is 1024 cycles of MMA): hence a converged warp with
+    // one elected lane, one barrier a stage and descriptors that only need an addition.
+    // D = f32 (bits 4-5 = 1), A = B = f16 (format 0), both K-major, N at bit 17, M at bit 24
+    constexpr unsigned idesc = (1u << 4) | (unsigned(BN >> 3) << 17) | (unsigned(Cfg::rows >> 4) << 24);
+    const unsigned long long bdesc = smem_desc(b_s, Cfg::b_lbo, 128);
+    const unsigned tmem_d = __shfl_sync(0xffffffffu, tmem_base, 0);
+    int s = 0;
+    unsigned parity = 0;
+    bool ok = true;
+    for (int kt = 0; kt < KT; ++kt) {
+      ok = __all_sync(0xffffffffu, mbar_wait<CTAS == 2>(full + 8 * s, parity, abort_flag, p.status, 3));
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if (elect_one()) {
+        const unsigned long long stage_desc = bdesc + unsigned(s * (Cfg::b_stage >> 4));
+        const unsigned stage_a = tmem_d + unsigned(BN + s * kAColumns);
+#pragma unroll
+        for (int j = 0; j < kBK / 16; ++j)
+          umma_f16<CTAS>(tmem_d, stage_a + unsigned(j * 8), stage_desc + unsigned(j * 2 * (Cfg::b_lbo >> 4)), idesc, j ? 1u : unsigned(kt != 0));
+        umma_commit<CTAS>(empty + 8 * s);  // frees the stage when these MMAs have read it
+      }
+      __syncwarp();
+      if (++s == S) {
+        s = 0;
+        parity ^= 1;
+      }
+    }
+    if (ok && elect_one()) umma_commit<CTAS>(accum);   // accumulators complete
+    __syncwarp();
+  } else if (lane == 0) {
+    // ---------------- second CTA of a pair: tell the issuing CTA when this one's half of a stage is there ----------------
+    // (one cluster-scope arrival a stage; from every producer warp it would wait for the warp's loads in flight each time)
+    int s = 0;
+    unsigned parity = 0;
+    for (int kt = 0; kt < KT; ++kt) {
+      if (!mbar_wait(full + 8 * s, parity, abort_flag, p.status, 3)) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      mbar_arrive_at(full + 8 * s, 0);
+      if (++s == S) {
+        s = 0;
+        parity ^= 1;
+      }
     }
   }
 
   // ---------------- epilogue: TMEM -> registers -> y ----------------
   if (warp < kProducerWarps) {
     grid_dependency_wait();                // xmul comes from the staging kernel
-    const bool ready = mbar_wait(accum, 0, abort_flag, p.status, 5);
+    const bool ready = __all_sync(0xffffffffu, mbar_wait(accum, 0, abort_flag, p.status, 5));
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (ready) {
-      const int quarter = warp & 3;
-      // the warps of one lane quarter share its MT x (BN/32) accumulator chunks
-      for (int item = warp >> 2; item < MT * (BN / 32); item += kProducerWarps / 4) {
-        const int m = item / (BN / 32), c = item % (BN / 32);
-        const int row = row0 + m * kMmaM + quarter * 32 + lane;
-        const float bias = (row < p.M && p.bias)
-                               ? (p.half_io ? __half2float(reinterpret_cast<const __half *>(p.bias)[row]) : __bfloat162float(p.bias[row]))
-                               : 0.f;
-        const float row_scale = row < p.M ? p.scales[row] : 0.f;
+    const int quarter = warp & 3, row = row0 + quarter * 32 + lane;
+    const float row_scale = row < p.M ? p.scales[row] : 0.f;
+    if (ready && gridDim.z > 1) {
+      // the warps of one lane quarter share its BN/32 accumulator chunks
+      for (int c = warp >> 2; c < BN / 32; c += kProducerWarps / 4) {
+        const float token_scale = tok0 + c * 32 + lane < p.T ? __ldcg(p.xmul + tok0 + c * 32 + lane) : 0.f;
+        float *dst = p.partial + (size_t(blockIdx.z) * p.T + tok0 + c * 32) * p.M + row;
         unsigned v[32];
-        tmem_load32(tmem_base + (unsigned(quarter * 32) << 16) + unsigned(m * BN + c * 32), v);
-        if (row < p.M) {
+        tmem_load32(tmem_base + (unsigned(quarter * 32) << 16) + unsigned(c * 32), v);
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const int tok = tok0 + c * 32 + j;
-            if (tok < p.T && gridDim.z > 1) {
-              p.partial[(size_t(blockIdx.z) * p.T + tok) * p.M + row] = __uint_as_float(v[j]) * (row_scale * __ldg(p.xmul + tok));
-            } else if (tok < p.T) {
-              const float value = fmaf(__uint_as_float(v[j]), row_scale * __ldg(p.xmul + tok), bias);
-              if (p.half_io) reinterpret_cast<__half *>(p.y)[size_t(tok) * p.M + row] = __float2half_rn(value);
-              else p.y[size_t(tok) * p.M + row] = __float2bfloat16(value);
-            }
-          }
+        for (int j = 0; j < 32; ++j) {
+          const float scale = row_scale * __shfl_sync(0xffffffffu, token_scale, j);
+          if (row < p.M && tok0 + c * 32 + j < p.T) dst[size_t(j) * p.M] = __uint_as_float(v[j]) * scale;
+        }
+      }
+    } else if (ready) {
+      // A lane holds one output row, so stores from here would be 64-byte pieces; the tile goes through shared memory (the
+      // activation stages are free now) and leaves as runs of 256 bytes.
+      const float bias = (row < p.M && p.bias)
+                             ? (p.half_io ? __half2float(reinterpret_cast<const __half *>(p.bias)[row]) : __bfloat162float(p.bias[row]))
+                             : 0.f;
+      uint16_t *out = reinterpret_cast<uint16_t *>(smem_raw + (b_s - sbase));   // [BN][128 rows]
+      for (int c = warp >> 2; c < BN / 32; c += kProducerWarps / 4) {
+        const float token_scale = tok0 + c * 32 + lane < p.T ? __ldcg(p.xmul + tok0 + c * 32 + lane) : 0.f;
+        unsigned v[32];
+        tmem_load32(tmem_base + (unsigned(quarter * 32) << 16) + unsigned(c * 32), v);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          const float value = fmaf(__uint_as_float(v[j]), row_scale * __shfl_sync(0xffffffffu, token_scale, j), bias);
+          out[(c * 32 + j) * kMmaM + quarter * 32 + lane] =
+              p.half_io ? __half_as_ushort(__float2half_rn(value)) : __bfloat16_as_ushort(__float2bfloat16(value));
+        }
+      }
+    }
+    asm volatile("bar.sync 1, %0;" ::"n"(kProducerWarps * 32) : "memory");
+    if (ready && gridDim.z == 1) {
+      const uint8_t *out = smem_raw + (b_s - sbase);
+      const int rows = min(kMmaM, p.M - row0), last = min(BN, p.T - tok0);
+      __nv_bfloat16 *dst = p.y + size_t(tok0) * p.M + row0;
+      if (p.M % 8 == 0) {                  // rows of y are 16-byte aligned
+        for (int i = tid; i < last * (kMmaM / 8); i += kProducerWarps * 32) {
+          const int tok = i / (kMmaM / 8), part = i % (kMmaM / 8);
+          if (part * 8 < rows)
+            *reinterpret_cast<uint4 *>(dst + size_t(tok) * p.M + part * 8) = *reinterpret_cast<const uint4 *>(out + (tok * kMmaM + part * 8) * 2);
+        }
+      } else {
+        for (int i = tid; i < last * kMmaM; i += kProducerWarps * 32) {
+          const int tok = i / kMmaM, r = i % kMmaM;
+          if (r < rows) dst[size_t(tok) * p.M + r] = reinterpret_cast<const __nv_bfloat16 *>(out)[i];
         }
       }
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if (CTAS == 2) cluster_sync();           // neither CTA leaves while the other's tensor core or barriers may still reach it
   if (warp == kMmaWarp) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(unsigned(Cfg::tmem_columns)) : "memory");
+    if (CTAS == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(unsigned(Cfg::tmem_columns)) : "memory");
+    else asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(unsigned(Cfg::tmem_columns)) : "memory");
   }
 }
 
@@ -436,24 +534,10 @@ static EncodeTiled encode_tiled_entry() {
 }
 
 // Tile candidates behind the reference's backend ids 5..9 (texelator/autotune.py:16-22):
-//   5: 128 rows x 256 tokens (baseline)   6: 256 x 256   7: 128 x 128   8: 128 x 64   9: 128 x 192
+//   5: 128 rows x 256 tokens (baseline)   6: 256 x 256 (a pair of CTAs)   7: 128 x 128   8: 128 x 64   9: 128 x 192
 // (192 tokens: 5120-row matrices at 512+ tokens launch 120 CTAs instead of 80 or 160 on the 148 SMs)
 // Tall tiles re-read the activations less often (tensor-bound prompts); narrow ones suit short prompts
 // where the weight stream is the bound.
-struct TileShape {
-  int mt, bn, bk;
-};
-static TileShape backend_shape(int backend) {
-  switch (backend) {
-    case 5: return {1, 256, 128};
-    case 6: return {2, 256, 64};
-    case 7: return {1, 128, 128};
-    case 8: return {1, 64, 128};
-    case 9: return {1, 192, 128};
-    default: return {0, 0, 0};
-  }
-}
-
 // Handles that were packed without a tuned backend.  Short prompts are paced by the producers, so the narrowest tile that
 // holds all tokens wins; from 192 tokens on, 192-token tiles unless the 256-token ones need fewer token blocks per SM.
 int prefill_choose_backend(const Handle *h, int tokens) {
@@ -465,7 +549,7 @@ int prefill_choose_backend(const Handle *h, int tokens) {
 }
 
 bool prefill_tile_eligible(const Handle *h, int backend, int tokens) {
-  return backend_shape(backend).mt != 0 && tokens >= 1 && h->K % 16 == 0 && encode_tiled_entry() != nullptr;
+  return backend >= 5 && backend <= 9 && tokens >= 1 && h->K % 16 == 0 && encode_tiled_entry() != nullptr;
 }
 
 // Short prompts on matrices with few rows leave most SMs without a CTA (5120 rows = 40 CTAs of 128 rows): K is
@@ -479,18 +563,21 @@ static int prefill_k_ranges(const Handle *h, int tokens, const Workspace *ws) {
   return std::max(ranges, 1);
 }
 
-template <int MT, int BN, int BK>
+template <int CTAS, int BN>
 static int launch_tile(const Handle *h, const __nv_bfloat16 *x, __nv_bfloat16 *y, int tokens, cudaStream_t stream, bool half_io) {
-  using Cfg = TileConfig<MT, BN, BK>;
+  using Cfg = TileConfig<CTAS, BN>;
   Workspace *ws = workspace_for(h->device);
   if (!ws) return TX_ECUDA;
+  // the lean variant decodes high-mode blocks of the software palette and nothing else
+  const bool generic = h->has_low_mode || h->palette == TX_PALETTE_HARDWARE;
+  const auto kernel = generic ? prefill_umma_kernel<CTAS, BN, true> : prefill_umma_kernel<CTAS, BN, false>;
   static std::mutex guard;
-  static std::map<int, bool> configured;
+  static std::map<std::pair<int, bool>, bool> configured;
   {
     std::lock_guard<std::mutex> lock(guard);
-    if (!configured[h->device]) {
-      TX_CUDA(cudaFuncSetAttribute(prefill_umma_kernel<MT, BN, BK>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(Cfg::smem)));
-      configured[h->device] = true;
+    if (!configured[{h->device, generic}]) {
+      TX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(Cfg::smem)));
+      configured[{h->device, generic}] = true;
     }
   }
   // Activations are staged once as fp16 after an exact per-token power-of-two rescale (the decode GEMV's
@@ -505,12 +592,12 @@ static int launch_tile(const Handle *h, const __nv_bfloat16 *x, __nv_bfloat16 *y
     stage_activations_kernel<<<dim3(padded_tokens / 8, slices), kStageThreads, 0, stream>>>(x + size_t(t0) * h->K, ws->xprep, ws->xmul, h->K, KP, n,
                                                                     padded_tokens, half_io ? 1 : 0);
     count_launch();
-    // staged X viewed as [KP/8 chunks][padded_tokens/32][32 tokens x 8 elements]: a box is BN/32 runs of
-    // 512 contiguous bytes per chunk and lands as BN-token core-matrix columns
+    // staged X viewed as [KP/8 chunks][padded_tokens/32][32 tokens x 8 elements]: a box is one run of
+    // 512 contiguous bytes per 32 tokens and chunk and lands as core-matrix columns
     CUtensorMap map;
     cuuint64_t dims[3] = {256, cuuint64_t(padded_tokens / 32), cuuint64_t(KP / 8)};
     cuuint64_t strides[2] = {512, cuuint64_t(padded_tokens) * 16};
-    cuuint32_t box[3] = {256, cuuint32_t(BN / 32), cuuint32_t(Cfg::chunks)};
+    cuuint32_t box[3] = {256, cuuint32_t(Cfg::tokens / 32), cuuint32_t(kChunks)};
     cuuint32_t elem[3] = {1, 1, 1};
     CUresult cr = encode_tiled_entry()(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, ws->xprep, dims, strides, box, elem,
                                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
@@ -533,8 +620,8 @@ static int launch_tile(const Handle *h, const __nv_bfloat16 *x, __nv_bfloat16 *y
     p.half_io = half_io ? 1 : 0;
     p.partial = ws->partial;
     const int ranges = prefill_k_ranges(h, n, ws);
-    dim3 grid((h->M + Cfg::rows - 1) / Cfg::rows, (n + BN - 1) / BN, ranges);
-    TX_CUDA(launch_pdl(prefill_umma_kernel<MT, BN, BK>, grid, dim3(kPrefillThreads), Cfg::smem, stream, p, map));
+    dim3 grid((h->M + Cfg::rows - 1) / Cfg::rows * CTAS, (n + BN - 1) / BN, ranges);
+    TX_CUDA(launch_pdl_cluster(kernel, CTAS, grid, dim3(kPrefillThreads), Cfg::smem, stream, p, map));
     count_launch();
     if (ranges > 1) {
       int rc = launch_combine(ws->partial, ranges, h->bias, y + size_t(t0) * h->M, n, h->M, half_io, ws->sm_count, stream);
@@ -550,42 +637,42 @@ static int launch_tile(const Handle *h, const __nv_bfloat16 *x, __nv_bfloat16 *y
 int launch_prefill_tile(const Handle *h, int backend, const __nv_bfloat16 *x, __nv_bfloat16 *y, int tokens, cudaStream_t stream,
                         bool half_io) {
   switch (backend) {
-    case 5: return launch_tile<1, 256, 128>(h, x, y, tokens, stream, half_io);
-    case 6: return launch_tile<2, 256, 64>(h, x, y, tokens, stream, half_io);
-    case 7: return launch_tile<1, 128, 128>(h, x, y, tokens, stream, half_io);
-    case 8: return launch_tile<1, 64, 128>(h, x, y, tokens, stream, half_io);
-    case 9: return launch_tile<1, 192, 128>(h, x, y, tokens, stream, half_io);
+    case 5: return launch_tile<1, 256>(h, x, y, tokens, stream, half_io);
+    case 6: return launch_tile<2, 256>(h, x, y, tokens, stream, half_io);
+    case 7: return launch_tile<1, 128>(h, x, y, tokens, stream, half_io);
+    case 8: return launch_tile<1, 64>(h, x, y, tokens, stream, half_io);
+    case 9: return launch_tile<1, 192>(h, x, y, tokens, stream, half_io);
     default: return fail(TX_EINVAL, "backend is not a tensor-core tile candidate");
   }
 }
 
-template <int MT, int BN, int BK>
+template <int CTAS, int BN>
 static int tile_info(int64_t out[9]) {
-  using Cfg = TileConfig<MT, BN, BK>;
+  using Cfg = TileConfig<CTAS, BN>;
   cudaFuncAttributes attributes{};
-  TX_CUDA(cudaFuncGetAttributes(&attributes, prefill_umma_kernel<MT, BN, BK>));
-  TX_CUDA(cudaFuncSetAttribute(prefill_umma_kernel<MT, BN, BK>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(Cfg::smem)));
+  TX_CUDA(cudaFuncGetAttributes(&attributes, prefill_umma_kernel<CTAS, BN, false>));
+  TX_CUDA(cudaFuncSetAttribute(prefill_umma_kernel<CTAS, BN, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(Cfg::smem)));
   int active = 0;
-  TX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&active, prefill_umma_kernel<MT, BN, BK>, kPrefillThreads, Cfg::smem));
+  TX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&active, prefill_umma_kernel<CTAS, BN, false>, kPrefillThreads, Cfg::smem));
   out[0] = attributes.numRegs;
   out[1] = int64_t(attributes.sharedSizeBytes);
   out[2] = int64_t(attributes.localSizeBytes);
   out[3] = attributes.maxThreadsPerBlock;
   out[4] = int64_t(Cfg::smem);
-  out[5] = Cfg::rows;   // output rows per CTA
-  out[6] = BN;          // tokens per CTA
-  out[7] = BK;          // columns per pipeline stage
+  out[5] = Cfg::rows;   // output rows per tile
+  out[6] = BN;          // tokens per tile
+  out[7] = kBK;         // columns per pipeline stage
   out[8] = active;
   return TX_OK;
 }
 
 int prefill_kernel_info(int backend, int64_t out[9]) {
   switch (backend) {
-    case 5: return tile_info<1, 256, 128>(out);
-    case 6: return tile_info<2, 256, 64>(out);
-    case 7: return tile_info<1, 128, 128>(out);
-    case 8: return tile_info<1, 64, 128>(out);
-    case 9: return tile_info<1, 192, 128>(out);
+    case 5: return tile_info<1, 256>(out);
+    case 6: return tile_info<2, 256>(out);
+    case 7: return tile_info<1, 128>(out);
+    case 8: return tile_info<1, 64>(out);
+    case 9: return tile_info<1, 192>(out);
     default: return fail(TX_EINVAL, "backend is not a tensor-core tile candidate");
   }
 }
