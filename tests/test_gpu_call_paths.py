@@ -126,3 +126,26 @@ def test_low_mode_entries_one_by_one(ext, lut, tokens, hardware):
     # 3e-5 of the endpoints' widening)
     bound = np.abs(want) * 2.0 ** -10 + 3e-6 + (0 if not hardware else 2.0 ** -9 + 6e-5) * ~np.repeat(e0 <= e1, 16, 1)
     assert (np.abs(got - want) <= bound).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("tokens,k,backend", [(1, 16, 8), (33, 144, 9), (31, 400, 6), (300, 1680, 6), (450, 80, 7), (600, 912, 5), (18, 102416, 8)])
+def test_staging_and_stage_ring_remainders(ext, lut, tokens, k, backend, dtype):
+    """Token counts around every number of tokens a staging block takes, rows that fit its shared memory and one that does
+    not, K of fewer units than the ring has stages and one past it, an odd number of 128-row blocks for the pair."""
+    m = 300
+    rng = np.random.default_rng(k)
+    ends = np.sort(rng.integers(-127, 128, (2, m, k // 16)), 0)[::-1].astype(np.int8)
+    blocks = O.pack_blocks(ends[0], ends[1], rng.integers(0, 8, (m, k // 16, 16)).astype(np.uint8))
+    scales = (rng.random(m) + 0.5).astype(np.float32)
+    h = ext.pack_encoded(torch.from_numpy(blocks).reshape(-1), torch.from_numpy(scales))
+    ext.set_prefill(h, 1, 1024)
+    ext.set_prefill_backend(h, backend)
+    x = (torch.randn(tokens, k, generator=torch.Generator().manual_seed(tokens)) / k ** 0.5).cuda().to(dtype)
+    y = ext.linear(h, x).double().cpu()
+    assert ext.kernel_status() == 0
+    w = torch.from_numpy(O.dequant_palette(blocks, m, lut).reshape(m, k)).double() * torch.from_numpy(scales).double()[:, None]
+    want = x.double().cpu() @ w.T
+    # exact products, fp32 sums, one rounding of the output (half a unit in its last place)
+    assert float((y - want).norm() / want.norm()) <= (2.0 ** -9 if dtype == torch.bfloat16 else 2.0 ** -12) + 1e-5
+    ext.free(h)

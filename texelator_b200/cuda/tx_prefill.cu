@@ -204,55 +204,71 @@ __device__ __forceinline__ unsigned long long smem_desc(unsigned addr, unsigned 
 // multiple of 32 -- which is the K-major core-matrix order of the B operand.  A TMA box then copies
 // runs of 32 tokens x 16 bytes = 512 contiguous bytes; with the row-major layout every 16-byte piece
 // was a TMA row of its own and the load, not the tensor pipe, set the pace of the wide tiles.
-// One CTA of 1024 threads stages eight tokens: four warps find the scaling of each token, then all
-// threads convert and write 128-byte runs (eight tokens of one chunk).
+//
+// A CTA stages `per_cta` tokens (1, 2 or 4: as many as leave every SM a CTA) in one trip to global memory: the rows wait in
+// shared memory while the magnitude scan finishes, then are converted and written out with neighbouring lanes on
+// neighbouring tokens.  Rows that do not fit are read again instead.
 //
 // Order of K.  A producer lane (g, t) holds whole 16-column blocks, and TMEM wants from it four K elements of every
 // 16-element MMA step, so the K elements are numbered the way the lanes hold them: element 4t + i of step j of a
 // 64-column half unit is column 16t + 4j + i.  The activations are written in that order here.
-constexpr int kStageThreads = 1024;
+constexpr int kStageThreads = 512;
+constexpr size_t kStageSmem = 200 * 1024;
+static size_t stage_row_bytes(int K) { return size_t(K) * 2 + 16; }   // + 16: rows start on different banks
 __global__ void __launch_bounds__(kStageThreads) stage_activations_kernel(const __nv_bfloat16 *__restrict__ x, __half *__restrict__ out,
                                                                           float *__restrict__ xmul, int K, int KP, int tokens,
-                                                                          int padded_tokens, int half_in) {
-  __shared__ unsigned warp_max[32];
+                                                                          int padded_tokens, int per_cta, int rows_fit, int half_in) {
+  extern __shared__ __align__(16) uint8_t rows_smem[];
+  __shared__ unsigned warp_max[kStageThreads / 32];
   grid_launch_dependents();      // the tile kernel may set up (barriers, TMEM, first weight loads) while this one runs
+  grid_dependency_wait();        // the scratch may still be read by an earlier call's tile kernel, and x be on its way
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int chunks = K / 8, padded = KP / 8;
-  const int first = blockIdx.x * 8;
+  const int chunks = K / 8, padded = KP / 8, row_bytes = K * 2 + 16;
+  const int first = blockIdx.x * per_cta, per_token = kStageThreads / per_cta;   // threads that read one row
   {
-    const int tok = first + (warp >> 2);
+    const int j = threadIdx.x / per_token, tok = first + j;
     unsigned m = 0;
-    if (tok < tokens && !half_in) {
+    if (tok < tokens && (rows_fit || !half_in)) {
       const uint4 *src = reinterpret_cast<const uint4 *>(x + size_t(tok) * K);
-      for (int i = (warp & 3) * 32 + lane; i < chunks; i += 128) m = max(m, chunk_absmax(src[i]));
-      m = __reduce_max_sync(0xffffffffu, m);
+      uint4 *row = reinterpret_cast<uint4 *>(rows_smem + size_t(j) * row_bytes);
+#pragma unroll 8
+      for (int i = threadIdx.x % per_token; i < chunks; i += per_token) {
+        const uint4 v = __ldcg(src + i);
+        if (rows_fit) row[i] = v;
+        if (!half_in) m = max(m, chunk_absmax(v));
+      }
     }
+    m = __reduce_max_sync(0xffffffffu, m);
     if (lane == 0) warp_max[warp] = m;
   }
   __syncthreads();
-  const int j = threadIdx.x & 7, tok = first + j;
-  const unsigned m = max(max(warp_max[4 * j], warp_max[4 * j + 1]), max(warp_max[4 * j + 2], warp_max[4 * j + 3]));
+  const int j = threadIdx.x % per_cta, tok = first + j;
+  const int warps = per_token / 32;
+  unsigned m = 0;
+  for (int w = 0; w < warps; ++w) m = max(m, warp_max[j * warps + w]);
   float mult, inverse;
   token_scaling(m, mult, inverse);
   if (half_in) inverse = 1.f;   // fp16 activations (x then points to fp16) are the operand as they are
-  if (threadIdx.x < 8 && tok < tokens && blockIdx.y == 0) xmul[tok] = inverse * kNumeratorScale;
+  if (int(threadIdx.x) < per_cta && tok < tokens) xmul[tok] = inverse * kNumeratorScale;
   uint4 *dst = reinterpret_cast<uint4 *>(out);
-  const __nv_bfloat16 *src = x + size_t(tok < tokens ? tok : 0) * K;
-  // few tokens give few CTAs: blockIdx.y cuts the conversion (not the scan above) into column slices
-  const int per_slice = (padded + int(gridDim.y) - 1) / int(gridDim.y);
-  const int slice_end = min(padded, (int(blockIdx.y) + 1) * per_slice);
-  for (int chunk = int(blockIdx.y) * per_slice + (threadIdx.x >> 3); chunk < slice_end; chunk += kStageThreads / 8) {
+  const uint8_t *row = rows_smem + size_t(j) * row_bytes;
+  const __nv_bfloat16 *again = x + size_t(tok < tokens ? tok : 0) * K;
+  const auto four = [&](int column) {
+    return rows_fit ? *reinterpret_cast<const uint2 *>(row + size_t(column) * 2) : __ldcg(reinterpret_cast<const uint2 *>(again + column));
+  };
+#pragma unroll 4
+  for (int chunk = threadIdx.x / per_cta; chunk < padded; chunk += per_token) {
     // chunk 2j + c of a half unit: columns 16(2c) + 4j .. + 3 and 16(2c + 1) + 4j .. + 3
     const int column = (chunk >> 3) * 64 + (chunk & 1) * 32 + ((chunk >> 1) & 3) * 4;
     uint4 v = make_uint4(0, 0, 0, 0);
     if (tok < tokens) {
       if (column < K) {
-        const uint2 low = *reinterpret_cast<const uint2 *>(src + column);
+        const uint2 low = four(column);
         v.x = low.x;
         v.y = low.y;
       }
       if (column + 16 < K) {
-        const uint2 high = *reinterpret_cast<const uint2 *>(src + column + 16);
+        const uint2 high = four(column + 16);
         v.z = high.x;
         v.w = high.y;
       }
@@ -577,6 +593,7 @@ static int launch_tile(const Handle *h, const __nv_bfloat16 *x, __nv_bfloat16 *y
     std::lock_guard<std::mutex> lock(guard);
     if (!configured[{h->device, generic}]) {
       TX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(Cfg::smem)));
+      TX_CUDA(cudaFuncSetAttribute(stage_activations_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kStageSmem)));
       configured[{h->device, generic}] = true;
     }
   }
@@ -588,9 +605,11 @@ static int launch_tile(const Handle *h, const __nv_bfloat16 *x, __nv_bfloat16 *y
   for (int t0 = 0; t0 < tokens; t0 += capacity) {
     const int n = std::min(capacity, tokens - t0);
     const int padded_tokens = (n + 31) & ~31;
-    const int slices = std::max(1, std::min(16, ws->sm_count / (padded_tokens / 8)));
-    stage_activations_kernel<<<dim3(padded_tokens / 8, slices), kStageThreads, 0, stream>>>(x + size_t(t0) * h->K, ws->xprep, ws->xmul, h->K, KP, n,
-                                                                    padded_tokens, half_io ? 1 : 0);
+    int per_cta = 4;
+    while (per_cta > 1 && (padded_tokens / per_cta < ws->sm_count * 3 / 4 || per_cta * stage_row_bytes(h->K) > kStageSmem)) per_cta /= 2;
+    const bool rows_fit = per_cta * stage_row_bytes(h->K) <= kStageSmem;
+    TX_CUDA(launch_pdl(stage_activations_kernel, dim3(padded_tokens / per_cta), dim3(kStageThreads), rows_fit ? per_cta * stage_row_bytes(h->K) : 0,
+                       stream, x + size_t(t0) * h->K, ws->xprep, ws->xmul, h->K, KP, n, padded_tokens, per_cta, rows_fit ? 1 : 0, half_io ? 1 : 0));
     count_launch();
     // staged X viewed as [KP/8 chunks][padded_tokens/32][32 tokens x 8 elements]: a box is one run of
     // 512 contiguous bytes per 32 tokens and chunk and lands as core-matrix columns
