@@ -1044,8 +1044,8 @@ int launch_gemv(const Handle *h, const __nv_bfloat16 *x, __nv_bfloat16 *y, int t
     if (plan.pre) {
       // scaled fp16 activations go through the per-device scratch (one pre-pass CTA per token)
       if (size_t(n) * KP > ws->xprep_halfs) return fail(TX_EINVAL, "tokens*K exceeds the activation scratch of the decode GEMV");
-      if (half_io) gemv_xprep_kernel<true><<<n, kGemvThreads, 0, stream>>>(p.x, ws->xprep, ws->xmul, h->K, KP);
-      else gemv_xprep_kernel<false><<<n, kGemvThreads, 0, stream>>>(p.x, ws->xprep, ws->xmul, h->K, KP);
+      TX_CUDA(launch_pdl(half_io ? gemv_xprep_kernel<true> : gemv_xprep_kernel<false>, dim3(n), dim3(kGemvThreads), 0, stream,
+                         static_cast<const void *>(p.x), ws->xprep, ws->xmul, h->K, KP));
       count_launch();
       p.xprep = ws->xprep;
       p.xmul = ws->xmul;

@@ -220,8 +220,8 @@ __global__ void __launch_bounds__(kStageThreads) stage_activations_kernel(const 
                                                                           int padded_tokens, int per_cta, int rows_fit, int half_in) {
   extern __shared__ __align__(16) uint8_t rows_smem[];
   __shared__ unsigned warp_max[kStageThreads / 32];
-  grid_launch_dependents();      // the tile kernel may set up (barriers, TMEM, first weight loads) while this one runs
   grid_dependency_wait();        // the scratch may still be read by an earlier call's tile kernel, and x be on its way
+  grid_launch_dependents();      // the tile kernel may set up (barriers, TMEM, first weight loads) while this one runs
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int chunks = K / 8, padded = KP / 8, row_bytes = K * 2 + 16;
   const int first = blockIdx.x * per_cta, per_token = kStageThreads / per_cta;   // threads that read one row
@@ -554,16 +554,6 @@ static EncodeTiled encode_tiled_entry() {
 // (192 tokens: 5120-row matrices at 512+ tokens launch 120 CTAs instead of 80 or 160 on the 148 SMs)
 // Tall tiles re-read the activations less often (tensor-bound prompts); narrow ones suit short prompts
 // where the weight stream is the bound.
-// Handles that were packed without a tuned backend.  Short prompts are paced by the producers, so the narrowest tile that
-// holds all tokens wins; from 192 tokens on, 192-token tiles unless the 256-token ones need fewer token blocks per SM.
-int prefill_choose_backend(const Handle *h, int tokens) {
-  if (tokens <= 64) return 8;
-  if (tokens <= 128) return 7;
-  const int blocks = (h->M + 127) / 128;
-  const auto waves = [&](int bn) { return (long(blocks) * ((tokens + bn - 1) / bn) + 147) / 148 * bn; };
-  return waves(192) < waves(256) ? 9 : 5;
-}
-
 bool prefill_tile_eligible(const Handle *h, int backend, int tokens) {
   return backend >= 5 && backend <= 9 && tokens >= 1 && h->K % 16 == 0 && encode_tiled_entry() != nullptr;
 }
@@ -577,6 +567,30 @@ static int prefill_k_ranges(const Handle *h, int tokens, const Workspace *ws) {
   int ranges = std::min(std::min(ws->sm_count / std::max(blocks, 1), 8), h->KI / 4);
   while (ranges > 1 && size_t(ranges) * tokens * h->M > ws->partial_floats) --ranges;
   return std::max(ranges, 1);
+}
+
+// The tile of handles without a tuned backend, and of the baseline id 5: all tiles give the same bits, so only time decides.
+// A wave of CTAs takes its 128-column stages at the pace of the MMAs or, below 128 tokens, of the producers, plus
+// what a CTA spends before and after them (TMEM, first loads, epilogue).  Measured on 5120x17408 with 512 tokens
+// (136 stages): 0.30, 0.35, 0.50 and 0.67 us a stage for 64, 128, 192 and 256 tokens and about 4 us a CTA; the tile with
+// the smallest sum over the waves wins, the wider one on a tie (it reads the activations less often).
+int prefill_choose_backend(const Handle *h, int tokens) {
+  const Workspace *ws = workspace_for(h->device);
+  if (!ws) return 5;
+  const struct { int backend, bn, stage; } tiles[4] = {{5, 256, 67}, {9, 192, 50}, {7, 128, 35}, {8, 64, 30}};   // stage: 10 ns
+  const int ranges = prefill_k_ranges(h, tokens, ws), stages = (h->KI + ranges - 1) / ranges;
+  const long blocks = long((h->M + 127) / 128) * ranges;
+  long best = 0;
+  int pick = 5;
+  for (const auto &tile : tiles) {
+    const long waves = (blocks * ((tokens + tile.bn - 1) / tile.bn) + ws->sm_count - 1) / ws->sm_count;
+    const long cost = waves * (400 + long(stages) * tile.stage);
+    if (best == 0 || cost < best) {
+      best = cost;
+      pick = tile.backend;
+    }
+  }
+  return pick;
 }
 
 template <int CTAS, int BN>
@@ -655,6 +669,7 @@ static int launch_tile(const Handle *h, const __nv_bfloat16 *x, __nv_bfloat16 *y
 // texelator_cuda.cu:996-1046; this kernel multiplies the exact numerators and scales in the epilogue)
 int launch_prefill_tile(const Handle *h, int backend, const __nv_bfloat16 *x, __nv_bfloat16 *y, int tokens, cudaStream_t stream,
                         bool half_io) {
+  if (backend == 5) backend = prefill_choose_backend(h, tokens);
   switch (backend) {
     case 5: return launch_tile<1, 256>(h, x, y, tokens, stream, half_io);
     case 6: return launch_tile<2, 256>(h, x, y, tokens, stream, half_io);
