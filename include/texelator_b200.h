@@ -180,7 +180,8 @@ int tx_set_palette(uint64_t handle, int palette);
  * [M, K] row-major, `hdiag` fp32 [K] (the activation second moments E[x_k^2] that weight the error),
  * `lut` fp32 [255, 255, 8] = palette[e1 + 127][e0 + 127][selector]; writes M * K / 2 bytes of row-major BC4
  * blocks (the .bc4 file content) and M fp32 row scales (the .scales.f32 content), which tx_pack_encoded
- * accepts as they are.  Asynchronous on `stream`. */
+ * accepts as they are.  `weight`, `hdiag` and `blocks_out` on 16-byte boundaries; `lut` may start at any float.
+ * Asynchronous on `stream`. */
 int tx_encode(const float *weight, const float *hdiag, const float *lut, int M, int K, uint8_t *blocks_out, float *scales_out,
               void *stream);
 

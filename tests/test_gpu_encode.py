@@ -113,3 +113,18 @@ def test_directory_written_by_the_reference_loads_and_runs(ext, lut, golden_dir)
         got_blocks, got_scales = ext.encode(torch.from_numpy(inputs[f"{key}/weight"]).cuda(), torch.from_numpy(inputs[f"{key}/hdiag"]).cuda(),
                                             torch.from_numpy(lut).cuda())
         assert np.array_equal(got_blocks.cpu().numpy(), blocks) and np.array_equal(got_scales.cpu().numpy(), scales)
+
+
+@pytest.mark.parametrize("shift", [0, 1, 2, 3])
+def test_palette_at_any_float(ext, lut, shift):
+    """A palette that is a slice of a larger buffer need not lie on a 16-byte boundary."""
+    gen = torch.Generator().manual_seed(shift)
+    w, hdiag = torch.randn(37, 592, generator=gen) * 0.05, torch.exp(torch.randn(592, generator=gen))
+    buffer = torch.zeros(lut.size + 8, device="cuda")
+    table = buffer[shift:shift + lut.size].view(255, 255, 8)
+    table.copy_(torch.from_numpy(lut))
+    assert buffer.data_ptr() % 16 == 0 and table.data_ptr() % 16 == 4 * shift
+    blocks, scales = ext.encode(w.cuda(), hdiag.cuda(), table)
+    want_blocks, want_scales = O.encode_linear(w, hdiag, lut)
+    assert np.array_equal(scales.cpu().numpy(), want_scales)
+    assert np.array_equal(blocks.cpu().numpy(), want_blocks.reshape(-1))

@@ -81,6 +81,12 @@ __device__ __forceinline__ int nearest_selector(float v, const float (&p)[8]) {
   return sel;
 }
 
+// half of a palette row (entries 0-3 or 4-7); WIDE: the table lies on a 16-byte boundary, so one load fetches it
+template <bool WIDE> __device__ __forceinline__ float4 palette_half(const float *row, int half) {
+  if (WIDE) return reinterpret_cast<const float4 *>(row)[half];
+  return make_float4(row[4 * half], row[4 * half + 1], row[4 * half + 2], row[4 * half + 3]);
+}
+
 __device__ __forceinline__ int clamp127(int e) { return min(max(e, -127), 127); }
 
 // value / scale, rounded to nearest: the residual correction of a quotient that is off by at most one unit in the last
@@ -99,7 +105,7 @@ constexpr int kEncodeThreads = 128;
 
 // A group of GROUP lanes encodes one row after another (rows group, group + groups, ...): the row's largest magnitude
 // first, then one 16-weight block per lane and step.
-template <int GROUP>
+template <int GROUP, bool WIDE>
 __global__ void __launch_bounds__(kEncodeThreads) encode_kernel(const float *__restrict__ weight, const float *__restrict__ hdiag,
                                                                 const float *__restrict__ lut, unsigned long long *__restrict__ blocks,
                                                                 float *__restrict__ scales, int M, int K) {
@@ -162,12 +168,12 @@ __global__ void __launch_bounds__(kEncodeThreads) encode_kernel(const float *__r
         h2[2 * j + 1] = pack2(g.z, g.w);
       }
       const int e0 = clamp127(int(rintf(__fmul_rn(vmax, 127.f)))), e1 = clamp127(int(rintf(__fmul_rn(vmin, 127.f))));
-      const auto palette_row = [&](int q0, int q1) { return reinterpret_cast<const float4 *>(lut + (size_t(q1 + 127) * 255 + (q0 + 127)) * 8); };
+      const auto palette_row = [&](int q0, int q1) { return lut + (size_t(q1 + 127) * 255 + (q0 + 127)) * 8; };
       unsigned long long start_bits = 0;
       float saa, sbb, sab, say, sby;
       {
         // weighted 2x2 normal equations on the start's selectors (encoder.py:72-84)
-        const float4 p_lo = palette_row(e0, e1)[0], p_hi = palette_row(e0, e1)[1];
+        const float4 p_lo = palette_half<WIDE>(palette_row(e0, e1), 0), p_hi = palette_half<WIDE>(palette_row(e0, e1), 1);
         const float p[8] = {p_lo.x, p_lo.y, p_lo.z, p_lo.w, p_hi.x, p_hi.y, p_hi.z, p_hi.w};
         const int high = e0 > e1;
         float taa[16], tbb[16], tab[16], tay[16], tby[16];
@@ -202,12 +208,13 @@ __global__ void __launch_bounds__(kEncodeThreads) encode_kernel(const float *__r
       // The next neighbour's palette is requested before this one's errors are computed.
       float best = INFINITY;
       int out = -1;
-      float4 p_lo = palette_row(clamp127(c0 - 1), clamp127(c1 - 1))[0], p_hi = palette_row(clamp127(c0 - 1), clamp127(c1 - 1))[1];
+      const float *first = palette_row(clamp127(c0 - 1), clamp127(c1 - 1));
+      float4 p_lo = palette_half<WIDE>(first, 0), p_hi = palette_half<WIDE>(first, 1);
 #pragma unroll 1
       for (int n = 0; n < 9; ++n) {
         const int next = min(n + 1, 8);
-        const float4 *ahead = palette_row(clamp127(c0 + next / 3 - 1), clamp127(c1 + next % 3 - 1));
-        const float4 next_lo = ahead[0], next_hi = ahead[1];
+        const float *ahead = palette_row(clamp127(c0 + next / 3 - 1), clamp127(c1 + next % 3 - 1));
+        const float4 next_lo = palette_half<WIDE>(ahead, 0), next_hi = palette_half<WIDE>(ahead, 1);
         unsigned long long d2[8];
         nearest_distances(v2, p_lo, p_hi, d2);
         // (scalar products and sums: ptxas contracts a packed multiply whose result meets a packed add, even with .rn on
@@ -231,7 +238,7 @@ __global__ void __launch_bounds__(kEncodeThreads) encode_kernel(const float *__r
       if (out >= 0) {                                   // (no neighbour wins only when the errors are not numbers)
         out0 = clamp127(c0 + out / 3 - 1);
         out1 = clamp127(c1 + out % 3 - 1);
-        const float4 q_lo = palette_row(out0, out1)[0], q_hi = palette_row(out0, out1)[1];
+        const float4 q_lo = palette_half<WIDE>(palette_row(out0, out1), 0), q_hi = palette_half<WIDE>(palette_row(out0, out1), 1);
         const float p[8] = {q_lo.x, q_lo.y, q_lo.z, q_lo.w, q_hi.x, q_hi.y, q_hi.z, q_hi.w};
         bits = 0;
 #pragma unroll
@@ -246,7 +253,9 @@ template <int GROUP>
 static void launch_encode_rows(const float *weight, const float *hdiag, const float *lut, int M, int K, uint8_t *blocks, float *scales, cudaStream_t stream) {
   const int per_cta = kEncodeThreads / GROUP;
   const int grid = int(std::min<size_t>((size_t(M) + per_cta - 1) / per_cta, size_t(1) << 20));
-  encode_kernel<GROUP><<<grid, kEncodeThreads, 0, stream>>>(weight, hdiag, lut, reinterpret_cast<unsigned long long *>(blocks), scales, M, K);
+  // a palette may start at any float (a slice of a larger buffer): the wide loads are for tables on a 16-byte boundary
+  const auto kernel = reinterpret_cast<uintptr_t>(lut) & 15 ? encode_kernel<GROUP, false> : encode_kernel<GROUP, true>;
+  kernel<<<grid, kEncodeThreads, 0, stream>>>(weight, hdiag, lut, reinterpret_cast<unsigned long long *>(blocks), scales, M, K);
 }
 
 int launch_encode(const float *weight, const float *hdiag, const float *lut, int M, int K, uint8_t *blocks, float *scales, cudaStream_t stream) {
