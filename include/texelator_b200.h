@@ -206,7 +206,8 @@ int tx_kernel_status(int device, int clear);
  *   rope_append      : rotate q and k of one token in place (rotate-half), append k and v to the
  *                      caches [kv_heads, max_len, head_dim] at *position (device int64)
  *   rope_append_prompt : the same for `tokens` rows of qkv at positions first, first + 1, ... (head_dim a
- *                      multiple of 16)
+ *                      multiple of 16).  The launch behind it starts when the rows are stored, so that an
+ *                      attention_step behind that launch may read them ahead
  *   attention_decode : one query per head over cache positions 0..*position, grouped-query; `scratch`
  *                      holds q_heads * ceil(max_len/128) * (head_dim+2) floats; head_dim must be 128
  *   attention_step   : rope_append + attention_decode of one token in one call (q is rotated on the
@@ -216,7 +217,9 @@ int tx_kernel_status(int device, int clear);
  *                      floats; head_dim 128; long caches are walked in 64-key chunks per CTA.  `position` and
  *                      the cache rows below it are read before the kernel waits for the launch in front of it
  *                      (they overlap that launch's tail): they must be complete when that launch starts, as they
- *                      are in a decode loop, where earlier steps wrote them
+ *                      are in a decode loop, where earlier steps wrote them, and behind rope_append_prompt;
+ *                      rope_append and attention_step itself let the launches behind them start early, so a
+ *                      step over rows they wrote needs a launch that is not one of this library's in between
  *   silu_mul         : out[t,i] = silu(gate_up[t,i]) * gate_up[t,intermediate+i]                     */
 int tx_aux_add_rmsnorm(void *h, const void *delta, const void *weight, void *y, int tokens, int hidden, float eps, void *stream);
 /* add_rmsnorm for one token with the extras of tx_linear_single: delta may come as `splits` fp32 partial

@@ -98,6 +98,36 @@ def test_attention_step_equals_two_kernel_path(ext):
     assert torch.allclose(a.float(), b.float(), atol=1e-2, rtol=1e-2)
 
 
+def test_attention_step_behind_an_appended_prompt(ext):
+    """A prompt's rows appended, a linear, one attention step over them, all on one stream: the step reads its rows
+    before it waits for the linear, and must see every row each time."""
+    q_heads, kv_heads, head_dim, tokens, max_len = 16, 2, 128, 3000, 3008
+    handle, gen = _packed_linear(ext, 64, 256, 5)
+    bf = dict(device="cuda", dtype=torch.bfloat16)
+    angles = torch.rand(max_len, head_dim // 2, device="cuda", generator=gen) * 6.28
+    cos, sin = angles.cos().contiguous(), angles.sin().contiguous()
+    prompt = torch.randn(tokens, (q_heads + 2 * kv_heads) * head_dim, generator=gen, **bf)
+    qkv = torch.randn(1, (q_heads + 2 * kv_heads) * head_dim, generator=gen, **bf)
+    x, y = torch.randn(8, 256, generator=gen, **bf), torch.empty(8, 64, **bf)
+    position = torch.full((1,), tokens, dtype=torch.int64, device="cuda")
+    scratch = torch.zeros(ext.attention_step_scratch_floats(q_heads, max_len), dtype=torch.float32, device="cuda")
+    outputs = []
+    for repeat in range(20):
+        k_cache, v_cache = torch.zeros(kv_heads, max_len, head_dim, **bf), torch.zeros(kv_heads, max_len, head_dim, **bf)
+        rows, out = prompt.clone(), torch.empty(1, q_heads * head_dim, **bf)
+        torch.cuda.synchronize()
+        ext.rope_append_prompt(rows, cos, sin, 0, k_cache, v_cache, q_heads, kv_heads, head_dim)
+        if repeat == 0:
+            torch.cuda.synchronize()
+        ext.linear_out(handle, x[:1 + repeat % 8], y[:1 + repeat % 8])
+        ext.attention_step(qkv, cos, sin, position, k_cache, v_cache, scratch, out, q_heads, kv_heads, head_dim)
+        torch.cuda.synchronize()
+        outputs.append(out)
+    ext.free(handle)
+    for out in outputs[1:]:
+        assert torch.equal(out, outputs[0])
+
+
 def test_attention_step_rejects_unsupported_shapes(ext):
     bf = dict(device="cuda", dtype=torch.bfloat16)
     cache = torch.zeros(1, 64, 64, **bf)

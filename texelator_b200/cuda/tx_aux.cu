@@ -562,11 +562,13 @@ __global__ void __launch_bounds__(64) rope_append_kernel(__nv_bfloat16 *__restri
 // rotated in place, k and v appended to the caches.  Bound by memory (every value is read once and written at most
 // twice): a thread owns eight dimensions of both halves of one head, so all accesses are 16 bytes and a warp
 // covers four heads of a token.
+// attention_step_kernel reads cache rows before it waits for the launch in front of it, and that launch (a linear) may
+// itself have started early.  So this kernel never signals its dependents: what follows starts when every block has
+// stored its rows and fenced, and whatever follows that sees them.
 __global__ void __launch_bounds__(256) rope_append_prompt_kernel(__nv_bfloat16 *__restrict__ qkv, const float *__restrict__ cos_table,
                                                                  const float *__restrict__ sin_table, int first, int tokens,
                                                                  __nv_bfloat16 *__restrict__ k_cache, __nv_bfloat16 *__restrict__ v_cache,
                                                                  int q_heads, int kv_heads, int head_dim, int max_len) {
-  grid_launch_dependents();
   grid_dependency_wait();
   const int half = head_dim / 2, per_head = half / 8, heads = q_heads + 2 * kv_heads;
   const size_t total = size_t(tokens) * heads * per_head;
@@ -599,6 +601,7 @@ __global__ void __launch_bounds__(256) rope_append_prompt_kernel(__nv_bfloat16 *
       *reinterpret_cast<uint4 *>(dst + half) = b;
     }
   }
+  __threadfence();
 }
 
 // Single-query attention over cache positions [0, pos], split along the sequence: CTA (split, kv head)
@@ -800,9 +803,9 @@ __global__ void __launch_bounds__(kStepThreads, 2) attention_step_kernel(const _
   out += size_t(blockIdx.z) * q_heads * kHeadDim;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   grid_launch_dependents();
-  // The position and the cache rows below it were written by earlier steps (no launch of this library writes
-  // them, and a foreign kernel directly in front would have to finish first), so they are read before the wait
-  // for the launch in front -- the qkv linear, whose tail these loads overlap.  Only qkv itself is new.
+  // The position and the cache rows below it are complete when the launch in front starts: earlier steps wrote them,
+  // or rope_append_prompt_kernel, which lets nothing start before its rows are stored.  So they are read before the
+  // wait for that launch -- the qkv linear, whose tail these loads overlap.  Only qkv itself is new.
   const long long pos = __ldcg(position);                       // attends to keys 0..pos; key pos is new
   const int live = int(pos / kStepKeys) + 1;                    // splits that hold at least one key
   if (split >= live) return;
