@@ -206,7 +206,7 @@ int tx_kernel_status(int device, int clear);
  *   rope_append      : rotate q and k of one token in place (rotate-half), append k and v to the
  *                      caches [kv_heads, max_len, head_dim] at *position (device int64)
  *   rope_append_prompt : the same for `tokens` rows of qkv at positions first, first + 1, ... (head_dim a
- *                      multiple of 16).  The launch behind it starts when the rows are stored, so that an
+ *                      multiple of 16, all pointers 16-byte aligned).  The launch behind it starts when the rows are stored, so that an
  *                      attention_step behind that launch may read them ahead
  *   attention_decode : one query per head over cache positions 0..*position, grouped-query; `scratch`
  *                      holds q_heads * ceil(max_len/128) * (head_dim+2) floats; head_dim must be 128

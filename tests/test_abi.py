@@ -46,6 +46,15 @@ def test_calls_without_a_gpu_fail_with_a_message(library):
     assert library.tx_launch_count() == 0
 
 
+@pytest.mark.parametrize("shifted", [0, 1, 2, 6, 7])
+def test_prompt_append_refuses_pointers_off_a_16_byte_boundary(library, shifted):
+    """Its loads and stores are 16 bytes wide; the check comes before any launch, so no device is needed."""
+    pointers = [4096 + (4 if index == shifted else 0) for index in range(8)]
+    qkv, cos, sin, k_cache, v_cache = pointers[0], pointers[1], pointers[2], pointers[6], pointers[7]
+    assert library.tx_aux_rope_append_prompt(qkv, cos, sin, 0, 0, k_cache, v_cache, 1, 1, 16, 1, None) == -1
+    assert b"16-byte aligned" in library.tx_last_error()
+
+
 def test_operator_refuses_cpu_tensors():
     import torch
     from texelator_b200 import runtime

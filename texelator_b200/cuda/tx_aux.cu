@@ -1614,6 +1614,9 @@ int tx_aux_rope_append_prompt(void *qkv, const float *cos_table, const float *si
                               void *v_cache, int q_heads, int kv_heads, int head_dim, int max_len, void *stream) {
   if (!qkv || !cos_table || !sin_table || !k_cache || !v_cache || q_heads < 1 || kv_heads < 1 || head_dim < 16 || head_dim % 16)
     return fail(TX_EINVAL, "tx_aux_rope_append_prompt: head_dim must be a multiple of 16 and no pointer null");
+  if ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(cos_table) | reinterpret_cast<uintptr_t>(sin_table) |
+       reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) & 15)
+    return fail(TX_EINVAL, "tx_aux_rope_append_prompt: pointers must be 16-byte aligned");
   if (tokens < 1 || first < 0 || max_len - first < tokens) return fail(TX_EINVAL, "tx_aux_rope_append_prompt: positions must lie inside the cache");
   const size_t total = size_t(tokens) * (q_heads + 2 * kv_heads) * (head_dim / 16);
   const int grid = int(std::min<size_t>((total + 255) / 256, 148 * 8));
