@@ -65,6 +65,28 @@ def test_operator_refuses_cpu_tensors():
         runtime.TexelatorLinear([])
 
 
+def test_operator_refuses_tensors_without_memory():
+    """Fake tensors pass for CUDA tensors; a view of one even has a nonzero address (its offset)."""
+    import torch
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    from texelator_b200 import runtime
+    ext = runtime.extension()
+    handle = 1 << 40                                        # never dereferenced: the call is refused before
+    ext._remember(handle, 32, 64, 0)
+    try:
+        with FakeTensorMode():
+            x = torch.empty(4, 64, device="cuda", dtype=torch.bfloat16)
+            y = torch.empty(4, 32, device="cuda", dtype=torch.bfloat16)
+        for rows in (slice(0, 4), slice(1, 4)):
+            with pytest.raises(RuntimeError, match="contiguous CUDA FP16 or BF16"):
+                ext.linear(handle, x[rows])
+            with pytest.raises(RuntimeError, match="contiguous CUDA FP16 or BF16"):
+                ext.linear_out(handle, x[rows], y[rows])
+    finally:
+        ext._shapes.pop(handle)
+        ext._binding.forget(handle)
+
+
 def test_no_product_code_imports_the_oracle():
     for path in list((ROOT / "texelator_b200").rglob("*.py")) + list((ROOT / "texelator_b200").rglob("*.cu")):
         text = path.read_text()

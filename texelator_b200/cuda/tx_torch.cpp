@@ -55,6 +55,10 @@ bool take_arguments(PyObject *const *args, Py_ssize_t nargs, PyObject *kwnames, 
   return fits;
 }
 
+// A fake tensor (shape propagation under torch.compile and its kin) calls itself a CUDA tensor but owns no memory, and
+// a view of one has its offset for an address: nothing may be launched on it.
+bool has_memory(const at::Tensor &t) { return t.numel() == 0 || (t.has_storage() && t.storage().data() != nullptr); }
+
 // the checks of texelator_cuda.cu:1332-1337; null with an exception set when one fails
 const Shape *check_input(PyObject *handle_object, PyObject *x_object, uint64_t *handle, const at::Tensor **x) {
   *handle = PyLong_AsUnsignedLongLong(handle_object);
@@ -74,6 +78,10 @@ const Shape *check_input(PyObject *handle_object, PyObject *x_object, uint64_t *
   *x = &THPVariable_Unpack(x_object);
   const at::Tensor &t = **x;
   if (!t.is_cuda() || (t.scalar_type() != at::kBFloat16 && t.scalar_type() != at::kHalf) || !t.is_contiguous()) {
+    raise("input must be contiguous CUDA FP16 or BF16");
+    return nullptr;
+  }
+  if (!has_memory(t)) {
     raise("input must be contiguous CUDA FP16 or BF16");
     return nullptr;
   }
@@ -140,7 +148,8 @@ PyObject *linear_out(PyObject *, PyObject *const *args, Py_ssize_t nargs, PyObje
   }
   const at::Tensor &y = THPVariable_Unpack(given[2]);
   const Shape shape = *found;
-  if (y.numel() != x->numel() / shape.k * shape.m || y.scalar_type() != x->scalar_type() || !y.is_contiguous() || y.device() != x->device())
+  if (y.numel() != x->numel() / shape.k * shape.m || y.scalar_type() != x->scalar_type() || !y.is_contiguous() || y.device() != x->device() ||
+      !has_memory(y))
     return raise("input shape/device mismatch");
   if (!launch(handle, *x, y, shape)) return nullptr;
   return Py_NewRef(given[2]);
