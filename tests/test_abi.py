@@ -65,6 +65,30 @@ def test_operator_refuses_cpu_tensors():
         runtime.TexelatorLinear([])
 
 
+@pytest.mark.parametrize("number", ["np.int64(5)", "np.uint64(5)", "None", "1.5", "-3", "2 ** 70", "'a'"])
+def test_unknown_handle_numbers_are_null_handles(number):
+    """An integer of any kind is a handle number; what names no handle is refused as the null handle is."""
+    import numpy as np
+    import torch
+    from texelator_b200 import runtime
+    with pytest.raises(RuntimeError, match="null Texelator handle"):
+        runtime.extension().linear(eval(number, {"np": np}), torch.zeros(1, 16, dtype=torch.bfloat16))
+
+
+def test_handle_numbers_of_numpy_are_known():
+    import numpy as np
+    import torch
+    from texelator_b200 import runtime
+    ext = runtime.extension()
+    ext._remember(1 << 40, 32, 64, 0)
+    try:
+        with pytest.raises(RuntimeError, match="contiguous CUDA"):      # the handle is found, the CPU tensor refused
+            ext.linear(np.int64(1 << 40), torch.zeros(1, 64, dtype=torch.bfloat16))
+    finally:
+        ext._shapes.pop(1 << 40)
+        ext._binding.forget(1 << 40)
+
+
 def test_operator_refuses_tensors_without_memory():
     """Fake tensors pass for CUDA tensors; a view of one even has a nonzero address (its offset)."""
     import torch

@@ -61,10 +61,13 @@ bool has_memory(const at::Tensor &t) { return t.numel() == 0 || (t.has_storage()
 
 // the checks of texelator_cuda.cu:1332-1337; null with an exception set when one fails
 const Shape *check_input(PyObject *handle_object, PyObject *x_object, uint64_t *handle, const at::Tensor **x) {
-  *handle = PyLong_AsUnsignedLongLong(handle_object);
-  if (*handle == uint64_t(-1) && PyErr_Occurred()) {
-    if (!PyErr_ExceptionMatches(PyExc_OverflowError)) return nullptr;
+  // any integer (NumPy's too); what is none, or does not fit, names no handle
+  PyObject *number = PyNumber_Index(handle_object);
+  *handle = number ? PyLong_AsUnsignedLongLong(number) : 0;
+  Py_XDECREF(number);
+  if (PyErr_Occurred()) {
     PyErr_Clear();
+    *handle = 0;
   }
   auto found = g_shapes.find(*handle);
   if (found == g_shapes.end()) {
