@@ -111,6 +111,24 @@ def test_operator_refuses_tensors_without_memory():
         ext._binding.forget(handle)
 
 
+def test_output_form_refuses_zero_tokens():
+    """``linear`` returns an empty tensor for no tokens; with an output of its own the caller must have some."""
+    import torch
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    from texelator_b200 import runtime
+    ext = runtime.extension()
+    ext._remember(1 << 40, 32, 64, 0)
+    try:
+        with FakeTensorMode():
+            x = torch.empty(0, 64, device="cuda", dtype=torch.bfloat16)
+            y = torch.empty(0, 32, device="cuda", dtype=torch.bfloat16)
+        with pytest.raises(RuntimeError, match="contiguous CUDA FP16 or BF16"):
+            ext.linear_out(1 << 40, x, y)
+    finally:
+        ext._shapes.pop(1 << 40)
+        ext._binding.forget(1 << 40)
+
+
 def test_no_product_code_imports_the_oracle():
     for path in list((ROOT / "texelator_b200").rglob("*.py")) + list((ROOT / "texelator_b200").rglob("*.cu")):
         text = path.read_text()

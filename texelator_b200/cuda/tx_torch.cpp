@@ -154,6 +154,7 @@ PyObject *linear_out(PyObject *, PyObject *const *args, Py_ssize_t nargs, PyObje
   if (y.numel() != x->numel() / shape.k * shape.m || y.scalar_type() != x->scalar_type() || !y.is_contiguous() || y.device() != x->device() ||
       !has_memory(y))
     return raise("input shape/device mismatch");
+  if (x->numel() == 0) return raise("input must be contiguous CUDA FP16 or BF16");   // tx_linear refuses a null activation pointer
   if (!launch(handle, *x, y, shape)) return nullptr;
   return Py_NewRef(given[2]);
   END_HANDLE_TH_ERRORS
