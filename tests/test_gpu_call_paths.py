@@ -44,6 +44,27 @@ def test_native_call_checks_and_keywords(ext, lut):
         ext.linear(h, x)
 
 
+def test_native_call_goes_to_the_library_that_packed_the_handle(ext, lut):
+    """Two loaded libraries (the second one a stand-in that launches nothing) serve their own handles."""
+    import ctypes
+    from types import SimpleNamespace
+    from texelator_b200 import runtime
+    blocks, scales, gen = _encoded(48, 64, 1, lut)
+    h = ext.pack_encoded(torch.from_numpy(blocks).reshape(-1), torch.from_numpy(scales))
+    x = torch.randn(3, 64, generator=gen).cuda().bfloat16()
+    before, calls = ext.linear(h, x), []
+    entry = ctypes.CFUNCTYPE(ctypes.c_int, ctypes.c_uint64, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_void_p)
+    stand_in = SimpleNamespace(tx_linear=entry(lambda *arguments: calls.append(arguments) or 0),
+                               tx_last_error=ctypes.CFUNCTYPE(ctypes.c_char_p)(lambda: b"stand-in"))
+    other = runtime._Extension(stand_in, runtime.load_binding())
+    other._remember(1 << 40, 32, 64, x.get_device())
+    assert other.linear(1 << 40, x).shape == (3, 32)
+    assert len(calls) == 1 and calls[0][:2] == (1 << 40, x.data_ptr()) and calls[0][3:5] == (3, 1)
+    assert torch.equal(ext.linear(h, x), before) and len(calls) == 1
+    other._binding.forget(1 << 40)
+    ext.free(h)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("tokens", [16, 64, 65, 128, 129, 400])
 def test_untuned_handle_matches_oracle(ext, lut, tokens, dtype):

@@ -5,8 +5,9 @@
 // per call.  Here the tensor is read through its C++ object, the output comes straight from the caching allocator
 // and the C-ABI entry point is called through its address: 4.8 us a call with the module's own Python on top.
 //
-// The module holds no CUDA code and links no library of this package: `bind` receives the addresses of the C-ABI
-// functions (include/texelator_b200.h), so the same build serves whichever library the loader chose.
+// The module holds no CUDA code and links no library of this package: every handle is remembered with the addresses
+// of the C-ABI functions (include/texelator_b200.h) of the library that packed it, so several loaded libraries keep
+// to their own handles.
 #include <Python.h>
 
 #include <ATen/ATen.h>
@@ -26,10 +27,10 @@ using ErrorFn = const char *(*)();
 struct Shape {
   int64_t m, k;
   int device;
+  LinearFn linear;
+  ErrorFn last_error;
 };
 
-LinearFn g_linear = nullptr;
-ErrorFn g_last_error = nullptr;
 std::unordered_map<uint64_t, Shape> g_shapes;   // every access holds the GIL
 
 PyObject *raise(const char *message) {
@@ -108,10 +109,10 @@ bool launch(uint64_t handle, const at::Tensor &x, const at::TensorBase &y, const
   const int dtype = x.scalar_type() == at::kBFloat16 ? 1 : 0;
   int status;
   Py_BEGIN_ALLOW_THREADS   // a launch can wait for room in the stream's queue
-  status = g_linear(handle, in, out, int(tokens), dtype, stream);
+  status = shape.linear(handle, in, out, int(tokens), dtype, stream);
   Py_END_ALLOW_THREADS
   if (status != 0) {
-    const char *message = g_last_error();
+    const char *message = shape.last_error();
     raise(message && message[0] ? message : "texelator_b200 call failed");
     return false;
   }
@@ -160,21 +161,15 @@ PyObject *linear_out(PyObject *, PyObject *const *args, Py_ssize_t nargs, PyObje
   END_HANDLE_TH_ERRORS
 }
 
-PyObject *bind(PyObject *, PyObject *args) {
-  unsigned long long linear_address, error_address;
-  if (!PyArg_ParseTuple(args, "KK", &linear_address, &error_address)) return nullptr;
-  g_linear = reinterpret_cast<LinearFn>(linear_address);
-  g_last_error = reinterpret_cast<ErrorFn>(error_address);
-  Py_RETURN_NONE;
-}
-
 PyObject *remember(PyObject *, PyObject *args) {
-  unsigned long long handle;
+  unsigned long long handle, linear_address, error_address;
   long long m, k;
   int device;
-  if (!PyArg_ParseTuple(args, "KLLi", &handle, &m, &k, &device)) return nullptr;
-  g_shapes[handle] = Shape{m, k, device};
+  if (!PyArg_ParseTuple(args, "KLLiKK", &handle, &m, &k, &device, &linear_address, &error_address)) return nullptr;
+  HANDLE_TH_ERRORS
+  g_shapes[handle] = Shape{m, k, device, reinterpret_cast<LinearFn>(linear_address), reinterpret_cast<ErrorFn>(error_address)};
   Py_RETURN_NONE;
+  END_HANDLE_TH_ERRORS
 }
 
 PyObject *forget(PyObject *, PyObject *args) {
@@ -188,8 +183,7 @@ PyObject *forget(PyObject *, PyObject *args) {
 PyMethodDef methods[] = {
     {"linear", TX_FAST(linear), "linear(handle, x) -> tensor [..., M]"},
     {"linear_out", TX_FAST(linear_out), "linear_out(handle, x, y) -> y, for outputs the caller keeps (CUDA graphs)"},
-    {"bind", bind, METH_VARARGS, "addresses of tx_linear and tx_last_error"},
-    {"remember", remember, METH_VARARGS, "remember(handle, m, k, device)"},
+    {"remember", remember, METH_VARARGS, "remember(handle, m, k, device, address of tx_linear, address of tx_last_error)"},
     {"forget", forget, METH_VARARGS, "forget(handle)"},
     {nullptr, nullptr, 0, nullptr}};
 

@@ -117,12 +117,12 @@ class _Extension:
         self._lib, self._binding = library, binding
         self._shapes: dict[int, tuple[int, int, int]] = {}   # handle -> (M, K, device)
         address = lambda function: ctypes.cast(function, ctypes.c_void_p).value
-        binding.bind(address(library.tx_linear), address(library.tx_last_error))
+        self._entry = address(library.tx_linear), address(library.tx_last_error)
         self.linear, self.linear_out = binding.linear, binding.linear_out
 
     def _remember(self, handle: int, m: int, k: int, device: int) -> int:
         self._shapes[handle] = (m, k, device)
-        self._binding.remember(handle, m, k, device)
+        self._binding.remember(handle, m, k, device, *self._entry)
         return handle
 
     # -- helpers -------------------------------------------------------------
