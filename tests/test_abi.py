@@ -85,8 +85,7 @@ def test_handle_numbers_of_numpy_are_known():
         with pytest.raises(RuntimeError, match="contiguous CUDA"):      # the handle is found, the CPU tensor refused
             ext.linear(np.int64(1 << 40), torch.zeros(1, 64, dtype=torch.bfloat16))
     finally:
-        ext._shapes.pop(1 << 40)
-        ext._binding.forget(1 << 40)
+        ext._forget(1 << 40)
 
 
 def test_operator_refuses_tensors_without_memory():
@@ -107,8 +106,7 @@ def test_operator_refuses_tensors_without_memory():
             with pytest.raises(RuntimeError, match="contiguous CUDA FP16 or BF16"):
                 ext.linear_out(handle, x[rows], y[rows])
     finally:
-        ext._shapes.pop(handle)
-        ext._binding.forget(handle)
+        ext._forget(handle)
 
 
 def test_output_form_refuses_zero_tokens():
@@ -125,8 +123,39 @@ def test_output_form_refuses_zero_tokens():
         with pytest.raises(RuntimeError, match="contiguous CUDA FP16 or BF16"):
             ext.linear_out(1 << 40, x, y)
     finally:
-        ext._shapes.pop(1 << 40)
-        ext._binding.forget(1 << 40)
+        ext._forget(1 << 40)
+
+
+def test_binding_for_another_torch_is_refused(monkeypatch):
+    import torch
+    from texelator_b200 import runtime
+    assert runtime.load_binding().built_for.startswith(f"torch {torch.__version__}, Python 3.")
+    monkeypatch.setattr(torch, "__version__", "1.0")
+    with pytest.raises(ImportError, match="was built for torch"):
+        runtime.load_binding()
+
+
+@pytest.mark.parametrize("reason", ["absent", "another torch"])
+def test_library_without_a_usable_binding_still_loads(monkeypatch, tmp_path, reason):
+    """A prebuilt library alone, or beside a binding for another torch, serves the operator through ctypes."""
+    import torch
+    from texelator_b200 import runtime
+    runtime.extension()                                     # both files exist from here on
+    monkeypatch.setenv("TEXELATOR_DISABLE_JIT", "1")
+    monkeypatch.setattr(runtime, "_EXTENSION", None)
+    if reason == "absent":
+        monkeypatch.setattr(runtime, "BINDING_PATH", tmp_path / "_tx_torch.so")
+    else:
+        monkeypatch.setattr(torch, "__version__", "1.0")
+    with pytest.warns(RuntimeWarning, match="through ctypes"):
+        ext = runtime.extension()
+    x = torch.zeros(1, 64, dtype=torch.bfloat16)
+    with pytest.raises(RuntimeError, match="null Texelator handle"):
+        ext.linear(1 << 40, x)
+    ext._remember(1 << 40, 32, 64, 0)
+    with pytest.raises(RuntimeError, match="contiguous CUDA FP16 or BF16"):
+        ext.linear(1 << 40, x)
+    ext._forget(1 << 40)
 
 
 def test_no_product_code_imports_the_oracle():

@@ -61,8 +61,29 @@ def test_native_call_goes_to_the_library_that_packed_the_handle(ext, lut):
     assert other.linear(1 << 40, x).shape == (3, 32)
     assert len(calls) == 1 and calls[0][:2] == (1 << 40, x.data_ptr()) and calls[0][3:5] == (3, 1)
     assert torch.equal(ext.linear(h, x), before) and len(calls) == 1
-    other._binding.forget(1 << 40)
+    other._forget(1 << 40)
     ext.free(h)
+
+
+def test_call_without_the_binding_gives_the_same_outputs(ext, lut):
+    import numpy as np
+    from texelator_b200 import runtime
+    blocks, scales, gen = _encoded(48, 64, 1, lut)
+    plain = runtime._Extension(ext._lib)
+    h = plain.pack_encoded(torch.from_numpy(blocks).reshape(-1), torch.from_numpy(scales))
+    ext._remember(h, *plain._shapes[h])
+    for tokens in (1, 3, 40):
+        for dtype in (torch.bfloat16, torch.float16):
+            x = torch.randn(tokens, 64, generator=gen).cuda().to(dtype)
+            out = torch.empty(tokens, 48, device="cuda", dtype=dtype)
+            assert torch.equal(plain.linear(h, x), ext.linear(h, x))
+            assert plain.linear_out(np.uint64(h), x, out) is out and torch.equal(out, ext.linear(np.uint64(h), x))
+    for one in (plain, ext):
+        assert one.linear(h, x[:0]).shape == (0, 48)
+        with pytest.raises(RuntimeError, match="contiguous CUDA FP16 or BF16"):
+            one.linear_out(h, x[:0], out[:0])
+    ext._forget(h)
+    plain.free(h)
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])

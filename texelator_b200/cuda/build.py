@@ -59,18 +59,37 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     return LIBRARY
 
 
+def binding_target() -> str:
+    """What the binding is compiled for; the compiled module carries this text and the loader compares it."""
+    import torch
+    return f"torch {torch.__version__}, Python {sys.version_info.major}.{sys.version_info.minor}"
+
+
+def binding_digest() -> str:
+    return hashlib.sha256(BINDING_SOURCE.read_bytes() + binding_target().encode() + sys.version.encode()).hexdigest()
+
+
+def binding_is_current() -> bool:
+    """Whether the module on disk is the one this source and this torch would build (a prebuilt one without a stamp is
+    left to the loader's check)."""
+    if not BINDING.exists():
+        return False
+    return not (BINDING_STAMP.exists() and BINDING_SOURCE.exists()) or BINDING_STAMP.read_text().strip() == binding_digest()
+
+
 def build_binding(force: bool = False, verbose: bool = False) -> Path:
     """The CPython module ``_tx_torch`` (host code only; g++ against the installed torch's headers)."""
     import sysconfig
 
     import torch
-    digest = hashlib.sha256(BINDING_SOURCE.read_bytes() + torch.__version__.encode() + sys.version.encode()).hexdigest()
+    digest = binding_digest()
     if not force and BINDING.exists() and BINDING_STAMP.exists() and BINDING_STAMP.read_text().strip() == digest:
         return BINDING
     root = Path(torch.__file__).resolve().parent
     cuda = Path(nvcc_path()).resolve().parent.parent
     include = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include", sysconfig.get_paths()["include"], cuda / "include"]
     command = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+               f'-DTX_BUILT_FOR="{binding_target()}"',
                *[f"-I{path}" for path in include], str(BINDING_SOURCE), "-o", str(BINDING), f"-L{root / 'lib'}", f"-Wl,-rpath,{root / 'lib'}",
                "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python"]
     result = subprocess.run(command, capture_output=True, text=True)

@@ -191,4 +191,12 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_tx_torch", nullptr, -1, methods};
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__tx_torch() { return PyModule_Create(&module); }
+// Tensors are read through inlined C++ accessors, which hold for one torch only; the loader compares this text.
+#ifndef TX_BUILT_FOR
+#define TX_BUILT_FOR "unknown"
+#endif
+PyMODINIT_FUNC PyInit__tx_torch() {
+  PyObject *self = PyModule_Create(&module);
+  if (self && PyModule_AddStringConstant(self, "built_for", TX_BUILT_FOR) != 0) Py_CLEAR(self);
+  return self;
+}

@@ -18,6 +18,7 @@ import ctypes
 import gc
 import json
 import os
+import warnings
 from pathlib import Path
 
 import numpy as np
@@ -96,13 +97,18 @@ def load_library(path: Path | None = None) -> ctypes.CDLL:
 
 
 def load_binding(path: Path | None = None):
-    """Import the CPython module of the operator call (raises if it does not fit the installed torch)."""
+    """Import the CPython module of the operator call; ``ImportError`` when it was built for another torch or Python
+    (it reads tensors through accessors that were inlined when it was built)."""
+    from .cuda.build import binding_target
     from importlib.machinery import ExtensionFileLoader
     from importlib.util import module_from_spec, spec_from_file_location
     location = str(path or BINDING_PATH)
     spec = spec_from_file_location("_tx_torch", location, loader=ExtensionFileLoader("_tx_torch", location))
     module = module_from_spec(spec)
     spec.loader.exec_module(module)
+    if getattr(module, "built_for", None) != binding_target():
+        raise ImportError(f"{location} was built for {getattr(module, 'built_for', 'an unknown torch')}, this is {binding_target()}; "
+                          "rebuild with `python -m texelator_b200.cuda.build`")
     return module
 
 
@@ -111,19 +117,27 @@ class _Extension:
     (texelator/cuda/extension.cpp:27-48): same function names and semantics.
 
     ``linear(handle, x)`` returns ``[..., M]`` in the input's type; ``linear_out(handle, x, y)`` writes into a
-    caller-provided output (static buffers for CUDA graphs).  Both are functions of the native binding."""
+    caller-provided output (static buffers for CUDA graphs).  Both are functions of the native binding; without one they
+    are the methods below, which make the same call through ctypes."""
 
-    def __init__(self, library: ctypes.CDLL, binding):
+    def __init__(self, library: ctypes.CDLL, binding=None):
         self._lib, self._binding = library, binding
         self._shapes: dict[int, tuple[int, int, int]] = {}   # handle -> (M, K, device)
-        address = lambda function: ctypes.cast(function, ctypes.c_void_p).value
-        self._entry = address(library.tx_linear), address(library.tx_last_error)
-        self.linear, self.linear_out = binding.linear, binding.linear_out
+        if binding is not None:
+            address = lambda function: ctypes.cast(function, ctypes.c_void_p).value
+            self._entry = address(library.tx_linear), address(library.tx_last_error)
+            self.linear, self.linear_out = binding.linear, binding.linear_out
 
     def _remember(self, handle: int, m: int, k: int, device: int) -> int:
         self._shapes[handle] = (m, k, device)
-        self._binding.remember(handle, m, k, device, *self._entry)
+        if self._binding is not None:
+            self._binding.remember(handle, m, k, device, *self._entry)
         return handle
+
+    def _forget(self, handle: int) -> None:
+        self._shapes.pop(handle, None)
+        if self._binding is not None:
+            self._binding.forget(handle)
 
     # -- helpers -------------------------------------------------------------
     def _check(self, status: int) -> None:
@@ -209,6 +223,22 @@ class _Extension:
             raise RuntimeError("input shape/device mismatch")
         return m, k, device, x.numel() // k
 
+    def _linear(self, handle: int, x: torch.Tensor, y: torch.Tensor, tokens: int, device: int) -> torch.Tensor:
+        dtype = DTYPE_BF16 if x.dtype == torch.bfloat16 else DTYPE_F16
+        self._check(self._lib.tx_linear(handle, x.data_ptr(), y.data_ptr(), tokens, dtype, torch.cuda.current_stream(device).cuda_stream))
+        return y
+
+    def linear(self, handle: int, x: torch.Tensor) -> torch.Tensor:
+        m, _, device, tokens = self._activation(handle, x)
+        y = torch.empty(x.shape[:-1] + (m,), dtype=x.dtype, device=x.device)
+        return self._linear(handle, x, y, tokens, device) if tokens else y
+
+    def linear_out(self, handle: int, x: torch.Tensor, y: torch.Tensor) -> torch.Tensor:
+        m, _, device, tokens = self._activation(handle, x)
+        if y.numel() != tokens * m or y.dtype != x.dtype or not y.is_contiguous() or y.device != x.device:
+            raise RuntimeError("input shape/device mismatch")
+        return self._linear(handle, x, y, tokens, device)
+
     def linear_static_scratch(self, handle: int, x: torch.Tensor) -> torch.Tensor:
         """``linear`` for a small token group through the entry point that allocates nothing on the
         device: its activation scratch is a fixed array inside the library (for callers whose memory
@@ -277,8 +307,7 @@ class _Extension:
         return self.kernel_info(9)
 
     def free(self, handle: int) -> None:
-        self._shapes.pop(handle, None)
-        self._binding.forget(handle)
+        self._forget(handle)
         self._check(self._lib.tx_free(handle))
 
     def palette_probe(self) -> torch.Tensor:
@@ -488,24 +517,37 @@ class _Extension:
         return int(self._lib.tx_launch_count())
 
 
+def _native_binding(build_allowed: bool, verbose: bool):
+    """The native operator call, or ``None`` with a warning where it cannot be had: no compiler, a build for another torch
+    that may not be rebuilt, a prebuilt library that came without it.  The kernels are the same either way."""
+    try:
+        from .cuda.build import binding_is_current, build_binding
+        if build_allowed and not binding_is_current():
+            build_binding(verbose=verbose)
+        return load_binding()
+    except (OSError, ImportError, RuntimeError) as error:
+        warnings.warn(f"the operator call goes through ctypes, about 7 us more a call on the host: {error}", RuntimeWarning, stacklevel=3)
+        return None
+
+
 def extension(verbose: bool = False):
     """Load (building in-tree with nvcc if needed) the CUDA library.  Like the reference
     (runtime.py:27-63) this raises instead of degrading when no native code is available;
     ``TEXELATOR_DISABLE_JIT`` forbids the nvcc build."""
     global _EXTENSION
     if _EXTENSION is None:
-        if not (LIBRARY_PATH.exists() and BINDING_PATH.exists()):
-            if os.environ.get("TEXELATOR_DISABLE_JIT", "").upper() in {"1", "ON", "YES", "TRUE"}:
+        build_allowed = os.environ.get("TEXELATOR_DISABLE_JIT", "").upper() not in {"1", "ON", "YES", "TRUE"}
+        if not LIBRARY_PATH.exists():
+            if not build_allowed:
                 raise RuntimeError(
                     "the prebuilt Texelator CUDA library is unavailable and JIT compilation is disabled")
-            from .cuda.build import build, build_binding
-            if not LIBRARY_PATH.exists():
-                build(verbose=verbose)
-            build_binding(verbose=verbose)
+            from .cuda.build import build
+            build(verbose=verbose)
         try:
-            _EXTENSION = _Extension(load_library(), load_binding())
-        except (OSError, AttributeError, ImportError) as error:
+            library = load_library()
+        except (OSError, AttributeError) as error:
             raise RuntimeError(f"the Texelator CUDA library could not be loaded: {error}") from error
+        _EXTENSION = _Extension(library, _native_binding(build_allowed, verbose))
     return _EXTENSION
 
 
