@@ -1,8 +1,11 @@
 """GPU parity of the tensor-core prefill tiles and of the tuners (run with ``-m gpu``)."""
+import re
+
 import numpy as np
 import pytest
 import torch
 
+from graph_kernels import launched
 from oracle import bc4_oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -62,6 +65,57 @@ def test_prefill_tiles_are_bitwise_identical(ext, lut):
             outs.append(ext.linear(h, x.cuda()))
         for other in outs[1:]:
             assert torch.equal(outs[0], other)
+    finally:
+        ext.free(h)
+
+
+TILES = {5: (1, 256), 6: (2, 256), 7: (1, 128), 8: (1, 64), 9: (1, 192)}      # id -> CTAs per tile, tokens
+
+
+def _tile_of(call):
+    """(CTAs, tokens) of the one tile kernel a call launches, or None."""
+    names = [re.search(r"prefill_umma_kernelILi(\d)ELi(\d+)E", name) for name, _ in launched(call)]
+    found = [(int(match[1]), int(match[2])) for match in names if match]
+    assert len(found) <= 1
+    return found[0] if found else None
+
+
+@pytest.mark.parametrize("tokens", [17, 600])
+@pytest.mark.parametrize("backend", sorted(TILES))
+def test_a_backend_id_launches_the_tile_it_names(ext, lut, backend, tokens):
+    blocks, scales, x = _case(3, 300, 912, tokens, lut)
+    h = _pack(ext, blocks, scales)
+    try:
+        ext.set_prefill_backend(h, backend)
+        x, y = x.cuda(), torch.empty(tokens, 300, dtype=torch.bfloat16, device="cuda")
+        assert _tile_of(lambda: ext.linear_out(h, x, y)) == TILES[backend]
+        info = ext.kernel_info(backend)
+        assert (info[5] // 128, info[6]) == TILES[backend]
+    finally:
+        ext.free(h)
+
+
+def test_untuned_handle_takes_every_single_tile_somewhere(ext, lut):
+    """Id 0 leaves the tile to the library; whichever it is, the output is the named tile's bit for bit."""
+    rng = np.random.default_rng(8)
+    m, k = 4250, 912
+    ends = np.sort(rng.integers(-127, 128, (2, m, k // 16)), 0)[::-1].astype(np.int8)
+    blocks = O.pack_blocks(ends[0], ends[1], rng.integers(0, 8, (m, k // 16, 16)).astype(np.uint8)).reshape(-1)
+    h = _pack(ext, blocks, (rng.random(m) + 0.5).astype(np.float32))
+    taken = set()
+    try:
+        for tokens in (16, 64, 160, 257, 600, 1000):
+            x = torch.randn(tokens, k, device="cuda", generator=torch.Generator(device="cuda").manual_seed(tokens)).bfloat16()
+            y = torch.empty(tokens, m, dtype=torch.bfloat16, device="cuda")
+            ext.set_prefill_backend(h, 0)
+            taken.add(_tile_of(lambda: ext.linear_out(h, x, y)))
+            ext.linear_out(h, x, y)
+            for backend in TILES:
+                ext.set_prefill_backend(h, backend)
+                assert torch.equal(ext.linear(h, x), y), (tokens, backend)
+        if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+            assert taken == {(1, 64), (1, 128), (1, 192), (1, 256)}
+        assert taken <= set(TILES.values())
     finally:
         ext.free(h)
 

@@ -569,7 +569,7 @@ static int prefill_k_ranges(const Handle *h, int tokens, const Workspace *ws) {
   return std::max(ranges, 1);
 }
 
-// The tile of handles without a tuned backend, and of the baseline id 5: all tiles give the same bits, so only time decides.
+// The tile of handles without a tuned backend (ids 0..4; 5..9 name one): all tiles give the same bits, so only time decides.
 // A wave of CTAs takes its 128-column stages at the pace of the MMAs or, below 128 tokens, of the producers, plus
 // what a CTA spends before and after them (TMEM, first loads, epilogue).  Measured on 5120x17408 with 512 tokens
 // (136 stages): 0.30, 0.35, 0.50 and 0.67 us a stage for 64, 128, 192 and 256 tokens and about 4 us a CTA; the tile with
@@ -669,7 +669,6 @@ static int launch_tile(const Handle *h, const __nv_bfloat16 *x, __nv_bfloat16 *y
 // texelator_cuda.cu:996-1046; this kernel multiplies the exact numerators and scales in the epilogue)
 int launch_prefill_tile(const Handle *h, int backend, const __nv_bfloat16 *x, __nv_bfloat16 *y, int tokens, cudaStream_t stream,
                         bool half_io) {
-  if (backend == 5) backend = prefill_choose_backend(h, tokens);
   switch (backend) {
     case 5: return launch_tile<1, 256>(h, x, y, tokens, stream, half_io);
     case 6: return launch_tile<2, 256>(h, x, y, tokens, stream, half_io);

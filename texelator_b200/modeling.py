@@ -153,11 +153,12 @@ class BC4Decoder:
     all-reduces after o/down over ``group``.  ``keep_dense`` also keeps ``bf16(pal*scale)``
     copies of every projection (from ``ext.dequant``) so that ``forward(..., dense=True)`` runs
     the same model through ``torch.matmul`` -- the dequantise-then-matmul comparison.
+    ``prefill_backend`` names a tile (5..9) or leaves the choice to the library for every prompt (0).
     """
 
     def __init__(self, config: DecoderConfig, device, max_len: int, seed: int = 0, tp_rank: int = 0,
                  tp_world: int = 1, group=None, lookahead: int = 3, keep_dense: bool = False,
-                 weight_std: float = 0.02, prefill_backend: int = 5, encoder: str = "minmax"):
+                 weight_std: float = 0.02, prefill_backend: int = 0, encoder: str = "minmax"):
         self.config, self.device, self.max_len = config, torch.device(device), max_len
         self.rank, self.world, self.group = tp_rank, tp_world, group
         if encoder not in ("minmax", "e3"):
