@@ -138,9 +138,12 @@ int tx_linear_single_info(uint64_t handle, int64_t out[3]);
 int tx_set_lookahead(uint64_t handle, int lookahead);
 /* set_prefill: texelator_cuda.cu:1480-1488.  threshold >= 1; tile_rows >= 16 and % 16 == 0. */
 int tx_set_prefill(uint64_t handle, int threshold, int tile_rows);
-/* set_prefill_backend: texelator_cuda.cu:1490-1503.  0..4: streamed small-batch path in token
- * groups; 5..9: tensor-core tile candidates (rows x tokens per CTA: 128x256, 256x256, 128x128, 128x64,
- * 128x192; see tx_kernel_info). */
+/* set_prefill_backend: texelator_cuda.cu:1490-1503; which kernel serves tokens >= threshold.  5..9: the tensor-core
+ * tile of that id (rows x tokens per CTA: 128x256, 256x256, 128x128, 128x64, 128x192; see tx_kernel_info).  0..4, which
+ * name the reference's fallback kernels: the library's choice by shape and token count, one of the tiles or, up to
+ * eight tokens, the decode kernel; TX_DECODE_ALU_EXACT handles stream their prompts through that path.  All tiles give
+ * the same bits; a tile adds a K range in one fp32 accumulator, the decode kernel in sixteen (raise the threshold to
+ * keep a handle's prompts there). */
 int tx_set_prefill_backend(uint64_t handle, int backend);
 /* New: choose the decode path (TX_DECODE_*). TX_DECODE_TEXTURE fails with TX_EUNSUPPORTED when
  * BC4 texture views are unavailable, and with TX_ESTATE when the hardware palette differs from

@@ -120,6 +120,26 @@ def test_untuned_handle_takes_every_single_tile_somewhere(ext, lut):
         ext.free(h)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("tokens", [1, 2, 8, 9, 15])
+def test_untuned_handle_with_a_low_threshold(ext, lut, tokens, dtype):
+    """Up to eight tokens the decode kernel serves the call as below a threshold, to the bit; from nine on a tile does."""
+    blocks, scales, x = _case(5, 300, 912, tokens, lut)
+    h = _pack(ext, blocks, scales)
+    try:
+        x, y = x.cuda().to(dtype), torch.empty(tokens, 300, dtype=dtype, device="cuda")
+        streamed = ext.linear(h, x)
+        ext.set_prefill(h, 1, 1024)
+        assert (_tile_of(lambda: ext.linear_out(h, x, y)) is None) == (tokens <= 8)
+        ext.linear_out(h, x, y)
+        if tokens <= 8:
+            assert torch.equal(y, streamed)
+        # otherwise the same products in another order, then one rounding: neighbours (2^-8, 2^-11 of the value) at most
+        assert float((y.double() - streamed.double()).norm() / streamed.double().norm()) <= (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11)
+    finally:
+        ext.free(h)
+
+
 def test_prefill_low_mode_blocks(ext, lut):
     blocks, scales, x = _case(4, 256, 512, 64, lut, sparse=0.9)
     h = _pack(ext, blocks, scales)

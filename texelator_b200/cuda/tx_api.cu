@@ -197,10 +197,12 @@ int tx_linear(uint64_t handle, const void *x, void *y, int tokens, int dtype, vo
   if (current != h->device) TX_CUDA(cudaSetDevice(h->device));
   int rc;
   // texelator_cuda.cu:1341 -- tokens >= threshold takes the prefill side of the dispatcher
-  // (ids 0..4 name the reference's fallback kernels; here they leave the choice of the tile to the library, and the
-  // exact-arithmetic and texture paths keep serving such handles' prompts themselves)
-  const int backend = h->prefill_backend >= 5 || h->decode_path != TX_DECODE_ALU_MMA ? h->prefill_backend : prefill_choose_backend(h, tokens);
-  if (tokens >= h->prefill_threshold && backend >= 5 && prefill_tile_eligible(h, backend, tokens)) {
+  // (ids 0..4 name the reference's fallback kernels; here they leave the choice to the library, and the exact-arithmetic
+  // and texture paths keep serving such handles' prompts themselves)
+  int backend = 0;
+  if (tokens >= h->prefill_threshold)
+    backend = h->prefill_backend >= 5 || h->decode_path != TX_DECODE_ALU_MMA ? h->prefill_backend : prefill_choose_backend(h, tokens);
+  if (backend >= 5 && prefill_tile_eligible(h, backend, tokens)) {
     rc = launch_prefill_tile(h, backend, xb, yb, tokens, stream, half_io);
   } else if (h->decode_path == TX_DECODE_ALU_EXACT) {
     rc = launch_gemv_exact(h, xb, yb, tokens, stream);

@@ -348,7 +348,7 @@ int launch_prefill_tile(const Handle *h, int backend, const __nv_bfloat16 *x, __
 // y = round(sum of `ranges` fp32 partial results [ranges][tokens][M] + bias): second step of a launch that cut K
 int launch_combine(const float *partial, int ranges, const void *bias, void *y, int tokens, int M, bool half_io, int sm_count,
                    cudaStream_t stream);
-int prefill_choose_backend(const Handle *h, int tokens);   // the tile a handle without a tuned backend takes
+int prefill_choose_backend(const Handle *h, int tokens);   // the tile a handle without a tuned backend takes; 0: the decode kernel
 bool prefill_tile_eligible(const Handle *h, int backend, int tokens);
 int gemv_kernel_info(int64_t out[9]);
 int prefill_kernel_info(int backend, int64_t out[9]);

@@ -574,7 +574,14 @@ static int prefill_k_ranges(const Handle *h, int tokens, const Workspace *ws) {
 // what a CTA spends before and after them (TMEM, first loads, epilogue).  Measured on 5120x17408 with 512 tokens
 // (136 stages): 0.30, 0.35, 0.50 and 0.67 us a stage for 64, 128, 192 and 256 tokens and about 4 us a CTA; the tile with
 // the smallest sum over the waves wins, the wider one on a tie (it reads the activations less often).
+//
+// Up to eight tokens (a threshold below the default of 16) the decode kernel keeps the call: it pays one group of MMA columns
+// there, and two from nine on.  Decode kernel against the 64-token tile, us a call from HBM: 256x2048 2.6 / 7.5 with one
+// token, 7.6 / 7.5 with eight, 11.2 / 7.6 with ten; 5120x5120 6.5 / 11.5, 11.6 / 11.8, 20.0 / 11.9; 34816x5120
+// 24.0 / 31.5, 30.8 / 32.0, 51.5 / 32.0.
+constexpr int kStreamedTokens = 8;
 int prefill_choose_backend(const Handle *h, int tokens) {
+  if (tokens <= kStreamedTokens) return 0;
   const Workspace *ws = workspace_for(h->device);
   if (!ws) return 5;
   const struct { int backend, bn, stage; } tiles[4] = {{5, 256, 67}, {9, 192, 50}, {7, 128, 35}, {8, 64, 30}};   // stage: 10 ns
