@@ -283,11 +283,14 @@ int tx_aux_silu_mul(const void *gate_up, void *out, int tokens, int intermediate
  *                          out [sequences, q_heads * head_dim]; `scratch` holds `sequences` times the floats of
  *                          attention_step; sequences * kv_heads <= 4096.
  *   silu_mul_pairs       : silu_mul for gate/up rows stored as alternating groups of eight (the row order the
- *                          SwiGLU-fused linear takes): out[t, 8j + e] = silu(gu[t, 16j + e]) * gu[t, 16j + 8 + e]. */
+ *                          SwiGLU-fused linear takes): out[t, 8j + e] = silu(gu[t, 16j + e]) * gu[t, 16j + 8 + e].
+ *   silu_mul_pairs_accurate : the same with expf in place of the fast exponential of the decode step (prompts: the
+ *                          outputs of PyTorch's silu(g.float()) * u.float()). */
 int tx_aux_attention_step_batch(const void *qkv, const float *cos_table, const float *sin_table, const void *positions, void *k_cache,
                                 void *v_cache, float *scratch, void *out, int sequences, int q_heads, int kv_heads, int head_dim,
                                 int max_len, float scale, void *stream);
 int tx_aux_silu_mul_pairs(const void *gate_up, void *out, int tokens, int intermediate, void *stream);
+int tx_aux_silu_mul_pairs_accurate(const void *gate_up, void *out, int tokens, int intermediate, void *stream);
 
 /* Number of this library's kernels launched by the calling process since load (all threads). */
 int64_t tx_launch_count(void);

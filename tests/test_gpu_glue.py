@@ -141,6 +141,33 @@ def test_attention_step_rejects_unsupported_shapes(ext):
         ext.attention_step(torch.zeros(1, 3 * 128, **bf), table, table, position, big, big, scratch, torch.zeros(1, 128, **bf), 1, 1, 128)
 
 
+def test_accurate_swiglu_is_pytorchs(ext):
+    """Every finite bf16 gate with 256 up values each: the prompt's SwiGLU gives PyTorch's bits."""
+    gates = torch.arange(-32768, 32768, dtype=torch.int32, device="cuda").to(torch.int16).view(torch.bfloat16)
+    gates = gates[gates.isfinite()]
+    gates = gates[:gates.numel() // 8 * 8]
+    tokens, columns = 256, gates.numel()
+    up = torch.randn(tokens, columns, device="cuda", generator=torch.Generator(device="cuda").manual_seed(4)).bfloat16()
+    gate_up = torch.stack([gates.view(1, -1, 8).expand(tokens, -1, -1), up.view(tokens, -1, 8)], 2).reshape(tokens, -1).contiguous()
+    out = torch.empty(tokens, columns, device="cuda", dtype=torch.bfloat16)
+    ext.silu_mul_pairs(gate_up, out, accurate=True)
+    want = (torch.nn.functional.silu(gates.float()) * up.float()).bfloat16()
+    assert torch.equal(out.view(torch.int16), want.view(torch.int16))
+
+
+def test_prompt_takes_the_accurate_swiglu(ext, monkeypatch):
+    from texelator_b200 import runtime
+    from texelator_b200.modeling import CONFIGS, BC4Decoder
+    calls = []
+    original = runtime._Extension.silu_mul_pairs
+    monkeypatch.setattr(runtime._Extension, "silu_mul_pairs",
+                        lambda self, gate_up, out, accurate=False: (calls.append(accurate), original(self, gate_up, out, accurate))[1])
+    model = BC4Decoder(CONFIGS["toy128"], "cuda:0", max_len=64, seed=3)
+    model.prefill(torch.arange(20))
+    model.free()
+    assert calls == [True] * CONFIGS["toy128"].layers
+
+
 def _packed_linear(ext, m, k, seed, bias=False):
     from texelator_b200.modeling import encode_minmax_cuda, software_palette_table
     gen = torch.Generator(device="cuda").manual_seed(seed)

@@ -1300,7 +1300,10 @@ __global__ void __launch_bounds__(256) silu_mul_kernel(const __nv_bfloat16 *__re
 }
 
 // the same for rows stored as (gate, up) groups of eight -- the row order of the SwiGLU-fused linear:
-// out[t, 8j + e] = silu(gu[t, 16j + e]) * gu[t, 16j + 8 + e]
+// out[t, 8j + e] = silu(gu[t, 16j + e]) * gu[t, 16j + 8 + e].  ACCURATE takes expf (2 units in the last place) where the
+// decode step's kernels take __expf, whose relative error grows with the argument: the prompt's arithmetic is then
+// PyTorch's silu(g.float()) * u.float() to the bit.  The pass is bound by memory either way.
+template <bool ACCURATE>
 __global__ void __launch_bounds__(256) silu_mul_pairs_kernel(const __nv_bfloat16 *__restrict__ gu, __nv_bfloat16 *__restrict__ out,
                                                              int inter, int tokens) {
   grid_launch_dependents();
@@ -1316,7 +1319,8 @@ __global__ void __launch_bounds__(256) silu_mul_pairs_kernel(const __nv_bfloat16
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const float2 g = __bfloat1622float2(pg[e]), u = __bfloat1622float2(pu[e]);
-      pr[e] = __floats2bfloat162_rn(g.x / (1.f + __expf(-g.x)) * u.x, g.y / (1.f + __expf(-g.y)) * u.y);
+      const float ex = ACCURATE ? expf(-g.x) : __expf(-g.x), ey = ACCURATE ? expf(-g.y) : __expf(-g.y);
+      pr[e] = __floats2bfloat162_rn(g.x / (1.f + ex) * u.x, g.y / (1.f + ey) * u.y);
     }
     *reinterpret_cast<uint4 *>(out + size_t(t) * inter + size_t(j) * 8) = result;
   }
@@ -1704,15 +1708,23 @@ int tx_aux_attention_step_batch(const void *qkv, const float *cos_table, const f
                             max_len, scale, stream);
 }
 
-int tx_aux_silu_mul_pairs(const void *gate_up, void *out, int tokens, int intermediate, void *stream) {
+static int launch_silu_mul_pairs(const void *gate_up, void *out, int tokens, int intermediate, bool accurate, void *stream) {
   if (!gate_up || !out || tokens < 1 || intermediate < 8 || intermediate % 8) return fail(TX_EINVAL, "tx_aux_silu_mul_pairs: bad argument");
   size_t chunks = size_t(tokens) * intermediate / 8;
   int grid = int(std::min<size_t>((chunks + 255) / 256, 148 * 8));
-  TX_CUDA(launch_pdl(silu_mul_pairs_kernel, dim3(grid), dim3(256), 0, static_cast<cudaStream_t>(stream),
+  TX_CUDA(launch_pdl(accurate ? silu_mul_pairs_kernel<true> : silu_mul_pairs_kernel<false>, dim3(grid), dim3(256), 0, static_cast<cudaStream_t>(stream),
                      static_cast<const __nv_bfloat16 *>(gate_up), static_cast<__nv_bfloat16 *>(out), intermediate, tokens));
   count_launch();
   TX_CUDA(cudaGetLastError());
   return TX_OK;
+}
+
+int tx_aux_silu_mul_pairs(const void *gate_up, void *out, int tokens, int intermediate, void *stream) {
+  return launch_silu_mul_pairs(gate_up, out, tokens, intermediate, false, stream);
+}
+
+int tx_aux_silu_mul_pairs_accurate(const void *gate_up, void *out, int tokens, int intermediate, void *stream) {
+  return launch_silu_mul_pairs(gate_up, out, tokens, intermediate, true, stream);
 }
 
 int tx_aux_silu_mul(const void *gate_up, void *out, int tokens, int intermediate, void *stream) {

@@ -364,7 +364,7 @@ class BC4Decoder:
             delta = self._reduce(ext.linear_out(self.h_o[layer], attended, out))
             ext.add_rmsnorm(h, delta, self.norm2[layer], x, c.rms_eps)
             ext.linear_out(self.h_gu[layer], x, gate_up)
-            ext.silu_mul_pairs(gate_up, act)
+            ext.silu_mul_pairs(gate_up, act, accurate=True)
             delta = self._reduce(ext.linear_out(self.h_down[layer], act, out))
         ext.add_rmsnorm(h, delta, self.final_norm, x, c.rms_eps)
         return x

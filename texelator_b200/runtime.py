@@ -74,6 +74,7 @@ C_API = {
     "tx_aux_attention_step": (_i32, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, ctypes.c_float, _vp]),
     "tx_aux_silu_mul": (_i32, [_vp, _vp, _i32, _i32, _vp]),
     "tx_aux_silu_mul_pairs": (_i32, [_vp, _vp, _i32, _i32, _vp]),
+    "tx_aux_silu_mul_pairs_accurate": (_i32, [_vp, _vp, _i32, _i32, _vp]),
     "tx_aux_attention_step_batch": (_i32, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, ctypes.c_float, _vp]),
     "tx_launch_count": (ctypes.c_int64, []),
     "tx_linear_single": (_i32, [_u64, _vp, _vp, _i32, _vp, _vp, _i32, ctypes.c_size_t, _vp]),
@@ -425,10 +426,12 @@ class _Extension:
                                                           sequences, q_heads, kv_heads, head_dim, max_len, float(head_dim) ** -0.5,
                                                           self._stream(qkv)))
 
-    def silu_mul_pairs(self, gate_up: torch.Tensor, out: torch.Tensor) -> None:
-        """``silu_mul`` for rows in ``interleave_gate_up`` order (gate and up rows in alternating groups of eight)."""
+    def silu_mul_pairs(self, gate_up: torch.Tensor, out: torch.Tensor, accurate: bool = False) -> None:
+        """``silu_mul`` for rows in ``interleave_gate_up`` order (gate and up rows in alternating groups of eight);
+        ``accurate`` takes the accurate exponential, as PyTorch's silu does."""
         tokens, two_i = gate_up.shape
-        self._check(self._lib.tx_aux_silu_mul_pairs(gate_up.data_ptr(), out.data_ptr(), tokens, two_i // 2, self._stream(gate_up)))
+        launch = self._lib.tx_aux_silu_mul_pairs_accurate if accurate else self._lib.tx_aux_silu_mul_pairs
+        self._check(launch(gate_up.data_ptr(), out.data_ptr(), tokens, two_i // 2, self._stream(gate_up)))
 
     def silu_mul(self, gate_up: torch.Tensor, out: torch.Tensor) -> None:
         tokens, two_i = gate_up.shape
