@@ -120,6 +120,29 @@ def test_untuned_handle_takes_every_single_tile_somewhere(ext, lut):
         ext.free(h)
 
 
+@pytest.mark.parametrize("m,k", [(512, 5120), (2048, 2048)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_untuned_prompt_is_as_close_to_64_bits_as_the_decode_kernel(ext, dtype, m, k):
+    """The tile adds a K range in one fp32 accumulator where the decode kernel has sixteen: on Gaussian rows both end at
+    the output's rounding (measured within 1e-4 of each other's distance; 1e-3 allowed)."""
+    from texelator_b200 import runtime
+    from texelator_b200.modeling import encode_minmax_cuda, software_palette_table
+    gen = torch.Generator(device="cuda").manual_seed(m + k)
+    h = ext.pack_encoded_device(*encode_minmax_cuda(torch.randn(m, k, device="cuda", generator=gen) * 0.02, software_palette_table("cuda")))
+    try:
+        w = ext.dequant(h, runtime.DEQUANT_SCALED_F32).double()
+        x = torch.randn(160, k, device="cuda", generator=gen).to(dtype)
+        want = x.double() @ w.T
+        distance = lambda y: float((y.double() - want).norm() / want.norm())
+        tile = distance(ext.linear(h, x))
+        ext.set_prefill(h, 1 << 30, 1024)
+        streamed = distance(ext.linear(h, x))
+        assert tile <= streamed * 1.001
+        assert tile <= (2.0 ** -9 if dtype == torch.bfloat16 else 2.0 ** -12)        # half a unit in the last place
+    finally:
+        ext.free(h)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("tokens", [1, 2, 8, 9, 15])
 def test_untuned_handle_with_a_low_threshold(ext, lut, tokens, dtype):
