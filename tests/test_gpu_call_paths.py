@@ -129,7 +129,7 @@ def test_rope_append_prompt(ext, tokens, first, q_heads, kv_heads, head_dim):
         ext.rope_append_prompt(qkv, cos, sin, max_len, k_cache, v_cache, q_heads, kv_heads, head_dim)
 
 
-@pytest.mark.parametrize("m,k", [(1, 16), (5, 528), (3, 1040), (130, 3168), (9, 2064)])
+@pytest.mark.parametrize("m,k", [(1, 16), (5, 528), (3, 1040), (130, 3168), (9, 2064), (1, 17408), (8, 11200), (7, 2064 * 4), (300, 5136), (593, 4096)])
 def test_encoder_ragged_rows_match_restatement(ext, lut, m, k):
     gen = torch.Generator().manual_seed(m + k)
     w = torch.randn(m, k, generator=gen) * torch.exp(4 * torch.randn(m, 1, generator=gen))

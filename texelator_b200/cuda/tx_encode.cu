@@ -102,9 +102,11 @@ __device__ __forceinline__ float divide_by_scale(float value, float scale, float
 }
 
 constexpr int kEncodeThreads = 128;
+constexpr int kEncodeWave = 148 * 4;   // blocks of threads resident at once (registers)
 
 // A group of GROUP lanes encodes one row after another (rows group, group + groups, ...): the row's largest magnitude
-// first, then one 16-weight block per lane and step.
+// first, then one 16-weight block per lane and step.  With gridDim.y > 1 that many groups share a row: each finds the
+// largest magnitude for itself (the row comes from L2) and takes every gridDim.y-th step.
 template <int GROUP, bool WIDE>
 __global__ void __launch_bounds__(kEncodeThreads) encode_kernel(const float *__restrict__ weight, const float *__restrict__ hdiag,
                                                                 const float *__restrict__ lut, unsigned long long *__restrict__ blocks,
@@ -148,9 +150,9 @@ __global__ void __launch_bounds__(kEncodeThreads) encode_kernel(const float *__r
     const float scale = fmaxf(m, 1e-12f), reciprocal = __frcp_rn(scale);
     const bool normal = scale >= 0x1p-60f && scale <= 0x1p60f;
     if (!live) continue;
-    if (in_group == 0) scales[row] = scale;
+    if (in_group == 0 && blockIdx.y == 0) scales[row] = scale;
 
-    for (int kb = in_group; kb < bpr; kb += GROUP) {
+    for (int kb = blockIdx.y * GROUP + in_group; kb < bpr; kb += gridDim.y * GROUP) {
       unsigned long long v2[8], h2[8];
       float vmax = -INFINITY, vmin = INFINITY;
 #pragma unroll
@@ -253,9 +255,15 @@ template <int GROUP>
 static void launch_encode_rows(const float *weight, const float *hdiag, const float *lut, int M, int K, uint8_t *blocks, float *scales, cudaStream_t stream) {
   const int per_cta = kEncodeThreads / GROUP;
   const int grid = int(std::min<size_t>((size_t(M) + per_cta - 1) / per_cta, size_t(1) << 20));
+  // Rows alone fill the chip from about 600 blocks of threads on (four to an SM).  Below that a row is shared, by as many
+  // groups as fit one wave and have a step each: 8 x 17408 84.6 -> 11.4 us, 100 x 11200 57.9 -> 16.6, 300 x 11200 74.9 -> 44.3
+  // (the kernel that spread single blocks over the chip took 29.2, 61.6 and 153.7).
+  const int steps = (K / 16 + GROUP - 1) / GROUP, shares = std::max(1, std::min(kEncodeWave / grid, steps));
+  const int rounds = (steps + shares - 1) / shares;   // steps of a group
+  const dim3 blocks_of_threads(grid, (steps + rounds - 1) / rounds);
   // a palette may start at any float (a slice of a larger buffer): the wide loads are for tables on a 16-byte boundary
   const auto kernel = reinterpret_cast<uintptr_t>(lut) & 15 ? encode_kernel<GROUP, false> : encode_kernel<GROUP, true>;
-  kernel<<<grid, kEncodeThreads, 0, stream>>>(weight, hdiag, lut, reinterpret_cast<unsigned long long *>(blocks), scales, M, K);
+  kernel<<<blocks_of_threads, kEncodeThreads, 0, stream>>>(weight, hdiag, lut, reinterpret_cast<unsigned long long *>(blocks), scales, M, K);
 }
 
 int launch_encode(const float *weight, const float *hdiag, const float *lut, int M, int K, uint8_t *blocks, float *scales, cudaStream_t stream) {
