@@ -50,6 +50,7 @@ constexpr int kLook = 2;                        // units of its row a producer w
 constexpr int kTmaWarp = kProducerWarps, kMmaWarp = kProducerWarps + 1;
 constexpr int kPrefillThreads = (kProducerWarps + 2) * 32;   // producer/epilogue warps + TMA warp + MMA warp
 constexpr unsigned kSpinLimit = 1u << 22;
+constexpr unsigned kDrainLimit = 1u << 20;      // polls per stage for copies in flight after an abort
 constexpr int kBK = 128;                        // columns per pipeline stage: one unit of the payload
 constexpr int kChunks = kBK / 8;                // 16-byte K chunks of the activation tile per stage
 constexpr int kAColumns = kBK / 2;              // TMEM columns of one A stage (two fp16 per 32-bit column)
@@ -409,9 +410,10 @@ prefill_umma_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap x
         }
       }
       if (*abort_flag) {
-        // give copies that were issued but never consumed time (bounded) to land before the CTA exits
+        // give copies that were issued but never consumed time (bounded) to land before the CTA exits; the wait ends early
+        // where a stage's producers arrived too, and is a delay where they left before it
         for (int kt = issued > S ? issued - S : 0; kt < issued; ++kt)
-          for (unsigned spin = 0; spin < (1u << 16) && !mbar_try_wait(full + 8 * (kt % S), (kt / S) & 1); ++spin) {}
+          for (unsigned spin = 0; spin < kDrainLimit && !mbar_try_wait(full + 8 * (kt % S), (kt / S) & 1); ++spin) {}
       }
     }
   } else if (rank == 0) {
