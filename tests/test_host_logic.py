@@ -150,3 +150,38 @@ def test_directory_written_by_the_reference_is_read_unchanged(golden_dir, lut):
         key = entry["artifact_key"]
         again_blocks, again_scales = O.encode_linear(inputs[f"{key}/weight"], inputs[f"{key}/hdiag"], lut)
         assert np.array_equal(again_blocks, blocks) and np.array_equal(again_scales, scales)
+
+
+def test_encoder_quotients_are_correctly_rounded():
+    """The encoder divides a weight by its row's scale through the reciprocal and two fused corrections where its guard
+    lets it (the guard's bounds are read from the source): every such quotient is the rounded one, at the corners of the
+    guarded range, next to midpoints between two quotients, and for scales near a power of two."""
+    import ctypes
+    import re
+    from pathlib import Path
+    source = (Path(autotune.__file__).parent / "cuda" / "tx_encode.cu").read_text()
+    low, high = (float.fromhex(v) for v in re.search(r"normal = scale >= (0x1p-\d+)f && scale <= (0x1p\d+)f", source).groups())
+    ratio = float.fromhex(re.search(r"fabsf\(value\) >= scale \* (0x1p-\d+)f", source)[1])
+    fma = ctypes.CDLL("libm.so.6").fmaf
+    fma.argtypes, fma.restype = [ctypes.c_float] * 3, ctypes.c_float
+    f32, rng = np.float32, np.random.default_rng(1)
+
+    def quotient(value, scale):
+        reciprocal = f32(1) / scale
+        q = f32(value * reciprocal)
+        q = f32(fma(fma(-q, scale, value), reciprocal, q))
+        return f32(fma(fma(-q, scale, value), reciprocal, q))
+
+    checked = 0
+    for exponent in (np.log2(low), np.log2(low) + 1, -13, 0, np.log2(high) - 1):
+        for depth in (np.log2(ratio), np.log2(ratio) + 1, -24, -3, -1):
+            mantissas = np.concatenate([1 + rng.random(1500), [1, 1 + 2.0 ** -23, 2 - 2.0 ** -23, 2 - 2.0 ** -22]])
+            for mantissa in mantissas:
+                scale = f32(np.ldexp(mantissa, int(exponent)))
+                middle = np.ldexp(1 + (2 * int(rng.integers(1 << 23)) + 1) * 2.0 ** -24, int(depth))       # between two quotients
+                for value in (f32(float(scale) * middle), f32(np.ldexp(1 + rng.random(), int(exponent + depth)))):
+                    if abs(value) < scale * f32(ratio) or abs(value) > scale:
+                        continue
+                    assert quotient(value, scale) == value / scale, (value, scale)
+                    checked += 1
+    assert checked > 50000

@@ -92,8 +92,9 @@ __device__ __forceinline__ int clamp127(int e) { return min(max(e, -127), 127); 
 // value / scale, rounded to nearest: the residual correction of a quotient that is off by at most one unit in the last
 // place is the correctly rounded quotient when the reciprocal is correctly rounded (Markstein 1990, "Computation of
 // elementary functions on the IBM RISC System/6000 processor"); the product with the reciprocal can be off by two, so
-// it takes a first correction too.  That holds while nothing underflows: `normal` says that the row's scale is far from the ends of the range, and values far below the
-// scale take the division.
+// it takes a first correction too.  The last residual has to be exact: it is a multiple of 2^-46 times the quotient's
+// and the scale's power of two, which is representable while the two exponents add up to -103 or more.  `normal` keeps
+// the scale at 2^-40 or more, and weights below 2^-60 of the scale take the division.
 __device__ __forceinline__ float divide_by_scale(float value, float scale, float reciprocal, bool normal) {
   if (!normal || !(fabsf(value) >= scale * 0x1p-60f || value == 0.f)) return __fdiv_rn(value, scale);
   float q = __fmul_rn(value, reciprocal);
@@ -148,7 +149,7 @@ __global__ void __launch_bounds__(kEncodeThreads) encode_kernel(const float *__r
       __syncthreads();
     }
     const float scale = fmaxf(m, 1e-12f), reciprocal = __frcp_rn(scale);
-    const bool normal = scale >= 0x1p-60f && scale <= 0x1p60f;
+    const bool normal = scale >= 0x1p-40f && scale <= 0x1p60f;
     if (!live) continue;
     if (in_group == 0 && blockIdx.y == 0) scales[row] = scale;
 
