@@ -93,12 +93,15 @@ struct PrefillParams {
 __device__ __forceinline__ void mbar_init(unsigned bar, unsigned count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
-// arrival on the barrier at this shared-memory offset of the CTA `rank` of the cluster, releasing at cluster scope
+// Arrival on the barrier at this shared-memory offset of the CTA `rank` of the cluster.  No cluster scope: it hands over
+// TMEM stores (complete since tcgen05.wait::st) and TMA copies that the tensor core reads, nothing that a thread of the
+// other CTA loads.  A release at cluster scope waits for all of the thread's loads in flight; with it in a relay thread, and
+// an acquire to match, 5120x17408 with 4096 tokens took 874 us (now 680; 34816x5120 1357, now 1225).
 __device__ __forceinline__ void mbar_arrive_at(unsigned bar, unsigned rank) {
   asm volatile(
       "{\n\t.reg .b32 remote;\n\t"
       "mapa.shared::cluster.u32 remote, %0, %1;\n\t"
-      "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [remote];\n\t}" ::"r"(bar), "r"(rank) : "memory");
+      "mbarrier.arrive.shared::cluster.b64 _, [remote];\n\t}" ::"r"(bar), "r"(rank) : "memory");
 }
 __device__ __forceinline__ void mbar_arrive(unsigned bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
@@ -106,28 +109,19 @@ __device__ __forceinline__ void mbar_arrive(unsigned bar) {
 __device__ __forceinline__ void mbar_expect_tx(unsigned bar, unsigned bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-template <bool CLUSTER = false>   // whether the arrivals it acquires come from another CTA of the cluster too
 __device__ __forceinline__ bool mbar_try_wait(unsigned bar, unsigned parity) {
   unsigned done;
-  if (CLUSTER)
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-  else
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(done) : "r"(bar), "r"(parity) : "memory");
   return done != 0;
 }
 // Bounded wait; returns false (after recording `code`) when the limit is reached or the CTA aborted.
-template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, volatile int *abort_flag, int *status, int code) {
   for (unsigned spin = 0; spin < kSpinLimit; ++spin) {
-    if (mbar_try_wait<CLUSTER>(bar, parity)) return true;
+    if (mbar_try_wait(bar, parity)) return true;
     if (*abort_flag) return false;
   }
   atomicCAS(status, 0, code);
@@ -306,8 +300,9 @@ prefill_umma_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap x
 
   if (tid == 0) {
     for (int s = 0; s < S; ++s) {
-      // the producer warps and the TMA lane of a stage; on the issuing CTA of a pair also one arrival for the other CTA's half
-      mbar_init(full + 8 * s, kProducerWarps / kGroups + 1 + (CTAS == 2 && rank == 0 ? 1 : 0));
+      // the producer warps and the TMA lane of a stage.  A pair counts on its issuing CTA: both CTAs' producers arrive there
+      // themselves, for the other CTA's TMA lane a relay does, and the other CTA's barrier takes its copy alone.
+      mbar_init(full + 8 * s, CTAS == 1 ? kProducerWarps / kGroups + 1 : rank == 0 ? CTAS * (kProducerWarps / kGroups + 1) : 1);
       mbar_init(empty + 8 * s, 1);
     }
     mbar_init(accum, 1);
@@ -385,7 +380,10 @@ prefill_umma_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap x
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
-        if (lane == 0) mbar_arrive(full + 8 * s);
+        if (lane == 0) {
+          if (CTAS == 1 || rank == 0) mbar_arrive(full + 8 * s);
+          else mbar_arrive_at(full + 8 * s, 0);
+        }
         s += kGroups;
         if (s >= S) {
           s -= S;
@@ -430,7 +428,7 @@ prefill_umma_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap x
     unsigned parity = 0;
     bool ok = true;
     for (int kt = 0; kt < KT; ++kt) {
-      ok = __all_sync(0xffffffffu, mbar_wait<CTAS == 2>(full + 8 * s, parity, abort_flag, p.status, 3));
+      ok = __all_sync(0xffffffffu, mbar_wait(full + 8 * s, parity, abort_flag, p.status, 3));
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       if (elect_one()) {
@@ -450,8 +448,7 @@ prefill_umma_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap x
     if (ok && elect_one()) umma_commit<CTAS>(accum);   // accumulators complete
     __syncwarp();
   } else if (lane == 0) {
-    // ---------------- second CTA of a pair: tell the issuing CTA when this one's half of a stage is there ----------------
-    // (one cluster-scope arrival a stage; from every producer warp it would wait for the warp's loads in flight each time)
+    // ---------------- second CTA of a pair: tell the issuing CTA when this one's activations of a stage are there ----------------
     int s = 0;
     unsigned parity = 0;
     for (int kt = 0; kt < KT; ++kt) {
@@ -575,7 +572,9 @@ static int prefill_k_ranges(const Handle *h, int tokens, const Workspace *ws) {
 // A wave of CTAs takes its 128-column stages at the pace of the MMAs or, below 128 tokens, of the producers, plus
 // what a CTA spends before and after them (TMEM, first loads, epilogue).  Measured on 5120x17408 with 512 tokens
 // (136 stages): 0.30, 0.35, 0.50 and 0.67 us a stage for 64, 128, 192 and 256 tokens and about 4 us a CTA; the tile with
-// the smallest sum over the waves wins, the wider one on a tie (it reads the activations less often).
+// the smallest sum over the waves wins, the wider one on a tie (it reads the activations less often).  The pair tile (id 6)
+// is left out: against the 256-token tile it measured between 6 % less and 13 % more for 512 to 4096 tokens, by the
+// GPU's power state more than by shape, and never less below that.
 //
 // Up to eight tokens (a threshold below the default of 16) the decode kernel keeps the call: it pays one group of MMA columns
 // there, and two from nine on.  Decode kernel against the 64-token tile, us a call from HBM: 256x2048 2.6 / 7.5 with one
