@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 import torch
 
+from graph_kernels import launched
 from oracle import bc4_oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -191,3 +192,51 @@ def test_staging_and_stage_ring_remainders(ext, lut, tokens, k, backend, dtype):
     # exact products, fp32 sums, one rounding of the output (half a unit in its last place)
     assert float((y - want).norm() / want.norm()) <= (2.0 ** -9 if dtype == torch.bfloat16 else 2.0 ** -12) + 1e-5
     ext.free(h)
+
+
+@pytest.mark.parametrize("variant", ["bias", "fp16 bias", "texture palette", "low mode"])
+@pytest.mark.parametrize("tokens,m,k", [(257, 300, 912), (600, 300, 912), (300, 130, 400)])
+@pytest.mark.parametrize("backend", [5, 6])
+def test_wide_tiles_with_remainders(ext, lut, backend, tokens, m, k, variant):
+    """The 256-token tiles with partial token, row and column tiles: bias in both types, both palettes, low-mode blocks."""
+    rng = np.random.default_rng(tokens + m)
+    ends = np.sort(rng.integers(-127, 128, (2, m, k // 16)), 0)[::-1].astype(np.int8)
+    ends[0] = np.maximum(ends[0], ends[1] + 1) if variant != "low mode" else ends[0]
+    if variant == "low mode":
+        swap = rng.random((m, k // 16)) < 0.3
+        ends = np.where(swap, ends[::-1], ends).astype(np.int8)
+    blocks = O.pack_blocks(ends[0], ends[1], rng.integers(0, 8, (m, k // 16, 16)).astype(np.uint8))
+    scales = (rng.random(m) + 0.5).astype(np.float32)
+    dtype = torch.float16 if variant == "fp16 bias" else torch.bfloat16
+    bias = torch.from_numpy(rng.standard_normal(m)).to(dtype).cuda() if "bias" in variant else None
+    table = O.hardware_palette() if variant == "texture palette" else lut
+    h = ext.pack_encoded(torch.from_numpy(blocks).reshape(-1), torch.from_numpy(scales), bias)
+    ext.set_palette(h, 1 if variant == "texture palette" else 0)
+    ext.set_prefill_backend(h, backend)
+    x = (torch.randn(tokens, k, generator=torch.Generator().manual_seed(tokens)) / k ** 0.5).cuda().to(dtype)
+    y = ext.linear(h, x).double().cpu()
+    ext.free(h)
+    assert ext.kernel_status() == 0
+    w = torch.from_numpy(O.dequant_palette(blocks, m, table).reshape(m, k)).double() * torch.from_numpy(scales).double()[:, None]
+    want = x.double().cpu() @ w.T + (bias.double().cpu() if bias is not None else 0)
+    # one rounding of the output (half a unit in its last place); the texture palette's step sizes and the low mode's entries
+    # are fp16 (2^-10 and 2^-11 of a weight at most)
+    weights = {"texture palette": 2.0 ** -10, "low mode": 2.0 ** -11}.get(variant, 0)
+    assert float((y - want).norm() / want.norm()) <= (2.0 ** -12 if dtype == torch.float16 else 2.0 ** -9) + weights + 1e-5
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("tokens", [33, 40, 100])
+def test_prompts_kept_on_the_decode_kernel(ext, lut, tokens, dtype):
+    """More tokens than one of its passes takes, with the threshold above them."""
+    blocks, scales, gen = _encoded(200, 656, tokens, lut)
+    h = ext.pack_encoded(torch.from_numpy(blocks).reshape(-1), torch.from_numpy(scales))
+    ext.set_prefill(h, tokens + 1, 1024)
+    x = torch.randn(tokens, 656, generator=gen).cuda().to(dtype)
+    y, out = ext.linear(h, x), torch.empty(tokens, 200, dtype=dtype, device="cuda")
+    names = [name for name, _ in launched(lambda: ext.linear_out(h, x, out))]
+    assert sum("gemv_tile_kernel" in name for name in names) > 1 and not any("prefill" in name for name in names)
+    w = ext.dequant(h, 1).double()
+    ext.free(h)
+    want = x.double() @ w.T
+    assert float((y.double() - want).norm() / want.norm()) <= (2.0 ** -9 if dtype == torch.bfloat16 else 2.0 ** -12) + 1e-5

@@ -29,6 +29,19 @@ def test_prefill_hidden_state_cosine(toy):
         assert _cosine(got, ref) >= 0.999, backend      # final hidden-state gate of the operator
 
 
+def test_prefill_through_the_decode_kernel(toy):
+    """The same gate with the prompt kept off the tiles."""
+    ids = torch.randint(0, toy.config.vocab, (40,), generator=torch.Generator().manual_seed(0))
+    before = [toy.ext.handle_info(h)[2:4] for h in toy.handles]
+    for h in toy.handles:
+        toy.ext.set_prefill(h, 1 << 30, 1024)
+    try:
+        assert _cosine(toy.prefill(ids), toy.prefill(ids, dense=True)) >= 0.999
+    finally:
+        for h, (threshold, rows) in zip(toy.handles, before):
+            toy.ext.set_prefill(h, threshold, rows)
+
+
 def test_decode_graph_matches_eager_and_dense(toy):
     ids = torch.randint(0, toy.config.vocab, (24,), generator=torch.Generator().manual_seed(1))
     toy.prefill(ids)
