@@ -179,7 +179,7 @@ int tx_set_palette(uint64_t handle, int palette);
 
 /* encode: the reference's offline encoder for one matrix, texelator/encoder.py:34-102 (endpoint_opt), :23-31
  * (nearest), :105-117 (pack_blocks) and :137-145 (row scales) -- there a chain of PyTorch tensor operations,
- * here two kernels whose output is byte-identical to it.  All pointers are device pointers: `weight` fp32
+ * here one kernel whose output is byte-identical to it.  All pointers are device pointers: `weight` fp32
  * [M, K] row-major, `hdiag` fp32 [K] (the activation second moments E[x_k^2] that weight the error),
  * `lut` fp32 [255, 255, 8] = palette[e1 + 127][e0 + 127][selector]; writes M * K / 2 bytes of row-major BC4
  * blocks (the .bc4 file content) and M fp32 row scales (the .scales.f32 content), which tx_pack_encoded
@@ -197,8 +197,8 @@ int tx_dequant(uint64_t handle, void *out, int what, void *stream);
 int tx_unpack_blocks(uint64_t handle, uint8_t *out_host);
 
 /* New: device status word.  Kernels never spin without a limit; when a bounded wait of the tensor-core
- * prefill kernel runs out it records a positive code (1..5 = producer, TMA, A-ready, X-ready,
- * accumulator wait) here and returns early.  Synchronises the device; returns the code (0 = healthy)
+ * prefill kernel runs out it records a positive code here and returns early (1: a producer, 2: the TMA lane waiting
+ * for a free stage; 3: a full stage; 5: the accumulators).  Synchronises the device; returns the code (0 = healthy)
  * or a negative TX_E* value; `clear` resets it. */
 int tx_kernel_status(int device, int clear);
 

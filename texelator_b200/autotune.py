@@ -28,7 +28,7 @@ from .runtime import extension, free, pack_entry_handles
 
 CANDIDATES = {
     "umma_128x256x128": 5,
-    "umma_256x256x64": 6,
+    "umma_256x256x128": 6,
     "umma_128x128x128": 7,
     "umma_128x64x128": 8,
     "umma_128x192x128": 9,

@@ -220,8 +220,8 @@ __global__ void __launch_bounds__(kEncodeThreads) encode_kernel(const float *__r
         const float4 next_lo = palette_half<WIDE>(ahead, 0), next_hi = palette_half<WIDE>(ahead, 1);
         unsigned long long d2[8];
         nearest_distances(v2, p_lo, p_hi, d2);
-        // (scalar products and sums: ptxas contracts a packed multiply whose result meets a packed add, even with .rn on
-        // both, and then four blocks of 5.6 million come out one neighbour off)
+        // (scalar products and sums: with packed multiplies and adds, .rn on both, 4 blocks of 5.6 million came out one
+        // neighbour off the reference's, as a fused multiply-add would have it)
         float te[16];
 #pragma unroll
         for (int j = 0; j < 16; ++j) {

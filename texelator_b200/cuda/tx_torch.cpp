@@ -3,7 +3,7 @@
 // What bounds a small linear is the host: a 256 x 2048 matrix runs 3.2 us on the GPU, and the same call written
 // in Python (tensor attribute reads, torch.empty, a stream object, ctypes conversions) cost 12.5 us of host time
 // per call.  Here the tensor is read through its C++ object, the output comes straight from the caching allocator
-// and the C-ABI entry point is called through its address: 4.8 us a call with the module's own Python on top.
+// and the C-ABI entry point is called through its address: 5.1 us a call with the module's own Python on top.
 //
 // The module holds no CUDA code and links no library of this package: every handle is remembered with the addresses
 // of the C-ABI functions (include/texelator_b200.h) of the library that packed it, so several loaded libraries keep
