@@ -1302,7 +1302,8 @@ __global__ void __launch_bounds__(256) silu_mul_kernel(const __nv_bfloat16 *__re
 // the same for rows stored as (gate, up) groups of eight -- the row order of the SwiGLU-fused linear:
 // out[t, 8j + e] = silu(gu[t, 16j + e]) * gu[t, 16j + 8 + e].  ACCURATE takes expf (2 units in the last place) where the
 // decode step's kernels take __expf, whose relative error grows with the argument: the prompt's arithmetic is then
-// PyTorch's silu(g.float()) * u.float() to the bit.  The pass is bound by memory either way.
+// PyTorch's silu(g.float()) * u.float() to the bit.  Close to memory either way: 700 x 11008 10.7 us against 10.4 (7.1 for
+// the bytes), 2000 x 28672 72.5 against 70.0 (52.6).
 template <bool ACCURATE>
 __global__ void __launch_bounds__(256) silu_mul_pairs_kernel(const __nv_bfloat16 *__restrict__ gu, __nv_bfloat16 *__restrict__ out,
                                                              int inter, int tokens) {
