@@ -1,0 +1,125 @@
+"""The decode kernel of one to sixteen tokens (``tx_stream.cu``) at the sizes where its cuts can go wrong: runs of a row of
+unequal length, ranges of a cluster, ragged rows, slabs (run with ``-m gpu``)."""
+import re
+
+import numpy as np
+import pytest
+import torch
+
+from oracle import bc4_oracle as O
+from graph_kernels import launched
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ext():
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    from texelator_b200 import runtime
+    return runtime.extension()
+
+
+def _distance(y, want):
+    return float((y.double() - want).norm() / want.norm())
+
+
+# One rounding of the output: half a unit in the last place, at most 2^-8 of a bf16 and 2^-11 of an fp16 value (8 and 11
+# significant bits).  The texture path rounds three times to fp16 on the way to a weight: its two multipliers and the sum.
+HALF_UNIT = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}
+TEXTURE = 3 * 2.0 ** -11
+
+
+@pytest.mark.parametrize("m,k", [
+    (1, 16), (17, 144), (40, 1008),                    # fewer units than runs, one ragged unit, eight units
+    (16, 1040), (250, 8176), (33, 8208),               # nine units; 64 units (sixteen runs) less and more a block
+    (4250, 2896), (1000, 17408), (64, 28672), (9472, 256),
+])
+@pytest.mark.parametrize("tokens", [1, 2, 8, 9, 16])
+def test_matches_64_bits(ext, lut, m, k, tokens):
+    from texelator_b200 import runtime
+    rng = np.random.default_rng(m + k + tokens)
+    weight = (rng.standard_normal((m, k)) * 0.02).astype(np.float32)
+    if m == 250:
+        weight[rng.random((m, k)) < 0.9] = 0           # low-mode blocks
+    for palette, table in ((runtime.PALETTE_SOFTWARE, lut), (runtime.PALETTE_HARDWARE, O.hardware_palette())):
+        blocks, scales = O.encode_minmax(weight, table)
+        for dtype in (torch.bfloat16, torch.float16):
+            bias = torch.from_numpy((rng.standard_normal(m) * 0.3).astype(np.float32)).to(dtype).cuda()
+            h = ext.pack_encoded(torch.from_numpy(blocks), torch.from_numpy(scales), bias)
+            try:
+                ext.set_palette(h, palette)
+                ext.set_prefill(h, 32, 1024)
+                x = torch.from_numpy(rng.standard_normal((tokens, k)).astype(np.float32)).to(dtype).cuda()
+                y = ext.linear(h, x)
+                want = x.double() @ ext.dequant(h, runtime.DEQUANT_SCALED_F32).double().T + bias.double()
+                bound = HALF_UNIT[dtype] + (TEXTURE if palette == runtime.PALETTE_HARDWARE else 1e-6)
+                assert _distance(y, want) <= bound, (palette, dtype)
+                assert torch.equal(ext.linear(h, x), y)
+            finally:
+                ext.free(h)
+
+
+def test_runs_of_different_magnitude(ext, lut):
+    """Every run of a row is rescaled by itself; the sum is what one scale for the whole token gives, at both ends of the
+    type's range and with runs of zeros."""
+    from texelator_b200 import runtime
+    rng = np.random.default_rng(11)
+    m, k = 48, 8192
+    blocks, scales = O.encode_minmax((rng.standard_normal((m, k)) * 0.02).astype(np.float32), lut)
+    h = ext.pack_encoded(torch.from_numpy(blocks), torch.from_numpy(scales))
+    try:
+        w = ext.dequant(h, runtime.DEQUANT_SCALED_F32).double()
+        for exponents in (rng.uniform(-30, 30, 16), rng.uniform(-37, -33, 16), rng.uniform(34, 36, 16), np.repeat(-300.0, 16)):
+            row = torch.from_numpy(rng.standard_normal((3, 16, k // 16)) * 10.0 ** exponents[None, :, None]).reshape(3, k)
+            x = row.to(torch.bfloat16).cuda()
+            want = x.double() @ w.T
+            y = ext.linear(h, x)
+            assert torch.isfinite(y).all()
+            if float(want.norm()) == 0:
+                assert not y.any()
+            else:
+                assert _distance(y, want) <= 2.0 ** -8
+    finally:
+        ext.free(h)
+
+
+@pytest.mark.parametrize("tokens", [1, 5, 16])
+def test_sums_do_not_depend_on_the_matrix_rows_or_the_look_ahead(ext, lut, tokens):
+    """The order of a row's sums follows K and whether there is one token: shards of a matrix, whatever clusters they run on, reassemble bit for bit."""
+    rng = np.random.default_rng(23)
+    m, k = 6400, 5120
+    blocks, scales = O.encode_minmax((rng.standard_normal((m, k)) * 0.02).astype(np.float32), lut)
+    x = torch.from_numpy(rng.standard_normal((tokens, k)).astype(np.float32)).bfloat16().cuda()
+    tb, ts = torch.from_numpy(blocks), torch.from_numpy(scales)
+    full = ext.pack_encoded(tb, ts)
+    shards = [ext.pack_encoded_shard(tb, ts, m, k, rows, (0, k // 16)) for rows in ((0, 16), (16, 1600), (1600, 1616), (1616, 6400))]
+    try:
+        for h in [full] + shards:
+            ext.set_prefill(h, 32, 1024)
+        y = ext.linear(full, x)
+        assert torch.equal(torch.cat([ext.linear(h, x) for h in shards], 1), y)
+        for lookahead in (1, 3, 6, 8):
+            ext.set_lookahead(full, lookahead)
+            assert torch.equal(ext.linear(full, x), y)
+        # a row of x gives the same bits in any company (one token has an order of its own, as have nine and more)
+        ext.set_lookahead(full, 2)
+        if tokens == 5:
+            assert torch.equal(torch.cat([ext.linear(full, x[:2]), ext.linear(full, x[2:])]), y)
+    finally:
+        for h in shards + [full]:
+            ext.free(h)
+
+
+def test_one_launch_below_seventeen_tokens(ext, lut):
+    rng = np.random.default_rng(3)
+    blocks, scales = O.encode_minmax((rng.standard_normal((96, 2048)) * 0.02).astype(np.float32), lut)
+    h = ext.pack_encoded(torch.from_numpy(blocks), torch.from_numpy(scales))
+    try:
+        ext.set_prefill(h, 64, 1024)
+        for tokens, passes in ((1, 1), (8, 1), (16, 1), (17, 2), (40, 3)):
+            x, y = torch.randn(tokens, 2048, device="cuda").bfloat16(), torch.empty(tokens, 96, device="cuda", dtype=torch.bfloat16)
+            names = [name for name, _ in launched(lambda: ext.linear_out(h, x, y))]
+            assert len(names) == passes and all(re.search("cluster_gemv_tile_kernel", name) for name in names)
+    finally:
+        ext.free(h)

@@ -300,9 +300,9 @@ __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddep
 
 bool pdl_enabled();
 
-// `ctas` consecutive CTAs along x form a cluster (1: none)
+// `ctas` consecutive CTAs along x form a cluster (1: none); `early`: may start while its predecessor drains
 template <typename... KernelArgs, typename... Args>
-cudaError_t launch_pdl_cluster(void (*kernel)(KernelArgs...), int ctas, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+cudaError_t launch_cluster(void (*kernel)(KernelArgs...), bool early, int ctas, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
   cudaLaunchConfig_t config{};
   config.gridDim = grid;
   config.blockDim = block;
@@ -310,7 +310,7 @@ cudaError_t launch_pdl_cluster(void (*kernel)(KernelArgs...), int ctas, dim3 gri
   config.stream = stream;
   cudaLaunchAttribute attributes[2]{};
   int count = 0;
-  if (pdl_enabled()) {
+  if (early && pdl_enabled()) {
     attributes[count].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attributes[count++].val.programmaticStreamSerializationAllowed = 1;
   }
@@ -325,6 +325,10 @@ cudaError_t launch_pdl_cluster(void (*kernel)(KernelArgs...), int ctas, dim3 gri
   return cudaLaunchKernelEx(&config, kernel, KernelArgs(args)...);
 }
 template <typename... KernelArgs, typename... Args>
+cudaError_t launch_pdl_cluster(void (*kernel)(KernelArgs...), int ctas, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+  return launch_cluster(kernel, true, ctas, grid, block, smem, stream, args...);
+}
+template <typename... KernelArgs, typename... Args>
 cudaError_t launch_pdl(void (*kernel)(KernelArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
   return launch_pdl_cluster(kernel, 1, grid, block, smem, stream, args...);
 }
@@ -336,6 +340,9 @@ int launch_dequant(const Handle *h, void *out, int what, cudaStream_t stream);
 int launch_gemv(const Handle *h, const __nv_bfloat16 *x, __nv_bfloat16 *y, int tokens, cudaStream_t stream, bool half_io = false);
 int launch_gemv_fused(const Handle *h, const __nv_bfloat16 *x, const __nv_bfloat16 *delta, const __nv_bfloat16 *gamma, float eps,
                       __nv_bfloat16 *residual_out, bool swiglu, __nv_bfloat16 *y, int tokens, cudaStream_t stream);
+// one launch for up to sixteen tokens (tx_stream.cu)
+int stream_tokens(const Handle *h, int tokens, bool half_io);   // tokens of one pass, at most `tokens`; 0: not for this matrix
+int launch_stream(const Handle *h, const void *x, void *y, int tokens, bool half_io, bool swiglu, cudaStream_t stream);
 bool gemv_single_eligible(const Handle *h);
 int gemv_suggest_splits(const Handle *h);
 int launch_gemv_single(const Handle *h, const __nv_bfloat16 *x, const uint8_t *staged, bool swiglu, __nv_bfloat16 *y,

@@ -1,5 +1,6 @@
-// Decode GEMV for tokens < prefill_threshold (reference: texelator_bc4_bf16_kernel,
-// texelator/cuda/texelator_cuda.cu:141-199, one warp per output row through the texture unit).
+// Decode GEMV, whole rows per CTA (reference: texelator_bc4_bf16_kernel, texelator/cuda/texelator_cuda.cu:141-199, one warp
+// per output row through the texture unit).  tx_linear streams up to sixteen tokens through tx_stream.cu; the kernel here
+// serves what that one does not: a fused norm in front, the allocation-free entry point, rows too long for it.
 //
 // B200 design.  A persistent CTA walks 16-row tiles of the tiled BC4 payload; its eight warps split
 // the tile's 1 KiB units (16 rows x 128 columns) round-robin, keep LOOKAHEAD units in flight as
@@ -125,7 +126,7 @@ __global__ void __launch_bounds__(kGemvThreads) gemv_xprep_kernel(const void *__
 template <int LOOKAHEAD, int NT, bool PRE, bool LOWMODE, int FUSE = 0>
 __global__ void __launch_bounds__(kGemvThreads, (NT == 1 && LOOKAHEAD <= 2) ? 3 : (NT <= 2 ? 2 : 1))
 gemv_tile_kernel(const GemvParams p) {
-  static_assert(FUSE == 0 || (NT == 1 && !PRE), "fused variants stage their activations in the CTA");
+  static_assert(PRE ? FUSE == 0 : NT == 1 && (FUSE & kFuseNorm), "the activations come from the pre-pass or from the fused norm");
   extern __shared__ __align__(16) uint8_t smem_raw[];
   const unsigned sbase = unsigned(__cvta_generic_to_shared(smem_raw));
   float *tokmul = reinterpret_cast<float *>(smem_raw);                  // 32 floats
@@ -195,12 +196,12 @@ gemv_tile_kernel(const GemvParams p) {
     if (tid < p.T) tokmul[tid] = __ldcg(p.xmul + tid);
   } else {
     for (int tok = 0; tok < p.T; ++tok) {
-      // one trip to global memory: the first kXChunks*256 chunks stay in registers between the
-      // magnitude scan and the conversion (covers K <= 18432); longer rows re-read the rest
+      // one trip to global memory: kXChunks*256 chunks stay in registers between the norm, the magnitude scan and the
+      // conversion (K <= 18432; the launcher rejects longer rows)
       const uint4 *xp = reinterpret_cast<const uint4 *>(p.x + size_t(tok) * p.K);
       uint4 held[kXChunks];
       unsigned m = 0;
-      if (FUSE & kFuseNorm) {
+      {
         // residual add and RMSNorm with the rounding points of separate kernels: r = bf16(x + delta),
         // a = bf16(r * inv * gamma).  Every CTA computes the row (K <= 18432 stays in registers); CTA 0
         // also stores r.  Rows longer than that are rejected by the launcher.
@@ -258,16 +259,6 @@ gemv_tile_kernel(const GemvParams p) {
             m = max(m, chunk_absmax(v));
           }
         }
-      } else {
-#pragma unroll
-        for (int c = 0; c < kXChunks; ++c) {
-          const int i = tid + c * kGemvThreads;
-          if (i < chunks) {
-            held[c] = __ldcg(xp + i);   // L2 read: another kernel wrote these moments ago
-            m = max(m, chunk_absmax(held[c]));
-          }
-        }
-        for (int i = tid + kXChunks * kGemvThreads; i < chunks; i += kGemvThreads) m = max(m, chunk_absmax(__ldcg(xp + i)));
       }
       m = __reduce_max_sync(0xffffffffu, m);
       if (lane == 0) red[warp] = m;
@@ -284,8 +275,6 @@ gemv_tile_kernel(const GemvParams p) {
         const int i = tid + c * kGemvThreads;
         if (i < padded) dst[i] = i < chunks ? convert_chunk(held[c], mult) : make_uint4(0, 0, 0, 0);
       }
-      for (int i = tid + kXChunks * kGemvThreads; i < padded; i += kGemvThreads)
-        dst[i] = i < chunks ? convert_chunk(__ldcg(xp + i), mult) : make_uint4(0, 0, 0, 0);
       __syncthreads();
     }
   }
@@ -347,16 +336,19 @@ gemv_tile_kernel(const GemvParams p) {
     for (int slot = 0; slot < LOOKAHEAD; ++slot) {
       const uint4 q = pend[slot][0], r = pend[slot][1];   // duos of rows g and g+8
       const unsigned flag = pflag[slot];
+        const bool texture = LOWMODE && (p.palette & 0xff) == TX_PALETTE_HARDWARE;   // uniform
+        const DuoConstants cq = texture ? duo_constants<true>(q.w) : duo_constants<false>(q.w);
+        const DuoConstants cr = texture ? duo_constants<true>(r.w) : duo_constants<false>(r.w);
       // ---- one unit: blocks (ki*8 + t) [sub 0] and (ki*8 + 4 + t) [sub 1] of rows g and g+8
 #pragma unroll
       for (int sub = 0; sub < 2; ++sub) {
         unsigned aq[8], ar[8];
-        if (LOWMODE && (p.palette & 0xff) == TX_PALETTE_HARDWARE) {   // uniform
-          if (sub == 0) { decode_duo_first<true>(q, aq); decode_duo_first<true>(r, ar); }
-          else { decode_duo_second<true>(q, aq); decode_duo_second<true>(r, ar); }
+        if (texture) {
+          if (sub == 0) { decode_duo_first<true>(q, cq, aq); decode_duo_first<true>(r, cr, ar); }
+          else { decode_duo_second<true>(q, cq, aq); decode_duo_second<true>(r, cr, ar); }
         } else {
-          if (sub == 0) { decode_duo_first(q, aq); decode_duo_first(r, ar); }
-          else { decode_duo_second(q, aq); decode_duo_second(r, ar); }
+          if (sub == 0) { decode_duo_first(q, cq, aq); decode_duo_first(r, cr, ar); }
+          else { decode_duo_second(q, cq, aq); decode_duo_second(r, cr, ar); }
         }
         if (LOWMODE && __any_sync(0xffffffffu, flag != 0)) {   // rare, warp-uniform: redo the low-mode blocks
           if (duo_block_is_low(q, sub)) decode_block_low(q, sub, aq, p.palette & 0xff);
@@ -834,8 +826,7 @@ static GemvKernel pick_lookahead(int lookahead) {
 }
 
 template <bool LOWMODE>
-static GemvKernel pick_tokens(int lookahead, int nt, bool pre) {
-  if (!pre) return pick_lookahead<1, false, LOWMODE>(lookahead);
+static GemvKernel pick_tokens(int lookahead, int nt) {
   switch (nt) {
     case 1: return pick_lookahead<1, true, LOWMODE>(lookahead);
     case 2: return pick_lookahead<2, true, LOWMODE>(lookahead);
@@ -855,12 +846,11 @@ static GemvKernel pick_fused_lookahead(int lookahead) {
   }
 }
 
-// fuse: kFuseNorm, kFuseSwiglu or both; fused variants exist for in-CTA staging (one token tile) only
-static GemvKernel pick_kernel(int lookahead, int nt, bool pre, bool low_mode, int fuse = 0) {
+// fuse: kFuseNorm with or without kFuseSwiglu (in-CTA staging, one token tile), or 0 behind the pre-pass
+static GemvKernel pick_kernel(int lookahead, int nt, bool low_mode, int fuse = 0) {
   switch (fuse) {
-    case 0: return low_mode ? pick_tokens<true>(lookahead, nt, pre) : pick_tokens<false>(lookahead, nt, pre);
+    case 0: return low_mode ? pick_tokens<true>(lookahead, nt) : pick_tokens<false>(lookahead, nt);
     case kFuseNorm: return low_mode ? pick_fused_lookahead<true, kFuseNorm>(lookahead) : pick_fused_lookahead<false, kFuseNorm>(lookahead);
-    case kFuseSwiglu: return low_mode ? pick_fused_lookahead<true, kFuseSwiglu>(lookahead) : pick_fused_lookahead<false, kFuseSwiglu>(lookahead);
     default:
       return low_mode ? pick_fused_lookahead<true, kFuseNorm | kFuseSwiglu>(lookahead)
                       : pick_fused_lookahead<false, kFuseNorm | kFuseSwiglu>(lookahead);
@@ -963,20 +953,22 @@ struct GemvPlan {
   size_t smem;
 };
 
-static int plan_gemv(const Handle *h, int tokens, GemvPlan &plan, int fuse = 0, bool single_token_kernel = false, bool force_pre = false,
-                     bool allow_splits = true) {
+// in-CTA activation conversion only while it stays a short prologue
+static bool fused_fits(const Handle *h, int tokens) { return tokens <= 2 && size_t(tokens) * h->K <= 36864; }
+
+static int plan_gemv(const Handle *h, int tokens, GemvPlan &plan, int fuse = 0, bool single_token_kernel = false) {
   Workspace *ws = workspace_for(h->device);
   if (!ws) return TX_ECUDA;
   int KP = h->KI * 128;
   plan.nt = token_tiles(tokens);
-  // in-CTA activation conversion only while it stays a short prologue
-  plan.pre = force_pre || !(tokens <= 2 && size_t(tokens) * h->K <= 36864);
-  if (fuse && plan.pre) return fail(TX_EINVAL, "fused linear handles at most 2 tokens with tokens * K <= 36864");
+  // a fused norm converts the activations in the CTA; without one they come through the pre-pass
+  plan.pre = !fuse;
+  if (fuse && !fused_fits(h, tokens)) return fail(TX_EINVAL, "fused linear handles at most 2 tokens with tokens * K <= 36864");
   // The single-token kernel (no per-weight arithmetic) is taken on request only (tx_linear_single): it
   // pays off when its token arrives staged; staging a bf16 row costs it more than the general kernel.
   plan.solo = single_token_kernel;
   plan.splits = 1;
-  if (plan.pre && !plan.solo && allow_splits) {
+  if (plan.pre && !plan.solo) {
     plan.splits = choose_splits(h, tokens, ws->sm_count, ws->partial_floats);
     if (plan.splits < 1) return fail(TX_EINVAL, "decode GEMV does not fit in shared memory for this K");
   }
@@ -986,7 +978,7 @@ static int plan_gemv(const Handle *h, int tokens, GemvPlan &plan, int fuse = 0, 
     plan.solo_kernel = (fuse & kFuseSwiglu) ? pick_solo<true>(h->lookahead) : pick_solo<false>(h->lookahead);
     plan.smem = solo_smem_bytes(h->KI);
   } else {
-    plan.kernel = pick_kernel(h->lookahead, plan.nt, plan.pre, needs_generic_variant(h), fuse);
+    plan.kernel = pick_kernel(h->lookahead, plan.nt, needs_generic_variant(h), fuse);
     plan.smem = plan.pre ? split_smem_bytes(h->KI, plan.splits, tokens) : gemv_smem_bytes(KP, tokens, plan.nt);
   }
   // attribute + occupancy queries are cached per (device, kernel, shared bytes)
@@ -1017,6 +1009,11 @@ static int plan_gemv(const Handle *h, int tokens, GemvPlan &plan, int fuse = 0, 
 // texelator_cuda.cu:94-139, which multiplies the un-rounded pal*scale in fp32 -- what this kernel computes
 // for either type); the activations then always take the pre-pass, which for fp16 is a padded copy.
 int launch_gemv(const Handle *h, const __nv_bfloat16 *x, __nv_bfloat16 *y, int tokens, cudaStream_t stream, bool half_io) {
+  for (int t0 = 0, pass = stream_tokens(h, tokens, half_io); pass > 0; t0 += pass) {
+    if (t0 >= tokens) return TX_OK;
+    const int rc = launch_stream(h, x + size_t(t0) * h->K, y + size_t(t0) * h->M, std::min(pass, tokens - t0), half_io, false, stream);
+    if (rc != TX_OK) return rc;
+  }
   Workspace *ws = workspace_for(h->device);
   if (!ws) return TX_ECUDA;
   int KP = h->KI * 128;
@@ -1025,7 +1022,7 @@ int launch_gemv(const Handle *h, const __nv_bfloat16 *x, __nv_bfloat16 *y, int t
   for (int t0 = 0; t0 < tokens; t0 += per_pass) {
     int n = std::min(per_pass, tokens - t0);
     GemvPlan plan;
-    int rc = plan_gemv(h, n, plan, 0, false, half_io);
+    int rc = plan_gemv(h, n, plan);
     if (rc != TX_OK) return rc;
     GemvParams p{};
     p.tiles = reinterpret_cast<const uint4 *>(h->tiles);
@@ -1083,6 +1080,8 @@ int launch_gemv_fused(const Handle *h, const __nv_bfloat16 *x, const __nv_bfloat
   }
   if (swiglu && h->M % 16) return fail(TX_EINVAL, "SwiGLU pairs need M to be a multiple of 16");
   if (fuse == 0) return launch_gemv(h, x, y, tokens, stream);
+  if (!fused_fits(h, tokens)) return fail(TX_EINVAL, "fused linear handles at most 2 tokens with tokens * K <= 36864");
+  if (!gamma) return launch_stream(h, x, y, tokens, false, true, stream);   // (rows this short always fit it)
   GemvPlan plan;
   int rc = plan_gemv(h, tokens, plan, fuse);
   if (rc != TX_OK) return rc;
@@ -1229,7 +1228,7 @@ int launch_gemv_static_scratch(const Handle *h, const __nv_bfloat16 *x, __nv_bfl
   StaticScratch *scratch = nullptr;
   int rc = static_scratch_for(h->device, &scratch);
   if (rc != TX_OK) return rc;
-  GemvKernel kernel = pick_kernel(h->lookahead, nt, true, needs_generic_variant(h));
+  GemvKernel kernel = pick_kernel(h->lookahead, nt, needs_generic_variant(h));
   // attribute and occupancy are looked up once per (device, kernel variant, shared bytes): host-side table, no allocation on the device
   static std::mutex guard;
   static std::map<std::tuple<int, const void *, size_t>, int> cache;
@@ -1270,26 +1269,6 @@ int launch_gemv_static_scratch(const Handle *h, const __nv_bfloat16 *x, __nv_bfl
   kernel<<<grid, kGemvThreads, smem, stream>>>(p);
   count_launch();
   TX_CUDA(cudaGetLastError());
-  return TX_OK;
-}
-
-int gemv_kernel_info(int64_t out[9]) {
-  cudaFuncAttributes attributes{};
-  GemvKernel kernel = gemv_tile_kernel<2, 1, false, false>;
-  TX_CUDA(cudaFuncGetAttributes(&attributes, kernel));
-  TX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemBudget + 1024)));
-  int active = 0;
-  size_t smem = gemv_smem_bytes(4096, 1, 1);
-  TX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&active, kernel, kGemvThreads, smem));
-  out[0] = attributes.numRegs;
-  out[1] = int64_t(attributes.sharedSizeBytes);
-  out[2] = int64_t(attributes.localSizeBytes);
-  out[3] = attributes.maxThreadsPerBlock;
-  out[4] = int64_t(smem);
-  out[5] = 16;   // rows per unit
-  out[6] = 8;    // tokens per mma tile
-  out[7] = 128;  // columns per unit
-  out[8] = active;
   return TX_OK;
 }
 

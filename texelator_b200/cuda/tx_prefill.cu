@@ -361,11 +361,13 @@ prefill_umma_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap x
         for (int h = 0; h < 2; ++h) {
           const uint4 duo = h == 0 ? q : r;
           if (GENERIC && p.palette == TX_PALETTE_HARDWARE) {   // uniform
-            decode_duo_first<true>(duo, a[0][h]);
-            decode_duo_second<true>(duo, a[1][h]);
+            const DuoConstants c = duo_constants<true>(duo.w);
+            decode_duo_first<true>(duo, c, a[0][h]);
+            decode_duo_second<true>(duo, c, a[1][h]);
           } else {
-            decode_duo_first(duo, a[0][h]);
-            decode_duo_second(duo, a[1][h]);
+            const DuoConstants c = duo_constants<false>(duo.w);
+            decode_duo_first(duo, c, a[0][h]);
+            decode_duo_second(duo, c, a[1][h]);
           }
           if (low) {
             if (duo_block_is_low(duo, 0)) decode_block_low(duo, 0, a[0][h], p.palette);
