@@ -135,3 +135,42 @@ def test_batch_of_sequences_equals_the_sequences_one_by_one(batch):
         model.check_status()
     finally:
         model.free()
+
+
+@pytest.mark.parametrize("kernel", ["gemv", "umma_128x64x128"])
+def test_replays_of_sixteen_sequences_equal_eager_steps(kernel):
+    """Forty replays of the captured step leave the bits of forty eager steps: tokens, hidden states and every cache row.
+    Both runs start where ``capture`` left the decoder."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    from texelator_b200.autotune import CANDIDATES
+    from texelator_b200.batched import BatchedBC4Decoder
+    from texelator_b200.modeling import CONFIGS
+    config = CONFIGS["toy128"]
+    model = BatchedBC4Decoder(config, "cuda:0", max_len=120, batch=16, seed=9)
+    try:
+        for handle in model.handles:
+            model.ext.set_prefill(handle, 17 if kernel == "gemv" else 16, 1024)
+            model.ext.set_prefill_backend(handle, CANDIDATES["umma_128x64x128"])
+        for sequence in range(16):
+            model.fill_context(sequence, 0, 5 + 4 * sequence, seed=3)
+        model.tok.copy_(torch.arange(16, device="cuda") * 100)
+        model.capture()
+        state = [t.clone() for t in (model.tok, model.pos, model.k_cache, model.v_cache)]
+        runs = []
+        for step in (model.decode_step, model.decode_graph):
+            for tensor, saved in zip((model.tok, model.pos, model.k_cache, model.v_cache), state):
+                tensor.copy_(saved)
+            torch.cuda.synchronize()
+            seen = []
+            for _ in range(40):
+                step()
+                seen.append((model.next_tok.clone(), model.last_hidden.clone()))
+            runs.append((seen, model.k_cache.clone(), model.v_cache.clone()))
+        torch.cuda.synchronize()
+        (eager, *eager_cache), (replayed, *replayed_cache) = runs
+        assert all(torch.equal(a, b) for e, r in zip(eager, replayed) for a, b in zip(e, r))
+        assert all(torch.equal(a, b) for a, b in zip(eager_cache, replayed_cache))
+        model.check_status()
+    finally:
+        model.free()

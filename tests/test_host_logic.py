@@ -185,3 +185,41 @@ def test_encoder_quotients_are_correctly_rounded():
                     assert quotient(value, scale) == value / scale, (value, scale)
                     checked += 1
     assert checked > 50000
+
+
+@pytest.mark.parametrize("times,kernel", [
+    ((14.0, 15.0, 13.9), "umma_128x64x128"), ((15.0, 14.0, 11.4), "umma_128x128x128"),   # within the margin: the faster tile
+    ((14.0, 15.0, 11.0), "gemv"), ((14.0, 13.9, 14.0), "umma_128x128x128"), ((30.0, 20.0, 15.0), "gemv"),
+])
+def test_a_batch_keeps_the_tile_unless_the_decode_kernel_is_clearly_faster(monkeypatch, times, kernel):
+    from types import SimpleNamespace
+    from texelator_b200 import batched
+    by_kernel = dict(zip(("umma_128x64x128", "umma_128x128x128", "gemv"), times))
+    state = {}
+
+    class Event:
+        def __init__(self, enable_timing):
+            pass
+
+        def record(self):
+            pass
+
+        def synchronize(self):
+            pass
+
+        def elapsed_time(self, end):       # milliseconds of three repeats over two layers
+            timed = "gemv" if state[1][0] > 16 else autotune_name[state[1][1]]
+            return by_kernel[timed] * 6 / 1000
+
+    autotune_name = {number: name for name, number in autotune.CANDIDATES.items()}
+    monkeypatch.setattr(torch.cuda, "Event", Event)
+    ext = SimpleNamespace(set_prefill=lambda h, threshold, rows: state.__setitem__(h, (threshold, None)),
+                          set_prefill_backend=lambda h, backend: state.__setitem__(h, (state[h][0], backend)), linear_out=lambda h, x, y: y)
+    layers = {name: [1, 2] for name in ("h_qkv", "h_o", "h_gu", "h_down")}
+    buffers = {name: None for name in ("buf_x", "buf_qkv", "buf_attn", "buf_o", "buf_gu", "buf_act", "buf_down")}
+    decoder = SimpleNamespace(ext=ext, batch=16, world=1, device="cpu", **layers, **buffers)
+    chosen = batched.BatchedBC4Decoder.tune_decode_kernel(decoder)
+    assert {entry[0] for entry in chosen.values()} == {kernel} and list(chosen) == ["qkv", "o", "gate_up", "down"]
+    assert abs(chosen["o"][1] - by_kernel[kernel]) < 1e-9 and set(chosen["o"][2]) == set(by_kernel)
+    threshold, backend = state[1]
+    assert (threshold > 16) == (kernel == "gemv") and backend == autotune.CANDIDATES["umma_128x64x128" if kernel == "gemv" else kernel]

@@ -22,6 +22,10 @@ import torch.nn.functional as F
 
 from .modeling import BC4Decoder, DecoderConfig, _rmsnorm
 
+# What the decode kernel has to gain before it takes a projection's rows from the tiles: it adds in another order, and two
+# timings of one kernel at start-up differ by up to 9 %.
+TUNE_MARGIN = 0.2
+
 
 class BatchedBC4Decoder(BC4Decoder):
     """``BC4Decoder`` with ``batch`` independent sequences: caches ``[layers, B, kv_heads, max_len, head_dim]``,
@@ -70,17 +74,21 @@ class BatchedBC4Decoder(BC4Decoder):
     @torch.no_grad()
     def tune_decode_kernel(self, repeats: int = 3) -> dict:
         """For batches at or above the reference's prefill threshold (16), time every projection's B-row linear
-        through the multi-token decode kernel and through the two narrow tensor-core tiles, over all layers (so
-        the weights come from HBM), and keep the fastest per projection -- the per-shape selection the reference's
-        autotuner makes for prompts (texelator/autotune.py:170-193), applied to the decode batch.  All ranks of a
-        tensor-parallel run take rank 0's choice.  Returns {projection: (kernel, microseconds per call)}."""
+        through the two narrow tensor-core tiles and the multi-token decode kernel, over all layers (so the weights
+        come from HBM), and keep one per projection -- the per-shape selection the reference's autotuner makes for
+        prompts (texelator/autotune.py:170-193), applied to the decode batch.  The tiles give the same bits, so the faster
+        one serves; the decode kernel adds a row in another order and is taken only when it is ``TUNE_MARGIN`` faster, so
+        that two instances of one decoder do not differ by a stopwatch (sixteen rows of 5120x5120: 13.7 to 14.2 us
+        through the 64-token tile, 14.1 to 14.8 through the decode kernel, now one and now the other in front).  All
+        ranks of a tensor-parallel run take rank 0's choice.  Returns {projection: (kernel, microseconds per call)}."""
         from .autotune import CANDIDATES
         from .runtime import PREFILL_THRESHOLD, PREFILL_TILE_ROWS
         ext, chosen = self.ext, {}
         if self.batch < PREFILL_THRESHOLD:
             return chosen
-        options = [("gemv", self.batch + 1, CANDIDATES["umma_128x64x128"]), ("umma_128x64x128", PREFILL_THRESHOLD, CANDIDATES["umma_128x64x128"]),
-                   ("umma_128x128x128", PREFILL_THRESHOLD, CANDIDATES["umma_128x128x128"])]
+        options = [("umma_128x64x128", PREFILL_THRESHOLD, CANDIDATES["umma_128x64x128"]),
+                   ("umma_128x128x128", PREFILL_THRESHOLD, CANDIDATES["umma_128x128x128"]),
+                   ("gemv", self.batch + 1, CANDIDATES["umma_128x64x128"])]
         groups = (("qkv", self.h_qkv, self.buf_x, self.buf_qkv), ("o", self.h_o, self.buf_attn, self.buf_o),
                   ("gate_up", self.h_gu, self.buf_x, self.buf_gu), ("down", self.h_down, self.buf_act, self.buf_down))
         for name, handles, x, y in groups:
@@ -99,7 +107,10 @@ class BatchedBC4Decoder(BC4Decoder):
                 end.record()
                 end.synchronize()
                 timings.append(begin.elapsed_time(end) * 1000 / (repeats * len(handles)))
-            best = torch.tensor([min(range(len(options)), key=timings.__getitem__)], device=self.device)
+            pick = 0 if timings[0] <= timings[1] else 1
+            if timings[2] < (1 - TUNE_MARGIN) * timings[pick]:
+                pick = 2
+            best = torch.tensor([pick], device=self.device)
             if self.world > 1:
                 torch.distributed.broadcast(best, src=0, group=self.group)
             pick = int(best.item())
