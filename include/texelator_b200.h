@@ -82,11 +82,12 @@ int tx_pack_encoded_shard(const uint8_t *blocks, size_t nbytes, const float *sca
  * (texelator_bc4_kernel, :94-139, un-rounded weight, fp32 accumulation, one fp16 rounding; for tokens >=
  * prefill_threshold the reference goes through fp16(pal*scale) and cuBLAS, :996-1046): the same kernels, the
  * fp16 activations are the tensor-core operand as they are.
- * Token groups below the threshold read the matrix once for all rows (the reference launches one grid row per
- * token, :1438-1468); for groups and for short prompts on matrices with few rows K may be cut into ranges whose
- * fp32 sums a second kernel adds in a fixed order (results repeat bit for bit; they can differ in the last bit
- * from the same rows taken one at a time).  All calls on one device share one activation scratch and one
- * partial-sum scratch: order them on one stream. */
+ * Token groups below the threshold read the matrix once for up to sixteen rows (the reference launches one grid row per
+ * token, :1438-1468).  K is cut into runs, and for short prompts on matrices with few rows into ranges, whose
+ * fp32 sums are added in a fixed order (results repeat bit for bit; they can differ in the last bit
+ * from the same rows taken one at a time).  On TX_DECODE_ALU_MMA `y` may overlap `x`: up to 32 tokens anyhow, any number
+ * where it is `x` itself (M = K).  Such calls, rows of more than 131072 columns and prompts go through one
+ * activation scratch and one partial-sum scratch of the device: order them on one stream. */
 int tx_linear(uint64_t handle, const void *x, void *y, int tokens, int dtype, void *stream);
 
 /* No counterpart in the reference.  The result of tx_linear for a small token group (1..32 tokens,
@@ -109,8 +110,8 @@ int tx_linear_static_scratch(uint64_t handle, const void *x, void *y, int tokens
  *   swiglu != 0         : the handle's rows are (gate, up) pairs -- in every group of 16 rows, rows 0-7
  *                         are gate rows and rows 8-15 the matching up rows -- and
  *                         y[t, 8*g + i] = silu(lin[16*g + i]) * lin[16*g + 8 + i]; y is [tokens, M/2].
- * Rounding points are those of the separate steps (bf16 after the add, after the norm, after each
- * linear output, after the product).  At most 2 tokens with tokens * K <= 36864; TX_DECODE_ALU_MMA only. */
+ * y must not overlap x or delta, which thread blocks still read while others store.  Rounding points are those of the
+ * separate steps (bf16 after the add, after the norm, after each linear output, after the product).  At most 2 tokens with tokens * K <= 36864; TX_DECODE_ALU_MMA only. */
 int tx_linear_fused(uint64_t handle, const void *x, const void *delta, const void *norm_weight, float eps, void *residual_out,
                     int swiglu, void *y, int tokens, int dtype, void *stream);
 

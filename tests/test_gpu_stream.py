@@ -123,3 +123,48 @@ def test_one_launch_below_seventeen_tokens(ext, lut):
             assert len(names) == passes and all(re.search("cluster_gemv_tile_kernel", name) for name in names)
     finally:
         ext.free(h)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("tokens,m,k,shift", [(1, 4096, 4096, 0), (8, 4096, 4096, 0), (16, 2048, 2048, 0), (40, 2048, 2048, 0),
+                                              (5, 8192, 2048, 1024), (12, 1024, 8192, -4096)])
+def test_output_over_the_input(ext, lut, dtype, tokens, m, k, shift):
+    """``y`` in the memory of ``x``, all of it or in part: every row is multiplied with the activations as they came."""
+    rng = np.random.default_rng(tokens + m)
+    blocks, scales = O.encode_minmax((rng.standard_normal((m, k)) * 0.02).astype(np.float32), lut)
+    h = ext.pack_encoded(torch.from_numpy(blocks), torch.from_numpy(scales))
+    try:
+        ext.set_prefill(h, 64, 1024)
+        w = ext.dequant(h, 1).double()
+        memory = torch.empty(tokens * (m + k) + 8192, dtype=dtype, device="cuda")
+        x = memory[4096:4096 + tokens * k].view(tokens, k)
+        y = memory[4096 + shift:4096 + shift + tokens * m].view(tokens, m)
+        for repeat in range(10):
+            source = torch.from_numpy(rng.standard_normal((tokens, k))).to(dtype).cuda()
+            x.copy_(source)
+            ext.linear_out(h, x, y)
+            assert _distance(y, source.double() @ w.T) <= HALF_UNIT[dtype] / 2 + 1e-6, repeat
+    finally:
+        ext.free(h)
+
+
+def test_output_over_the_input_of_a_call_in_slabs(ext):
+    """Rows too many for one launch: the second launch reads the activations after the first has stored its rows."""
+    m, k, tokens = 28688, 8192, 16
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    blocks = torch.randint(0, 256, (m * k // 2,), device="cuda", generator=gen, dtype=torch.uint8)
+    h = ext.pack_encoded_device(blocks, torch.rand(m, device="cuda", generator=gen) + 0.5)
+    try:
+        ext.set_prefill(h, 64, 1024)
+        source = torch.randn(tokens, k, device="cuda", generator=gen).bfloat16()
+        memory = torch.empty(tokens * m, dtype=torch.bfloat16, device="cuda")
+        apart = torch.empty(tokens, m, dtype=torch.bfloat16, device="cuda")
+        grids = [grid for name, grid in launched(lambda: ext.linear_out(h, source, apart)) if "cluster_gemv" in name]
+        assert len(grids) > 1
+        x, y = memory[:tokens * k].view(tokens, k), memory.view(tokens, m)
+        x.copy_(source)
+        ext.linear_out(h, x, y)
+        # both are one rounding away from the same sums
+        assert _distance(y, apart.double()) <= 2 * 2.0 ** -9
+    finally:
+        ext.free(h)
