@@ -168,3 +168,26 @@ def test_output_over_the_input_of_a_call_in_slabs(ext):
         assert _distance(y, apart.double()) <= 2 * 2.0 ** -9
     finally:
         ext.free(h)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("tokens", [1, 9, 33])
+def test_rows_too_long_for_one_launch(ext, dtype, tokens):
+    """1025 units of 128 columns: the row walk behind its pre-pass, in K ranges."""
+    m, k = 40, 131088
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    blocks = torch.randint(0, 256, (m * k // 2,), device="cuda", generator=gen, dtype=torch.uint8)
+    bias = torch.randn(m, device="cuda", generator=gen).to(dtype)
+    h = ext.pack_encoded_device(blocks, torch.rand(m, device="cuda", generator=gen) + 0.5, bias)
+    try:
+        ext.set_prefill(h, 64, 1024)
+        x = (torch.randn(tokens, k, device="cuda", generator=gen) / k ** 0.5).to(dtype)
+        y = torch.empty(tokens, m, device="cuda", dtype=dtype)
+        names = [name for name, _ in launched(lambda: ext.linear_out(h, x, y))]
+        assert any("gemv_xprep_kernel" in name for name in names) and not any("cluster_gemv" in name for name in names)
+        want = x.double() @ ext.dequant(h, 1).double().T + bias.double()
+        # one rounding of the output; entries of low-mode blocks (about half of these) are fp16
+        assert _distance(y, want) <= HALF_UNIT[dtype] / 2 + 2.0 ** -11
+        assert torch.equal(ext.linear(h, x), y)
+    finally:
+        ext.free(h)

@@ -1006,8 +1006,8 @@ static int plan_gemv(const Handle *h, int tokens, GemvPlan &plan, int fuse = 0, 
 }
 
 // `half_io`: x, y and the handle's bias are fp16 (the reference's texelator_bc4_kernel,
-// texelator_cuda.cu:94-139, which multiplies the un-rounded pal*scale in fp32 -- what this kernel computes
-// for either type); the activations then always take the pre-pass, which for fp16 is a padded copy.
+// texelator_cuda.cu:94-139, which multiplies the un-rounded pal*scale in fp32 -- what the kernels compute
+// for either type).
 //
 // Where x and y overlap, the row walk behind its pre-pass serves the call: the pre-pass copies the activations of all tokens of
 // a pass before a row of y is stored, while a cluster of the one-launch kernel may still read x when another stores.
@@ -1016,6 +1016,7 @@ int launch_gemv(const Handle *h, const __nv_bfloat16 *x, __nv_bfloat16 *y, int t
   for (int t0 = 0, pass = apart ? stream_tokens(h, tokens, half_io) : 0; pass > 0; t0 += pass) {
     if (t0 >= tokens) return TX_OK;
     const int rc = launch_stream(h, x + size_t(t0) * h->K, y + size_t(t0) * h->M, std::min(pass, tokens - t0), half_io, false, stream);
+    if (rc == TX_EUNSUPPORTED) break;   // no cluster of it fits this device: the row walk below serves all tokens
     if (rc != TX_OK) return rc;
   }
   Workspace *ws = workspace_for(h->device);

@@ -416,10 +416,9 @@ static int resident_clusters(int device, StreamKernel kernel, int cluster, int p
     attribute.val.clusterDim.y = attribute.val.clusterDim.z = 1;
     config.attrs = &attribute;
     config.numAttrs = 1;
-    if (cudaOccupancyMaxActiveClusters(&found, kernel, &config) != cudaSuccess) found = 0;
+    if (cudaOccupancyMaxActiveClusters(&found, kernel, &config) != cudaSuccess) found = 0;   // (the error is read below)
   }
-  cudaGetLastError();
-  cache[key] = found;
+  if (cudaGetLastError() == cudaSuccess) cache[key] = found;   // (a failed query may succeed next time)
   return found;
 }
 
@@ -492,7 +491,7 @@ int launch_stream(const Handle *h, const void *x, void *y, int tokens, bool half
   p.T = tokens;
   p.mode = h->palette | (stream_runs(h->KI, tokens, half_io).strided ? kStreamStrided : 0) | (half_io ? kStreamHalf : 0) | (swiglu ? kStreamSwiglu : 0);
   StreamPlan plan{};
-  if (!plan_stream(h, kernel, tokens, half_io, ws->sm_count, plan)) return fail(TX_EINVAL, "decode GEMV does not fit in shared memory for this K");
+  if (!plan_stream(h, kernel, tokens, half_io, ws->sm_count, plan)) return fail(TX_EUNSUPPORTED, "no thread-block cluster of the decode kernel fits this device");
   p.chain_shift = plan.chain_shift;
   p.cluster_shift = plan.cluster_shift;
   for (int begin = 0; begin < h->MT; begin += plan.slab) {
