@@ -191,3 +191,17 @@ def test_rows_too_long_for_one_launch(ext, dtype, tokens):
         assert torch.equal(ext.linear(h, x), y)
     finally:
         ext.free(h)
+
+
+@pytest.mark.parametrize("m,k", [(256, 8192), (512, 5120), (2048, 11008), (1000, 17600)])
+def test_one_token_takes_small_clusters(ext, m, k):
+    """At most two thread blocks for each sixteen rows: a token's eight runs occupy no more warps than one block has."""
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    blocks = torch.randint(0, 256, (m * k // 2,), device="cuda", generator=gen, dtype=torch.uint8)
+    h = ext.pack_encoded_device(blocks, torch.ones(m, device="cuda"))
+    try:
+        x, y = torch.randn(1, k, device="cuda").bfloat16(), torch.empty(1, m, device="cuda", dtype=torch.bfloat16)
+        (_, grid), = launched(lambda: ext.linear_out(h, x, y))
+        assert grid[0] <= 2 * ((m + 15) // 16)
+    finally:
+        ext.free(h)

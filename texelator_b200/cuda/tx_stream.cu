@@ -422,22 +422,32 @@ static int resident_clusters(int device, StreamKernel kernel, int cluster, int p
   return found;
 }
 
-// Cluster size and number of launches.  The estimate, in us, fitted to 14 shapes of 256 x 2048 to 57344 x 8192 with 1 to 15
-// tokens: a warp takes 0.5 us a unit with sixteen warps on an SM (0.8 beyond eight tokens, where it issues twice the MMAs; a
-// third less with eight warps), half of it counted by the warp with most units and half by the average; 0.35 us for
-// each (token, run) a warp stages and the bytes staged by all CTAs at 8 TB/s, both smaller in a larger cluster; what a cluster
-// costs at its barriers and in SMs that no whole cluster fits; 2.5 us a launch.  With eight tokens, clusters of 1, 2, 4, 8:
-// 256 x 2048 6.7, 4.9, 3.8, 3.2 us; 34816 x 5120 37.2, 28.7, 30.6, 29.4; with one token 34816 x 5120 22.2, 23.2, 24.0, 25.8.
+// Cluster size and number of launches.  The estimate, in us: a warp takes 0.35 us a unit (0.55 beyond eight tokens, where it
+// issues twice the MMAs) with sixteen warps on an SM and two thirds of that with eight, half of it counted by the warp with most
+// units and half by the average; 0.35 us for each (token, run) a warp stages and the bytes staged by all CTAs at 8 TB/s, both
+// smaller in a larger cluster; what a cluster costs at its barriers, in SMs that no whole cluster fits and, for four and
+// eight, in an early start lost (launch_stream); 2.5 us a launch.  The constants are fitted to 34 shapes of 200 x 256 to
+// 57344 x 8192 with 1, 2, 3, 5, 8, 12 and 15 tokens, each timed with clusters of 1, 2, 4 and 8 in a graph of 30 calls over three
+// matrices: the pick is 0.4 % slower than the best of the four on average, 10 % at worst.  us a call, by cluster:
+//
+//   256 x 2048     one token 2.6, 2.7, 3.3, 3.5      eight tokens 7.0, 4.8, 4.2, 3.9
+//   512 x 5120     one token 3.5, 3.4, 4.1, 4.2      eight tokens 8.4, 5.8, 5.2, 4.6
+//   2048 x 11008   one token 7.9, 5.6, 6.5, 6.2      eight tokens (too large), 12.4, 9.5, 7.9
+//   34816 x 5120   one token 21.1, 22.2, 23.9, 25.9  eight tokens 36.3, 27.6, 27.5, 28.7
+//
+// One bf16 token never takes clusters of more than two: its eight runs are fixed, so a warp's longest run stays as long while
+// warps idle, and the early start is worth 0.5 us (512 x 5120 with four CTAs 4.1 us, 3.4 with two).
 static bool plan_stream(const Handle *h, StreamKernel kernel, int tokens, bool half_io, int sm_count, StreamPlan &best) {
   const Runs runs = stream_runs(h->KI, tokens, half_io);
   const int NS = runs.shift, NC = 1 << NS;
-  const double step = tokens <= 8 ? 0.5 : 0.8, cluster_cost[4] = {0.0, 0.35, 0.6, 0.9};
+  const double step = tokens <= 8 ? 0.35 : 0.55, cluster_cost[4] = {0.0, 0.35, 1.1, 1.1};
   double best_cost = 0;
   for (int slabs = 1; slabs <= h->MT; slabs *= 2) {
     const int tiles = (h->MT + slabs - 1) / slabs;
     for (int CS = 0; CS <= 3 && CS <= NS; ++CS) {
       const int C = 1 << CS, n = NC >> CS;
       if (n > kStreamWarps) continue;
+      if (runs.strided && CS > 1 && best_cost != 0) break;
       const int units = n * runs.longest(), fixed = stream_head_bytes(tokens, NC) + tokens * (units * 256 + 16);
       for (int per_sm = 2; per_sm >= 1; --per_sm) {
         const int clusters = std::min(tiles, resident_clusters(h->device, kernel, C, per_sm, sm_count));
