@@ -161,12 +161,24 @@ __global__ void __launch_bounds__(kStreamThreads, 2) cluster_gemv_tile_kernel(co
     unsigned m = 0;
 #pragma unroll
     for (int j = 0; j < kHeldChunks; ++j) held[j] = fetch(lane + j * 32);
+    // what a lane does not keep waits in shared memory as it came: no trip to L2 for it a second time
+#pragma unroll 1
+    for (int i0 = kHeldChunks * 32; i0 < count; i0 += kHeldChunks * 32) {
+      uint4 more[kHeldChunks];
+#pragma unroll
+      for (int j = 0; j < kHeldChunks; ++j) more[j] = fetch(i0 + lane + j * 32);
+#pragma unroll
+      for (int j = 0; j < kHeldChunks; ++j) {
+        const int i = i0 + lane + j * 32;
+        if (i < count) dst[i] = more[j];
+        m = max(m, chunk_absmax(more[j]));
+      }
+    }
     int exponent = 0;
     float mult = 1.f;
     if (!half_io) {                                       // (fp16 activations are the operand as they are)
 #pragma unroll
       for (int j = 0; j < kHeldChunks; ++j) m = max(m, chunk_absmax(held[j]));
-      for (int i = lane + kHeldChunks * 32; i < count; i += 32) m = max(m, chunk_absmax(fetch(i)));
       m = __reduce_max_sync(0xffffffffu, m);
       float inverse;
       token_scaling(m, mult, inverse);
@@ -178,10 +190,9 @@ __global__ void __launch_bounds__(kStreamThreads, 2) cluster_gemv_tile_kernel(co
       const int i = lane + j * 32;
       if (i < count) dst[i] = half_io ? held[j] : convert_chunk(held[j], mult);
     }
-    for (int i = lane + kHeldChunks * 32; i < count; i += 32) {
-      const uint4 v = fetch(i);
-      dst[i] = half_io ? v : convert_chunk(v, mult);
-    }
+    if (!half_io)
+#pragma unroll 1
+      for (int i = lane + kHeldChunks * 32; i < count; i += 32) dst[i] = convert_chunk(dst[i], mult);
     if (lane == 0) exps_g[tok * NC + c] = exponent;
   }
   __syncthreads();
