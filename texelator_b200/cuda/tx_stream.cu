@@ -37,7 +37,7 @@ constexpr int kStreamThreads = 256;
 constexpr int kStreamWarps = kStreamThreads / 32;
 constexpr int kStreamTokens = 16;
 constexpr int kHeldChunks = 4;              // 16-byte pieces of a run a lane keeps while it looks for the largest magnitude
-constexpr int kStreamHalf = 0x100, kStreamSwiglu = 0x200, kStreamStrided = 0x400;   // flags beside the palette in StreamParams::mode
+constexpr int kStreamHalf = 1, kStreamSwiglu = 2, kStreamStrided = 4;   // flags in StreamParams::mode
 
 struct StreamParams {
   const uint4 *tiles;
@@ -92,7 +92,8 @@ __host__ __device__ __forceinline__ int stream_part_bytes(int tiles_of_cluster, 
   return (owned * chains * tokens * 64 + 127) & ~127;
 }
 
-// MODE 0: high-mode blocks of the software palette; 1: high-mode blocks of the texture palette; 2: anything
+// MODE: 0 software palette, 1 texture palette, + 2 where the payload has low-mode blocks.  (One instance for both palettes with such
+// blocks chose at run time: 34816 x 5120, nine weights of ten zero, one token, 69.7 us, 61.4 with an instance each.)
 template <int LOOKAHEAD, int NT, int MODE>
 __global__ void __launch_bounds__(kStreamThreads, 2) cluster_gemv_tile_kernel(const StreamParams p) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
@@ -132,7 +133,7 @@ __global__ void __launch_bounds__(kStreamThreads, 2) cluster_gemv_tile_kernel(co
       const uint4 *src = base + size_t(unext) * 64;
       pend[slot][0] = ldg_stream(src);
       pend[slot][1] = ldg_stream(src + 32);
-      if (MODE == 2) pflag[slot] = p.flags[unext];
+      if (MODE >= 2) pflag[slot] = p.flags[unext];
     }
     --left;
     const bool wrap = --run_left == 0;
@@ -252,22 +253,17 @@ __global__ void __launch_bounds__(kStreamThreads, 2) cluster_gemv_tile_kernel(co
       for (int slot = 0; slot < LOOKAHEAD; ++slot) {
         const uint4 q = pend[slot][0], r = pend[slot][1];   // duos of rows g and g + 8
         const unsigned flag = pflag[slot];
-        const bool texture = MODE == 1 || (MODE == 2 && (p.mode & 0xff) == TX_PALETTE_HARDWARE);   // uniform
-        const DuoConstants cq = texture ? duo_constants<true>(q.w) : duo_constants<false>(q.w);
-        const DuoConstants cr = texture ? duo_constants<true>(r.w) : duo_constants<false>(r.w);
+        constexpr bool texture = MODE & 1;
+        constexpr int palette = texture ? TX_PALETTE_HARDWARE : TX_PALETTE_SOFTWARE;
+        const DuoConstants cq = duo_constants<texture>(q.w), cr = duo_constants<texture>(r.w);
 #pragma unroll
         for (int sub = 0; sub < 2; ++sub) {
           unsigned aq[8], ar[8];
-          if (texture) {
-            if (sub == 0) { decode_duo_first<true>(q, cq, aq); decode_duo_first<true>(r, cr, ar); }
-            else { decode_duo_second<true>(q, cq, aq); decode_duo_second<true>(r, cr, ar); }
-          } else {
-            if (sub == 0) { decode_duo_first(q, cq, aq); decode_duo_first(r, cr, ar); }
-            else { decode_duo_second(q, cq, aq); decode_duo_second(r, cr, ar); }
-          }
-          if (MODE == 2 && __any_sync(0xffffffffu, flag != 0)) {   // warp-uniform: redo the low-mode blocks
-            if (duo_block_is_low(q, sub)) decode_block_low(q, sub, aq, p.mode & 0xff);
-            if (duo_block_is_low(r, sub)) decode_block_low(r, sub, ar, p.mode & 0xff);
+          if (sub == 0) { decode_duo_first<texture>(q, cq, aq); decode_duo_first<texture>(r, cr, ar); }
+          else { decode_duo_second<texture>(q, cq, aq); decode_duo_second<texture>(r, cr, ar); }
+          if (MODE >= 2 && __any_sync(0xffffffffu, flag != 0)) {   // warp-uniform: redo the low-mode blocks
+            if (duo_block_is_low(q, sub)) decode_block_low(q, sub, aq, palette);
+            if (duo_block_is_low(r, sub)) decode_block_low(r, sub, ar, palette);
           }
 #pragma unroll
           for (int nt = 0; nt < NT; ++nt) {
@@ -386,8 +382,9 @@ static StreamKernel pick_lookahead(int lookahead) {
 }
 template <int NT>
 static StreamKernel pick_mode(const Handle *h) {
-  if (h->has_low_mode) return pick_lookahead<NT, 2>(h->lookahead);
-  return h->palette == TX_PALETTE_HARDWARE ? pick_lookahead<NT, 1>(h->lookahead) : pick_lookahead<NT, 0>(h->lookahead);
+  const bool texture = h->palette == TX_PALETTE_HARDWARE;
+  if (h->has_low_mode) return texture ? pick_lookahead<NT, 3>(h->lookahead) : pick_lookahead<NT, 2>(h->lookahead);
+  return texture ? pick_lookahead<NT, 1>(h->lookahead) : pick_lookahead<NT, 0>(h->lookahead);
 }
 
 constexpr int kStreamSmem[3] = {0, 200 * 1024, 112 * 1024};   // dynamic shared memory of a CTA that has an SM to itself, and of two
@@ -510,7 +507,7 @@ int launch_stream(const Handle *h, const void *x, void *y, int tokens, bool half
   p.K = h->K;
   p.KI = h->KI;
   p.T = tokens;
-  p.mode = h->palette | (stream_runs(h->KI, tokens, half_io).strided ? kStreamStrided : 0) | (half_io ? kStreamHalf : 0) | (swiglu ? kStreamSwiglu : 0);
+  p.mode = (stream_runs(h->KI, tokens, half_io).strided ? kStreamStrided : 0) | (half_io ? kStreamHalf : 0) | (swiglu ? kStreamSwiglu : 0);
   StreamPlan plan{};
   if (!plan_stream(h, kernel, tokens, half_io, ws->sm_count, plan)) return fail(TX_EUNSUPPORTED, "no thread-block cluster of the decode kernel fits this device");
   p.chain_shift = plan.chain_shift;
