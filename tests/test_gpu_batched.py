@@ -174,3 +174,39 @@ def test_replays_of_sixteen_sequences_equal_eager_steps(kernel):
         model.check_status()
     finally:
         model.free()
+
+
+@pytest.mark.parametrize("batch", [1, 3])
+def test_capture_on_the_last_cache_row(batch):
+    """A sequence with room for one more token: ``capture`` touches no row but those of the next positions."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    from texelator_b200.batched import BatchedBC4Decoder
+    from texelator_b200.modeling import BC4Decoder, CONFIGS
+    config, max_len = CONFIGS["toy128"], 40
+    if batch == 1:
+        model, positions = BC4Decoder(config, "cuda:0", max_len=max_len, seed=2), [max_len - 1]
+    else:
+        model, positions = BatchedBC4Decoder(config, "cuda:0", max_len=max_len, batch=batch, seed=2), [max_len - 1, 5, 20]
+    try:
+        gen = torch.Generator(device="cuda").manual_seed(1)
+        for cache in (model.k_cache, model.v_cache):
+            cache.copy_(torch.randn(cache.shape, device="cuda", generator=gen))
+        model.pos.copy_(torch.tensor(positions, device="cuda"))
+        if batch == 1:
+            model.mask[..., :max_len - 1] = True
+        before = (model.tok.clone(), model.pos.clone(), model.k_cache.clone(), model.v_cache.clone())
+        model.capture()
+        torch.cuda.synchronize()
+        assert torch.equal(model.tok, before[0]) and torch.equal(model.pos, before[1])
+        for cache, saved in ((model.k_cache, before[2]), (model.v_cache, before[3])):
+            changed = (cache != saved).any(-1)                               # [layers, (sequences,) heads, rows]
+            changed = changed.unsqueeze(1) if batch == 1 else changed
+            for sequence, position in enumerate(positions):
+                rows = changed[:, sequence].any(0).any(0).nonzero().reshape(-1).tolist()
+                assert rows == [position]
+        model.decode_graph()
+        model.check_status()
+        assert model.pos.tolist() == [p + 1 for p in positions]
+    finally:
+        model.free()

@@ -236,11 +236,17 @@ class BatchedBC4Decoder(BC4Decoder):
     def capture(self) -> None:
         """Record ``decode_step`` in a CUDA graph (NCCL all-reduces included when tensor-parallel)."""
         stream = torch.cuda.Stream(self.device)
-        saved = (self.tok.clone(), self.pos.clone())     # the warm-up steps write cache rows that the real steps rewrite
+        # the warm-up steps write two cache rows of every sequence, its position's and the next one's (which follows from the
+        # token the first step picked); the real steps rewrite them before they read them.  Where a sequence has one row
+        # left, both write that one.
+        saved = (self.tok.clone(), self.pos.clone())
+        full = int(self.pos.max()) + 1 >= self.max_len
         stream.wait_stream(torch.cuda.current_stream(self.device))
         with torch.cuda.stream(stream):
             for _ in range(2):
                 self.decode_step()
+                if full:
+                    self.tok.copy_(saved[0]); self.pos.copy_(saved[1])
             self.tok.copy_(saved[0]); self.pos.copy_(saved[1])
             stream.synchronize()
             before = self.ext.launch_count()

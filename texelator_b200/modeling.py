@@ -565,13 +565,18 @@ class BC4Decoder:
         use_fused = self.fused if fused is None else fused
         step = self._decode_step if not use_fused else (self._decode_step_single if self.single and fused is None and not self.fuse_norm and self.prefer_single() else self._decode_step_fused)
         stream = torch.cuda.Stream(self.device)
+        # the warm-up steps write two cache rows, the position's and the next one's (which follows from the token the first step
+        # picked); the real steps rewrite them before they read them.  Where one row is left, both write that one.
         saved = (self.tok.clone(), self.pos.clone(), self.mask.clone())
+        full = int(self.pos.max()) + 1 >= self.max_len
         # the capture stream is non-blocking: everything queued so far (the prompt's cache writes, the clones
         # above) has to be ordered before the first warm-up step on it
         stream.wait_stream(torch.cuda.current_stream(self.device))
         with torch.cuda.stream(stream):
             for _ in range(2):
                 step()
+                if full:
+                    self.tok.copy_(saved[0]); self.pos.copy_(saved[1]); self.mask.copy_(saved[2])
             self.tok.copy_(saved[0]); self.pos.copy_(saved[1]); self.mask.copy_(saved[2])
             stream.synchronize()
             before = self.ext.launch_count()
