@@ -28,10 +28,10 @@ ROOT = Path(__file__).resolve().parent
 sys.path.insert(0, str(ROOT))
 
 # DRAM bytes moved per algorithmic byte by the decode GEMV: dram__bytes_read.sum + dram__bytes_write.sum of
-# one ncu-captured gemv_tile_kernel<4,1,0,0,0> launch on a 34816x5120 matrix (89.34 MB + 3.27 MB) over its
+# one ncu-captured cluster_gemv_tile_kernel<3,1,0> launch on a 34816x5120 matrix (89.32 MB + 2.78 MB) over its
 # algorithmic 89.35 MB.  The kernel reads every payload byte once, so the ratio carries over to the other
 # shapes; re-capture when the kernel's memory access pattern changes.
-GEMV_DRAM_BYTES_PER_ALGORITHMIC_BYTE = (89.34 + 3.27) / 89.35
+GEMV_DRAM_BYTES_PER_ALGORITHMIC_BYTE = (89.32 + 2.78) / 89.35
 
 METRIC = "bc4_decode_tokens_per_second_bs1"
 UNIT = "tok/s"
@@ -280,7 +280,7 @@ def gemv_roofline(model, config, world: int) -> dict:
     traffic_ratio = GEMV_DRAM_BYTES_PER_ALGORITHMIC_BYTE
     return {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
             "traffic": traffic_ratio * total, "traffic_source": "ncu capture of one 34816x5120 launch (ratio to algorithmic bytes), scaled by algorithmic bytes",
-            "peak_source": source, "kernel": "gemv_tile_kernel (all %d decode GEMV launches of one token)" % len(jobs),
+            "peak_source": source, "kernel": "cluster_gemv_tile_kernel (all %d decode GEMV launches of one token)" % len(jobs),
             "algorithmic_bytes_per_token": total, "ms_per_token_linear_only": ms, "launches": len(jobs)}
 
 

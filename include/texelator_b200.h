@@ -11,8 +11,8 @@
  * same meaning; the Python wrapper turns a non-zero status into RuntimeError).
  *
  * Threading: like the reference, a handle is not safe for concurrent use from several host
- * threads, and setters are plain field writes.  All launches of one process on one device share
- * a per-device activation scratch (multi-token decode), so tx_linear calls on the same device must
+ * threads, and setters are plain field writes.  Prompts, and decode calls that go through a pre-pass (tx_linear names them),
+ * share a per-device activation scratch, so such tx_linear calls on the same device must
  * be ordered on one stream (or otherwise serialised) with respect to each other.
  */
 #ifndef TEXELATOR_B200_H
@@ -135,7 +135,7 @@ int tx_linear_single(uint64_t handle, const void *x, const void *staged, int swi
 int tx_linear_single_info(uint64_t handle, int64_t out[3]);
 
 /* set_lookahead: texelator_cuda.cu:1471-1478.  k in {1,2,3,4,6,8}: 1 KiB weight requests each
- * warp keeps in flight (the reference: texture requests in flight). */
+ * warp keeps in flight (the reference: texture requests in flight); tx_linear takes 1 as 2. */
 int tx_set_lookahead(uint64_t handle, int lookahead);
 /* set_prefill: texelator_cuda.cu:1480-1488.  threshold >= 1; tile_rows >= 16 and % 16 == 0. */
 int tx_set_prefill(uint64_t handle, int threshold, int tile_rows);

@@ -4,7 +4,7 @@ The reference has no serving loop of its own; a batch reaches its operator as th
 ``linear`` call, and every token count below the prefill threshold goes to the decode GEMV with one grid
 row per token (``texelator/cuda/texelator_cuda.cu:1438-1468``), which streams the whole matrix once per
 token.  Here the B rows of a step go through the multi-token decode kernel, which reads the matrix once
-for all of them (K ranges per CTA, so that the B activation rows of a range fit in shared memory), and the
+for up to sixteen of them (each CTA of a cluster stages its share of every activation row), and the
 steps between the linears are the library's glue kernels with a batch dimension:
 
     add_rmsnorm [B, hidden] -> qkv linear -> attention_step_batch (RoPE, cache append, attention of every

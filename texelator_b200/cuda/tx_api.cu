@@ -33,9 +33,9 @@ bool pdl_enabled() {
   return enabled;
 }
 
-// The scratch is sized once per device: 48 Mi scaled fp16 activations (96 MiB; multi-token decode
-// passes use the first 32 tokens' worth, the prefill GEMM stages whole token chunks) plus one
-// multiplier per staged token, and 16 Mi floats (64 MiB) for the K-range sums of multi-token decode passes.
+// The scratch is sized once per device: 48 Mi scaled fp16 activations (96 MiB; the prefill GEMM stages whole token
+// chunks, the decode row walk the first 32 tokens' worth) plus one multiplier per staged token, and 16 Mi floats
+// (64 MiB) for the K-range sums of both.
 Workspace *workspace_for(int device) {
   std::lock_guard<std::mutex> lock(g_workspace_guard);
   auto found = g_workspaces.find(device);

@@ -160,10 +160,10 @@ struct Handle {
 
 // Per-device scratch shared by every handle of the process on that device.
 struct Workspace {
-  __half *xprep = nullptr;        // scaled fp16 activations of multi-token decode passes
+  __half *xprep = nullptr;        // scaled fp16 activations of prompts and of the row walk's decode passes
   size_t xprep_halfs = 0;
   float *xmul = nullptr;          // per-token multipliers, one per staged token
-  float *partial = nullptr;       // fp32 sums of the K ranges of a multi-token decode pass, [splits][tokens][M]
+  float *partial = nullptr;       // fp32 sums of the K ranges of a short prompt or of such a pass, [ranges][tokens][M]
   size_t partial_floats = 0;
   int *status = nullptr;          // first non-zero code a kernel recorded when a bounded wait ran out
   int sm_count = 0;

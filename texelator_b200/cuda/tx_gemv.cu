@@ -1,6 +1,7 @@
 // Decode GEMV, whole rows per CTA (reference: texelator_bc4_bf16_kernel, texelator/cuda/texelator_cuda.cu:141-199, one warp
 // per output row through the texture unit).  tx_linear streams up to sixteen tokens through tx_stream.cu; the kernel here
-// serves what that one does not: a fused norm in front, the allocation-free entry point, rows too long for it.
+// serves what that one does not: a fused norm in front, the allocation-free entry point, rows too long for it, outputs that
+// overlap the activations.
 //
 // B200 design.  A persistent CTA walks 16-row tiles of the tiled BC4 payload; its eight warps split
 // the tile's 1 KiB units (16 rows x 128 columns) round-robin, keep LOOKAHEAD units in flight as
@@ -336,9 +337,9 @@ gemv_tile_kernel(const GemvParams p) {
     for (int slot = 0; slot < LOOKAHEAD; ++slot) {
       const uint4 q = pend[slot][0], r = pend[slot][1];   // duos of rows g and g+8
       const unsigned flag = pflag[slot];
-        const bool texture = LOWMODE && (p.palette & 0xff) == TX_PALETTE_HARDWARE;   // uniform
-        const DuoConstants cq = texture ? duo_constants<true>(q.w) : duo_constants<false>(q.w);
-        const DuoConstants cr = texture ? duo_constants<true>(r.w) : duo_constants<false>(r.w);
+      const bool texture = LOWMODE && (p.palette & 0xff) == TX_PALETTE_HARDWARE;   // uniform
+      const DuoConstants cq = texture ? duo_constants<true>(q.w) : duo_constants<false>(q.w);
+      const DuoConstants cr = texture ? duo_constants<true>(r.w) : duo_constants<false>(r.w);
       // ---- one unit: blocks (ki*8 + t) [sub 0] and (ki*8 + 4 + t) [sub 1] of rows g and g+8
 #pragma unroll
       for (int sub = 0; sub < 2; ++sub) {

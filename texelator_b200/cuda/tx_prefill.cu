@@ -579,9 +579,10 @@ static int prefill_k_ranges(const Handle *h, int tokens, const Workspace *ws) {
 // GPU's power state more than by shape, and never less below that.
 //
 // Up to eight tokens (a threshold below the default of 16) the decode kernel keeps the call: it pays one group of MMA columns
-// there, and two from nine on.  Decode kernel against the 64-token tile, us a call from HBM: 256x2048 2.6 / 7.5 with one
-// token, 7.6 / 7.5 with eight, 11.2 / 7.6 with ten; 5120x5120 6.5 / 11.5, 11.6 / 11.8, 20.0 / 11.9; 34816x5120
-// 24.0 / 31.5, 30.8 / 32.0, 51.5 / 32.0.
+// there, and two from nine on.  Decode kernel against the 64-token tile, us a call from HBM with one, eight, ten and fifteen
+// tokens: 256x2048 2.7 / 6.9, 3.8 / 7.3, 4.6 / 7.4, 4.9 / 7.5; 5120x5120 6.3 / 11.4, 9.4 / 11.9, 11.3 / 12.1, 11.8 / 12.6;
+// 34816x5120 22.4 / 31.6, 29.3 / 31.9, 35.5 / 32.1, 38.3 / 32.0.  From nine tokens on the tile is the faster one on the widest
+// matrices alone; the line was drawn for a decode kernel that took 11.2, 20.0 and 51.5 us for ten.
 //
 // Distance from 64 bits, tile against decode kernel, which adds a row in sixteen shorter chains: on Gaussian activations
 // both end at the output's rounding (fp16, 11008x2048, 160 tokens: 2.0759e-4 and 2.0757e-4 of the result; bf16 equal to

@@ -14,13 +14,16 @@
 //   * the order of the sums does not depend on the rows of the matrix, the cluster size or the look-ahead, so row shards
 //     reassemble bit for bit.
 //
-// What bounds it: instruction issue.  With the weights in L2 a call takes as long as with the weights in HBM; a unit is about
-// 170 instructions of a warp, and what comes before the first unit (index arithmetic on kernel parameters alone, no
-// division) and after the last one counts on small matrices.  us a call from HBM, the row walk with its pre-pass and combine
-// launches before / this kernel, for one, eight and fifteen bf16 tokens: 34816 x 5120 24.0 / 22.4, 31.2 / 29.0, 55.7 / 41;
-// 5120 x 17408 16.7 / 16.5, 24.8 / 19.1, 39.7 / 24.9; 22016 x 2048 9.0 / 8.0, 13.3 / 13.0, 22.8 / 17.4; 2048 x 11008 8.4 / 8.9,
-// 14.7 / 9.0, 23.1 / 11.8; 256 x 2048 2.6 / 2.7, 7.7 / 3.9, 12.6 / 5.0; one fp16 token on the texture palette, 5120 x 17408,
-// 30.6 / 20.6.
+// What bounds it: instruction issue.  With the weights in L2 a call takes as long as with the weights in HBM; one token of
+// 34816 x 5120 is 154 warp instructions a unit, all counted, on 3.7 warps a scheduler that issue in 58 % of the cycles.  What comes
+// before the first unit (index arithmetic on kernel parameters alone, no division) and after the last one counts on small
+// matrices.  us a call (a graph over copies larger than L2, look-ahead 3), the row walk with its pre-pass and combine
+// launches / this kernel, for one, eight and fifteen bf16 tokens:
+//
+//   34816 x 5120   24.3 / 22.4   31.2 / 29.3   55.2 / 38.3        2048 x 11008   8.3 / 6.8   14.1 / 8.8   23.1 / 11.7
+//   5120 x 17408   16.8 / 16.1   24.8 / 18.9   38.9 / 24.3        512 x 5120     3.5 / 3.6    9.2 / 4.8   15.4 / 6.0
+//   22016 x 2048    9.2 / 8.1    13.3 / 12.6   23.0 / 17.1        256 x 2048     2.6 / 2.7    7.7 / 3.8   12.8 / 4.9
+//   one fp16 token on the texture palette, 5120 x 17408: 30.7 / 20.5
 //
 // The only waits are CTA and cluster barriers.
 #include <algorithm>
@@ -93,7 +96,7 @@ __host__ __device__ __forceinline__ int stream_part_bytes(int tiles_of_cluster, 
 }
 
 // MODE: 0 software palette, 1 texture palette, + 2 where the payload has low-mode blocks.  (One instance for both palettes with such
-// blocks chose at run time: 34816 x 5120, nine weights of ten zero, one token, 69.7 us, 61.4 with an instance each.)
+// blocks chose at run time: 34816 x 5120, nine weights of ten zero, one token, 69.7 us, 61.2 with an instance each.)
 template <int LOOKAHEAD, int NT, int MODE>
 __global__ void __launch_bounds__(kStreamThreads, 2) cluster_gemv_tile_kernel(const StreamParams p) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
