@@ -180,7 +180,7 @@ int tx_set_palette(uint64_t handle, int palette);
 
 /* encode: the reference's offline encoder for one matrix, texelator/encoder.py:34-102 (endpoint_opt), :23-31
  * (nearest), :105-117 (pack_blocks) and :137-145 (row scales) -- there a chain of PyTorch tensor operations,
- * here one kernel whose output is byte-identical to it.  All pointers are device pointers: `weight` fp32
+ * here with output that is byte-identical to it.  All pointers are device pointers: `weight` fp32
  * [M, K] row-major, `hdiag` fp32 [K] (the activation second moments E[x_k^2] that weight the error),
  * `lut` fp32 [255, 255, 8] = palette[e1 + 127][e0 + 127][selector]; writes M * K / 2 bytes of row-major BC4
  * blocks (the .bc4 file content) and M fp32 row scales (the .scales.f32 content), which tx_pack_encoded

@@ -128,3 +128,43 @@ def test_palette_at_any_float(ext, lut, shift):
     want_blocks, want_scales = O.encode_linear(w, hdiag, lut)
     assert np.array_equal(scales.cpu().numpy(), want_scales)
     assert np.array_equal(blocks.cpu().numpy(), want_blocks.reshape(-1))
+
+
+def _rows(kind, m, k, gen):
+    w = torch.randn(m, k, device="cuda", generator=gen)
+    if kind == "uniform":                    # endpoints at their limit
+        w = torch.rand(m, k, device="cuda", generator=gen) - 0.5
+    elif kind == "cubed":                    # blocks far below the row's largest weight: endpoints close together
+        w = w ** 3
+    elif kind == "pruned":
+        w = w * (torch.rand(m, k, device="cuda", generator=gen) < 0.1)
+    elif kind == "ties":                     # weights on and half way between palette entries
+        w = torch.randint(-14 * 127, 14 * 127 + 1, (m, k), device="cuda", generator=gen).float() / (14 * 127)
+    elif kind == "numbers":                  # not numbers, infinities, weights far below the scale
+        w[::3, 5], w[::5, 9], w[1::5, 17] = float("nan"), float("inf"), -float("inf")
+        w[::4, ::3] *= 1e-25
+    return w
+
+
+@pytest.mark.parametrize("kind,m,k,palette", [
+    ("normal", 2051, 2048, "software"), ("uniform", 4096, 1040, "software"), ("cubed", 1200, 4096, "software"),
+    ("pruned", 1024, 4160, "software"), ("ties", 1024, 4096, "software"), ("numbers", 1024, 4096, "software"),
+    ("normal", 90000, 48, "software"), ("normal", 593, 8208, "software"), ("normal", 300, 17408, "software"),
+    ("normal", 1024, 4096, "hardware"), ("normal", 1024, 4096, "one entry off"), ("moments", 1024, 4096, "software")])
+def test_large_matrices_get_the_bytes_of_their_slabs(ext, lut, kind, m, k, palette):
+    """Matrices of 2^21 weights and more have blocks that are searched by a quadratic form; slabs of fewer rows are searched
+    neighbour by neighbour.  A row's bytes do not depend on the rows beside it, so both have to agree."""
+    gen = torch.Generator(device="cuda").manual_seed(k)
+    table = (ext.hardware_palette().reshape(255, 255, 8) if palette == "hardware" else torch.from_numpy(lut)).cuda().clone()
+    if palette == "one entry off":
+        table[60, 190, 4] += 1e-3            # high mode, endpoints apart
+    w = _rows(kind, m, k, gen)
+    hdiag = torch.exp(torch.randn(k, device="cuda", generator=gen))
+    if kind == "moments":
+        hdiag[::7], hdiag[5], hdiag[100], hdiag[200] = 0, -1, float("nan"), float("inf")
+    assert m * k >= 1 << 21
+    blocks, scales = ext.encode(w, hdiag, table)
+    rows = ((1 << 21) - 1) // k
+    slabs = [ext.encode(w[i:i + rows], hdiag, table) for i in range(0, m, rows)]
+    assert torch.equal(blocks, torch.cat([b for b, _ in slabs]))
+    assert torch.equal(scales.view(torch.int32), torch.cat([s for _, s in slabs]).view(torch.int32))
