@@ -544,7 +544,6 @@ __global__ void __launch_bounds__(kEncodeThreads, 4) encode_kernel(const float *
     }
     const float scale = fmaxf(m, 1e-12f), reciprocal = __frcp_rn(scale);
     const bool normal = scale >= 0x1p-40f && scale <= 0x1p60f;
-    const unsigned tiny = __float_as_uint(scale * 0x1p-60f) * 2 - 1;
     if (!live) continue;
     if (in_group == 0 && blockIdx.y == 0) scales[row] = scale;
 
@@ -560,7 +559,7 @@ __global__ void __launch_bounds__(kEncodeThreads, 4) encode_kernel(const float *
         b.h2[2 * j + 1] = pack2(g.z, g.w);
         // (no weight of the row is above the scale, so the quotients need no clamp)
         const auto quotient = [&](float value) {
-          rough |= __float_as_uint(value) * 2 - 1 < tiny;     // below 2^-60 of the scale, and not zero
+          rough |= !(fabsf(value) >= scale * 0x1p-60f || value == 0.f);   // (true for a weight that is not a number)
           return divide_by_scale(value, scale, reciprocal);
         };
         const float a0 = quotient(w[j].x), a1 = quotient(w[j].y), a2 = quotient(w[j].z), a3 = quotient(w[j].w);
