@@ -226,6 +226,10 @@ int tx_kernel_status(int device, int clear);
  *                      step over rows they wrote needs a launch that is not one of this library's in between
  *   silu_mul         : out[t,i] = silu(gate_up[t,i]) * gate_up[t,intermediate+i]                     */
 int tx_aux_add_rmsnorm(void *h, const void *delta, const void *weight, void *y, int tokens, int hidden, float eps, void *stream);
+/* The same with rows of h taken from an embedding table [vocab, hidden] first: h[r] = table[row_tokens[r]]; a token outside the table records
+ * code 33 in the device status word (tx_kernel_status) and takes row 0. */
+int tx_aux_embed_rmsnorm(const void *table, int64_t vocab, const int64_t *row_tokens, void *h, const void *weight, void *y, int tokens, int hidden,
+                         float eps, int device, void *stream);
 /* add_rmsnorm for one token with the extras of tx_linear_single: delta may come as `splits` fp32 partial
  * vectors (partials[s * partial_stride + i], added in split order, rounded to bf16, then added to h), and
  * the normalised row may also (or only: y may be NULL then) be written in staged form to `staged`

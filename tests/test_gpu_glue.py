@@ -330,3 +330,20 @@ def test_allreduce_wait_is_bounded_and_reports(ext):
     assert ext.kernel_status() == 0
     torch.zeros(1, device="cuda").add_(1)                        # the context is still usable
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("tokens,hidden", [(1, 256), (1, 5120), (3, 2056), (16, 4096), (2, 16384)])
+def test_embed_rmsnorm_is_a_gather_and_a_norm(ext, tokens, hidden):
+    gen = torch.Generator(device="cuda").manual_seed(hidden)
+    table = torch.randn(50, hidden, device="cuda", generator=gen).bfloat16()
+    weight = torch.randn(hidden, device="cuda", generator=gen).bfloat16()
+    ids = torch.randint(0, 50, (tokens,), device="cuda", generator=gen)
+    ids[0] = 49
+    want_h, want_y = table[ids], torch.empty(tokens, hidden, dtype=torch.bfloat16, device="cuda")
+    ext.add_rmsnorm(want_h.clone(), None, weight, want_y, 1e-6)
+    h, y = torch.zeros_like(want_h), torch.zeros_like(want_y)
+    ext.embed_rmsnorm(table, ids, h, weight, y, 1e-6)
+    assert torch.equal(h, want_h) and torch.equal(y, want_y) and ext.kernel_status() == 0
+    ids[-1] = 50                                # outside the table: reported, and row 0 in its place
+    ext.embed_rmsnorm(table, ids, h, weight, y, 1e-6)
+    assert ext.kernel_status(clear=True) == 33 and torch.equal(h[-1], table[0])

@@ -166,11 +166,11 @@ class BatchedBC4Decoder(BC4Decoder):
             torch.distributed.all_reduce(t, group=self.group)
 
     def _pick_tokens(self, hidden: torch.Tensor) -> None:
-        logits = (hidden @ self.lm_head.T).float()
+        logits = hidden @ self.lm_head.T
         if not self.vocab_parallel:
-            self.next_tok.copy_(logits.argmax(-1))
+            torch.argmax(logits, -1, out=self.next_tok)     # the bf16 order is the fp32 order
             return
-        score, index = logits.max(-1)
+        score, index = logits.float().max(-1)
         self.best_local[:, 0].copy_(score)
         self.best_local[:, 1].copy_(index + self.vocab_offset)             # token ids are exact in fp32 (< 2^24)
         torch.distributed.all_gather_into_tensor(self.best_all, self.best_local, group=self.group)
@@ -182,10 +182,12 @@ class BatchedBC4Decoder(BC4Decoder):
         """One token for every sequence, library kernels only (this is what ``capture`` records)."""
         c, ext = self.config, self.ext
         q_heads, kv_heads = c.q_heads // self.world, c.kv_heads // self.world
-        torch.index_select(self.embed, 0, self.tok, out=self.buf_h)
         delta = None
         for layer in range(c.layers):
-            ext.add_rmsnorm(self.buf_h, delta, self.norm1[layer], self.buf_x, c.rms_eps)
+            if layer == 0:
+                ext.embed_rmsnorm(self.embed, self.tok, self.buf_h, self.norm1[layer], self.buf_x, c.rms_eps)
+            else:
+                ext.add_rmsnorm(self.buf_h, delta, self.norm1[layer], self.buf_x, c.rms_eps)
             ext.linear_out(self.h_qkv[layer], self.buf_x, self.buf_qkv)
             ext.attention_step_batch(self.buf_qkv, self.cos, self.sin, self.pos, self.k_cache[layer], self.v_cache[layer],
                                      self.attn_scratch, self.buf_attn, q_heads, kv_heads, c.head_dim)
@@ -197,9 +199,8 @@ class BatchedBC4Decoder(BC4Decoder):
             ext.linear_out(self.h_down[layer], self.buf_act, self.buf_down)
             self._all_reduce(self.buf_down)
             delta = self.buf_down
-        ext.add_rmsnorm(self.buf_h, delta, self.final_norm, self.buf_x, c.rms_eps)
-        self.last_hidden.copy_(self.buf_x)
-        self._pick_tokens(self.buf_x)
+        ext.add_rmsnorm(self.buf_h, delta, self.final_norm, self.last_hidden, c.rms_eps)
+        self._pick_tokens(self.last_hidden)
         self.tok.copy_(self.next_tok)
         self.pos.add_(1)
 

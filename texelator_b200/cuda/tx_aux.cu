@@ -26,9 +26,18 @@ __device__ __forceinline__ float warp_max(float v) {
 constexpr int kNormThreads = 512;
 constexpr int kNormChunks = 4;            // hidden <= 512 * 8 * 4 = 16384 stays in registers
 
+// EMBED: the first norm of a decode step.  A row of h is the embedding of the row's token, fetched here and stored for the residual
+// (a launch of its own before: 16 rows of 5120 14.2 us, of which the wait for one more kernel in the chain is most; one row 2.0).
+struct EmbedRows {
+  const __nv_bfloat16 *table;   // [vocab, hidden]
+  const long long *tokens;
+  long long vocab;
+  int *status;                  // code 33: a token outside the table (row 0 is taken)
+};
+template <bool EMBED>
 __global__ void __launch_bounds__(kNormThreads) add_rmsnorm_kernel(__nv_bfloat16 *__restrict__ h, const __nv_bfloat16 *__restrict__ delta,
                                                                    const __nv_bfloat16 *__restrict__ weight, __nv_bfloat16 *__restrict__ y,
-                                                                   int hidden, float eps) {
+                                                                   int hidden, float eps, const EmbedRows embed) {
   __shared__ float partial[kNormThreads / 32];
   grid_launch_dependents();
   const int row = blockIdx.x, chunks = hidden / 8;
@@ -43,13 +52,23 @@ __global__ void __launch_bounds__(kNormThreads) add_rmsnorm_kernel(__nv_bfloat16
   grid_dependency_wait();
   uint4 *hr = reinterpret_cast<uint4 *>(h + size_t(row) * hidden);
   const uint4 *dr = delta ? reinterpret_cast<const uint4 *>(delta + size_t(row) * hidden) : nullptr;
+  const uint4 *er = nullptr;
+  if (EMBED) {
+    long long token = __ldcg(embed.tokens + row);
+    if (token < 0 || token >= embed.vocab) {
+      if (threadIdx.x == 0) atomicCAS(embed.status, 0, 33);
+      token = 0;
+    }
+    er = reinterpret_cast<const uint4 *>(embed.table + size_t(token) * hidden);
+  }
   uint4 keep[kNormChunks];
   float ss = 0.f;
 #pragma unroll
   for (int c = 0; c < kNormChunks; ++c) {
     const int i = threadIdx.x + c * kNormThreads;
     if (i < chunks) {
-      uint4 v = __ldcg(hr + i);   // inputs come from the previous kernel: read through L2
+      uint4 v = __ldcg((EMBED ? er : hr) + i);   // inputs come from the previous kernel: read through L2
+      if (EMBED) hr[i] = v;
       __nv_bfloat162 *pv = reinterpret_cast<__nv_bfloat162 *>(&v);
       if (dr) {
         uint4 d = __ldcg(dr + i);
@@ -1447,9 +1466,23 @@ extern "C" {
 int tx_aux_add_rmsnorm(void *h, const void *delta, const void *weight, void *y, int tokens, int hidden, float eps, void *stream) {
   if (!h || !weight || !y || tokens < 1 || hidden < 8 || hidden % 8 || hidden > kNormThreads * 8 * kNormChunks)
     return fail(TX_EINVAL, "tx_aux_add_rmsnorm: hidden must be a multiple of 8 and at most 16384");
-  TX_CUDA(launch_pdl(add_rmsnorm_kernel, dim3(tokens), dim3(kNormThreads), 0, static_cast<cudaStream_t>(stream),
+  TX_CUDA(launch_pdl(add_rmsnorm_kernel<false>, dim3(tokens), dim3(kNormThreads), 0, static_cast<cudaStream_t>(stream),
                      static_cast<__nv_bfloat16 *>(h), static_cast<const __nv_bfloat16 *>(delta),
-                     static_cast<const __nv_bfloat16 *>(weight), static_cast<__nv_bfloat16 *>(y), hidden, eps));
+                     static_cast<const __nv_bfloat16 *>(weight), static_cast<__nv_bfloat16 *>(y), hidden, eps, EmbedRows{}));
+  count_launch();
+  TX_CUDA(cudaGetLastError());
+  return TX_OK;
+}
+
+int tx_aux_embed_rmsnorm(const void *table, int64_t vocab, const int64_t *row_tokens, void *h, const void *weight, void *y, int tokens, int hidden,
+                         float eps, int device, void *stream) {
+  if (!table || !row_tokens || !h || !weight || !y || vocab < 1 || tokens < 1 || hidden < 8 || hidden % 8 || hidden > kNormThreads * 8 * kNormChunks)
+    return fail(TX_EINVAL, "tx_aux_embed_rmsnorm: hidden must be a multiple of 8 and at most 16384");
+  Workspace *ws = workspace_for(device);
+  if (!ws) return TX_ECUDA;
+  const EmbedRows embed{static_cast<const __nv_bfloat16 *>(table), reinterpret_cast<const long long *>(row_tokens), vocab, ws->status};
+  TX_CUDA(launch_pdl(add_rmsnorm_kernel<true>, dim3(tokens), dim3(kNormThreads), 0, static_cast<cudaStream_t>(stream), static_cast<__nv_bfloat16 *>(h),
+                     static_cast<const __nv_bfloat16 *>(nullptr), static_cast<const __nv_bfloat16 *>(weight), static_cast<__nv_bfloat16 *>(y), hidden, eps, embed));
   count_launch();
   TX_CUDA(cudaGetLastError());
   return TX_OK;

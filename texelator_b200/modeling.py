@@ -412,11 +412,11 @@ class BC4Decoder:
 
     def _pick_token(self, hidden):
         """Greedy next token from the final hidden state (bf16 output head, fp32 argmax)."""
-        logits = (hidden @ self.lm_head.T).float()
+        logits = hidden @ self.lm_head.T
         if not self.vocab_parallel:
-            self.next_tok.copy_(logits.argmax(-1))
+            torch.argmax(logits, -1, out=self.next_tok)     # the bf16 order is the fp32 order
             return
-        score, index = logits.max(-1)
+        score, index = logits.float().max(-1)
         if self.peers is not None and self.single:
             self.ext.peer_best_token(score.contiguous(), index.contiguous(), self.vocab_offset, self.peers, self.next_tok)
             return
@@ -426,12 +426,13 @@ class BC4Decoder:
         winner = self.best_all[:, 0].argmax().reshape(1)
         self.next_tok.copy_(torch.index_select(self.best_all[:, 1], 0, winner).long())   # no host round trip
 
-    def _add_norm(self, residual, delta, weight):
-        """residual += delta (all-reduced first when it is a tensor-parallel partial); buf_x = rmsnorm(residual) * weight."""
+    def _add_norm(self, residual, delta, weight, out=None):
+        """residual += delta (all-reduced first when it is a tensor-parallel partial); out (buf_x) = rmsnorm(residual) * weight."""
+        out = self.buf_x if out is None else out
         if delta is not None and self.peers is not None and not self.fuse_norm:
-            self.ext.allreduce_add_rmsnorm(residual, delta, weight, self.buf_x, self.config.rms_eps, self.peers)
+            self.ext.allreduce_add_rmsnorm(residual, delta, weight, out, self.config.rms_eps, self.peers)
         else:
-            self.ext.add_rmsnorm(residual, delta, weight, self.buf_x, self.config.rms_eps)
+            self.ext.add_rmsnorm(residual, delta, weight, out, self.config.rms_eps)
 
     def enable_peer_exchange(self) -> bool:
         """Switch the fused decode step of a tensor-parallel model from NCCL all-reduces to the all-reduce
@@ -504,12 +505,16 @@ class BC4Decoder:
         split merge), o linear, gate/up linear (add + norm in front, SwiGLU behind), down linear."""
         c, ext = self.config, self.ext
         q_heads, kv_heads = c.q_heads // self.world, c.kv_heads // self.world
-        torch.index_select(self.embed, 0, self.tok, out=self.buf_h)
+        if self.fuse_norm:
+            torch.index_select(self.embed, 0, self.tok, out=self.buf_h)
         residual, spare = self.buf_h, self.buf_h2       # the fused linears write x + delta to the other buffer
         delta = None
         for layer in range(c.layers):
             if not self.fuse_norm:
-                self._add_norm(residual, delta, self.norm1[layer])
+                if layer == 0:
+                    ext.embed_rmsnorm(self.embed, self.tok, residual, self.norm1[layer], self.buf_x, c.rms_eps)
+                else:
+                    self._add_norm(residual, delta, self.norm1[layer])
                 ext.linear_out(self.h_qkv[layer], self.buf_x, self.buf_qkv)
             elif delta is None:
                 ext.linear_fused_out(self.h_qkv[layer], residual, self.buf_qkv, norm_weight=self.norm1[layer], eps=c.rms_eps)
@@ -535,9 +540,8 @@ class BC4Decoder:
             delta = self.buf_down
         if residual is not self.buf_h:
             self.buf_h.copy_(residual)
-        self._add_norm(self.buf_h, delta, self.final_norm)
-        self.last_hidden.copy_(self.buf_x)
-        self._pick_token(self.buf_x)
+        self._add_norm(self.buf_h, delta, self.final_norm, self.last_hidden)
+        self._pick_token(self.last_hidden)
         self.tok.copy_(self.next_tok)
         self.mask.index_fill_(3, self.pos, True)
         self.pos.add_(1)

@@ -67,6 +67,7 @@ C_API = {
     "tx_unpack_blocks": (_i32, [_u64, _vp]),
     "tx_kernel_status": (_i32, [_i32, _i32]),
     "tx_aux_add_rmsnorm": (_i32, [_vp, _vp, _vp, _vp, _i32, _i32, ctypes.c_float, _vp]),
+    "tx_aux_embed_rmsnorm": (_i32, [_vp, ctypes.c_int64, _vp, _vp, _vp, _vp, _i32, _i32, ctypes.c_float, _i32, _vp]),
     "tx_aux_rope_append": (_i32, [_vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp]),
     "tx_aux_rope_append_prompt": (_i32, [_vp, _vp, _vp, _i32, _i32, _vp, _vp, _i32, _i32, _i32, _i32, _vp]),
     "tx_aux_attention_decode": (_i32, [_vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, ctypes.c_float, _vp]),
@@ -370,6 +371,12 @@ class _Extension:
         tokens, hidden = h.shape
         self._check(self._lib.tx_aux_add_rmsnorm(h.data_ptr(), delta.data_ptr() if delta is not None else None,
                                                  weight.data_ptr(), y.data_ptr(), tokens, hidden, eps, self._stream(h)))
+
+    def embed_rmsnorm(self, table: torch.Tensor, row_tokens: torch.Tensor, h: torch.Tensor, weight: torch.Tensor, y: torch.Tensor, eps: float) -> None:
+        """``h = table[row_tokens]`` (int64, one per row), ``y = rmsnorm(h) * weight``."""
+        tokens, hidden = h.shape
+        self._check(self._lib.tx_aux_embed_rmsnorm(table.data_ptr(), table.shape[0], row_tokens.data_ptr(), h.data_ptr(), weight.data_ptr(),
+                                                   y.data_ptr(), tokens, hidden, eps, h.device.index, self._stream(h)))
 
     def rope_append(self, qkv, cos, sin, position, k_cache, v_cache, q_heads: int, kv_heads: int, head_dim: int) -> None:
         self._check(self._lib.tx_aux_rope_append(qkv.data_ptr(), cos.data_ptr(), sin.data_ptr(), position.data_ptr(),
