@@ -347,3 +347,35 @@ def test_embed_rmsnorm_is_a_gather_and_a_norm(ext, tokens, hidden):
     ids[-1] = 50                                # outside the table: reported, and row 0 in its place
     ext.embed_rmsnorm(table, ids, h, weight, y, 1e-6)
     assert ext.kernel_status(clear=True) == 33 and torch.equal(h[-1], table[0])
+
+
+@pytest.mark.parametrize("sequences,q_heads,kv_heads,max_len,positions", [
+    (16, 40, 8, 1040, [0, 1, 15, 16, 17, 63, 64, 65, 127, 128, 500, 640, 1000, 1023, 1024, 1039]),   # two splits: a cluster
+    (3, 8, 8, 700, [699, 16, 448]),                          # eleven splits: merged behind
+    (5, 64, 8, 600, [599, 0, 64, 300, 15]),                  # eight heads a kv head, a cluster of seven
+    (40, 16, 8, 400, [(37 * i) % 400 for i in range(40)]),   # one split: written directly
+])
+def test_attention_step_batch_matches_64_bits(ext, sequences, q_heads, kv_heads, max_len, positions):
+    """The edges of sixteen-key tiles and 64-key chunks, and each way the splits are merged, against 64-bit attention over the same
+    bf16 keys and rotated queries: what is left is the rounding of the output (2^-9 of a value at most)."""
+    gen = torch.Generator(device="cuda").manual_seed(max_len)
+    bf = dict(device="cuda", dtype=torch.bfloat16)
+    k_cache, v_cache = torch.randn(sequences, kv_heads, max_len, 128, generator=gen, **bf), torch.randn(sequences, kv_heads, max_len, 128, generator=gen, **bf)
+    k_cache[:, :, :8] *= 4                                   # a few large scores, so that the running maximum moves late
+    for b, pos in enumerate(positions):                      # nothing behind the position may be read
+        k_cache[b, :, pos:], v_cache[b, :, pos:] = float("nan"), float("nan")
+    angles = torch.rand(max_len, 64, device="cuda", generator=gen) * 6.28
+    cos, sin = angles.cos().contiguous(), angles.sin().contiguous()
+    qkv = torch.randn(sequences, (q_heads + 2 * kv_heads) * 128, generator=gen, **bf)
+    scratch = torch.zeros(sequences * ext.attention_step_scratch_floats(q_heads, max_len), dtype=torch.float32, device="cuda")
+    out = torch.zeros(sequences, q_heads * 128, **bf)
+    ext.attention_step_batch(qkv, cos, sin, torch.tensor(positions, device="cuda"), k_cache, v_cache, scratch, out, q_heads, kv_heads, 128)
+    for b, pos in enumerate(positions):
+        c, s = cos[pos], sin[pos]
+        q = qkv[b, :q_heads * 128].view(q_heads, 128).float()
+        q = torch.cat([q[:, :64] * c - q[:, 64:] * s, q[:, 64:] * c + q[:, :64] * s], -1).bfloat16().double()
+        keys, values = (t[b, :, :pos + 1].double().repeat_interleave(q_heads // kv_heads, 0) for t in (k_cache, v_cache))
+        want = torch.einsum("hk,hkd->hd", torch.softmax(torch.einsum("hd,hkd->hk", q, keys) * 128 ** -0.5, -1), values)
+        got = out[b].view(q_heads, 128).double()
+        # (a rotated query may be rounded the other way where the product was contracted: 2^-8 of one element)
+        assert float((got - want).norm() / want.norm()) <= 4e-3, (b, pos)
