@@ -351,12 +351,13 @@ def test_embed_rmsnorm_is_a_gather_and_a_norm(ext, tokens, hidden):
 
 @pytest.mark.parametrize("sequences,q_heads,kv_heads,max_len,positions", [
     (16, 40, 8, 1040, [0, 1, 15, 16, 17, 63, 64, 65, 127, 128, 500, 640, 1000, 1023, 1024, 1039]),   # two splits: a cluster
-    (3, 8, 8, 700, [699, 16, 448]),                          # eleven splits: merged behind
-    (5, 64, 8, 600, [599, 0, 64, 300, 15]),                  # eight heads a kv head, a cluster of seven
+    (3, 8, 8, 700, [699, 16, 448]),                          # a chunk a CTA, merged behind
+    (5, 64, 8, 1000, [999, 0, 64, 300, 15]),                 # eight heads a kv head, a cluster of seven
+    (2, 24, 8, 2900, [2899, 1300]),                          # eighteen splits of several chunks: merged behind
     (40, 16, 8, 400, [(37 * i) % 400 for i in range(40)]),   # one split: written directly
 ])
 def test_attention_step_batch_matches_64_bits(ext, sequences, q_heads, kv_heads, max_len, positions):
-    """The edges of sixteen-key tiles and 64-key chunks, and each way the splits are merged, against 64-bit attention over the same
+    """The edges of 64-key chunks, and each way the splits are merged, against 64-bit attention over the same
     bf16 keys and rotated queries: what is left is the rounding of the output (2^-9 of a value at most)."""
     gen = torch.Generator(device="cuda").manual_seed(max_len)
     bf = dict(device="cuda", dtype=torch.bfloat16)

@@ -582,7 +582,7 @@ __global__ void __launch_bounds__(64) rope_append_kernel(__nv_bfloat16 *__restri
 // rotated in place, k and v appended to the caches.  Bound by memory (every value is read once and written at most
 // twice): a thread owns eight dimensions of both halves of one head, so all accesses are 16 bytes and a warp
 // covers four heads of a token.
-// attention_tile_kernel reads cache rows before it waits for the launch in front of it, and that launch (a linear) may
+// attention_step_kernel reads cache rows before it waits for the launch in front of it, and that launch (a linear) may
 // itself have started early.  So this kernel never signals its dependents: what follows starts when every block has
 // stored its rows and fenced, and whatever follows that sees them.
 __global__ void __launch_bounds__(256) rope_append_prompt_kernel(__nv_bfloat16 *__restrict__ qkv, const float *__restrict__ cos_table,
@@ -765,14 +765,14 @@ __global__ void __launch_bounds__(kHeadDim) attention_combine_kernel(const float
   out[size_t(head) * kHeadDim + tid] = __float2bfloat16(num / den);
 }
 
-// The attention block of a decode step: RoPE of q and of the new key, append of the new key and value to the caches, single-query
-// grouped-query attention over positions 0..pos.  attention_tile_kernel below does it, with attention_merge_kernel behind it where the
-// splits are many.  attention_step_loop_kernel is the step in one launch, merge included (TEXELATOR_B200_ATTENTION_MERGE=inline): at most two CTAs an SM,
-// CTA `split` walks 64-key chunks split, split + gridDim.x, ... with running soft-max statistics:
+// One launch for the attention block of a decode step: RoPE of q and of the new key, append of the new
+// key and value to the caches, single-query grouped-query attention over positions 0..pos, and the
+// merge of the sequence splits.  CTA (split, kv head) owns kStepKeys cache positions:
 //   prologue  rotated q of the GROUP query heads -> shared memory (rounded to bf16 like a stored q);
 //             the CTA whose range holds `pos` rotates the new key and writes key and value rows to the
 //             caches (visible to the whole CTA after the barrier);
-//   loads     keys eight lanes per row (four rows per warp instruction), values one row per warp instruction;
+//   loads     every key and value row of the CTA is requested before any arithmetic: keys eight lanes
+//             per row (four rows per warp instruction), values one row per warp instruction;
 //   scores    16 products per lane, three shuffles per (key, head); soft-max statistics per head;
 //   values    p * v accumulated per warp, summed over the eight warps through shared memory;
 //   merge     each CTA publishes its unnormalised output and (max, sum); the CTA that arrives last for
@@ -797,19 +797,18 @@ __device__ __forceinline__ void unpack_bf16x8(const uint4 &raw, float (&out)[8])
 }
 
 template <int GROUP>
-__global__ void __launch_bounds__(kStepThreads, 2) attention_step_loop_kernel(const __nv_bfloat16 *__restrict__ qkv,
+__global__ void __launch_bounds__(kStepThreads, 2) attention_step_kernel(const __nv_bfloat16 *__restrict__ qkv,
                                                                       const float *__restrict__ cos_table,
                                                                       const float *__restrict__ sin_table,
                                                                       const long long *__restrict__ position,
                                                                       __nv_bfloat16 *__restrict__ k_cache,
                                                                       __nv_bfloat16 *__restrict__ v_cache, float *__restrict__ partial,
                                                                       __nv_bfloat16 *__restrict__ out, int q_heads, int kv_heads,
-                                                                      int max_len, int split_capacity, float scale) {
+                                                                      int max_len, int split_capacity, float scale, int merge_here) {
   __shared__ __align__(16) float q_s[GROUP][kHeadDim];
   __shared__ float p_s[GROUP][kStepKeys];
   __shared__ __align__(16) float red_s[kStepThreads / 32][GROUP][kHeadDim];   // per-warp partial sums
   __shared__ float stat_s[GROUP][2];
-  __shared__ float rescale_s[GROUP];
   __shared__ float weight_s[GROUP][kStepMaxSplits];   // merge weights of the splits
   __shared__ int last_s;
   constexpr int kHalf = kHeadDim / 2, kWarps = kStepThreads / 32;
@@ -824,13 +823,37 @@ __global__ void __launch_bounds__(kStepThreads, 2) attention_step_loop_kernel(co
   out += size_t(blockIdx.z) * q_heads * kHeadDim;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   grid_launch_dependents();
-  grid_dependency_wait();
+  // The position and the cache rows below it are complete when the launch in front starts: earlier steps wrote them,
+  // or rope_append_prompt_kernel, which lets nothing start before its rows are stored.  So they are read before the
+  // wait for that launch -- the qkv linear, whose tail these loads overlap.  Only qkv itself is new.
   const long long pos = __ldcg(position);                       // attends to keys 0..pos; key pos is new
-  const int chunks = int(pos / kStepKeys) + 1;                  // 64-key chunks that hold at least one key
-  const int splits = gridDim.x;                                 // CTA `split` takes chunks split, split + splits, ...
-  const int live = min(splits, chunks);                         // CTAs with work
+  const int live = int(pos / kStepKeys) + 1;                    // splits that hold at least one key
   if (split >= live) return;
+  const int key0 = split * kStepKeys;
+  const int count = int(min((long long)kStepKeys, pos + 1 - key0));
   const size_t q_rows = size_t(q_heads) * kHeadDim, kv_rows = size_t(kv_heads) * kHeadDim;
+
+  // ---- all old cache rows of this CTA in flight at once ----
+  // keys: lane (r = lane >> 3, j = lane & 7) holds dimensions 8j..8j+7 and 64+8j..64+8j+7 of key
+  // warp*8 + batch*4 + r; values: lane holds dimensions 4*lane..4*lane+3 of key warp*8 + i
+  const int r = lane >> 3, j = lane & 7;
+  uint4 key_raw[2][2];
+  uint2 val_raw[8];
+#pragma unroll
+  for (int b = 0; b < 2; ++b) {
+    const int key = warp * 8 + b * 4 + r;
+    const uint4 *row = reinterpret_cast<const uint4 *>(k_cache + (size_t(kvh) * max_len + key0 + key) * kHeadDim);
+    const bool old_row = key0 + key < pos;
+    key_raw[b][0] = old_row ? __ldcg(row + j) : make_uint4(0, 0, 0, 0);
+    key_raw[b][1] = old_row ? __ldcg(row + 8 + j) : make_uint4(0, 0, 0, 0);
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int key = warp * 8 + i;
+    val_raw[i] = key0 + key < pos ? __ldcg(reinterpret_cast<const uint2 *>(v_cache + (size_t(kvh) * max_len + key0 + key) * kHeadDim) + lane)
+                                  : make_uint2(0, 0);
+  }
+  grid_dependency_wait();
 
   // ---- prologue: rotate-half RoPE of q (and of the new key by its owner) ----
   for (int idx = tid; idx < GROUP * kHalf; idx += kStepThreads) {
@@ -841,7 +864,7 @@ __global__ void __launch_bounds__(kStepThreads, 2) attention_step_loop_kernel(co
     q_s[g][i] = __bfloat162float(__float2bfloat16(x1 * c - x2 * sn)) * scale;
     q_s[g][i + kHalf] = __bfloat162float(__float2bfloat16(x2 * c + x1 * sn)) * scale;
   }
-  if (split == (chunks - 1) % splits) {          // the CTA whose last chunk holds the new position
+  if (split == live - 1) {
     if (tid < kHalf) {
       const int i = tid;
       const float c = cos_table[pos * kHalf + i], sn = sin_table[pos * kHalf + i];
@@ -858,48 +881,21 @@ __global__ void __launch_bounds__(kStepThreads, 2) attention_step_loop_kernel(co
   }
   __syncthreads();
 
-  // ---- all cache rows of a chunk in flight at once ----
-  // keys: lane (r = lane >> 3, j = lane & 7) holds dimensions 8j..8j+7 and 64+8j..64+8j+7 of key
-  // warp*8 + batch*4 + r; values: lane holds dimensions 4*lane..4*lane+3 of key warp*8 + i
-  const int r = lane >> 3, j = lane & 7;
-  uint4 key_raw[2][2];
-  uint2 val_raw[8];
-  auto request_keys = [&](int chunk) {
-    const int key0 = chunk * kStepKeys;
-    const int count = int(min((long long)kStepKeys, pos + 1 - key0));
+  // ---- the new row (written above by this CTA when it owns the last split) ----
 #pragma unroll
-    for (int b = 0; b < 2; ++b) {
-      const int key = warp * 8 + b * 4 + r;
-      const uint4 *row = reinterpret_cast<const uint4 *>(k_cache + (size_t(kvh) * max_len + key0 + key) * kHeadDim);
-      key_raw[b][0] = key < count ? __ldcg(row + j) : make_uint4(0, 0, 0, 0);
-      key_raw[b][1] = key < count ? __ldcg(row + 8 + j) : make_uint4(0, 0, 0, 0);
+  for (int b = 0; b < 2; ++b) {
+    const int key = warp * 8 + b * 4 + r;
+    if (key0 + key == pos) {
+      const uint4 *row = reinterpret_cast<const uint4 *>(k_cache + (size_t(kvh) * max_len + pos) * kHeadDim);
+      key_raw[b][0] = __ldcg(row + j);
+      key_raw[b][1] = __ldcg(row + 8 + j);
     }
-  };
-  auto request_values = [&](int chunk) {
-    const int key0 = chunk * kStepKeys;
-    const int count = int(min((long long)kStepKeys, pos + 1 - key0));
+  }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int key = warp * 8 + i;
-      val_raw[i] = key < count ? __ldcg(reinterpret_cast<const uint2 *>(v_cache + (size_t(kvh) * max_len + key0 + key) * kHeadDim) + lane)
-                               : make_uint2(0, 0);
-    }
-  };
-  request_keys(split);
-  request_values(split);
+  for (int i = 0; i < 8; ++i)
+    if (key0 + warp * 8 + i == pos)
+      val_raw[i] = __ldcg(reinterpret_cast<const uint2 *>(v_cache + (size_t(kvh) * max_len + pos) * kHeadDim) + lane);
 
-  // Long caches give a CTA several chunks: running soft-max statistics per head (kept by warp g for head
-  // g), accumulators rescaled when the maximum moves, the next chunk's rows requested before this one is
-  // processed.  With one chunk per CTA (up to about 2300 positions on 8 kv heads) the loop runs once.
-  // The next chunk's keys are requested as soon as this chunk's scores are done with the key registers,
-  // its values after the value registers are consumed (no second register set: two CTAs per SM).
-  float acc[GROUP][4];
-#pragma unroll
-  for (int g = 0; g < GROUP; ++g) acc[g][0] = acc[g][1] = acc[g][2] = acc[g][3] = 0.f;
-  float run_max = -INFINITY, run_sum = 0.f;
-  for (int chunk = split; chunk < chunks; chunk += splits) {
-  const int count = int(min((long long)kStepKeys, pos + 1 - (long long)chunk * kStepKeys));
-  const bool more = chunk + splits < chunks;                    // uniform
   // ---- scores (q of one head at a time, so that two CTAs fit the register file of an SM) ----
   {
     float k[2][16];
@@ -926,15 +922,301 @@ __global__ void __launch_bounds__(kStepThreads, 2) attention_step_loop_kernel(co
       }
     }
   }
-  if (more) request_keys(chunk + splits);
   __syncthreads();
   // ---- per head: max and exp-sum over the CTA's keys (warp g handles head g; GROUP <= 8 warps) ----
   if (warp < GROUP) {
     const float a = p_s[warp][lane], b = p_s[warp][lane + 32];
-    const float m = fmaxf(run_max, warp_max(fmaxf(a, b)));     // finite: every chunk of the walk holds a key
+    const float m = warp_max(fmaxf(a, b));              // finite: key 0 of a live split exists
     const float ea = __expf(a - m), eb = __expf(b - m);
     p_s[warp][lane] = ea;
     p_s[warp][lane + 32] = eb;
+    const float sum = warp_sum(ea + eb);
+    if (lane == 0) {
+      stat_s[warp][0] = m;
+      stat_s[warp][1] = sum;
+    }
+  }
+  __syncthreads();
+  // ---- values ----
+  {
+    float acc[GROUP][4];
+#pragma unroll
+    for (int g = 0; g < GROUP; ++g) acc[g][0] = acc[g][1] = acc[g][2] = acc[g][3] = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float v0 = __uint_as_float(val_raw[i].x << 16), v1 = __uint_as_float(val_raw[i].x & 0xffff0000u);
+      const float v2 = __uint_as_float(val_raw[i].y << 16), v3 = __uint_as_float(val_raw[i].y & 0xffff0000u);
+#pragma unroll
+      for (int g = 0; g < GROUP; ++g) {
+        const float pw = p_s[g][warp * 8 + i];
+        acc[g][0] = fmaf(pw, v0, acc[g][0]);
+        acc[g][1] = fmaf(pw, v1, acc[g][1]);
+        acc[g][2] = fmaf(pw, v2, acc[g][2]);
+        acc[g][3] = fmaf(pw, v3, acc[g][3]);
+      }
+    }
+#pragma unroll
+    for (int g = 0; g < GROUP; ++g)
+      *reinterpret_cast<float4 *>(&red_s[warp][g][4 * lane]) = make_float4(acc[g][0], acc[g][1], acc[g][2], acc[g][3]);
+  }
+  __syncthreads();
+  for (int idx = tid; idx < GROUP * kHeadDim; idx += kStepThreads) {
+    const int g = idx / kHeadDim, d = idx % kHeadDim;
+    float sum = 0.f;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) sum += red_s[w][g][d];
+    partial[(size_t(kvh * GROUP + g) * split_capacity + split) * kStepRow + d] = sum;
+  }
+  if (tid < GROUP) {
+    float *rec = partial + (size_t(kvh * GROUP + tid) * split_capacity + split) * kStepRow;
+    rec[kHeadDim] = stat_s[tid][0];
+    rec[kHeadDim + 1] = stat_s[tid][1];
+  }
+  if (!merge_here) return;      // attention_merge_kernel, the next launch on the stream, merges the splits
+  // ---- publish; the CTA that arrives last for this kv head merges ----
+  // The barrier makes every thread's stores visible to thread 0, whose device-scope fence orders them
+  // before its arrival (the grid-synchronisation idiom); the last arriver fences again before reading.
+  __syncthreads();
+  if (tid == 0) {
+    __threadfence();
+    const unsigned before = atomicAdd(&g_attention_arrivals[arrival_slot], 1u);
+    last_s = before == unsigned(live - 1);
+    if (last_s) {
+      g_attention_arrivals[arrival_slot] = 0;      // every CTA of this launch has arrived: ready for the next launch
+      __threadfence();
+    }
+  }
+  __syncthreads();
+  if (!last_s) return;
+  // merge: warps 0..GROUP-1 turn the (max, sum) records of their head into weights (each record is read
+  // once, eight per lane at most); then all warps accumulate weighted outputs over interleaved splits
+  // and the CTA adds the eight partial sums
+  if (warp < GROUP) {
+    const float *base = partial + size_t(kvh * GROUP + warp) * split_capacity * kStepRow;
+    constexpr int kPerLane = kStepMaxSplits / 32;
+    float2 rec[kPerLane];
+#pragma unroll
+    for (int i = 0; i < kPerLane; ++i) {
+      const int sp = lane + 32 * i;
+      rec[i] = sp < live ? __ldcg(reinterpret_cast<const float2 *>(base + size_t(sp) * kStepRow + kHeadDim)) : make_float2(-INFINITY, 0.f);
+    }
+    float m = -INFINITY;
+#pragma unroll
+    for (int i = 0; i < kPerLane; ++i) m = fmaxf(m, rec[i].x);
+    m = warp_max(m);
+    float den = 0.f;
+#pragma unroll
+    for (int i = 0; i < kPerLane; ++i) {
+      const int sp = lane + 32 * i;
+      const float w = __expf(rec[i].x - m);        // 0 for the padding records
+      if (sp < live) weight_s[warp][sp] = w;
+      den = fmaf(w, rec[i].y, den);
+    }
+    den = warp_sum(den);
+    if (lane == 0) stat_s[warp][0] = 1.f / den;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int g = 0; g < GROUP; ++g) {
+    const float *base = partial + size_t(kvh * GROUP + g) * split_capacity * kStepRow;
+    float4 num = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+    for (int sp = warp; sp < live; sp += kWarps) {
+      const float w = weight_s[g][sp];
+      const float4 v = __ldcg(reinterpret_cast<const float4 *>(base + size_t(sp) * kStepRow) + lane);
+      num.x = fmaf(w, v.x, num.x);
+      num.y = fmaf(w, v.y, num.y);
+      num.z = fmaf(w, v.z, num.z);
+      num.w = fmaf(w, v.w, num.w);
+    }
+    *reinterpret_cast<float4 *>(&red_s[warp][g][4 * lane]) = num;
+  }
+  __syncthreads();
+  for (int idx = tid; idx < GROUP * kHeadDim; idx += kStepThreads) {
+    const int g = idx / kHeadDim, d = idx % kHeadDim;
+    float sum = 0.f;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) sum += red_s[w][g][d];
+    out[size_t(kvh * GROUP + g) * kHeadDim + d] = __float2bfloat16(sum * stat_s[g][0]);
+  }
+}
+
+// The same step for long caches and batches: the grid is capped at two resident CTAs per SM and every CTA walks several
+// 64-key chunks (chunk = split, split + gridDim.x, ...) with running soft-max statistics.  A ring of chunks in shared memory, filled by cp.async, keeps
+// HBM busy across the chunk's barriers; the first chunks are requested before the wait for the launch in front, like the kernel above.  Products,
+// sums and their order are the kernel's above.
+//
+// DIRECT (a batch with up to eight splits, which are a cluster): the splits meet in distributed shared memory, with the arithmetic of
+// attention_merge_kernel, and that launch falls away.
+//
+// What bounds it: HBM for long batches, else the chain of a chunk (three barriers).  us a call with the merge (a graph over caches larger than L2), 40 query
+// heads on 8 kv heads, rows in registers requested when the ones before were used up / this: 16 sequences of 500 to 1000 positions 31.7 / 26.1, 32 of 2000
+// to 4000 193 / 152; 64 heads on 8, 8 of 1000 to 2000 42.7 / 33.9.  (Tensor cores, a warp to sixteen keys and no barriers, take 14.0, 73 and 15.2, but add in
+// another order: with logits that tie, a decoder then picks other tokens than the one-sequence kernel above.)
+constexpr int kRingStages = 3, kChunkBytes = kStepKeys * kHeadDim * 2 * 2;   // keys, then values
+constexpr size_t kRingSmem = size_t(kRingStages) * kChunkBytes;
+__device__ __forceinline__ void cluster_barrier() { asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ float load_remote(const float *mine, int rank) {   // the float at this place in the shared memory of another CTA of the cluster
+  float v;
+  asm volatile("{\n\t.reg .b32 remote;\n\tmapa.shared::cluster.u32 remote, %1, %2;\n\tld.shared::cluster.f32 %0, [remote];\n\t}"
+               : "=f"(v) : "r"(unsigned(__cvta_generic_to_shared(mine))), "r"(rank) : "memory");
+  return v;
+}
+
+template <int GROUP, bool DIRECT>
+__global__ void __launch_bounds__(kStepThreads, 2) attention_step_loop_kernel(const __nv_bfloat16 *__restrict__ qkv,
+                                                                      const float *__restrict__ cos_table,
+                                                                      const float *__restrict__ sin_table,
+                                                                      const long long *__restrict__ position,
+                                                                      __nv_bfloat16 *k_cache,
+                                                                      __nv_bfloat16 *v_cache, float *__restrict__ partial,
+                                                                      __nv_bfloat16 *__restrict__ out, int q_heads, int kv_heads,
+                                                                      int max_len, int split_capacity, float scale, int merge_here) {
+  extern __shared__ __align__(128) uint8_t ring_smem[];
+  __shared__ __align__(16) float q_s[GROUP][4][8][4];                 // a lane's sixteen dimensions in four loads that meet every bank once
+  constexpr int kHeads = (GROUP + 1) / 2;                             // of a warp in the scores
+  constexpr int kPitch = GROUP <= 4 ? 4 : 8;                          // a key's weights lie together: one or two loads for all heads
+  __shared__ __align__(16) float p_s[kStepKeys][kPitch];
+  __shared__ float stat_s[GROUP][2];
+  __shared__ float rescale_s[GROUP];
+  __shared__ __align__(16) __nv_bfloat16 fresh_s[2][kHeadDim];        // the new key, rotated, and value
+  __shared__ float weight_s[DIRECT ? 1 : GROUP][DIRECT ? 1 : kStepMaxSplits];   // merge weights of the splits
+  __shared__ int last_s;
+  auto red_s = reinterpret_cast<float(*)[GROUP][kHeadDim]>(ring_smem);   // per-warp partial sums, where the chunks were
+  constexpr int kHalf = kHeadDim / 2, kWarps = kStepThreads / 32;
+  const int split = blockIdx.x, kvh = blockIdx.y;
+  // batched step: blockIdx.z is the sequence; every array is [sequences][the one-sequence extent]
+  const int arrival_slot = int(blockIdx.z) * kv_heads + kvh;
+  qkv += size_t(blockIdx.z) * size_t(q_heads + 2 * kv_heads) * kHeadDim;
+  position += blockIdx.z;
+  k_cache += (size_t(blockIdx.z) * kv_heads + kvh) * max_len * kHeadDim;
+  v_cache += (size_t(blockIdx.z) * kv_heads + kvh) * max_len * kHeadDim;
+  partial += size_t(blockIdx.z) * q_heads * split_capacity * kStepRow;
+  out += size_t(blockIdx.z) * q_heads * kHeadDim;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  grid_launch_dependents();
+  const int pos = int(__ldcg(position));                        // attends to keys 0..pos; key pos is new
+  const int chunks = pos / kStepKeys + 1;                       // 64-key chunks that hold at least one key
+  const int splits = gridDim.x;                                 // CTA `split` takes chunks split, split + splits, ...
+  const int live = min(splits, chunks);                         // CTAs with work
+  if (split >= live) {
+    if (DIRECT && splits > 1) {                                 // the others count on every CTA of the cluster
+      cluster_barrier();
+      cluster_barrier();
+    }
+    return;
+  }
+  const size_t q_rows = size_t(q_heads) * kHeadDim, kv_rows = size_t(kv_heads) * kHeadDim;
+  const unsigned ring = unsigned(__cvta_generic_to_shared(ring_smem));
+  // old rows of a chunk: 1024 pieces of 16 bytes of keys, as many of values (rows from pos on are never read from the ring)
+  const auto request = [&](int chunk, int stage) {
+    const int rows = min(kStepKeys, pos - chunk * kStepKeys);
+    const uint4 *keys = reinterpret_cast<const uint4 *>(k_cache + size_t(chunk) * kStepKeys * kHeadDim), *values = reinterpret_cast<const uint4 *>(v_cache + size_t(chunk) * kStepKeys * kHeadDim);
+    const unsigned to = ring + unsigned(stage * kChunkBytes);
+#pragma unroll
+    for (int i = 0; i < kStepKeys * 16 / kStepThreads; ++i) {
+      const int piece = tid + i * kStepThreads;
+      if ((piece >> 4) < rows) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + unsigned(piece * 16)), "l"(keys + piece) : "memory");
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + unsigned(kChunkBytes / 2 + piece * 16)), "l"(values + piece) : "memory");
+      }
+    }
+  };
+#pragma unroll
+  for (int i = 0; i < kRingStages - 1; ++i) {
+    if (split + i * splits < chunks) request(split + i * splits, i);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  grid_dependency_wait();                                       // qkv
+
+  // ---- prologue: rotate-half RoPE of q (and of the new key by its owner) ----
+  for (int idx = tid; idx < GROUP * kHalf; idx += kStepThreads) {
+    const int g = idx / kHalf, i = idx % kHalf;
+    const float c = cos_table[size_t(pos) * kHalf + i], sn = sin_table[size_t(pos) * kHalf + i];
+    const __nv_bfloat16 *vec = qkv + size_t(kvh * GROUP + g) * kHeadDim;
+    const float x1 = __bfloat162float(__ldcg(vec + i)), x2 = __bfloat162float(__ldcg(vec + i + kHalf));
+    q_s[g][(i >> 2) & 1][i >> 3][i & 3] = __bfloat162float(__float2bfloat16(x1 * c - x2 * sn)) * scale;
+    q_s[g][2 + ((i >> 2) & 1)][i >> 3][i & 3] = __bfloat162float(__float2bfloat16(x2 * c + x1 * sn)) * scale;
+  }
+  if (split == (chunks - 1) % splits) {          // the CTA whose last chunk holds the new position
+    if (tid < kHalf) {
+      const int i = tid;
+      const float c = cos_table[size_t(pos) * kHalf + i], sn = sin_table[size_t(pos) * kHalf + i];
+      const __nv_bfloat16 *vec = qkv + q_rows + size_t(kvh) * kHeadDim;
+      const float x1 = __bfloat162float(__ldcg(vec + i)), x2 = __bfloat162float(__ldcg(vec + i + kHalf));
+      __nv_bfloat16 *dst = k_cache + size_t(pos) * kHeadDim;
+      dst[i] = fresh_s[0][i] = __float2bfloat16(x1 * c - x2 * sn);
+      dst[i + kHalf] = fresh_s[0][i + kHalf] = __float2bfloat16(x2 * c + x1 * sn);
+    } else if (tid < 2 * kHalf) {
+      const int i = tid - kHalf;
+      const __nv_bfloat162 pair = __ldcg(reinterpret_cast<const __nv_bfloat162 *>(qkv + q_rows + kv_rows + size_t(kvh) * kHeadDim) + i);
+      reinterpret_cast<__nv_bfloat162 *>(v_cache + size_t(pos) * kHeadDim)[i] = pair;
+      reinterpret_cast<__nv_bfloat162 *>(fresh_s[1])[i] = pair;
+    }
+  }
+
+  // keys: lane (r = lane >> 3, j = lane & 7) reads dimensions 8j..8j+7 and 64+8j..64+8j+7 of keys
+  // (warp & 3)*16 + batch*4 + r for half of the heads (a warp that had eight keys and all heads read q twice as often: shared memory
+  // was what the scores waited for); values: lane reads dimensions 4*lane..4*lane+3 of key warp*8 + i
+  const int r = lane >> 3, j = lane & 7;
+  float acc[GROUP][4];
+#pragma unroll
+  for (int g = 0; g < GROUP; ++g) acc[g][0] = acc[g][1] = acc[g][2] = acc[g][3] = 0.f;
+  float run_max = -INFINITY, run_sum = 0.f;                     // kept by warp g for head g
+  int stage = 0;
+  for (int chunk = split; chunk < chunks; chunk += splits) {
+  const int count = min(kStepKeys, pos + 1 - chunk * kStepKeys);   // the last of them is the new one when count is not 64, and may be when it is
+  const int fresh = pos - chunk * kStepKeys;                    // its place in the chunk (64 or more: not here)
+  asm volatile("cp.async.wait_group %0;" ::"n"(kRingStages - 2) : "memory");
+  __syncthreads();                                              // the chunk is there, and the stage of the one before is free
+  {
+    const int ahead = chunk + (kRingStages - 1) * splits;
+    if (ahead < chunks) request(ahead, stage == 0 ? kRingStages - 1 : stage - 1);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  const uint8_t *const rows = ring_smem + stage * kChunkBytes;
+  stage = stage + 1 == kRingStages ? 0 : stage + 1;
+  // ---- scores ----
+  {
+    float k[4][16];
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      const int key = (warp & 3) * 16 + b * 4 + r;
+      const uint4 *row = key == fresh ? reinterpret_cast<const uint4 *>(fresh_s[0]) : reinterpret_cast<const uint4 *>(rows + key * kHeadDim * 2);
+      unpack_bf16x8(row[j], *reinterpret_cast<float(*)[8]>(&k[b][0]));
+      unpack_bf16x8(row[8 + j], *reinterpret_cast<float(*)[8]>(&k[b][8]));
+    }
+    // The eight lanes of a key add their parts with partners 1, 2 and 4 lanes away.  Four keys go together: a lane hands over half of the
+    // keys at each step, so that four sums take four exchanges instead of twelve.
+#pragma unroll
+    for (int i = 0; i < kHeads; ++i) {
+      const int g = (warp >> 2) * kHeads + i;
+      if (g < GROUP) {                                           // (uniform in the warp)
+        float q[16], dot[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) *reinterpret_cast<float4 *>(&q[4 * e]) = *reinterpret_cast<const float4 *>(&q_s[g][e][j][0]);
+#pragma unroll
+        for (int e = 0; e < 16; ++e)
+#pragma unroll
+          for (int b = 0; b < 4; ++b) dot[b] = fmaf(k[b][e], q[e], dot[b]);
+        const bool odd = j & 1, upper = j & 2;                   // this lane's keys after the exchanges: b = odd + 2 * upper
+        const float keep0 = odd ? dot[1] : dot[0], keep1 = odd ? dot[3] : dot[2], give0 = odd ? dot[0] : dot[1], give1 = odd ? dot[2] : dot[3];
+        const float sum0 = keep0 + __shfl_xor_sync(0xffffffffu, give0, 1), sum1 = keep1 + __shfl_xor_sync(0xffffffffu, give1, 1);
+        float sum = (upper ? sum1 : sum0) + __shfl_xor_sync(0xffffffffu, upper ? sum0 : sum1, 2);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 4);
+        const int key = (warp & 3) * 16 + (odd ? 4 : 0) + (upper ? 8 : 0) + r;
+        if (j < 4) p_s[key][g] = key < count ? sum : -INFINITY;
+      }
+    }
+  }
+  __syncthreads();
+  // ---- per head: max and exp-sum over the CTA's keys (warp g handles head g; GROUP <= 8 warps) ----
+  if (warp < GROUP) {
+    const float a = p_s[lane][warp], b = p_s[lane + 32][warp];
+    const float m = fmaxf(run_max, warp_max(fmaxf(a, b)));     // finite: every chunk of the walk holds a key
+    const float ea = __expf(a - m), eb = __expf(b - m);
+    p_s[lane][warp] = ea;
+    p_s[lane + 32][warp] = eb;
     const float factor = __expf(run_max - m);                   // 0 on the first chunk
     run_sum = fmaf(run_sum, factor, warp_sum(ea + eb));
     run_max = m;
@@ -954,11 +1236,17 @@ __global__ void __launch_bounds__(kStepThreads, 2) attention_step_loop_kernel(co
     }
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const float v0 = __uint_as_float(val_raw[i].x << 16), v1 = __uint_as_float(val_raw[i].x & 0xffff0000u);
-      const float v2 = __uint_as_float(val_raw[i].y << 16), v3 = __uint_as_float(val_raw[i].y & 0xffff0000u);
+      const int key = warp * 8 + i;                             // (uniform in the warp)
+      const uint8_t *row = key == fresh ? reinterpret_cast<const uint8_t *>(fresh_s[1]) : rows + kChunkBytes / 2 + key * kHeadDim * 2;
+      const uint2 raw = key < count ? reinterpret_cast<const uint2 *>(row)[lane] : make_uint2(0, 0);
+      const float v0 = __uint_as_float(raw.x << 16), v1 = __uint_as_float(raw.x & 0xffff0000u);
+      const float v2 = __uint_as_float(raw.y << 16), v3 = __uint_as_float(raw.y & 0xffff0000u);
+      float p[kPitch];
+#pragma unroll
+      for (int g = 0; g < kPitch; g += 4) *reinterpret_cast<float4 *>(&p[g]) = *reinterpret_cast<const float4 *>(&p_s[key][g]);
 #pragma unroll
       for (int g = 0; g < GROUP; ++g) {
-        const float pw = p_s[g][warp * 8 + i];
+        const float pw = p[g];
         acc[g][0] = fmaf(pw, v0, acc[g][0]);
         acc[g][1] = fmaf(pw, v1, acc[g][1]);
         acc[g][2] = fmaf(pw, v2, acc[g][2]);
@@ -966,11 +1254,9 @@ __global__ void __launch_bounds__(kStepThreads, 2) attention_step_loop_kernel(co
       }
     }
   }
-  if (more) {
-    request_values(chunk + splits);
-    __syncthreads();                                            // p_s and rescale_s are rewritten by the next chunk
-  }
   }   // chunk loop
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();                                              // the ring makes room for the sums
 #pragma unroll
   for (int g = 0; g < GROUP; ++g)
     *reinterpret_cast<float4 *>(&red_s[warp][g][4 * lane]) = make_float4(acc[g][0], acc[g][1], acc[g][2], acc[g][3]);
@@ -980,13 +1266,48 @@ __global__ void __launch_bounds__(kStepThreads, 2) attention_step_loop_kernel(co
     float sum = 0.f;
 #pragma unroll
     for (int w = 0; w < kWarps; ++w) sum += red_s[w][g][d];
-    partial[(size_t(kvh * GROUP + g) * split_capacity + split) * kStepRow + d] = sum;
+    if (DIRECT) red_s[0][g][d] = sum;            // (this thread alone reads and writes the column)
+    else partial[(size_t(kvh * GROUP + g) * split_capacity + split) * kStepRow + d] = sum;
+  }
+  if (DIRECT) {
+    // the merge of attention_merge_kernel for up to eight splits, sum for sum: its four thread groups take splits part and part + 4, its warp adds
+    // the weights' sums with the partner 4, 2 and 1 lanes away.  CTA `split` merges heads split, split + live, ...
+    if (splits > 1) cluster_barrier();
+    else __syncthreads();
+    for (int idx = tid; idx < GROUP * kHeadDim; idx += kStepThreads) {
+      const int g = idx / kHeadDim, d = idx % kHeadDim;
+      if (g % live != split) continue;
+      float top[8], weight[8], part[8], m = -INFINITY;
+#pragma unroll
+      for (int sp = 0; sp < 8; ++sp) {
+        top[sp] = sp < live ? (splits > 1 ? load_remote(&stat_s[g][0], sp) : stat_s[g][0]) : -INFINITY;
+        m = fmaxf(m, top[sp]);
+      }
+#pragma unroll
+      for (int sp = 0; sp < 8; ++sp) {
+        weight[sp] = __expf(top[sp] - m);
+        part[sp] = fmaf(weight[sp], sp < live ? (splits > 1 ? load_remote(&stat_s[g][1], sp) : stat_s[g][1]) : 0.f, 0.f);
+      }
+      const float den = ((part[0] + part[4]) + (part[2] + part[6])) + ((part[1] + part[5]) + (part[3] + part[7]));
+      float sum[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        sum[q] = 0.f;
+#pragma unroll
+        for (int sp = q; sp < 8; sp += 4)
+          if (sp < live) sum[q] = fmaf(weight[sp], splits > 1 ? load_remote(&red_s[0][g][d], sp) : red_s[0][g][d], sum[q]);
+      }
+      out[size_t(kvh * GROUP + g) * kHeadDim + d] = __float2bfloat16((((sum[0] + sum[1]) + sum[2]) + sum[3]) * (1.f / den));
+    }
+    if (splits > 1) cluster_barrier();           // no CTA leaves while another reads its sums
+    return;
   }
   if (tid < GROUP) {
     float *rec = partial + (size_t(kvh * GROUP + tid) * split_capacity + split) * kStepRow;
     rec[kHeadDim] = stat_s[tid][0];
     rec[kHeadDim + 1] = stat_s[tid][1];
   }
+  if (!merge_here) return;      // attention_merge_kernel, the next launch on the stream, merges the splits
   // ---- publish; the CTA that arrives last for this kv head merges ----
   // The barrier makes every thread's stores visible to thread 0, whose device-scope fence orders them
   // before its arrival (the grid-synchronisation idiom); the last arriver fences again before reading.
@@ -1182,316 +1503,6 @@ __global__ void __launch_bounds__(kHeadDim * kMergeParts) attention_merge_kernel
   }
 }
 
-// ---------------------------------------------------------------------------------------------------------------------
-// Attention of one new token a sequence, a warp to a tile of sixteen keys.
-//
-// blockIdx = (split, kv head, sequence); CTA `split` takes the 64-key chunks split, split + gridDim.x, ..., each of its four warps sixteen
-// keys of every chunk, with running soft-max statistics of its own.  Both products run on the tensor cores (mma.sync m16n8k16, up to eight query
-// heads of the kv head as rows), and a warp meets no barrier before the end, where the four warps are merged.
-//
-//   tiles    every warp has a ring of three in shared memory, filled by cp.async: two CTAs an SM keep 190 KB in flight without a register.
-//   scores   a lane (g, t) reads dimensions 32 i + 8 t .. + 7 of keys g and g + 8: eight consecutive ones are its elements of two MMA steps (a
-//            dot product does not mind the order).  q and the new key are rotated in the same arrangement, both halves of a pair in one lane.
-//   values   a lane reads dimensions 8 g .. + 7 and 64 + 8 g .. + 7 of keys 2 t, 2 t + 1, 2 t + 8, 2 t + 9 and packs neighbouring keys; column n
-//            of MMA j is dimension 8 n + j.
-//   weights  stay fp32: a weight is the exact sum of three bf16 parts; the first two are rows g and g + 8 of one MMA, the third its own.
-//   splits   of a batch (eight at most) are a cluster that adds its sums in order; CLUSTER false: attention_merge_kernel adds them.
-//
-// Old cache rows of the first tiles are requested before the wait for the launch in front: earlier steps wrote them, or rope_append_prompt_kernel, which
-// lets nothing start before its rows are stored.  Only qkv itself is new.
-//
-// What bounds it: HBM for long batches, latencies otherwise.  us a call (a graph over caches larger than L2), one product a lane and three
-// barriers a chunk, with a merge behind / this kernel, 40 query heads on 8 kv heads: 16 sequences of 500 to 1000 positions 31.7 / 14.0
-// (fragments loaded from global memory and merged behind: 19.7; the same from the ring: 17.0), 32 of 2000 to 4000 193 / 73 (6.1 TB/s), one of 2080
-// 7.8 / 7.6; 16 heads on 2, one of 1500 7.0 / 6.2.
-// ---------------------------------------------------------------------------------------------------------------------
-constexpr int kTileWarps = 4, kTileThreads = kTileWarps * 32, kTileCtas = 2;   // CTAs of an SM, by registers and shared memory
-constexpr int kTileStages = 3, kTileBytes = 8192;
-constexpr size_t kTileSmem = size_t(kTileWarps) * kTileStages * kTileBytes;
-static_assert(kTileSmem >= sizeof(float) * kTileWarps * kMaxGroup * (kHeadDim + 4), "the sums fit where the tiles were");
-__device__ __forceinline__ void mma_bf16(float (&c)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1) {
-  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-// dimensions 32 i + 8 t .. + 7 (i = 0..3) of a head, rotated and rounded to bf16: i and i + 2 are the halves of its pairs
-__device__ __forceinline__ void rotate_head(uint4 (&x)[4], const float *__restrict__ cos_row, const float *__restrict__ sin_row, int t) {
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    float lo[8], hi[8];
-    unpack_bf16x8(x[i], lo);
-    unpack_bf16x8(x[i + 2], hi);
-    unsigned a[4], b[4];
-#pragma unroll
-    for (int e = 0; e < 8; e += 2) {
-      const float2 c = *reinterpret_cast<const float2 *>(cos_row + 32 * i + 8 * t + e), sn = *reinterpret_cast<const float2 *>(sin_row + 32 * i + 8 * t + e);
-      const __nv_bfloat162 first = __floats2bfloat162_rn(lo[e] * c.x - hi[e] * sn.x, lo[e + 1] * c.y - hi[e + 1] * sn.y);
-      const __nv_bfloat162 second = __floats2bfloat162_rn(hi[e] * c.x + lo[e] * sn.x, hi[e + 1] * c.y + lo[e + 1] * sn.y);
-      a[e / 2] = *reinterpret_cast<const unsigned *>(&first);
-      b[e / 2] = *reinterpret_cast<const unsigned *>(&second);
-    }
-    x[i] = make_uint4(a[0], a[1], a[2], a[3]);
-    x[i + 2] = make_uint4(b[0], b[1], b[2], b[3]);
-  }
-}
-__device__ __forceinline__ void cluster_barrier() { asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-__device__ __forceinline__ float load_remote(unsigned addr, int rank) {   // this shared-memory address of another CTA of the cluster
-  float v;
-  asm volatile("{\n\t.reg .b32 remote;\n\tmapa.shared::cluster.u32 remote, %1, %2;\n\tld.shared::cluster.f32 %0, [remote];\n\t}" : "=f"(v) : "r"(addr), "r"(rank) : "memory");
-  return v;
-}
-__device__ __forceinline__ unsigned upper_halves(float a, float b) { return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632); }
-__device__ __forceinline__ float below_upper_half(float v) { return v - __uint_as_float(__float_as_uint(v) & 0xffff0000u); }   // exact
-
-template <bool CLUSTER>
-__global__ void __launch_bounds__(kTileThreads, kTileCtas) attention_tile_kernel(const __nv_bfloat16 *__restrict__ qkv, const float *__restrict__ cos_table,
-                                                                                 const float *__restrict__ sin_table, const long long *__restrict__ position,
-                                                                                 __nv_bfloat16 *k_cache, __nv_bfloat16 *v_cache, float *__restrict__ partial,
-                                                                                 __nv_bfloat16 *__restrict__ out, int q_heads, int kv_heads, int group,
-                                                                                 int max_len, int split_capacity, float scale) {
-  extern __shared__ __align__(128) uint8_t tile_smem[];          // a ring of tiles for every warp; sums at the end
-  auto sum_s = reinterpret_cast<float(*)[kMaxGroup][kHeadDim + 4]>(tile_smem);
-  __shared__ float stat_s[kTileWarps][kMaxGroup][2];
-  __shared__ uint4 fresh_s[2][kHeadDim / 8];                     // the new key, rotated, and value
-  const int split = blockIdx.x, kvh = blockIdx.y;
-  qkv += size_t(blockIdx.z) * size_t(q_heads + 2 * kv_heads) * kHeadDim;
-  k_cache += (size_t(blockIdx.z) * kv_heads + kvh) * max_len * kHeadDim;
-  v_cache += (size_t(blockIdx.z) * kv_heads + kvh) * max_len * kHeadDim;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
-  grid_launch_dependents();
-  const int pos = int(__ldcg(position + blockIdx.z));           // attends to keys 0..pos; key pos is new
-  const int chunks = pos / kStepKeys + 1, splits = gridDim.x;
-  if (split >= chunks) {
-    if (CLUSTER) {                                               // the others count on every CTA of the cluster
-      cluster_barrier();
-      cluster_barrier();
-    }
-    return;
-  }
-
-  // a tile in shared memory: sixteen key rows, then sixteen value rows, 256 bytes each; 16-byte piece c of a row lies at c ^ turn(row), which
-  // spreads both the keys' and the values' fragment loads over all banks
-  const auto turn = [](int row) { return (row & 6) ^ ((row & 1) << 2); };
-  const unsigned ring = unsigned(__cvta_generic_to_shared(tile_smem)) + unsigned(warp * kTileStages * kTileBytes);
-  const int step = splits * kStepKeys;
-  const auto request = [&](int base, int stage) {
-    if (base < pos) {
-      const unsigned to = ring + unsigned(stage * kTileBytes);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int row = 2 * i + (lane >> 4), c = lane & 15;
-        const bool old_row = base + row < pos;                   // (others become zeros)
-        const size_t at = old_row ? size_t(base + row) * kHeadDim + c * 8 : 0;
-        const unsigned dst = to + unsigned(row * 256 + (c ^ turn(row)) * 16);
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(k_cache + at), "r"(old_row ? 16 : 0) : "memory");
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + 4096), "l"(v_cache + at), "r"(old_row ? 16 : 0) : "memory");
-      }
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  int base = split * kStepKeys + warp * 16;
-#pragma unroll
-  for (int i = 0; i < kTileStages; ++i) request(base + i * step, i);
-  grid_dependency_wait();                                        // qkv
-
-  const float *cos_row = cos_table + size_t(pos) * (kHeadDim / 2), *sin_row = sin_table + size_t(pos) * (kHeadDim / 2);
-  uint4 q[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-    q[i] = g < group ? __ldcg(reinterpret_cast<const uint4 *>(qkv + size_t(kvh * group + g) * kHeadDim) + 4 * i + t) : make_uint4(0, 0, 0, 0);
-  rotate_head(q, cos_row, sin_row, t);
-  // the warp whose tile holds the new row takes it from qkv to the caches, and keeps a copy
-  if (split == (chunks - 1) % splits && warp == (pos % kStepKeys) / 16) {
-    uint4 fresh[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) fresh[i] = __ldcg(reinterpret_cast<const uint4 *>(qkv + size_t(q_heads + kvh) * kHeadDim) + 4 * i + t);
-    rotate_head(fresh, cos_row, sin_row, t);
-    if (g == 0) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        fresh_s[0][4 * i + t] = fresh[i];
-        reinterpret_cast<uint4 *>(k_cache + size_t(pos) * kHeadDim)[4 * i + t] = fresh[i];
-      }
-    } else if (g < 5) {                                          // lanes 4..19: the value row
-      const uint4 row = __ldcg(reinterpret_cast<const uint4 *>(qkv + size_t(q_heads + kv_heads + kvh) * kHeadDim) + lane - 4);
-      fresh_s[1][lane - 4] = row;
-      reinterpret_cast<uint4 *>(v_cache + size_t(pos) * kHeadDim)[lane - 4] = row;
-    }
-    __syncwarp();
-  }
-
-  float acc[2][8][4];
-#pragma unroll
-  for (int h = 0; h < 2; ++h)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc[h][j][0] = acc[h][j][1] = acc[h][j][2] = acc[h][j][3] = 0.f;
-  float run_max = -INFINITY, run_sum = 0.f;
-  int stage = 0;
-  for (; base <= pos; base += step) {                            // (a tile with no key up to pos is the warp's last)
-    asm volatile("cp.async.wait_group %0;" ::"n"(kTileStages - 1) : "memory");
-    __syncwarp();
-    const unsigned tile = ring + unsigned(stage * kTileBytes);
-    const int at = pos - base;
-    if (at < 16) {                                               // the new row is one of these
-      const uint4 piece = fresh_s[lane >> 4][lane & 15];
-      asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(tile + unsigned((lane >> 4) * 4096 + at * 256 + ((lane & 15) ^ turn(at)) * 16)),
-                   "r"(piece.x), "r"(piece.y), "r"(piece.z), "r"(piece.w) : "memory");
-      if (base >= pos) {                                         // (it is the first, and nothing was fetched: the rows behind it count as zeros)
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int row = 2 * i + (lane >> 4);
-          const unsigned dst = tile + unsigned(row * 256 + (lane & 15) * 16);
-          if (row != at) {
-            asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(dst), "r"(0) : "memory");
-            asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(dst + 4096), "r"(0) : "memory");
-          }
-        }
-      }
-      __syncwarp();
-    }
-    // ---- scores: rows are heads, columns keys ----
-    float s[2][4];
-#pragma unroll
-    for (int n = 0; n < 2; ++n) {
-      s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const uint4 key = lds128(tile + unsigned((8 * n + g) * 256 + ((4 * i + t) ^ turn(g)) * 16));
-        mma_bf16(s[n], q[i].x, 0, q[i].y, 0, key.x, key.y);
-        mma_bf16(s[n], q[i].z, 0, q[i].w, 0, key.z, key.w);
-      }
-    }
-    float p[4], top = run_max;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int column = 8 * (e >> 1) + 2 * t + (e & 1);
-      p[e] = column <= at ? s[e >> 1][e & 1] * scale : -INFINITY;
-      top = fmaxf(top, p[e]);
-    }
-    top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
-    top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));      // finite: key `base` exists
-    if (__any_sync(0xffffffffu, top > run_max)) {
-      const float factor = __expf(run_max - top);                // 0 on the first tile
-      run_sum *= factor;
-      run_max = top;
-#pragma unroll
-      for (int h = 0; h < 2; ++h)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          acc[h][j][0] *= factor;
-          acc[h][j][1] *= factor;
-          acc[h][j][2] *= factor;
-          acc[h][j][3] *= factor;
-        }
-    }
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      p[e] = __expf(p[e] - top);
-      run_sum += p[e];
-    }
-    // ---- values: weights in three exact parts ----
-    float rest[4], last[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      rest[e] = below_upper_half(p[e]);
-      last[e] = below_upper_half(rest[e]);
-    }
-    const unsigned a0 = upper_halves(p[0], p[1]), a2 = upper_halves(p[2], p[3]), a1 = upper_halves(rest[0], rest[1]), a3 = upper_halves(rest[2], rest[3]);
-    const unsigned c0 = upper_halves(last[0], last[1]), c2 = upper_halves(last[2], last[3]);
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      unsigned v0[4], v1[4], v2[4], v3[4];
-      const auto value = [&](int r, unsigned (&v)[4]) {
-        const int row = 2 * t + (r & 1) + 8 * (r >> 1);
-        const uint4 piece = lds128(tile + unsigned(4096 + row * 256 + ((g + 8 * h) ^ turn(row)) * 16));
-        v[0] = piece.x;
-        v[1] = piece.y;
-        v[2] = piece.z;
-        v[3] = piece.w;
-      };
-      value(0, v0);
-      value(1, v1);
-      value(2, v2);
-      value(3, v3);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const unsigned order = j & 1 ? 0x7632 : 0x5410, b0 = __byte_perm(v0[j / 2], v1[j / 2], order), b1 = __byte_perm(v2[j / 2], v3[j / 2], order);
-        mma_bf16(acc[h][j], a0, a1, a2, a3, b0, b1);
-        mma_bf16(acc[h][j], c0, 0, c2, 0, b0, b1);
-      }
-    }
-    __syncwarp();                                                // all lanes have read the tile
-    request(base + kTileStages * step, stage);
-    stage = stage + 1 == kTileStages ? 0 : stage + 1;
-  }
-  asm volatile("cp.async.wait_all;" ::: "memory");
-  __syncthreads();                                               // the rings make room for the sums
-  run_sum += __shfl_xor_sync(0xffffffffu, run_sum, 1);
-  run_sum += __shfl_xor_sync(0xffffffffu, run_sum, 2);
-
-  // ---- the four warps: lane (g, t) holds dimensions 64 h + 16 t + 0..15 of head g ----
-  if (t == 0) {
-    stat_s[warp][g][0] = run_max;
-    stat_s[warp][g][1] = run_sum;
-  }
-#pragma unroll
-  for (int h = 0; h < 2; ++h)
-#pragma unroll
-    for (int c = 0; c < 2; ++c)
-#pragma unroll
-      for (int j = 0; j < 8; j += 4)
-        *reinterpret_cast<float4 *>(&sum_s[warp][g][64 * h + 16 * t + 8 * c + j]) =
-            make_float4(acc[h][j][c] + acc[h][j][c + 2], acc[h][j + 1][c] + acc[h][j + 1][c + 2], acc[h][j + 2][c] + acc[h][j + 2][c + 2],
-                        acc[h][j + 3][c] + acc[h][j + 3][c + 2]);
-  __syncthreads();
-  static_assert(kTileThreads == kHeadDim, "a thread a dimension");
-  for (int head = 0; head < group; ++head) {
-    float top = stat_s[0][head][0];                              // finite: the first key of a live chunk is warp 0's
-#pragma unroll
-    for (int w = 1; w < kTileWarps; ++w) top = fmaxf(top, stat_s[w][head][0]);
-    float total = 0.f, sum = 0.f;
-#pragma unroll
-    for (int w = 0; w < kTileWarps; ++w) {
-      const float factor = __expf(stat_s[w][head][0] - top);     // 0 for a warp without keys
-      total = fmaf(factor, stat_s[w][head][1], total);
-      sum = fmaf(factor, sum_s[w][head][threadIdx.x], sum);
-    }
-    if (CLUSTER) {
-      // (every thread rewrites what it alone has read of this head; the statistics go behind the dimensions)
-      sum_s[0][head][threadIdx.x] = sum;
-      if (threadIdx.x == 0) {
-        sum_s[0][head][kHeadDim] = top;
-        sum_s[0][head][kHeadDim + 1] = total;
-      }
-    } else if (splits == 1) {
-      out[(size_t(blockIdx.z) * q_heads + kvh * group + head) * kHeadDim + threadIdx.x] = __float2bfloat16(sum / total);
-    } else {
-      float *rec = partial + ((size_t(blockIdx.z) * q_heads + kvh * group + head) * split_capacity + split) * kStepRow;
-      rec[threadIdx.x] = sum;
-      if (threadIdx.x == 0) {
-        rec[kHeadDim] = top;
-        rec[kHeadDim + 1] = total;
-      }
-    }
-  }
-  if (!CLUSTER) return;
-  // ---- the splits, which are the cluster: CTA `split` merges heads split, split + live, ... in the order of the splits ----
-  cluster_barrier();
-  const int live = min(splits, chunks);
-  for (int head = split; head < group; head += live) {
-    const unsigned mine = unsigned(__cvta_generic_to_shared(&sum_s[0][head][0]));
-    float top = -INFINITY;
-    for (int r = 0; r < live; ++r) top = fmaxf(top, load_remote(mine + kHeadDim * 4, r));
-    float total = 0.f, sum = 0.f;
-    for (int r = 0; r < live; ++r) {
-      const float factor = __expf(load_remote(mine + kHeadDim * 4, r) - top);
-      total = fmaf(factor, load_remote(mine + kHeadDim * 4 + 4, r), total);
-      sum = fmaf(factor, load_remote(mine + threadIdx.x * 4, r), sum);
-    }
-    out[(size_t(blockIdx.z) * q_heads + kvh * group + head) * kHeadDim + threadIdx.x] = __float2bfloat16(sum / total);
-  }
-  cluster_barrier();                                             // no CTA leaves while another reads its sums
-}
-
 // TEXELATOR_B200_ATTENTION_MERGE=inline keeps the merge inside the step kernel (one launch per step instead of
 // two; 27B-class decode measured 193.0 tok/s that way against 198.7 with the separate merge)
 static bool merge_inline() {
@@ -1502,45 +1513,33 @@ static bool merge_inline() {
   return value;
 }
 
-struct StepCall {
-  const __nv_bfloat16 *qkv;
-  const float *cos_table, *sin_table;
-  const long long *position;
-  __nv_bfloat16 *k_cache, *v_cache;
-  float *scratch;
-  __nv_bfloat16 *out;
-  int sequences, q_heads, kv_heads, max_len;
-  float scale;
-  int device;
-};
-
-template <int GROUP>
-static cudaError_t launch_attention_inline(const StepCall &c, int splits, cudaStream_t s) {
-  return launch_pdl(attention_step_loop_kernel<GROUP>, dim3(splits, c.kv_heads, c.sequences), dim3(kStepThreads), 0, s, c.qkv, c.cos_table, c.sin_table,
-                    c.position, c.k_cache, c.v_cache, c.scratch, c.out, c.q_heads, c.kv_heads, c.max_len, splits, c.scale);
-}
-
-// One 64-key chunk a CTA while all of them are resident at once; beyond that every CTA takes several (fewer records to merge).
-static cudaError_t launch_attention_step(const StepCall &c, int sm_count, cudaStream_t s) {
-  const int chunks_max = (c.max_len + kStepKeys - 1) / kStepKeys;
-  const int splits = std::min(std::min(chunks_max, kStepMaxSplits), std::max(1, kTileCtas * sm_count / (c.kv_heads * c.sequences)));
-  // A batch's splits are few: they are a cluster and need no merge behind them.  One sequence keeps the launch behind its splits, which are many.
-  const bool cluster = c.sequences > 1 && splits > 1 && splits <= 8;
-  const auto kernel = cluster ? attention_tile_kernel<true> : attention_tile_kernel<false>;
-  static std::atomic<unsigned long long> configured[2];         // a bit a device
-  if (c.device >= 64 || !(configured[cluster].load(std::memory_order_relaxed) >> c.device & 1)) {
-    cudaError_t set = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTileSmem));
-    if (set == cudaSuccess) set = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-    if (set != cudaSuccess) return set;
-    if (c.device < 64) configured[cluster].fetch_or(1ull << c.device, std::memory_order_relaxed);
+template <int GROUP, bool LOOP>
+static cudaError_t launch_attention_step(int splits, int kv_heads, int sequences, cudaStream_t s, const __nv_bfloat16 *qkv, const float *cos_table,
+                                         const float *sin_table, const long long *position, __nv_bfloat16 *k_cache,
+                                         __nv_bfloat16 *v_cache, float *scratch, __nv_bfloat16 *out, int q_heads, int max_len, float scale, int device) {
+  const int merge_here = merge_inline() ? 1 : 0;
+  // (one sequence keeps the launch behind its splits: as a dependent it is resident and waiting when the last split ends)
+  const bool direct = LOOP && !merge_here && sequences > 1 && splits <= 8;
+  cudaError_t status;
+  if (LOOP) {
+    const auto kernel = direct ? attention_step_loop_kernel<GROUP, true> : attention_step_loop_kernel<GROUP, false>;
+    static std::atomic<unsigned long long> configured[2];       // a bit a device
+    if (device >= 64 || !(configured[direct].load(std::memory_order_relaxed) >> device & 1)) {
+      status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kRingSmem));
+      if (status == cudaSuccess) status = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+      if (status != cudaSuccess) return status;
+      if (device < 64) configured[direct].fetch_or(1ull << device, std::memory_order_relaxed);
+    }
+    status = launch_pdl_cluster(kernel, direct ? splits : 1, dim3(splits, kv_heads, sequences), dim3(kStepThreads), kRingSmem, s, qkv, cos_table, sin_table,
+                                position, k_cache, v_cache, scratch, out, q_heads, kv_heads, max_len, splits, scale, merge_here);
+  } else {
+    status = launch_pdl(attention_step_kernel<GROUP>, dim3(splits, kv_heads, sequences), dim3(kStepThreads), 0, s, qkv, cos_table, sin_table,
+                        position, k_cache, v_cache, scratch, out, q_heads, kv_heads, max_len, splits, scale, merge_here);
   }
-  const cudaError_t status = launch_pdl_cluster(kernel, cluster ? splits : 1, dim3(splits, c.kv_heads, c.sequences), dim3(kTileThreads), kTileSmem, s, c.qkv, c.cos_table,
-                                                c.sin_table, c.position, c.k_cache, c.v_cache, c.scratch, c.out, c.q_heads, c.kv_heads, c.q_heads / c.kv_heads,
-                                                c.max_len, splits, c.scale);
-  if (status != cudaSuccess || splits == 1 || cluster) return status;
+  if (status != cudaSuccess || merge_here || direct) return status;
   count_launch();
-  return launch_pdl(attention_merge_kernel, dim3(c.q_heads, c.sequences), dim3(kHeadDim * kMergeParts), 0, s, static_cast<const float *>(c.scratch), c.position, c.out,
-                    c.q_heads, splits, splits);
+  return launch_pdl(attention_merge_kernel, dim3(q_heads, sequences), dim3(kHeadDim * kMergeParts), 0, s, static_cast<const float *>(scratch), position, out,
+                    q_heads, splits, LOOP ? splits : kStepMaxSplits);
 }
 
 }  // namespace tx
@@ -1781,25 +1780,32 @@ static int attention_step_any(const void *qkv, const float *cos_table, const flo
     return fail(TX_EUNSUPPORTED, "tx_aux_attention_step supports head_dim 128, up to 128 kv heads, up to 4096 (sequence, kv head) pairs and "
                                  "up to 8 query heads per kv head");
   if (max_len < 1) return fail(TX_EINVAL, "tx_aux_attention_step: max_len must be positive");
+  // one CTA per 64-key chunk while that fits two resident CTAs per SM; longer caches give every CTA several chunks
   int device = 0;
   TX_CUDA(cudaGetDevice(&device));
   Workspace *ws = workspace_for(device);
-  const int sm_count = ws ? ws->sm_count : 128;
+  const int resident = std::max(1, (ws ? 2 * ws->sm_count : 256) / (kv_heads * sequences));
+  const int chunks_max = (max_len + kStepKeys - 1) / kStepKeys;
+  // up to two waves of one-chunk CTAs (most of them idle while the cache is short) run the leaner variant
+  const bool loop = chunks_max > 2 * resident || chunks_max > kStepMaxSplits;
+  const int splits = loop ? std::min(std::min(chunks_max, resident), kStepMaxSplits) : chunks_max;
   auto s = static_cast<cudaStream_t>(stream);
-  const StepCall call{static_cast<const __nv_bfloat16 *>(qkv), cos_table, sin_table, static_cast<const long long *>(position),
-                      static_cast<__nv_bfloat16 *>(k_cache), static_cast<__nv_bfloat16 *>(v_cache), scratch, static_cast<__nv_bfloat16 *>(out),
-                      sequences, q_heads, kv_heads, max_len, scale, device};
+  auto q = static_cast<const __nv_bfloat16 *>(qkv);
+  auto pos = static_cast<const long long *>(position);
+  auto kc = static_cast<__nv_bfloat16 *>(k_cache), vc = static_cast<__nv_bfloat16 *>(v_cache);
+  auto o = static_cast<__nv_bfloat16 *>(out);
   cudaError_t err = cudaSuccess;
-  if (!merge_inline()) {
-    err = launch_attention_step(call, sm_count, s);
-  } else {
-    const int splits = std::min(std::min((max_len + kStepKeys - 1) / kStepKeys, std::max(1, 2 * sm_count / (kv_heads * sequences))), kStepMaxSplits);
-    switch (q_heads / kv_heads) {
-#define TX_STEP_CASE(G) case G: err = launch_attention_inline<G>(call, splits, s); break;
-      TX_STEP_CASE(1) TX_STEP_CASE(2) TX_STEP_CASE(3) TX_STEP_CASE(4) TX_STEP_CASE(5) TX_STEP_CASE(6) TX_STEP_CASE(7) TX_STEP_CASE(8)
+  switch (q_heads / kv_heads) {
+#define TX_STEP_CASE(G)                                                                                                          \
+  case G:                                                                                                                        \
+    err = loop ? launch_attention_step<G, true>(splits, kv_heads, sequences, s, q, cos_table, sin_table, pos, kc, vc, scratch, o, \
+                                                q_heads, max_len, scale, device)                                                  \
+               : launch_attention_step<G, false>(splits, kv_heads, sequences, s, q, cos_table, sin_table, pos, kc, vc, scratch,   \
+                                                 o, q_heads, max_len, scale, device);                                             \
+    break;
+    TX_STEP_CASE(1) TX_STEP_CASE(2) TX_STEP_CASE(3) TX_STEP_CASE(4) TX_STEP_CASE(5) TX_STEP_CASE(6) TX_STEP_CASE(7) TX_STEP_CASE(8)
 #undef TX_STEP_CASE
-      default: return fail(TX_EUNSUPPORTED, "tx_aux_attention_step: unsupported query group");
-    }
+    default: return fail(TX_EUNSUPPORTED, "tx_aux_attention_step: unsupported query group");
   }
   TX_CUDA(err);
   count_launch();
