@@ -101,6 +101,14 @@ int tx_linear(uint64_t handle, const void *x, void *y, int tokens, int dtype, vo
  * stream capture.  Every call on a device uses the same array: calls that overlap on the GPU race. */
 int tx_linear_static_scratch(uint64_t handle, const void *x, void *y, int tokens, int dtype, void *stream);
 
+/* New: a prompt's activations in the form that the tensor-core tiles read (fp16 after an exact power-of-two rescale per token, in the tile's order
+ * of K, and a multiplier per token), written by tx_aux_add_rmsnorm_staged or tx_aux_silu_mul_pairs_staged into a buffer of
+ * tx_staged_prompt_bytes(K, tokens), 16-byte aligned.  tx_linear_staged multiplies it (bf16 in and out); the result is tx_linear's of the rows, bit for
+ * bit.  tx_linear_takes_staged: 1 where tx_linear would serve that many tokens with a tile, else 0. */
+size_t tx_staged_prompt_bytes(int K, int tokens);
+int tx_linear_takes_staged(uint64_t handle, int tokens);
+int tx_linear_staged(uint64_t handle, const void *staged, void *y, int tokens, void *stream);
+
 /* No counterpart in the reference (its decode loop leaves these steps to PyTorch kernels between the
  * linears, texelator/cli.py:189-219).  Decode linear with its neighbours fused into the same launch:
  *   norm_weight != NULL : r = bf16(x + delta) (delta may be NULL), a = bf16(rmsnorm(r, eps) * norm_weight)
@@ -230,6 +238,9 @@ int tx_aux_add_rmsnorm(void *h, const void *delta, const void *weight, void *y, 
  * code 33 in the device status word (tx_kernel_status) and takes row 0. */
 int tx_aux_embed_rmsnorm(const void *table, int64_t vocab, const int64_t *row_tokens, void *h, const void *weight, void *y, int tokens, int hidden,
                          float eps, int device, void *stream);
+/* tx_aux_add_rmsnorm and tx_aux_silu_mul_pairs with the result in staged form (tx_linear_staged) instead of rows */
+int tx_aux_add_rmsnorm_staged(void *h, const void *delta, const void *weight, void *staged, int tokens, int hidden, float eps, void *stream);
+int tx_aux_silu_mul_pairs_staged(const void *gate_up, void *staged, int tokens, int intermediate, int accurate, void *stream);
 /* add_rmsnorm for one token with the extras of tx_linear_single: delta may come as `splits` fp32 partial
  * vectors (partials[s * partial_stride + i], added in split order, rounded to bf16, then added to h), and
  * the normalised row may also (or only: y may be NULL then) be written in staged form to `staged`

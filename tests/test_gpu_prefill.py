@@ -263,3 +263,41 @@ def test_hardware_palettes_and_texture_gate(ext, lut, tmp_path, monkeypatch):
             assert ext.handle_info(h)[5] == 0
     finally:
         ext.free(h)
+
+
+@pytest.mark.parametrize("tokens,k,m", [(16, 256, 200), (17, 1168, 300), (33, 2048, 128), (700, 5120, 640), (1, 144, 64), (40, 16384, 128),
+                                        (303, 2064, 64), (595, 4096, 64), (601, 8192, 64), (593, 8208, 64)])     # two and four rows a CTA
+def test_staged_activations_give_the_linear_of_their_rows(ext, lut, tokens, k, m):
+    """A norm or a SwiGLU that writes the tile's form, then the tile: the bits of the rows' own linear, at edges of 128-column units and 32
+    tokens, whichever tile; and refused where the linear would not take one."""
+    blocks, scales, x = _case(k, m, k, tokens, lut)
+    bias = torch.from_numpy(np.random.default_rng(2).standard_normal(m).astype(np.float32)).bfloat16().cuda()
+    h = _pack(ext, blocks, scales, bias)
+    try:
+        gen = torch.Generator(device="cuda").manual_seed(k)
+        weight, delta = torch.randn(k, device="cuda", generator=gen).bfloat16(), torch.randn(tokens, k, device="cuda", generator=gen).bfloat16()
+        gate_up = (torch.randn(tokens, 2 * k, device="cuda", generator=gen) * 3).bfloat16()
+        x[0] = 0
+        x = x.cuda()
+        ext.set_prefill(h, 1, 1024)
+        staged = ext.staged_buffer(k, tokens, "cuda").fill_(0x7e)
+        y = torch.empty(tokens, m, dtype=torch.bfloat16, device="cuda")
+        for backend in (5, 6, 7, 8, 9):
+            ext.set_prefill_backend(h, backend)
+            assert ext.takes_staged(h, tokens)
+            rows, residual, residual_staged = torch.empty_like(x), x.clone(), x.clone()
+            ext.add_rmsnorm(residual, delta, weight, rows, 1e-6)
+            ext.add_rmsnorm_staged(residual_staged, delta, weight, staged, 1e-6)
+            assert torch.equal(residual, residual_staged)
+            assert torch.equal(ext.linear_staged(h, staged, y), ext.linear(h, rows))
+            for accurate in (False, True):
+                ext.silu_mul_pairs(gate_up, rows, accurate)
+                ext.silu_mul_pairs_staged(gate_up, staged, accurate)
+                assert torch.equal(ext.linear_staged(h, staged, y), ext.linear(h, rows))
+        ext.set_prefill(h, tokens + 1, 1024)
+        assert not ext.takes_staged(h, tokens)
+        with pytest.raises(RuntimeError, match="does not take staged"):
+            ext.linear_staged(h, staged, y)
+        assert ext.kernel_status() == 0
+    finally:
+        ext.free(h)

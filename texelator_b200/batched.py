@@ -59,6 +59,7 @@ class BatchedBC4Decoder(BC4Decoder):
             self.buf_down = torch.zeros(batch, c.hidden, **bf)
             self.attn_scratch = torch.zeros(batch * self.ext.attention_step_scratch_floats(q_heads, max_len),
                                             dtype=torch.float32, device=self.device)
+            self.buf_staged = self.ext.staged_buffer(max(c.hidden, self.i_loc), batch, self.device)
             if self.vocab_parallel:
                 self.best_local = torch.zeros(batch, 2, dtype=torch.float32, device=self.device)
                 self.best_all = torch.zeros(self.world, batch, 2, dtype=torch.float32, device=self.device)
@@ -182,21 +183,34 @@ class BatchedBC4Decoder(BC4Decoder):
         """One token for every sequence, library kernels only (this is what ``capture`` records)."""
         c, ext = self.config, self.ext
         q_heads, kv_heads = c.q_heads // self.world, c.kv_heads // self.world
+        staged = lambda handle: ext.takes_staged(handle, self.batch)     # the tile reads what the kernel in front leaves in its form
         delta = None
         for layer in range(c.layers):
-            if layer == 0:
-                ext.embed_rmsnorm(self.embed, self.tok, self.buf_h, self.norm1[layer], self.buf_x, c.rms_eps)
+            if layer and staged(self.h_qkv[layer]):
+                ext.add_rmsnorm_staged(self.buf_h, delta, self.norm1[layer], self.buf_staged, c.rms_eps)
+                ext.linear_staged(self.h_qkv[layer], self.buf_staged, self.buf_qkv)
             else:
-                ext.add_rmsnorm(self.buf_h, delta, self.norm1[layer], self.buf_x, c.rms_eps)
-            ext.linear_out(self.h_qkv[layer], self.buf_x, self.buf_qkv)
+                if layer == 0:
+                    ext.embed_rmsnorm(self.embed, self.tok, self.buf_h, self.norm1[layer], self.buf_x, c.rms_eps)
+                else:
+                    ext.add_rmsnorm(self.buf_h, delta, self.norm1[layer], self.buf_x, c.rms_eps)
+                ext.linear_out(self.h_qkv[layer], self.buf_x, self.buf_qkv)
             ext.attention_step_batch(self.buf_qkv, self.cos, self.sin, self.pos, self.k_cache[layer], self.v_cache[layer],
                                      self.attn_scratch, self.buf_attn, q_heads, kv_heads, c.head_dim)
             ext.linear_out(self.h_o[layer], self.buf_attn, self.buf_o)
             self._all_reduce(self.buf_o)
-            ext.add_rmsnorm(self.buf_h, self.buf_o, self.norm2[layer], self.buf_x, c.rms_eps)
-            ext.linear_out(self.h_gu[layer], self.buf_x, self.buf_gu)
-            ext.silu_mul_pairs(self.buf_gu, self.buf_act)
-            ext.linear_out(self.h_down[layer], self.buf_act, self.buf_down)
+            if staged(self.h_gu[layer]):
+                ext.add_rmsnorm_staged(self.buf_h, self.buf_o, self.norm2[layer], self.buf_staged, c.rms_eps)
+                ext.linear_staged(self.h_gu[layer], self.buf_staged, self.buf_gu)
+            else:
+                ext.add_rmsnorm(self.buf_h, self.buf_o, self.norm2[layer], self.buf_x, c.rms_eps)
+                ext.linear_out(self.h_gu[layer], self.buf_x, self.buf_gu)
+            if ext.stages_swiglu(self.batch, self.i_loc) and staged(self.h_down[layer]):
+                ext.silu_mul_pairs_staged(self.buf_gu, self.buf_staged)
+                ext.linear_staged(self.h_down[layer], self.buf_staged, self.buf_down)
+            else:
+                ext.silu_mul_pairs(self.buf_gu, self.buf_act)
+                ext.linear_out(self.h_down[layer], self.buf_act, self.buf_down)
             self._all_reduce(self.buf_down)
             delta = self.buf_down
         ext.add_rmsnorm(self.buf_h, delta, self.final_norm, self.last_hidden, c.rms_eps)

@@ -137,6 +137,8 @@ static int pack_common(const uint8_t *blocks, size_t src_pitch_blocks, const flo
 
 using namespace tx;
 
+static constexpr int kStagedPromptTokens = 65536;   // as many as one launch of a tile takes
+
 extern "C" {
 
 const char *tx_last_error(void) { return g_error.c_str(); }
@@ -177,6 +179,38 @@ int tx_pack_encoded_shard(const uint8_t *blocks, size_t nbytes, const float *sca
                      device, out_handle);
 }
 
+// The tile that serves a call, 0: a decode kernel.  texelator_cuda.cu:1341 -- tokens >= threshold takes the prefill side of the dispatcher
+// (ids 0..4 name the reference's fallback kernels; here they leave the choice to the library, and the exact-arithmetic
+// and texture paths keep serving such handles' prompts themselves)
+static int tile_of_call(const Handle *h, int tokens) {
+  if (tokens < h->prefill_threshold) return 0;
+  const int backend = h->prefill_backend >= 5 || h->decode_path != TX_DECODE_ALU_MMA ? h->prefill_backend : prefill_choose_backend(h, tokens);
+  return backend >= 5 && prefill_tile_eligible(h, backend, tokens) ? backend : 0;
+}
+
+size_t tx_staged_prompt_bytes(int K, int tokens) { return K > 0 && tokens > 0 ? staged_prompt_bytes(K, tokens) : 0; }
+
+int tx_linear_takes_staged(uint64_t handle, int tokens) {
+  Handle *h = as_handle(handle);
+  if (!h) return fail(TX_EINVAL, "null Texelator handle");
+  return tokens > 0 && tokens <= kStagedPromptTokens && (!h->bias || h->bias_dtype == TX_DTYPE_BF16) && tile_of_call(h, tokens) ? 1 : 0;
+}
+
+int tx_linear_staged(uint64_t handle, const void *staged, void *y, int tokens, void *stream_ptr) {
+  Handle *h = as_handle(handle);
+  if (!h) return fail(TX_EINVAL, "null Texelator handle");
+  if (!staged || !y || ((reinterpret_cast<uintptr_t>(staged) | reinterpret_cast<uintptr_t>(y)) & 15))
+    return fail(TX_EINVAL, "activation and output pointers must be 16-byte aligned");
+  if (tx_linear_takes_staged(handle, tokens) != 1) return fail(TX_EUNSUPPORTED, "this call does not take staged activations (tx_linear_takes_staged)");
+  int current = 0;
+  TX_CUDA(cudaGetDevice(&current));
+  if (current != h->device) TX_CUDA(cudaSetDevice(h->device));
+  const int rc = launch_prefill_staged(h, tile_of_call(h, tokens), static_cast<const uint8_t *>(staged), static_cast<__nv_bfloat16 *>(y), tokens,
+                                       static_cast<cudaStream_t>(stream_ptr));
+  if (current != h->device) cudaSetDevice(current);
+  return rc;
+}
+
 int tx_linear(uint64_t handle, const void *x, void *y, int tokens, int dtype, void *stream_ptr) {
   Handle *h = as_handle(handle);
   if (!h) return fail(TX_EINVAL, "null Texelator handle");
@@ -196,13 +230,8 @@ int tx_linear(uint64_t handle, const void *x, void *y, int tokens, int dtype, vo
   TX_CUDA(cudaGetDevice(&current));
   if (current != h->device) TX_CUDA(cudaSetDevice(h->device));
   int rc;
-  // texelator_cuda.cu:1341 -- tokens >= threshold takes the prefill side of the dispatcher
-  // (ids 0..4 name the reference's fallback kernels; here they leave the choice to the library, and the exact-arithmetic
-  // and texture paths keep serving such handles' prompts themselves)
-  int backend = 0;
-  if (tokens >= h->prefill_threshold)
-    backend = h->prefill_backend >= 5 || h->decode_path != TX_DECODE_ALU_MMA ? h->prefill_backend : prefill_choose_backend(h, tokens);
-  if (backend >= 5 && prefill_tile_eligible(h, backend, tokens)) {
+  const int backend = tile_of_call(h, tokens);
+  if (backend) {
     rc = launch_prefill_tile(h, backend, xb, yb, tokens, stream, half_io);
   } else if (h->decode_path == TX_DECODE_ALU_EXACT) {
     rc = launch_gemv_exact(h, xb, yb, tokens, stream);

@@ -27,6 +27,54 @@ __device__ __forceinline__ float warp_max(float v) {
 constexpr int kNormThreads = 512;
 constexpr int kNormChunks = 4;            // hidden <= 512 * 8 * 4 = 16384 stays in registers
 
+// A row whose piece threadIdx.x + c * kNormThreads is piece(c) (zeros behind the row) in staged form
+template <typename Piece>
+__device__ __forceinline__ void stage_row(uint8_t *staged, int K, int tokens, int tok, unsigned peak, Piece piece) {
+  float mult, inverse;
+  token_scaling(peak, mult, inverse);
+  const int pieces = (K + 127) / 128 * 16, padded = padded_prompt(tokens);
+#pragma unroll
+  for (int c = 0; c < kNormChunks; ++c) {
+    const int i = threadIdx.x + c * kNormThreads;
+    if (c * kNormThreads < pieces) stage_piece(reinterpret_cast<uint4 *>(staged), padded, tok, i, convert_chunk(piece(c), mult), i < pieces);
+  }
+  if (threadIdx.x == 0) reinterpret_cast<float *>(staged + staged_prompt_multipliers(K, tokens))[tok] = inverse * kNumeratorScale;
+}
+
+// Several rows of a CTA in staged form: they wait in shared memory (rows `row_bytes` apart) and leave with neighbouring lanes on neighbouring
+// tokens, in runs of ROWS * 16 bytes.  us a call with one, two and four rows a CTA: 200 x 2048 4.3, 3.3, 4.1; 700 x 2048 9.8, 5.4, 6.4;
+// 2000 x 2048 25.6, 8.5, 9.2 (the norm alone 2.2, 4.5, 10.1); so two, and one below a CTA an SM.
+__host__ __device__ inline size_t staged_row_bytes(int K) { return size_t(K) * 2 + 16; }   // + 16: rows start on different banks
+template <int ROWS>
+__device__ __forceinline__ void stage_rows(uint8_t *staged, const uint8_t *rows_smem, int K, int tokens, const unsigned (&peaks)[ROWS][kNormThreads / 32]) {
+  const int j = threadIdx.x % ROWS, tok = blockIdx.x * ROWS + j, padded = padded_prompt(tokens), chunks = (K + 127) / 128 * 16;
+  if (tok >= tokens) return;
+  unsigned peak = 0;
+#pragma unroll
+  for (int w = 0; w < kNormThreads / 32; ++w) peak = max(peak, peaks[j][w]);
+  float mult, inverse;
+  token_scaling(peak, mult, inverse);
+  if (threadIdx.x < ROWS) reinterpret_cast<float *>(staged + staged_prompt_multipliers(K, tokens))[tok] = inverse * kNumeratorScale;
+  const uint8_t *row = rows_smem + j * staged_row_bytes(K);
+  uint4 *dst = reinterpret_cast<uint4 *>(staged) + tok;
+#pragma unroll 4
+  for (int chunk = threadIdx.x / ROWS; chunk < chunks; chunk += kNormThreads / ROWS) {
+    // chunk 2j + c of a half unit: columns 16(2c) + 4j .. + 3 and 16(2c + 1) + 4j .. + 3
+    const int column = (chunk >> 3) * 64 + (chunk & 1) * 32 + ((chunk >> 1) & 3) * 4;
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (column < K) {
+      const uint2 low = *reinterpret_cast<const uint2 *>(row + column * 2);
+      v.x = low.x;
+      v.y = low.y;
+    }
+    if (column + 16 < K) {
+      const uint2 high = *reinterpret_cast<const uint2 *>(row + column * 2 + 32);
+      v.z = high.x;
+      v.w = high.y;
+    }
+    dst[size_t(chunk) * padded] = convert_chunk(v, mult);
+  }
+}
 // EMBED: the first norm of a decode step.  A row of h is the embedding of the row's token, fetched here and stored for the residual
 // (a launch of its own before: 16 rows of 5120 14.2 us, of which the wait for one more kernel in the chain is most; one row 2.0).
 struct EmbedRows {
@@ -35,7 +83,8 @@ struct EmbedRows {
   long long vocab;
   int *status;                  // code 33: a token outside the table (row 0 is taken)
 };
-template <bool EMBED>
+// STAGED: y is the staged form of the rows (tx_decode.cuh) that the next linear's tile reads, instead of rows: no staging launch in between.
+template <bool EMBED, bool STAGED>
 __global__ void __launch_bounds__(kNormThreads) add_rmsnorm_kernel(__nv_bfloat16 *__restrict__ h, const __nv_bfloat16 *__restrict__ delta,
                                                                    const __nv_bfloat16 *__restrict__ weight, __nv_bfloat16 *__restrict__ y,
                                                                    int hidden, float eps, const EmbedRows embed) {
@@ -97,11 +146,13 @@ __global__ void __launch_bounds__(kNormThreads) add_rmsnorm_kernel(__nv_bfloat16
   for (int w = 0; w < kNormThreads / 32; ++w) total += partial[w];
   const float inv = rsqrtf(total / float(hidden) + eps);
   uint4 *yr = reinterpret_cast<uint4 *>(y + size_t(row) * hidden);
+  unsigned peak = 0;
 #pragma unroll
   for (int c = 0; c < kNormChunks; ++c) {
     const int i = threadIdx.x + c * kNormThreads;
+    uint4 o = make_uint4(0, 0, 0, 0);
     if (i < chunks) {
-      uint4 v = keep[c], w = gain[c], o;
+      uint4 v = keep[c], w = gain[c];
       const __nv_bfloat162 *pv = reinterpret_cast<const __nv_bfloat162 *>(&v), *pw = reinterpret_cast<const __nv_bfloat162 *>(&w);
       __nv_bfloat162 *po = reinterpret_cast<__nv_bfloat162 *>(&o);
 #pragma unroll
@@ -109,9 +160,102 @@ __global__ void __launch_bounds__(kNormThreads) add_rmsnorm_kernel(__nv_bfloat16
         float2 a = __bfloat1622float2(pv[e]), g = __bfloat1622float2(pw[e]);
         po[e] = __floats2bfloat162_rn(a.x * inv * g.x, a.y * inv * g.y);
       }
-      yr[i] = o;
+      if (!STAGED) yr[i] = o;
+    }
+    if (STAGED) {
+      keep[c] = o;
+      peak = max(peak, chunk_absmax(o));
     }
   }
+  if (STAGED) {
+    __shared__ unsigned peaks[kNormThreads / 32];
+    peak = __reduce_max_sync(0xffffffffu, peak);
+    if ((threadIdx.x & 31) == 0) peaks[threadIdx.x >> 5] = peak;
+    __syncthreads();
+    for (int w = 0; w < kNormThreads / 32; ++w) peak = max(peak, peaks[w]);
+    stage_row(reinterpret_cast<uint8_t *>(y), hidden, gridDim.x, row, peak, [&](int c) { return keep[c]; });
+  }
+}
+
+// add_rmsnorm_kernel<false, true> for ROWS rows a CTA: 512 / ROWS threads a row, each with the pieces of ROWS threads of that kernel, whose order of
+// sums it keeps (a sum for each of those threads, warp by warp, the warps in order).
+template <int ROWS, int CHUNKS>
+__global__ void __launch_bounds__(kNormThreads) add_rmsnorm_rows_staged_kernel(__nv_bfloat16 *__restrict__ h, const __nv_bfloat16 *__restrict__ delta,
+                                                                               const __nv_bfloat16 *__restrict__ weight, uint8_t *__restrict__ staged, int hidden,
+                                                                               int tokens, float eps) {
+  extern __shared__ __align__(16) uint8_t rows_smem[];
+  __shared__ float partial[ROWS][kNormThreads / 32];
+  __shared__ unsigned peaks[ROWS][kNormThreads / 32];
+  constexpr int kPerRow = kNormThreads / ROWS;
+  const int chunks = hidden / 8, j = threadIdx.x / kPerRow, t = threadIdx.x % kPerRow, tok = blockIdx.x * ROWS + j, lane = threadIdx.x & 31;
+  grid_launch_dependents();
+  grid_dependency_wait();
+  const bool live = tok < tokens;
+  uint4 *hr = reinterpret_cast<uint4 *>(h + size_t(live ? tok : 0) * hidden);
+  const uint4 *dr = delta ? reinterpret_cast<const uint4 *>(delta + size_t(live ? tok : 0) * hidden) : nullptr;
+  uint4 keep[ROWS][CHUNKS];
+  float ss[ROWS];
+#pragma unroll
+  for (int v = 0; v < ROWS; ++v) {                       // thread t + v * kPerRow of the other kernel
+    ss[v] = 0.f;
+#pragma unroll
+    for (int c = 0; c < CHUNKS; ++c) {
+      const int i = t + v * kPerRow + c * kNormThreads;
+      if (live && i < chunks) {
+        uint4 x = __ldcg(hr + i);
+        __nv_bfloat162 *px = reinterpret_cast<__nv_bfloat162 *>(&x);
+        if (dr) {
+          const uint4 d = __ldcg(dr + i);
+          const __nv_bfloat162 *pd = reinterpret_cast<const __nv_bfloat162 *>(&d);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float2 a = __bfloat1622float2(px[e]), b = __bfloat1622float2(pd[e]);
+            px[e] = __floats2bfloat162_rn(a.x + b.x, a.y + b.y);
+          }
+          hr[i] = x;
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 a = __bfloat1622float2(px[e]);
+          ss[v] += a.x * a.x + a.y * a.y;
+        }
+        keep[v][c] = x;
+      }
+    }
+    ss[v] = warp_sum(ss[v]);
+    if (lane == 0) partial[j][(t + v * kPerRow) >> 5] = ss[v];
+  }
+  __syncthreads();
+  float total = 0.f;
+#pragma unroll
+  for (int w = 0; w < kNormThreads / 32; ++w) total += partial[j][w];
+  const float inv = rsqrtf(total / float(hidden) + eps);
+  uint4 *row = reinterpret_cast<uint4 *>(rows_smem + j * staged_row_bytes(hidden));
+  const uint4 *wr = reinterpret_cast<const uint4 *>(weight);
+#pragma unroll
+  for (int v = 0; v < ROWS; ++v) {
+    unsigned peak = 0;
+#pragma unroll
+    for (int c = 0; c < CHUNKS; ++c) {
+      const int i = t + v * kPerRow + c * kNormThreads;
+      if (live && i < chunks) {
+        uint4 x = keep[v][c], w = wr[i], o;
+        const __nv_bfloat162 *px = reinterpret_cast<const __nv_bfloat162 *>(&x), *pw = reinterpret_cast<const __nv_bfloat162 *>(&w);
+        __nv_bfloat162 *po = reinterpret_cast<__nv_bfloat162 *>(&o);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 a = __bfloat1622float2(px[e]), g = __bfloat1622float2(pw[e]);
+          po[e] = __floats2bfloat162_rn(a.x * inv * g.x, a.y * inv * g.y);
+        }
+        row[i] = o;
+        peak = max(peak, chunk_absmax(o));
+      }
+    }
+    peak = __reduce_max_sync(0xffffffffu, peak);
+    if (lane == 0) peaks[j][(t + v * kPerRow) >> 5] = peak;
+  }
+  __syncthreads();
+  stage_rows<ROWS>(staged, rows_smem, hidden, tokens, peaks);
 }
 
 // The same step for one token with the two extras of the single-token decode path:
@@ -1397,6 +1541,18 @@ __global__ void __launch_bounds__(256) silu_mul_kernel(const __nv_bfloat16 *__re
 // decode step's kernels take __expf, whose relative error grows with the argument: the prompt's arithmetic is then
 // PyTorch's silu(g.float()) * u.float() to the bit.  Close to memory either way: 700 x 11008 10.7 us against 10.4 (7.1 for
 // the bytes), 2000 x 28672 72.5 against 70.0 (52.6).
+template <bool ACCURATE> __device__ __forceinline__ uint4 silu_mul_chunk(const uint4 gate, const uint4 up) {
+  const __nv_bfloat162 *pg = reinterpret_cast<const __nv_bfloat162 *>(&gate), *pu = reinterpret_cast<const __nv_bfloat162 *>(&up);
+  uint4 result;
+  __nv_bfloat162 *pr = reinterpret_cast<__nv_bfloat162 *>(&result);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const float2 g = __bfloat1622float2(pg[e]), u = __bfloat1622float2(pu[e]);
+    const float ex = ACCURATE ? expf(-g.x) : __expf(-g.x), ey = ACCURATE ? expf(-g.y) : __expf(-g.y);
+    pr[e] = __floats2bfloat162_rn(g.x / (1.f + ex) * u.x, g.y / (1.f + ey) * u.y);
+  }
+  return result;
+}
 template <bool ACCURATE>
 __global__ void __launch_bounds__(256) silu_mul_pairs_kernel(const __nv_bfloat16 *__restrict__ gu, __nv_bfloat16 *__restrict__ out,
                                                              int inter, int tokens) {
@@ -1406,18 +1562,20 @@ __global__ void __launch_bounds__(256) silu_mul_pairs_kernel(const __nv_bfloat16
   for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < size_t(tokens) * chunks; i += size_t(gridDim.x) * blockDim.x) {
     const int t = int(i / chunks), j = int(i % chunks);
     const uint4 *src = reinterpret_cast<const uint4 *>(gu + size_t(t) * 2 * inter + size_t(j) * 16);
-    const uint4 gate = __ldcg(src), up = __ldcg(src + 1);
-    const __nv_bfloat162 *pg = reinterpret_cast<const __nv_bfloat162 *>(&gate), *pu = reinterpret_cast<const __nv_bfloat162 *>(&up);
-    uint4 result;
-    __nv_bfloat162 *pr = reinterpret_cast<__nv_bfloat162 *>(&result);
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float2 g = __bfloat1622float2(pg[e]), u = __bfloat1622float2(pu[e]);
-      const float ex = ACCURATE ? expf(-g.x) : __expf(-g.x), ey = ACCURATE ? expf(-g.y) : __expf(-g.y);
-      pr[e] = __floats2bfloat162_rn(g.x / (1.f + ex) * u.x, g.y / (1.f + ey) * u.y);
-    }
-    *reinterpret_cast<uint4 *>(out + size_t(t) * inter + size_t(j) * 8) = result;
+    *reinterpret_cast<uint4 *>(out + size_t(t) * inter + size_t(j) * 8) = silu_mul_chunk<ACCURATE>(__ldcg(src), __ldcg(src + 1));
   }
+}
+
+// The same for few tokens into the staged form (tx_decode.cuh) that the down projection's tile reads, a cluster a row: 16 x 17408
+// 4.6 us, 1.9 and 9.8 for rows and a staging launch of a CTA a row.
+// With more tokens the two launches are as fast, because here a row's exponentials are a few CTAs' (700 x 11008 10.1 + 4.5 us, 15.4 with a CTA a row).
+template <bool ACCURATE>
+__global__ void __launch_bounds__(kSplitThreads) silu_mul_pairs_staged_kernel(const __nv_bfloat16 *__restrict__ gu, uint8_t *__restrict__ staged, int inter) {
+  grid_launch_dependents();
+  grid_dependency_wait();
+  const uint4 *src = reinterpret_cast<const uint4 *>(gu + size_t(blockIdx.y) * 2 * inter);
+  stage_split_row(reinterpret_cast<uint4 *>(staged), reinterpret_cast<float *>(staged + staged_prompt_multipliers(inter, gridDim.y)), inter, padded_prompt(gridDim.y), false,
+                  [&](int i) { return silu_mul_chunk<ACCURATE>(__ldcg(src + 2 * i), __ldcg(src + 2 * i + 1)); });
 }
 
 // The merge of the splits as a launch of its own: one CTA per query head and sequence, thread d owns output
@@ -1551,9 +1709,32 @@ extern "C" {
 int tx_aux_add_rmsnorm(void *h, const void *delta, const void *weight, void *y, int tokens, int hidden, float eps, void *stream) {
   if (!h || !weight || !y || tokens < 1 || hidden < 8 || hidden % 8 || hidden > kNormThreads * 8 * kNormChunks)
     return fail(TX_EINVAL, "tx_aux_add_rmsnorm: hidden must be a multiple of 8 and at most 16384");
-  TX_CUDA(launch_pdl(add_rmsnorm_kernel<false>, dim3(tokens), dim3(kNormThreads), 0, static_cast<cudaStream_t>(stream),
+  TX_CUDA(launch_pdl(add_rmsnorm_kernel<false, false>, dim3(tokens), dim3(kNormThreads), 0, static_cast<cudaStream_t>(stream),
                      static_cast<__nv_bfloat16 *>(h), static_cast<const __nv_bfloat16 *>(delta),
                      static_cast<const __nv_bfloat16 *>(weight), static_cast<__nv_bfloat16 *>(y), hidden, eps, EmbedRows{}));
+  count_launch();
+  TX_CUDA(cudaGetLastError());
+  return TX_OK;
+}
+
+int tx_aux_add_rmsnorm_staged(void *h, const void *delta, const void *weight, void *staged, int tokens, int hidden, float eps, void *stream) {
+  if (!h || !weight || !staged || tokens < 1 || hidden < 8 || hidden % 8 || hidden > kNormThreads * 8 * kNormChunks || (reinterpret_cast<uintptr_t>(staged) & 15))
+    return fail(TX_EINVAL, "tx_aux_add_rmsnorm_staged: hidden must be a multiple of 8 and at most 16384, the staged buffer 16-byte aligned");
+  int device = 0;
+  TX_CUDA(cudaGetDevice(&device));
+  const Workspace *ws = workspace_for(device);
+  if (hidden <= kNormThreads * 8 * 2 && ws && tokens >= ws->sm_count) {
+    const auto kernel = hidden <= kNormThreads * 8 ? add_rmsnorm_rows_staged_kernel<2, 1> : add_rmsnorm_rows_staged_kernel<2, 2>;
+    const size_t smem = 2 * staged_row_bytes(hidden);   // (33 KB at most)
+    TX_CUDA(launch_pdl(kernel, dim3((tokens + 1) / 2), dim3(kNormThreads), smem, static_cast<cudaStream_t>(stream), static_cast<__nv_bfloat16 *>(h),
+                       static_cast<const __nv_bfloat16 *>(delta), static_cast<const __nv_bfloat16 *>(weight), static_cast<uint8_t *>(staged), hidden, tokens, eps));
+    count_launch();
+    TX_CUDA(cudaGetLastError());
+    return TX_OK;
+  }
+  TX_CUDA(launch_pdl(add_rmsnorm_kernel<false, true>, dim3(tokens), dim3(kNormThreads), 0, static_cast<cudaStream_t>(stream),
+                     static_cast<__nv_bfloat16 *>(h), static_cast<const __nv_bfloat16 *>(delta),
+                     static_cast<const __nv_bfloat16 *>(weight), static_cast<__nv_bfloat16 *>(staged), hidden, eps, EmbedRows{}));
   count_launch();
   TX_CUDA(cudaGetLastError());
   return TX_OK;
@@ -1566,7 +1747,7 @@ int tx_aux_embed_rmsnorm(const void *table, int64_t vocab, const int64_t *row_to
   Workspace *ws = workspace_for(device);
   if (!ws) return TX_ECUDA;
   const EmbedRows embed{static_cast<const __nv_bfloat16 *>(table), reinterpret_cast<const long long *>(row_tokens), vocab, ws->status};
-  TX_CUDA(launch_pdl(add_rmsnorm_kernel<true>, dim3(tokens), dim3(kNormThreads), 0, static_cast<cudaStream_t>(stream), static_cast<__nv_bfloat16 *>(h),
+  TX_CUDA(launch_pdl(add_rmsnorm_kernel<true, false>, dim3(tokens), dim3(kNormThreads), 0, static_cast<cudaStream_t>(stream), static_cast<__nv_bfloat16 *>(h),
                      static_cast<const __nv_bfloat16 *>(nullptr), static_cast<const __nv_bfloat16 *>(weight), static_cast<__nv_bfloat16 *>(y), hidden, eps, embed));
   count_launch();
   TX_CUDA(cudaGetLastError());
@@ -1844,6 +2025,21 @@ int tx_aux_silu_mul_pairs(const void *gate_up, void *out, int tokens, int interm
 
 int tx_aux_silu_mul_pairs_accurate(const void *gate_up, void *out, int tokens, int intermediate, void *stream) {
   return launch_silu_mul_pairs(gate_up, out, tokens, intermediate, true, stream);
+}
+
+int tx_aux_silu_mul_pairs_staged(const void *gate_up, void *staged, int tokens, int intermediate, int accurate, void *stream) {
+  if (!gate_up || !staged || tokens < 1 || intermediate < 8 || intermediate % 8 || (reinterpret_cast<uintptr_t>(staged) & 15))
+    return fail(TX_EINVAL, "tx_aux_silu_mul_pairs_staged: bad argument");
+  if (tokens > 65535) return fail(TX_EUNSUPPORTED, "tx_aux_silu_mul_pairs_staged: up to 65535 tokens");
+  int device = 0;
+  TX_CUDA(cudaGetDevice(&device));
+  const Workspace *ws = workspace_for(device);
+  const int shares = staging_shares(intermediate, tokens, ws ? ws->sm_count : 148);
+  TX_CUDA(launch_pdl_cluster(accurate ? silu_mul_pairs_staged_kernel<true> : silu_mul_pairs_staged_kernel<false>, shares, dim3(shares, tokens), dim3(kSplitThreads), 0,
+                             static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16 *>(gate_up), static_cast<uint8_t *>(staged), intermediate));
+  count_launch();
+  TX_CUDA(cudaGetLastError());
+  return TX_OK;
 }
 
 int tx_aux_silu_mul(const void *gate_up, void *out, int tokens, int intermediate, void *stream) {

@@ -352,6 +352,7 @@ int launch_gemv_exact(const Handle *h, const __nv_bfloat16 *x, __nv_bfloat16 *y,
 int launch_gemv_texture(const Handle *h, const __nv_bfloat16 *x, __nv_bfloat16 *y, int tokens, cudaStream_t stream);
 int launch_prefill_tile(const Handle *h, int backend, const __nv_bfloat16 *x, __nv_bfloat16 *y, int tokens,
                         cudaStream_t stream, bool half_io = false);
+int launch_prefill_staged(const Handle *h, int backend, const uint8_t *staged, __nv_bfloat16 *y, int tokens, cudaStream_t stream);
 // y = round(sum of `ranges` fp32 partial results [ranges][tokens][M] + bias): second step of a launch that cut K
 int launch_combine(const float *partial, int ranges, const void *bias, void *y, int tokens, int M, bool half_io, int sm_count,
                    cudaStream_t stream);

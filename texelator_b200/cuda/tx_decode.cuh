@@ -308,4 +308,78 @@ __device__ __forceinline__ void solo_stage_chunk(int i, uint4 raw, float mult, u
   }
 }
 
+// ---------------------------------------------------------------------------------------------
+// Staged form of a prompt's activations for the tensor-core tiles: fp16 after an exact power-of-two rescale per token, chunk-major
+// [K/8][tokens padded to 32][8] with K padded to 128, the order of K in which the tile's producers hold the weights (element 4t + i of step j of a
+// 64-column half unit is column 16t + 4j + i), then one fp32 multiplier 2^s * 65536/889 a token.  stage_activations_kernel writes it
+// from rows in memory; a kernel that has a row in registers writes it with stage_piece.
+// ---------------------------------------------------------------------------------------------
+__host__ __device__ inline int padded_prompt(int tokens) { return (tokens + 31) & ~31; }
+__host__ __device__ inline size_t staged_prompt_multipliers(int K, int tokens) { return size_t((K + 127) / 128) * 16 * padded_prompt(tokens) * 16; }   // byte offset
+__host__ __device__ inline size_t staged_prompt_bytes(int K, int tokens) { return staged_prompt_multipliers(K, tokens) + size_t(padded_prompt(tokens)) * 4; }
+// Eight consecutive columns (converted) of piece i of a token; neighbouring lanes hold neighbouring pieces, lane 0 of eight the first of a half unit.
+// Lanes q and q ^ 2 swap halves, so that each stores one whole chunk.  `inside`: the piece exists (all lanes of the warp call).
+__device__ __forceinline__ void stage_piece(uint4 *staged, int padded_tokens, int tok, int i, uint4 v, bool inside) {
+  const int q = i & 7, odd = (q >> 1) & 1;               // block column parity
+  const unsigned give0 = odd ? v.x : v.z, give1 = odd ? v.y : v.w;
+  const unsigned get0 = __shfl_xor_sync(0xffffffffu, give0, 2), get1 = __shfl_xor_sync(0xffffffffu, give1, 2);
+  // even columns keep steps 2(q & 1), odd ones steps 2(q & 1) + 1; chunk 2j + c of the half unit
+  const int chunk = (i & ~7) + 2 * (2 * (q & 1) + odd) + (q >> 2);
+  if (inside) staged[size_t(chunk) * padded_tokens + tok] = odd ? make_uint4(get0, get1, v.z, v.w) : make_uint4(v.x, v.y, get0, get1);
+}
+
+// One row by the CTAs of a cluster (blockIdx.x the share, blockIdx.y the token): every CTA takes a run of half units, the largest magnitudes meet
+// through distributed shared memory.  For few tokens: a CTA a row leaves most SMs idle and a long row is a long chain (16 rows of 17408 columns
+// took 9.8 us that way).  From kSplitColumns columns on: a linear of 5120 x 17408 with 16 and 64 tokens
+// 26.8 -> 23.5 and 28.4 -> 24.3 us, 8192 x 28672 49.0 -> 41.4 and 51.3 -> 46.9, but 2048 x 11008 with 29 13.4 -> 14.1 and 5120 x 5120 with 16 12.0 -> 13.6 (a cluster's
+// launch).  piece(i): eight columns as bf16 (or, half_in, fp16), asked for once where a thread has up to kSplitHeld of them.
+constexpr int kSplitThreads = 256, kSplitHeld = 4, kSplitColumns = 12288;
+template <typename Piece>
+__device__ __forceinline__ void stage_split_row(uint4 *staged, float *multipliers, int K, int padded_tokens, bool half_in, Piece piece) {
+  __shared__ unsigned warp_peak[kSplitThreads / 32], peak_s;
+  const int shares = gridDim.x, share = blockIdx.x, tok = blockIdx.y, pieces = (K + 127) / 128 * 16, exist = K / 8;
+  const int first = int((long long)share * (pieces / 8) / shares) * 8, last = int((long long)(share + 1) * (pieces / 8) / shares) * 8;
+  const auto fetch = [&](int i) { return i < last && i < exist ? piece(i) : make_uint4(0, 0, 0, 0); };
+  uint4 held[kSplitHeld];
+  unsigned peak = 0;
+#pragma unroll
+  for (int c = 0; c < kSplitHeld; ++c) held[c] = fetch(first + int(threadIdx.x) + c * kSplitThreads);
+  float mult = 1.f, inverse = 1.f;
+  if (!half_in) {
+#pragma unroll
+    for (int c = 0; c < kSplitHeld; ++c) peak = max(peak, chunk_absmax(held[c]));
+    for (int i = first + int(threadIdx.x) + kSplitHeld * kSplitThreads; i < last; i += kSplitThreads) peak = max(peak, chunk_absmax(fetch(i)));
+    peak = __reduce_max_sync(0xffffffffu, peak);
+    if ((threadIdx.x & 31) == 0) warp_peak[threadIdx.x >> 5] = peak;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < kSplitThreads / 32; ++w) peak = max(peak, warp_peak[w]);
+    if (shares > 1) {
+      if (threadIdx.x == 0) peak_s = peak;
+      asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+      for (int r = 0; r < shares; ++r) {
+        unsigned other;
+        asm volatile("{\n\t.reg .b32 remote;\n\tmapa.shared::cluster.u32 remote, %1, %2;\n\tld.shared::cluster.u32 %0, [remote];\n\t}"
+                     : "=r"(other) : "r"(unsigned(__cvta_generic_to_shared(&peak_s))), "r"(r) : "memory");
+        peak = max(peak, other);
+      }
+      asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // (waited for at the end: nobody leaves while another reads)
+    }
+    token_scaling(peak, mult, inverse);
+  }
+  const auto store = [&](int i, uint4 v) { stage_piece(staged, padded_tokens, tok, i, half_in ? v : convert_chunk(v, mult), i < last); };
+#pragma unroll
+  for (int c = 0; c < kSplitHeld; ++c)
+    if (first + c * kSplitThreads < last) store(first + int(threadIdx.x) + c * kSplitThreads, held[c]);
+  for (int i0 = first + kSplitHeld * kSplitThreads; i0 < last; i0 += kSplitThreads) store(i0 + int(threadIdx.x), fetch(i0 + int(threadIdx.x)));
+  if (share == 0 && threadIdx.x == 0) multipliers[tok] = inverse * kNumeratorScale;
+  if (!half_in && shares > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// CTAs of a row: up to eight while two CTAs an SM are not exceeded and each has eight half units or more
+inline int staging_shares(int K, int tokens, int sm_count) {
+  int shares = 8;
+  while (shares > 1 && (tokens * shares > 2 * sm_count || (K + 63) / 64 < 8 * shares)) shares /= 2;
+  return shares;
+}
+
 }  // namespace tx

@@ -273,6 +273,15 @@ __global__ void __launch_bounds__(kStageThreads) stage_activations_kernel(const 
   }
 }
 
+// Few tokens with long rows: a cluster a row (stage_split_row)
+__global__ void __launch_bounds__(kSplitThreads) stage_split_kernel(const __nv_bfloat16 *__restrict__ x, __half *__restrict__ out, float *__restrict__ xmul, int K,
+                                                                    int padded_tokens, int half_in) {
+  grid_dependency_wait();        // the scratch may still be read by an earlier call's tile kernel, and x be on its way
+  grid_launch_dependents();
+  const uint4 *row = reinterpret_cast<const uint4 *>(x + size_t(blockIdx.y) * K);
+  stage_split_row(reinterpret_cast<uint4 *>(out), xmul, K, padded_tokens, half_in != 0, [&](int i) { return __ldcg(row + i); });
+}
+
 template <int CTAS, int BN, bool GENERIC>
 __global__ void __launch_bounds__(kPrefillThreads, 1)
 prefill_umma_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap x_map) {
@@ -609,11 +618,10 @@ int prefill_choose_backend(const Handle *h, int tokens) {
   return pick;
 }
 
+// One launch of the tile over `n` staged tokens, and the combine behind it where K is cut.
 template <int CTAS, int BN>
-static int launch_tile(const Handle *h, const __nv_bfloat16 *x, __nv_bfloat16 *y, int tokens, cudaStream_t stream, bool half_io) {
+static int launch_staged_tile(const Handle *h, const Workspace *ws, const __half *staged, const float *xmul, __nv_bfloat16 *y, int n, cudaStream_t stream, bool half_io) {
   using Cfg = TileConfig<CTAS, BN>;
-  Workspace *ws = workspace_for(h->device);
-  if (!ws) return TX_ECUDA;
   // the lean variant decodes high-mode blocks of the software palette and nothing else
   const bool generic = h->has_low_mode || h->palette == TX_PALETTE_HARDWARE;
   const auto kernel = generic ? prefill_umma_kernel<CTAS, BN, true> : prefill_umma_kernel<CTAS, BN, false>;
@@ -623,8 +631,56 @@ static int launch_tile(const Handle *h, const __nv_bfloat16 *x, __nv_bfloat16 *y
     std::lock_guard<std::mutex> lock(guard);
     if (!configured[{h->device, generic}]) {
       TX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(Cfg::smem)));
-      TX_CUDA(cudaFuncSetAttribute(stage_activations_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kStageSmem)));
       configured[{h->device, generic}] = true;
+    }
+  }
+  const int KP = h->KI * 128, padded_tokens = padded_prompt(n);
+  // staged X viewed as [KP/8 chunks][padded_tokens/32][32 tokens x 8 elements]: a box is one run of
+  // 512 contiguous bytes per 32 tokens and chunk and lands as core-matrix columns
+  CUtensorMap map;
+  cuuint64_t dims[3] = {256, cuuint64_t(padded_tokens / 32), cuuint64_t(KP / 8)};
+  cuuint64_t strides[2] = {512, cuuint64_t(padded_tokens) * 16};
+  cuuint32_t box[3] = {256, cuuint32_t(Cfg::tokens / 32), cuuint32_t(kChunks)};
+  cuuint32_t elem[3] = {1, 1, 1};
+  CUresult cr = encode_tiled_entry()(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<__half *>(staged), dims, strides, box, elem,
+                                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (cr != CUDA_SUCCESS) return fail(TX_ECUDA, "cuTensorMapEncodeTiled failed with code " + std::to_string(int(cr)));
+  PrefillParams p{};
+  p.tiles = reinterpret_cast<const uint4 *>(h->tiles);
+  p.flags = h->unit_flags;
+  p.scales = h->scales;
+  p.bias = h->bias;
+  p.xmul = xmul;
+  p.y = y;
+  p.status = ws->status;
+  p.M = h->M;
+  p.K = h->K;
+  p.KI = h->KI;
+  p.MT = h->MT;
+  p.T = n;
+  p.palette = h->palette;
+  p.half_io = half_io ? 1 : 0;
+  p.partial = ws->partial;
+  const int ranges = prefill_k_ranges(h, n, ws);
+  dim3 grid((h->M + Cfg::rows - 1) / Cfg::rows * CTAS, (n + BN - 1) / BN, ranges);
+  TX_CUDA(launch_pdl_cluster(kernel, CTAS, grid, dim3(kPrefillThreads), Cfg::smem, stream, p, map));
+  count_launch();
+  if (ranges > 1) return launch_combine(ws->partial, ranges, h->bias, y, n, h->M, half_io, ws->sm_count, stream);
+  return TX_OK;
+}
+
+template <int CTAS, int BN>
+static int launch_tile(const Handle *h, const __nv_bfloat16 *x, __nv_bfloat16 *y, int tokens, cudaStream_t stream, bool half_io) {
+  Workspace *ws = workspace_for(h->device);
+  if (!ws) return TX_ECUDA;
+  static std::mutex guard;
+  static std::map<int, bool> configured;
+  {
+    std::lock_guard<std::mutex> lock(guard);
+    if (!configured[h->device]) {
+      TX_CUDA(cudaFuncSetAttribute(stage_activations_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kStageSmem)));
+      configured[h->device] = true;
     }
   }
   // Activations are staged once as fp16 after an exact per-token power-of-two rescale (the decode GEMV's
@@ -634,48 +690,20 @@ static int launch_tile(const Handle *h, const __nv_bfloat16 *x, __nv_bfloat16 *y
   if (capacity < 32) return fail(TX_EINVAL, "K is too large for the prefill activation scratch");
   for (int t0 = 0; t0 < tokens; t0 += capacity) {
     const int n = std::min(capacity, tokens - t0);
-    const int padded_tokens = (n + 31) & ~31;
+    const int padded_tokens = padded_prompt(n);
+    const int shares = h->K >= kSplitColumns && n <= ws->sm_count ? staging_shares(h->K, n, ws->sm_count) : 1;
     int per_cta = 4;
     while (per_cta > 1 && (padded_tokens / per_cta < ws->sm_count * 3 / 4 || per_cta * stage_row_bytes(h->K) > kStageSmem)) per_cta /= 2;
     const bool rows_fit = per_cta * stage_row_bytes(h->K) <= kStageSmem;
-    TX_CUDA(launch_pdl(stage_activations_kernel, dim3(padded_tokens / per_cta), dim3(kStageThreads), rows_fit ? per_cta * stage_row_bytes(h->K) : 0,
+    if (shares > 1)
+      TX_CUDA(launch_pdl_cluster(stage_split_kernel, shares, dim3(shares, n), dim3(kSplitThreads), 0, stream, x + size_t(t0) * h->K, ws->xprep, ws->xmul, h->K,
+                                 padded_tokens, half_io ? 1 : 0));
+    else
+      TX_CUDA(launch_pdl(stage_activations_kernel, dim3(padded_tokens / per_cta), dim3(kStageThreads), rows_fit ? per_cta * stage_row_bytes(h->K) : 0,
                        stream, x + size_t(t0) * h->K, ws->xprep, ws->xmul, h->K, KP, n, padded_tokens, per_cta, rows_fit ? 1 : 0, half_io ? 1 : 0));
     count_launch();
-    // staged X viewed as [KP/8 chunks][padded_tokens/32][32 tokens x 8 elements]: a box is one run of
-    // 512 contiguous bytes per 32 tokens and chunk and lands as core-matrix columns
-    CUtensorMap map;
-    cuuint64_t dims[3] = {256, cuuint64_t(padded_tokens / 32), cuuint64_t(KP / 8)};
-    cuuint64_t strides[2] = {512, cuuint64_t(padded_tokens) * 16};
-    cuuint32_t box[3] = {256, cuuint32_t(Cfg::tokens / 32), cuuint32_t(kChunks)};
-    cuuint32_t elem[3] = {1, 1, 1};
-    CUresult cr = encode_tiled_entry()(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, ws->xprep, dims, strides, box, elem,
-                                       CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                                       CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (cr != CUDA_SUCCESS) return fail(TX_ECUDA, "cuTensorMapEncodeTiled failed with code " + std::to_string(int(cr)));
-    PrefillParams p{};
-    p.tiles = reinterpret_cast<const uint4 *>(h->tiles);
-    p.flags = h->unit_flags;
-    p.scales = h->scales;
-    p.bias = h->bias;
-    p.xmul = ws->xmul;
-    p.y = y + size_t(t0) * h->M;
-    p.status = ws->status;
-    p.M = h->M;
-    p.K = h->K;
-    p.KI = h->KI;
-    p.MT = h->MT;
-    p.T = n;
-    p.palette = h->palette;
-    p.half_io = half_io ? 1 : 0;
-    p.partial = ws->partial;
-    const int ranges = prefill_k_ranges(h, n, ws);
-    dim3 grid((h->M + Cfg::rows - 1) / Cfg::rows * CTAS, (n + BN - 1) / BN, ranges);
-    TX_CUDA(launch_pdl_cluster(kernel, CTAS, grid, dim3(kPrefillThreads), Cfg::smem, stream, p, map));
-    count_launch();
-    if (ranges > 1) {
-      int rc = launch_combine(ws->partial, ranges, h->bias, y + size_t(t0) * h->M, n, h->M, half_io, ws->sm_count, stream);
-      if (rc != TX_OK) return rc;
-    }
+    const int rc = launch_staged_tile<CTAS, BN>(h, ws, ws->xprep, ws->xmul, y + size_t(t0) * h->M, n, stream, half_io);
+    if (rc != TX_OK) return rc;
   }
   TX_CUDA(cudaGetLastError());
   return TX_OK;
@@ -693,6 +721,26 @@ int launch_prefill_tile(const Handle *h, int backend, const __nv_bfloat16 *x, __
     case 9: return launch_tile<1, 192>(h, x, y, tokens, stream, half_io);
     default: return fail(TX_EINVAL, "backend is not a tensor-core tile candidate");
   }
+}
+
+// The same for activations that the kernel in front wrote in staged form (bf16 in and out), in a buffer of the caller's.
+int launch_prefill_staged(const Handle *h, int backend, const uint8_t *staged, __nv_bfloat16 *y, int tokens, cudaStream_t stream) {
+  Workspace *ws = workspace_for(h->device);
+  if (!ws) return TX_ECUDA;
+  const __half *x = reinterpret_cast<const __half *>(staged);
+  const float *xmul = reinterpret_cast<const float *>(staged + staged_prompt_multipliers(h->K, tokens));
+  int rc;
+  switch (backend) {
+    case 5: rc = launch_staged_tile<1, 256>(h, ws, x, xmul, y, tokens, stream, false); break;
+    case 6: rc = launch_staged_tile<2, 256>(h, ws, x, xmul, y, tokens, stream, false); break;
+    case 7: rc = launch_staged_tile<1, 128>(h, ws, x, xmul, y, tokens, stream, false); break;
+    case 8: rc = launch_staged_tile<1, 64>(h, ws, x, xmul, y, tokens, stream, false); break;
+    case 9: rc = launch_staged_tile<1, 192>(h, ws, x, xmul, y, tokens, stream, false); break;
+    default: return fail(TX_EINVAL, "backend is not a tensor-core tile candidate");
+  }
+  if (rc != TX_OK) return rc;
+  TX_CUDA(cudaGetLastError());
+  return TX_OK;
 }
 
 template <int CTAS, int BN>

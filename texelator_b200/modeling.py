@@ -352,20 +352,33 @@ class BC4Decoder:
         make = lambda columns: torch.empty(tokens, columns, dtype=torch.bfloat16, device=self.device)
         x, qkv, gate_up, act, out = make(c.hidden), make(self.q_loc + 2 * self.kv_loc), make(2 * self.i_loc), make(self.i_loc), make(c.hidden)
         q = qkv[:, :self.q_loc].view(tokens, q_heads, c.head_dim).transpose(0, 1).unsqueeze(0)
+        staged = ext.staged_buffer(max(c.hidden, self.i_loc), tokens, self.device)
+
+        def normed(handle, delta, weight, out):
+            if ext.takes_staged(handle, tokens):
+                ext.add_rmsnorm_staged(h, delta, weight, staged, c.rms_eps)
+                ext.linear_staged(handle, staged, out)
+            else:
+                ext.add_rmsnorm(h, delta, weight, x, c.rms_eps)
+                ext.linear_out(handle, x, out)
+
         delta = None
         for layer in range(c.layers):
-            ext.add_rmsnorm(h, delta, self.norm1[layer], x, c.rms_eps)
-            ext.linear_out(self.h_qkv[layer], x, qkv)
+            normed(self.h_qkv[layer], delta, self.norm1[layer], qkv)
             k_cache, v_cache = self.k_cache[layer], self.v_cache[layer]
             ext.rope_append_prompt(qkv, self.cos, self.sin, 0, k_cache, v_cache, q_heads, kv_heads, c.head_dim)
             attended = F.scaled_dot_product_attention(q, k_cache[:, :tokens].unsqueeze(0), v_cache[:, :tokens].unsqueeze(0),
                                                       is_causal=True, enable_gqa=True)
             attended = attended.squeeze(0).transpose(0, 1).reshape(tokens, self.q_loc).contiguous()
             delta = self._reduce(ext.linear_out(self.h_o[layer], attended, out))
-            ext.add_rmsnorm(h, delta, self.norm2[layer], x, c.rms_eps)
-            ext.linear_out(self.h_gu[layer], x, gate_up)
-            ext.silu_mul_pairs(gate_up, act, accurate=True)
-            delta = self._reduce(ext.linear_out(self.h_down[layer], act, out))
+            normed(self.h_gu[layer], delta, self.norm2[layer], gate_up)
+            if ext.stages_swiglu(tokens, self.i_loc) and ext.takes_staged(self.h_down[layer], tokens):
+                ext.silu_mul_pairs_staged(gate_up, staged, accurate=True)
+                ext.linear_staged(self.h_down[layer], staged, out)
+            else:
+                ext.silu_mul_pairs(gate_up, act, accurate=True)
+                ext.linear_out(self.h_down[layer], act, out)
+            delta = self._reduce(out)
         ext.add_rmsnorm(h, delta, self.final_norm, x, c.rms_eps)
         return x
 

@@ -68,6 +68,11 @@ C_API = {
     "tx_kernel_status": (_i32, [_i32, _i32]),
     "tx_aux_add_rmsnorm": (_i32, [_vp, _vp, _vp, _vp, _i32, _i32, ctypes.c_float, _vp]),
     "tx_aux_embed_rmsnorm": (_i32, [_vp, ctypes.c_int64, _vp, _vp, _vp, _vp, _i32, _i32, ctypes.c_float, _i32, _vp]),
+    "tx_staged_prompt_bytes": (_sz, [_i32, _i32]),
+    "tx_linear_takes_staged": (_i32, [_u64, _i32]),
+    "tx_linear_staged": (_i32, [_u64, _vp, _vp, _i32, _vp]),
+    "tx_aux_add_rmsnorm_staged": (_i32, [_vp, _vp, _vp, _vp, _i32, _i32, ctypes.c_float, _vp]),
+    "tx_aux_silu_mul_pairs_staged": (_i32, [_vp, _vp, _i32, _i32, _i32, _vp]),
     "tx_aux_rope_append": (_i32, [_vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp]),
     "tx_aux_rope_append_prompt": (_i32, [_vp, _vp, _vp, _i32, _i32, _vp, _vp, _i32, _i32, _i32, _i32, _vp]),
     "tx_aux_attention_decode": (_i32, [_vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, ctypes.c_float, _vp]),
@@ -371,6 +376,42 @@ class _Extension:
         tokens, hidden = h.shape
         self._check(self._lib.tx_aux_add_rmsnorm(h.data_ptr(), delta.data_ptr() if delta is not None else None,
                                                  weight.data_ptr(), y.data_ptr(), tokens, hidden, eps, self._stream(h)))
+
+    # -- activations in the form the tiles read: from the kernel that makes them to the linear, without a staging launch --------
+    def staged_buffer(self, columns: int, tokens: int, device) -> torch.Tensor:
+        """A buffer for ``tokens`` rows of up to ``columns`` activations in staged form."""
+        return torch.empty(self._lib.tx_staged_prompt_bytes(columns, tokens), dtype=torch.uint8, device=device)
+
+    def takes_staged(self, handle: int, tokens: int) -> bool:
+        """Whether ``linear_staged`` serves this many tokens (``linear`` would take a tile for them)."""
+        return self._lib.tx_linear_takes_staged(handle, tokens) == 1
+
+    def linear_staged(self, handle: int, staged: torch.Tensor, y: torch.Tensor) -> torch.Tensor:
+        """``linear_out`` of rows in staged form: the same result bit for bit."""
+        m, k, _ = self._shapes[handle]
+        tokens = y.numel() // m
+        if y.numel() != tokens * m or y.dtype != torch.bfloat16 or not y.is_contiguous() or staged.numel() < self._lib.tx_staged_prompt_bytes(k, tokens):
+            raise RuntimeError("input shape/device mismatch")
+        self._check(self._lib.tx_linear_staged(handle, staged.data_ptr(), y.data_ptr(), tokens, self._stream(y)))
+        return y
+
+    def add_rmsnorm_staged(self, h: torch.Tensor, delta: torch.Tensor | None, weight: torch.Tensor, staged: torch.Tensor, eps: float) -> None:
+        tokens, hidden = h.shape
+        if staged.numel() < self._lib.tx_staged_prompt_bytes(hidden, tokens):
+            raise RuntimeError("the staged buffer is too small")
+        self._check(self._lib.tx_aux_add_rmsnorm_staged(h.data_ptr(), delta.data_ptr() if delta is not None else None, weight.data_ptr(),
+                                                        staged.data_ptr(), tokens, hidden, eps, self._stream(h)))
+
+    @staticmethod
+    def stages_swiglu(tokens: int, intermediate: int) -> bool:
+        """Whether a SwiGLU that writes the tile's form is faster than one that writes rows and a staging launch behind it: few long rows."""
+        return tokens <= 64 and intermediate >= 12288
+
+    def silu_mul_pairs_staged(self, gate_up: torch.Tensor, staged: torch.Tensor, accurate: bool = False) -> None:
+        tokens, two_i = gate_up.shape
+        if staged.numel() < self._lib.tx_staged_prompt_bytes(two_i // 2, tokens):
+            raise RuntimeError("the staged buffer is too small")
+        self._check(self._lib.tx_aux_silu_mul_pairs_staged(gate_up.data_ptr(), staged.data_ptr(), tokens, two_i // 2, int(accurate), self._stream(gate_up)))
 
     def embed_rmsnorm(self, table: torch.Tensor, row_tokens: torch.Tensor, h: torch.Tensor, weight: torch.Tensor, y: torch.Tensor, eps: float) -> None:
         """``h = table[row_tokens]`` (int64, one per row), ``y = rmsnorm(h) * weight``."""
