@@ -194,6 +194,45 @@ __device__ __forceinline__ unsigned long long smem_desc(unsigned addr, unsigned 
          ((unsigned long long)((sbo >> 4) & 0x3FFF) << 32) | (1ull << 46);
 }
 
+// Sums of 32 tokens (a register each) of a lane's row, scaled and rounded, to out[token * kMmaM].  Eight at a time and step by step, two to a
+// conversion: with all steps of one token behind one another a chunk took 1250 cycles of sixteen warps.
+template <bool HALF>
+__device__ __forceinline__ void round_to(uint16_t *out, const unsigned (&v)[32], float row_scale, float bias, float token_scale) {
+#pragma unroll
+  for (int j0 = 0; j0 < 32; j0 += 8) {
+    float value[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) value[j] = __shfl_sync(0xffffffffu, token_scale, j0 + j);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) value[j] = fmaf(__uint_as_float(v[j0 + j]), row_scale * value[j], bias);
+#pragma unroll
+    for (int j = 0; j < 8; j += 2) {
+      unsigned pair;
+      if (HALF) {
+        const __half2 h = __floats2half2_rn(value[j], value[j + 1]);
+        pair = *reinterpret_cast<const unsigned *>(&h);
+      } else {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(value[j], value[j + 1]);
+        pair = *reinterpret_cast<const unsigned *>(&h);
+      }
+      out[(j0 + j) * kMmaM] = uint16_t(pair);
+      out[(j0 + j + 1) * kMmaM] = uint16_t(pair >> 16);
+    }
+  }
+}
+// the same for a K range: fp32, to dst[token * M], of the first `last` tokens
+__device__ __forceinline__ void scale_to(float *dst, int M, const unsigned (&v)[32], float row_scale, float token_scale, int last) {
+#pragma unroll
+  for (int j0 = 0; j0 < 32; j0 += 8) {
+    float value[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) value[j] = __uint_as_float(v[j0 + j]) * (row_scale * __shfl_sync(0xffffffffu, token_scale, j0 + j));
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (j0 + j < last) dst[size_t(j0 + j) * M] = value[j];
+  }
+}
+
 // Activation staging for the GEMM: per token an exact power-of-two rescale to fp16 (the decode GEMV's
 // arithmetic), stored chunk-major -- out[(chunk * padded_tokens + token) * 8 .. +8], padded_tokens a
 // multiple of 32 -- which is the K-major core-matrix order of the B operand.  A TMA box then copies
@@ -504,11 +543,7 @@ prefill_umma_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap x
         float *dst = p.partial + (size_t(blockIdx.z) * p.T + tok0 + c * 32) * p.M + row;
         unsigned v[32];
         tmem_load32(tmem_base + (unsigned(quarter * 32) << 16) + unsigned(c * 32), v);
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          const float scale = row_scale * __shfl_sync(0xffffffffu, token_scale[i], j);
-          if (row < p.M && tok0 + c * 32 + j < p.T) dst[size_t(j) * p.M] = __uint_as_float(v[j]) * scale;
-        }
+        scale_to(dst, p.M, v, row_scale, token_scale[i], row < p.M ? p.T - tok0 - c * 32 : 0);
       }
     } else if (ready) {
       // A lane holds one output row, so stores from here would be 64-byte pieces; the tile goes through shared memory (the
@@ -520,12 +555,9 @@ prefill_umma_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap x
         if (c >= BN / 32) break;
         unsigned v[32];
         tmem_load32(tmem_base + (unsigned(quarter * 32) << 16) + unsigned(c * 32), v);
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          const float value = fmaf(__uint_as_float(v[j]), row_scale * __shfl_sync(0xffffffffu, token_scale[i], j), bias);
-          out[(c * 32 + j) * kMmaM + quarter * 32 + lane] =
-              p.half_io ? __half_as_ushort(__float2half_rn(value)) : __bfloat16_as_ushort(__float2bfloat16(value));
-        }
+        uint16_t *to = out + c * 32 * kMmaM + quarter * 32 + lane;
+        if (p.half_io) round_to<true>(to, v, row_scale, bias, token_scale[i]);   // (uniform)
+        else round_to<false>(to, v, row_scale, bias, token_scale[i]);
       }
     }
     asm volatile("bar.sync 1, %0;" ::"n"(kProducerWarps * 32) : "memory");
