@@ -949,7 +949,7 @@ __global__ void __launch_bounds__(kStepThreads, 2) attention_step_kernel(const _
                                                                       __nv_bfloat16 *__restrict__ v_cache, float *__restrict__ partial,
                                                                       __nv_bfloat16 *__restrict__ out, int q_heads, int kv_heads,
                                                                       int max_len, int split_capacity, float scale, int merge_here) {
-  __shared__ __align__(16) float q_s[GROUP][kHeadDim];
+  __shared__ __align__(16) float q_s[GROUP][4][8][4];                 // a lane's sixteen dimensions in four loads that meet every bank once
   __shared__ float p_s[GROUP][kStepKeys];
   __shared__ __align__(16) float red_s[kStepThreads / 32][GROUP][kHeadDim];   // per-warp partial sums
   __shared__ float stat_s[GROUP][2];
@@ -1005,8 +1005,8 @@ __global__ void __launch_bounds__(kStepThreads, 2) attention_step_kernel(const _
     const float c = cos_table[pos * kHalf + i], sn = sin_table[pos * kHalf + i];
     const __nv_bfloat16 *vec = qkv + size_t(kvh * GROUP + g) * kHeadDim;
     const float x1 = __bfloat162float(__ldcg(vec + i)), x2 = __bfloat162float(__ldcg(vec + i + kHalf));
-    q_s[g][i] = __bfloat162float(__float2bfloat16(x1 * c - x2 * sn)) * scale;
-    q_s[g][i + kHalf] = __bfloat162float(__float2bfloat16(x2 * c + x1 * sn)) * scale;
+    q_s[g][(i >> 2) & 1][i >> 3][i & 3] = __bfloat162float(__float2bfloat16(x1 * c - x2 * sn)) * scale;
+    q_s[g][2 + ((i >> 2) & 1)][i >> 3][i & 3] = __bfloat162float(__float2bfloat16(x2 * c + x1 * sn)) * scale;
   }
   if (split == live - 1) {
     if (tid < kHalf) {
@@ -1050,9 +1050,9 @@ __global__ void __launch_bounds__(kStepThreads, 2) attention_step_kernel(const _
     }
 #pragma unroll
     for (int g = 0; g < GROUP; ++g) {
-      const float4 *src = reinterpret_cast<const float4 *>(&q_s[g][0]);
-      const float4 qa = src[2 * j], qb = src[2 * j + 1], qc = src[16 + 2 * j], qd = src[16 + 2 * j + 1];
-      const float q[16] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w, qc.x, qc.y, qc.z, qc.w, qd.x, qd.y, qd.z, qd.w};
+      float q[16];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) *reinterpret_cast<float4 *>(&q[4 * e]) = *reinterpret_cast<const float4 *>(&q_s[g][e][j][0]);
 #pragma unroll
       for (int b = 0; b < 2; ++b) {
         const int key = warp * 8 + b * 4 + r;
@@ -1219,8 +1219,7 @@ __global__ void __launch_bounds__(kStepThreads, 2) attention_step_loop_kernel(co
   extern __shared__ __align__(128) uint8_t ring_smem[];
   __shared__ __align__(16) float q_s[GROUP][4][8][4];                 // a lane's sixteen dimensions in four loads that meet every bank once
   constexpr int kHeads = (GROUP + 1) / 2;                             // of a warp in the scores
-  constexpr int kPitch = GROUP <= 4 ? 4 : 8;                          // a key's weights lie together: one or two loads for all heads
-  __shared__ __align__(16) float p_s[kStepKeys][kPitch];
+  __shared__ float p_s[GROUP][kStepKeys];
   __shared__ float stat_s[GROUP][2];
   __shared__ float rescale_s[GROUP];
   __shared__ __align__(16) __nv_bfloat16 fresh_s[2][kHeadDim];        // the new key, rotated, and value
@@ -1349,18 +1348,18 @@ __global__ void __launch_bounds__(kStepThreads, 2) attention_step_loop_kernel(co
         float sum = (upper ? sum1 : sum0) + __shfl_xor_sync(0xffffffffu, upper ? sum0 : sum1, 2);
         sum += __shfl_xor_sync(0xffffffffu, sum, 4);
         const int key = (warp & 3) * 16 + (odd ? 4 : 0) + (upper ? 8 : 0) + r;
-        if (j < 4) p_s[key][g] = key < count ? sum : -INFINITY;
+        if (j < 4) p_s[g][key] = key < count ? sum : -INFINITY;
       }
     }
   }
   __syncthreads();
   // ---- per head: max and exp-sum over the CTA's keys (warp g handles head g; GROUP <= 8 warps) ----
   if (warp < GROUP) {
-    const float a = p_s[lane][warp], b = p_s[lane + 32][warp];
+    const float a = p_s[warp][lane], b = p_s[warp][lane + 32];
     const float m = fmaxf(run_max, warp_max(fmaxf(a, b)));     // finite: every chunk of the walk holds a key
     const float ea = __expf(a - m), eb = __expf(b - m);
-    p_s[lane][warp] = ea;
-    p_s[lane + 32][warp] = eb;
+    p_s[warp][lane] = ea;
+    p_s[warp][lane + 32] = eb;
     const float factor = __expf(run_max - m);                   // 0 on the first chunk
     run_sum = fmaf(run_sum, factor, warp_sum(ea + eb));
     run_max = m;
@@ -1385,12 +1384,9 @@ __global__ void __launch_bounds__(kStepThreads, 2) attention_step_loop_kernel(co
       const uint2 raw = key < count ? reinterpret_cast<const uint2 *>(row)[lane] : make_uint2(0, 0);
       const float v0 = __uint_as_float(raw.x << 16), v1 = __uint_as_float(raw.x & 0xffff0000u);
       const float v2 = __uint_as_float(raw.y << 16), v3 = __uint_as_float(raw.y & 0xffff0000u);
-      float p[kPitch];
-#pragma unroll
-      for (int g = 0; g < kPitch; g += 4) *reinterpret_cast<float4 *>(&p[g]) = *reinterpret_cast<const float4 *>(&p_s[key][g]);
 #pragma unroll
       for (int g = 0; g < GROUP; ++g) {
-        const float pw = p[g];
+        const float pw = p_s[g][key];
         acc[g][0] = fmaf(pw, v0, acc[g][0]);
         acc[g][1] = fmaf(pw, v1, acc[g][1]);
         acc[g][2] = fmaf(pw, v2, acc[g][2]);

@@ -20,8 +20,8 @@
 //   encode_block_spaced  the software palette: weights are assigned by rounding, the nine errors come from a quadratic form and what is
 //                        too close to call is evaluated the first way.  About 1600 instructions, 64 % of the issue slots.
 //
-// us a call, all blocks the first way / as launched: 4096 x 4096 156.8 / 79.6, 11000 x 11008 1097 / 491, 9000 x 2000 182.6 / 96.7;
-// 4096 x 4096 with nine weights of ten zero 166 / 177, under the texture palette 157 / 168 (5 of it the verdict).
+// us a call, all blocks the first way / as launched: 4096 x 4096 156.8 / 80.4, 11000 x 11008 1097 / 505, 9000 x 2000 182.6 / 99.0;
+// 4096 x 4096 with nine weights of ten zero 166 / 171, under the texture palette 156 / 162 (the verdict).
 #include "tx_common.cuh"
 
 namespace tx {
@@ -585,10 +585,11 @@ __global__ void __launch_bounds__(kEncodeThreads, 4) encode_kernel(const float *
 template <int GROUP>
 static void launch_encode_rows(const float *weight, const float *hdiag, const float *lut, int M, int K, uint8_t *blocks, float *scales, cudaStream_t stream) {
   const int per_cta = kEncodeThreads / GROUP, ctas = (M + per_cta - 1) / per_cta;
-  // Rows alone fill the chip from about 600 blocks of threads on (four to an SM), and the blocks then take several each.  Below that
+  // Rows alone fill the chip from about 600 blocks of threads on (four to an SM); beyond three times that the blocks take several each (4096 x 4096 79.6,
+  // 80.4, 84.4 us with one wave of blocks, three and a block a row; under the texture palette 171, 162, 164).  Below that
   // a row is shared, by as many groups as fit one wave and have a step each: 8 x 17408 84.6 -> 11.4 us, 100 x 11200 57.9 -> 16.6,
   // 300 x 11200 74.9 -> 44.3 (the kernel that spread single blocks over the chip took 29.2, 61.6 and 153.7).
-  const int grid = std::min(ctas, kEncodeWave);
+  const int grid = std::min(ctas, 3 * kEncodeWave);
   const int steps = (K / 16 + GROUP - 1) / GROUP, most = std::max(1, std::min(kEncodeWave / grid, steps));
   const int rounds = (steps + most - 1) / most;   // steps of a group
   const int shares = (steps + rounds - 1) / rounds;
