@@ -301,3 +301,32 @@ def test_staged_activations_give_the_linear_of_their_rows(ext, lut, tokens, k, m
         assert ext.kernel_status() == 0
     finally:
         ext.free(h)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("m,k,tokens", [(128, 1024, 16), (132, 1024, 33), (130, 1040, 64), (257, 2064, 65), (1024, 4096, 127), (3000, 1536, 1),
+                                        (4250, 2896, 29), (5120, 1024, 17), (2304, 8192, 40), (9216, 1024, 31), (9344, 1024, 31)])
+def test_k_ranges_add_to_the_sums_of_their_columns(ext, lut, m, k, tokens, dtype):
+    """K in two to eight ranges, added by a cluster where all clusters fit and by a second launch elsewhere (the pair tile): the same bits from
+    every tile, and the 64-bit sums within the output's rounding and the fp32 adds."""
+    blocks, scales, x = _case(m + k, m, k, tokens, lut)
+    bias = torch.from_numpy(np.random.default_rng(2).standard_normal(m).astype(np.float32)).to(dtype).cuda()
+    h = _pack(ext, blocks, scales, bias)
+    try:
+        from texelator_b200 import runtime
+        x = x.cuda().to(dtype)
+        ext.set_prefill(h, 1, 1024)
+        outs = []
+        for backend in (6, 5, 7, 8, 9):                       # the pair tile always adds by the second launch
+            ext.set_prefill_backend(h, backend)
+            outs.append(ext.linear(h, x))
+        assert all(torch.equal(y, outs[0]) for y in outs[1:])
+        want = x.double() @ ext.dequant(h, runtime.DEQUANT_SCALED_F32).double().T + bias.double()
+        size = x.double().abs() @ ext.dequant(h, runtime.DEQUANT_SCALED_F32).double().abs().T + bias.double().abs()
+        # half a unit of the output (2^-8 or 2^-11 of a value's power of two), and fp32 chains of k / 16 adds that may truncate (2^-23 of the
+        # absolute sum each); 2^-24 is under fp16's smallest step
+        half = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+        assert bool(((outs[0].double() - want).abs() <= half * want.abs() + k / 16 * 2.0 ** -23 * size + 2.0 ** -24).all())
+        assert ext.kernel_status() == 0
+    finally:
+        ext.free(h)

@@ -300,9 +300,9 @@ __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddep
 
 bool pdl_enabled();
 
-// `ctas` consecutive CTAs along x form a cluster (1: none); `early`: may start while its predecessor drains
+// `cluster` CTAs along x, y and z form a cluster (1: none); `early`: may start while its predecessor drains
 template <typename... KernelArgs, typename... Args>
-cudaError_t launch_cluster(void (*kernel)(KernelArgs...), bool early, int ctas, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+cudaError_t launch_cluster(void (*kernel)(KernelArgs...), bool early, dim3 cluster, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
   cudaLaunchConfig_t config{};
   config.gridDim = grid;
   config.blockDim = block;
@@ -314,10 +314,11 @@ cudaError_t launch_cluster(void (*kernel)(KernelArgs...), bool early, int ctas, 
     attributes[count].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attributes[count++].val.programmaticStreamSerializationAllowed = 1;
   }
-  if (ctas > 1) {
+  if (cluster.x * cluster.y * cluster.z > 1) {
     attributes[count].id = cudaLaunchAttributeClusterDimension;
-    attributes[count].val.clusterDim.x = unsigned(ctas);
-    attributes[count].val.clusterDim.y = attributes[count].val.clusterDim.z = 1;
+    attributes[count].val.clusterDim.x = cluster.x;
+    attributes[count].val.clusterDim.y = cluster.y;
+    attributes[count].val.clusterDim.z = cluster.z;
     ++count;
   }
   config.attrs = attributes;
@@ -325,8 +326,8 @@ cudaError_t launch_cluster(void (*kernel)(KernelArgs...), bool early, int ctas, 
   return cudaLaunchKernelEx(&config, kernel, KernelArgs(args)...);
 }
 template <typename... KernelArgs, typename... Args>
-cudaError_t launch_pdl_cluster(void (*kernel)(KernelArgs...), int ctas, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
-  return launch_cluster(kernel, true, ctas, grid, block, smem, stream, args...);
+cudaError_t launch_pdl_cluster(void (*kernel)(KernelArgs...), dim3 cluster, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+  return launch_cluster(kernel, true, cluster, grid, block, smem, stream, args...);
 }
 template <typename... KernelArgs, typename... Args>
 cudaError_t launch_pdl(void (*kernel)(KernelArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {

@@ -72,7 +72,7 @@ template <int CTAS, int BN> struct TileConfig {
   static_assert(stages >= 2, "tile does not fit two pipeline stages");
   static_assert(BN + stages * kAColumns <= tmem_columns, "accumulator and A stages must fit TMEM");
   static_assert(tokens % 32 == 0 && BN % 32 == 0 && BN <= 256, "the activation box is made of 32-token runs; N is at most 256");
-  static_assert(stages * b_stage >= BN * kMmaM * 2, "the output tile is staged where the activations were");
+  static_assert(stages * b_stage >= BN * kMmaM * (CTAS == 1 ? 4 : 2), "the output tile, or its fp32 sums, are staged where the activations were");
 };
 
 struct PrefillParams {
@@ -86,7 +86,8 @@ struct PrefillParams {
   int M, K, KI, MT, T;
   int palette;
   int half_io;   // bias and y are fp16 (the staged activations are fp16 either way)
-  float *partial;   // gridDim.z > 1: K is cut into gridDim.z ranges of units and the scaled fp32 sums go to partial[range][T][M]
+  float *partial;   // gridDim.z > 1: K is cut into gridDim.z ranges of units and the scaled fp32 sums go to partial[range][T][M]; null: the ranges
+                    // of a tile are a cluster that adds them in shared memory
 };
 
 // ---- PTX wrappers -------------------------------------------------------------------------------
@@ -345,6 +346,7 @@ prefill_umma_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap x
   const int u0 = int(blockIdx.z) * p.KI / int(gridDim.z), u1 = (int(blockIdx.z) + 1) * p.KI / int(gridDim.z);
   const int KT = u1 - u0;
   const int row0 = blockIdx.x * kMmaM, tok0 = blockIdx.y * BN;
+  const bool merge = CTAS == 1 && gridDim.z > 1 && p.partial == nullptr;
 
   if (tid == 0) {
     for (int s = 0; s < S; ++s) {
@@ -535,7 +537,17 @@ prefill_umma_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap x
     }
     const bool ready = __all_sync(0xffffffffu, mbar_wait(accum, 0, abort_flag, p.status, 5));
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (ready && gridDim.z > 1) {
+    if (ready && merge) {
+      float *sums = reinterpret_cast<float *>(smem_raw + (b_s - sbase));        // [BN][128 rows], where the activations were
+#pragma unroll
+      for (int i = 0; i < kMost; ++i) {
+        const int c = (warp >> 2) + i * kParts;
+        if (c >= BN / 32) break;
+        unsigned v[32];
+        tmem_load32(tmem_base + (unsigned(quarter * 32) << 16) + unsigned(c * 32), v);
+        scale_to(sums + c * 32 * kMmaM + quarter * 32 + lane, kMmaM, v, row_scale, token_scale[i], 32);
+      }
+    } else if (ready && gridDim.z > 1) {
 #pragma unroll
       for (int i = 0; i < kMost; ++i) {
         const int c = (warp >> 2) + i * kParts;
@@ -579,6 +591,50 @@ prefill_umma_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap x
       }
     }
   }
+  if (merge) {
+    // The ranges of this tile, in order, bias, one rounding: launch_combine's sums to the bit, without its launch and without [ranges][T][M] floats
+    // through global memory.  A CTA takes every gridDim.z-th token, a warp a token, a lane four rows (a row of sums is one conflict-free read).
+    cluster_sync();
+    const bool whole = !*abort_flag;       // (an abort is reported; what this CTA would add is not there)
+    if (warp < kProducerWarps && whole) {
+      const int row = row0 + lane * 4, rows = min(4, p.M - row), last = min(BN, p.T - tok0), ranges = int(gridDim.z);
+      const bool wide = p.M % 4 == 0;      // rows of y are 8-byte aligned
+      float bias[4] = {};
+      if (p.bias) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (i < rows) bias[i] = p.half_io ? __half2float(reinterpret_cast<const __half *>(p.bias)[row + i]) : __bfloat162float(p.bias[row + i]);
+      }
+      for (int tok = int(blockIdx.z) + ranges * warp; tok < last; tok += ranges * kProducerWarps) {
+        const unsigned at = b_s + unsigned((tok * kMmaM + lane * 4) * 4);
+        float sum[4] = {};
+        for (int r = 0; r < ranges; ++r) {
+          float4 part;
+          asm volatile("{\n\t.reg .b32 remote;\n\tmapa.shared::cluster.u32 remote, %4, %5;\n\tld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [remote];\n\t}"
+                       : "=f"(part.x), "=f"(part.y), "=f"(part.z), "=f"(part.w) : "r"(at), "r"(r) : "memory");
+          sum[0] += part.x;
+          sum[1] += part.y;
+          sum[2] += part.z;
+          sum[3] += part.w;
+        }
+        uint16_t out[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          if (p.bias) sum[i] += bias[i];
+          out[i] = p.half_io ? __half_as_ushort(__float2half_rn(sum[i])) : __bfloat16_as_ushort(__float2bfloat16(sum[i]));
+        }
+        uint16_t *dst = reinterpret_cast<uint16_t *>(p.y) + size_t(tok0 + tok) * p.M + row;
+        if (wide) {
+          if (rows == 4) *reinterpret_cast<uint2 *>(dst) = make_uint2(out[0] | (unsigned(out[1]) << 16), out[2] | (unsigned(out[3]) << 16));
+        } else {
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            if (i < rows) dst[i] = out[i];
+        }
+      }
+    }
+    cluster_sync();                        // no CTA leaves while another reads its sums
+  }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (CTAS == 2) cluster_sync();           // neither CTA leaves while the other's tensor core or barriers may still reach it
@@ -616,7 +672,7 @@ bool prefill_tile_eligible(const Handle *h, int backend, int tokens) {
 }
 
 // Short prompts on matrices with few rows leave most SMs without a CTA (5120 rows = 40 CTAs of 128 rows): K is
-// then cut into ranges, one CTA per (row block, token block, range), fp32 sums combined by a second kernel.  The
+// then cut into ranges, one CTA per (row block, token block, range), whose fp32 sums are added in the order of the ranges.  The
 // number of ranges depends on the matrix and the token count only -- never on the tile -- so that all tiles keep
 // adding in the same order and stay bitwise identical to each other (the autotuner's admission rule).
 static int prefill_k_ranges(const Handle *h, int tokens, const Workspace *ws) {
@@ -665,20 +721,56 @@ int prefill_choose_backend(const Handle *h, int tokens) {
   return pick;
 }
 
-// One launch of the tile over `n` staged tokens, and the combine behind it where K is cut.
+// What a tile's instance is asked for once per device: its shared memory, and how many clusters of 2 to 8 K ranges are resident at once.
+struct TileSetup {
+  bool ready = false;
+  int clusters[9] = {-1, -1, -1, -1, -1, -1, -1, -1, -1};   // -1: not asked yet
+};
+
+template <int CTAS, int BN, typename Kernel>
+static int resident_clusters(Kernel kernel, int ranges, int sm_count) {
+  cudaLaunchConfig_t config{};
+  cudaLaunchAttribute attribute{};
+  config.gridDim = dim3(unsigned(sm_count / ranges), 1, unsigned(ranges));
+  config.blockDim = dim3(kPrefillThreads);
+  config.dynamicSmemBytes = TileConfig<CTAS, BN>::smem;
+  attribute.id = cudaLaunchAttributeClusterDimension;
+  attribute.val.clusterDim.x = attribute.val.clusterDim.y = 1;
+  attribute.val.clusterDim.z = unsigned(ranges);
+  config.attrs = &attribute;
+  config.numAttrs = 1;
+  int found = 0;
+  if (cudaOccupancyMaxActiveClusters(&found, kernel, &config) == cudaSuccess) return found;
+  cudaGetLastError();
+  return 0;
+}
+
+// One launch of the tile over `n` staged tokens, and where K is cut the sum of its ranges: inside the launch, by clusters, where all of them are
+// resident at once (a cluster waits for as many free SMs of one GPC as it has CTAs), else by a combine behind it.  By clusters / by a combine, us a
+// call from HBM with 16, 64 and 128 tokens on the 64-token tile: 256x2048 6.3, 6.9, 7.3 / 7.7, 7.9, 8.9; 5120x5120 10.2, 12.6, 21.7 / 12.1, 14.0,
+// 22.7; 5120x17408 19.8, 24.4, 42.5 / 22.7, 26.8, 46.5; 8192x28672 39.5, 44.5, 84.6 / 44.1, 48.4, 88.3.  No shape was slower.
 template <int CTAS, int BN>
 static int launch_staged_tile(const Handle *h, const Workspace *ws, const __half *staged, const float *xmul, __nv_bfloat16 *y, int n, cudaStream_t stream, bool half_io) {
   using Cfg = TileConfig<CTAS, BN>;
   // the lean variant decodes high-mode blocks of the software palette and nothing else
   const bool generic = h->has_low_mode || h->palette == TX_PALETTE_HARDWARE;
   const auto kernel = generic ? prefill_umma_kernel<CTAS, BN, true> : prefill_umma_kernel<CTAS, BN, false>;
+  const int ranges = prefill_k_ranges(h, n, ws);
+  dim3 grid((h->M + Cfg::rows - 1) / Cfg::rows * CTAS, (n + BN - 1) / BN, ranges);
+  bool merge = CTAS == 1 && ranges > 1;
   static std::mutex guard;
-  static std::map<std::pair<int, bool>, bool> configured;
+  static std::map<std::pair<int, bool>, TileSetup> configured;
   {
     std::lock_guard<std::mutex> lock(guard);
-    if (!configured[{h->device, generic}]) {
+    TileSetup &setup = configured[{h->device, generic}];
+    if (!setup.ready) {
       TX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(Cfg::smem)));
-      configured[{h->device, generic}] = true;
+      setup.ready = true;
+    }
+    if (merge) {
+      int &clusters = setup.clusters[ranges];        // (at most 8 ranges)
+      if (clusters < 0) clusters = resident_clusters<CTAS, BN>(kernel, ranges, ws->sm_count);
+      merge = int(grid.x * grid.y) <= clusters;
     }
   }
   const int KP = h->KI * 128, padded_tokens = padded_prompt(n);
@@ -708,12 +800,10 @@ static int launch_staged_tile(const Handle *h, const Workspace *ws, const __half
   p.T = n;
   p.palette = h->palette;
   p.half_io = half_io ? 1 : 0;
-  p.partial = ws->partial;
-  const int ranges = prefill_k_ranges(h, n, ws);
-  dim3 grid((h->M + Cfg::rows - 1) / Cfg::rows * CTAS, (n + BN - 1) / BN, ranges);
-  TX_CUDA(launch_pdl_cluster(kernel, CTAS, grid, dim3(kPrefillThreads), Cfg::smem, stream, p, map));
+  p.partial = merge ? nullptr : ws->partial;
+  TX_CUDA(launch_pdl_cluster(kernel, merge ? dim3(1, 1, ranges) : dim3(CTAS), grid, dim3(kPrefillThreads), Cfg::smem, stream, p, map));
   count_launch();
-  if (ranges > 1) return launch_combine(ws->partial, ranges, h->bias, y, n, h->M, half_io, ws->sm_count, stream);
+  if (ranges > 1 && !merge) return launch_combine(ws->partial, ranges, h->bias, y, n, h->M, half_io, ws->sm_count, stream);
   return TX_OK;
 }
 
