@@ -330,3 +330,24 @@ def test_k_ranges_add_to_the_sums_of_their_columns(ext, lut, m, k, tokens, dtype
         assert ext.kernel_status() == 0
     finally:
         ext.free(h)
+
+
+@pytest.mark.parametrize("m,k,tokens", [(19072, 16, 17), (18945, 144, 64), (22016, 400, 65), (37889, 128, 33), (9600, 272, 200), (7000, 2080, 900)])
+def test_two_tiles_an_sm_are_bitwise_the_tile_of_one(ext, lut, m, k, tokens):
+    """Grids of more CTAs than SMs run the 64- and 128-token tiles as two small CTAs an SM (three and two stages): the bits of the wide tiles,
+    with one unit, fewer units than stages, ragged rows and tokens."""
+    rng = np.random.default_rng(m)
+    ends = np.sort(rng.integers(-127, 128, (2, m, k // 16)), 0)[::-1].astype(np.int8)
+    blocks = O.pack_blocks(ends[0], ends[1], rng.integers(0, 8, (m, k // 16, 16)).astype(np.uint8)).reshape(-1)
+    h = _pack(ext, blocks, (rng.random(m) + 0.5).astype(np.float32))
+    try:
+        x = torch.randn(tokens, k, device="cuda", generator=torch.Generator(device="cuda").manual_seed(k)).bfloat16()
+        ext.set_prefill(h, 1, 1024)
+        outs = []
+        for backend in (5, 7, 8):
+            ext.set_prefill_backend(h, backend)
+            outs.append(ext.linear(h, x))
+        assert torch.equal(outs[1], outs[0]) and torch.equal(outs[2], outs[0])
+        assert ext.kernel_status() == 0
+    finally:
+        ext.free(h)

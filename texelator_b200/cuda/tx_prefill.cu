@@ -42,13 +42,11 @@
 namespace tx {
 
 constexpr int kMmaM = 128;               // rows of a CTA's accumulator (TMEM lanes)
-// Sixteen producer warps: warp w reaches the TMEM lanes of quarter w & 3 only, holds one of that quarter's two 16-row
-// tiles and decodes whole 128-column units of it on alternate pipeline stages.
-constexpr int kProducerWarps = 16;
-constexpr int kGroups = 2;                      // groups of producer warps that take alternate units
+// Eight producer warps a group: warp w reaches the TMEM lanes of quarter w & 3 only, holds one of that quarter's two 16-row
+// tiles and decodes whole 128-column units of it.  Two groups take alternate pipeline stages;
+// a CTA of one group (tiles up to 128 tokens) is small enough for two on an SM, which then set up, fill their pipelines and store at different
+// times (two_an_sm).
 constexpr int kLook = 2;                        // units of its row a producer warp keeps in flight as register loads
-constexpr int kTmaWarp = kProducerWarps, kMmaWarp = kProducerWarps + 1;
-constexpr int kPrefillThreads = (kProducerWarps + 2) * 32;   // producer/epilogue warps + TMA warp + MMA warp
 constexpr unsigned kSpinLimit = 1u << 22;
 constexpr unsigned kDrainLimit = 1u << 20;      // polls per stage for copies in flight after an abort
 constexpr int kBK = 128;                        // columns per pipeline stage: one unit of the payload
@@ -58,17 +56,19 @@ constexpr int kAColumns = kBK / 2;              // TMEM columns of one A stage (
 // One tile shape: CTAS x 128 output rows x BN tokens.  The accumulator takes BN columns of every CTA's TMEM, the ring of
 // decoded A stages the columns behind it; shared memory holds the activations alone, and with CTAS = 2 each CTA keeps
 // half of the tokens (the tensor cores of a pair read both halves).
-template <int CTAS, int BN> struct TileConfig {
+template <int CTAS, int BN, int GROUPS = 2> struct TileConfig {
+  static constexpr int producers = 8 * GROUPS;
+  static constexpr int threads = (producers + 2) * 32;        // producer/epilogue warps + TMA warp + MMA warp
+  static constexpr int tmem_columns = GROUPS == 2 ? 512 : 256;
   static constexpr int rows = CTAS * kMmaM;
   static constexpr int tokens = BN / CTAS;                    // tokens this CTA stages
   static constexpr int b_lbo = tokens * 16;
   static constexpr int b_stage = kChunks * b_lbo;
   static constexpr int fixed = 1024 /*alignment*/ + 256 /*barriers*/;
-  static constexpr int fit_smem = (220 * 1024 - fixed) / b_stage, fit_tmem = (512 - BN) / kAColumns;
+  static constexpr int fit_smem = (220 * 1024 - fixed) / b_stage, fit_tmem = (tmem_columns - BN) / kAColumns;
   static constexpr int fit = fit_smem < fit_tmem ? fit_smem : fit_tmem;
   static constexpr int stages = fit > 6 ? 6 : fit;
   static constexpr size_t smem = fixed + size_t(stages) * b_stage;
-  static constexpr int tmem_columns = 512;
   static_assert(stages >= 2, "tile does not fit two pipeline stages");
   static_assert(BN + stages * kAColumns <= tmem_columns, "accumulator and A stages must fit TMEM");
   static_assert(tokens % 32 == 0 && BN % 32 == 0 && BN <= 256, "the activation box is made of 32-token runs; N is at most 256");
@@ -322,10 +322,11 @@ __global__ void __launch_bounds__(kSplitThreads) stage_split_kernel(const __nv_b
   stage_split_row(reinterpret_cast<uint4 *>(out), xmul, K, padded_tokens, half_in != 0, [&](int i) { return __ldcg(row + i); });
 }
 
-template <int CTAS, int BN, bool GENERIC>
-__global__ void __launch_bounds__(kPrefillThreads, 1)
+template <int CTAS, int BN, bool GENERIC, int GROUPS>
+__global__ void __launch_bounds__(TileConfig<CTAS, BN, GROUPS>::threads, GROUPS == 2 ? 1 : 2)
 prefill_umma_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap x_map) {
-  using Cfg = TileConfig<CTAS, BN>;
+  using Cfg = TileConfig<CTAS, BN, GROUPS>;
+  constexpr int kProducerWarps = Cfg::producers, kGroups = GROUPS, kTmaWarp = kProducerWarps, kMmaWarp = kProducerWarps + 1;
   constexpr int S = Cfg::stages;
   extern __shared__ uint8_t smem_raw[];
   const unsigned sbase = unsigned(__cvta_generic_to_shared(smem_raw));
@@ -346,7 +347,7 @@ prefill_umma_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap x
   const int u0 = int(blockIdx.z) * p.KI / int(gridDim.z), u1 = (int(blockIdx.z) + 1) * p.KI / int(gridDim.z);
   const int KT = u1 - u0;
   const int row0 = blockIdx.x * kMmaM, tok0 = blockIdx.y * BN;
-  const bool merge = CTAS == 1 && gridDim.z > 1 && p.partial == nullptr;
+  const bool merge = CTAS == 1 && GROUPS == 2 && gridDim.z > 1 && p.partial == nullptr;
 
   if (tid == 0) {
     for (int s = 0; s < S; ++s) {
@@ -682,11 +683,24 @@ static int prefill_k_ranges(const Handle *h, int tokens, const Workspace *ws) {
   return std::max(ranges, 1);
 }
 
+// Whether a tile of at most 128 tokens runs as two small CTAs an SM (half the producers, registers and TMEM each).  A CTA alone on its SM spends
+// 3 to 4 us before and after its stages with the tensor core and the memory idle, and 272 CTAs on 148 SMs cost as much as 296; two on an SM fill
+// each other's gaps.  They lose where rounding the grid up to two an SM costs a wave and the rows are long enough to show it.  One / two an SM, us a
+// call from HBM, waves of one an SM before the figures -- 64 tokens: 24576x1024 2: 11.9 / 9.6; 22016x2048 2: 16.3 / 14.2; 34816x5120 2: 32.8 / 30.3;
+// 57344x8192 4: 85.9 / 79.6.  With the 128-token tile: 22016x2048 2: 20.1 / 17.5, 3: 29.1 / 27.1, 7: 65.0 / 59.8; 19200x4096 3: 43.0 / 44.9,
+// 7: 106.4 / 101.0; 28672x8192 4: 100.3 / 92.8, 5: 141.6 / 144.1; 24576x1024 8: 52.0 / 38.6.
+static bool two_an_sm(long ctas, int ranges, int units, int sm_count) {
+  const long one = (ctas + sm_count - 1) / sm_count, two = (ctas + 2 * sm_count - 1) / (2 * sm_count);
+  return ranges == 1 && one > 1 && (2 * two <= one || one >= 7 || units <= 16);
+}
+
 // The tile of handles without a tuned backend (ids 0..4; 5..9 name one): all tiles give the same bits, so only time decides.
 // A wave of CTAs takes its 128-column stages at the pace of the MMAs or, below 128 tokens, of the producers, plus
 // what a CTA spends before and after them (TMEM, first loads, epilogue).  Measured on 5120x17408 with 512 tokens
 // (136 stages): 0.30, 0.35, 0.50 and 0.67 us a stage for 64, 128, 192 and 256 tokens and about 4 us a CTA; the tile with
-// the smallest sum over the waves wins, the wider one on a tie (it reads the activations less often).  The pair tile (id 6)
+// the smallest sum over the waves wins, the wider one on a tie (it reads the activations less often).  The sums are those of one CTA an SM also where
+// two_an_sm would take two: the line then lies a little late for short rows (24576x1024 with 700 tokens: 128-token tile 38.6, 192 tokens 42.5 us).
+// The pair tile (id 6)
 // is left out: against the 256-token tile it measured between 6 % less and 13 % more for 512 to 4096 tokens, by the
 // GPU's power state more than by shape, and never less below that.
 //
@@ -732,7 +746,7 @@ static int resident_clusters(Kernel kernel, int ranges, int sm_count) {
   cudaLaunchConfig_t config{};
   cudaLaunchAttribute attribute{};
   config.gridDim = dim3(unsigned(sm_count / ranges), 1, unsigned(ranges));
-  config.blockDim = dim3(kPrefillThreads);
+  config.blockDim = dim3(TileConfig<CTAS, BN>::threads);
   config.dynamicSmemBytes = TileConfig<CTAS, BN>::smem;
   attribute.id = cudaLaunchAttributeClusterDimension;
   attribute.val.clusterDim.x = attribute.val.clusterDim.y = 1;
@@ -749,15 +763,15 @@ static int resident_clusters(Kernel kernel, int ranges, int sm_count) {
 // resident at once (a cluster waits for as many free SMs of one GPC as it has CTAs), else by a combine behind it.  By clusters / by a combine, us a
 // call from HBM with 16, 64 and 128 tokens on the 64-token tile: 256x2048 6.3, 6.9, 7.3 / 7.7, 7.9, 8.9; 5120x5120 10.2, 12.6, 21.7 / 12.1, 14.0,
 // 22.7; 5120x17408 19.8, 24.4, 42.5 / 22.7, 26.8, 46.5; 8192x28672 39.5, 44.5, 84.6 / 44.1, 48.4, 88.3.  No shape was slower.
-template <int CTAS, int BN>
-static int launch_staged_tile(const Handle *h, const Workspace *ws, const __half *staged, const float *xmul, __nv_bfloat16 *y, int n, cudaStream_t stream, bool half_io) {
-  using Cfg = TileConfig<CTAS, BN>;
+template <int CTAS, int BN, int GROUPS>
+static int launch_staged_groups(const Handle *h, const Workspace *ws, const __half *staged, const float *xmul, __nv_bfloat16 *y, int n, cudaStream_t stream, bool half_io) {
+  using Cfg = TileConfig<CTAS, BN, GROUPS>;
   // the lean variant decodes high-mode blocks of the software palette and nothing else
   const bool generic = h->has_low_mode || h->palette == TX_PALETTE_HARDWARE;
-  const auto kernel = generic ? prefill_umma_kernel<CTAS, BN, true> : prefill_umma_kernel<CTAS, BN, false>;
+  const auto kernel = generic ? prefill_umma_kernel<CTAS, BN, true, GROUPS> : prefill_umma_kernel<CTAS, BN, false, GROUPS>;
   const int ranges = prefill_k_ranges(h, n, ws);
   dim3 grid((h->M + Cfg::rows - 1) / Cfg::rows * CTAS, (n + BN - 1) / BN, ranges);
-  bool merge = CTAS == 1 && ranges > 1;
+  bool merge = CTAS == 1 && GROUPS == 2 && ranges > 1;
   static std::mutex guard;
   static std::map<std::pair<int, bool>, TileSetup> configured;
   {
@@ -801,10 +815,18 @@ static int launch_staged_tile(const Handle *h, const Workspace *ws, const __half
   p.palette = h->palette;
   p.half_io = half_io ? 1 : 0;
   p.partial = merge ? nullptr : ws->partial;
-  TX_CUDA(launch_pdl_cluster(kernel, merge ? dim3(1, 1, ranges) : dim3(CTAS), grid, dim3(kPrefillThreads), Cfg::smem, stream, p, map));
+  TX_CUDA(launch_pdl_cluster(kernel, merge ? dim3(1, 1, ranges) : dim3(CTAS), grid, dim3(Cfg::threads), Cfg::smem, stream, p, map));
   count_launch();
   if (ranges > 1 && !merge) return launch_combine(ws->partial, ranges, h->bias, y, n, h->M, half_io, ws->sm_count, stream);
   return TX_OK;
+}
+
+template <int CTAS, int BN>
+static int launch_staged_tile(const Handle *h, const Workspace *ws, const __half *staged, const float *xmul, __nv_bfloat16 *y, int n, cudaStream_t stream, bool half_io) {
+  constexpr bool small = CTAS == 1 && BN <= 128;
+  if (small && two_an_sm(long(h->M + kMmaM - 1) / kMmaM * ((n + BN - 1) / BN), prefill_k_ranges(h, n, ws), h->KI, ws->sm_count))
+    return launch_staged_groups<CTAS, BN, small ? 1 : 2>(h, ws, staged, xmul, y, n, stream, half_io);
+  return launch_staged_groups<CTAS, BN, 2>(h, ws, staged, xmul, y, n, stream, half_io);
 }
 
 template <int CTAS, int BN>
@@ -884,10 +906,10 @@ template <int CTAS, int BN>
 static int tile_info(int64_t out[9]) {
   using Cfg = TileConfig<CTAS, BN>;
   cudaFuncAttributes attributes{};
-  TX_CUDA(cudaFuncGetAttributes(&attributes, prefill_umma_kernel<CTAS, BN, false>));
-  TX_CUDA(cudaFuncSetAttribute(prefill_umma_kernel<CTAS, BN, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(Cfg::smem)));
+  TX_CUDA(cudaFuncGetAttributes(&attributes, prefill_umma_kernel<CTAS, BN, false, 2>));
+  TX_CUDA(cudaFuncSetAttribute(prefill_umma_kernel<CTAS, BN, false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(Cfg::smem)));
   int active = 0;
-  TX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&active, prefill_umma_kernel<CTAS, BN, false>, kPrefillThreads, Cfg::smem));
+  TX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&active, prefill_umma_kernel<CTAS, BN, false, 2>, Cfg::threads, Cfg::smem));
   out[0] = attributes.numRegs;
   out[1] = int64_t(attributes.sharedSizeBytes);
   out[2] = int64_t(attributes.localSizeBytes);
