@@ -4,10 +4,11 @@ The reference has no serving loop of its own; a batch reaches its operator as th
 ``linear`` call, and every token count below the prefill threshold goes to the decode GEMV with one grid
 row per token (``texelator/cuda/texelator_cuda.cu:1438-1468``), which streams the whole matrix once per
 token.  Here the B rows of a step go through the multi-token decode kernel, which reads the matrix once
-for up to sixteen of them (each CTA of a cluster stages its share of every activation row), and the
-steps between the linears are the library's glue kernels with a batch dimension:
+for up to sixteen of them (each CTA of a cluster stages its share of every activation row), or through a
+tensor-core tile (``tune_decode_kernel``), and the steps between the linears are the library's glue kernels with a
+batch dimension; where a tile takes the rows, norms (and SwiGLU with long rows) write the form that it reads:
 
-    add_rmsnorm [B, hidden] -> qkv linear -> attention_step_batch (RoPE, cache append, attention of every
+    embed_rmsnorm / add_rmsnorm [B, hidden] -> qkv linear -> attention_step_batch (RoPE, cache append, attention of every
     sequence at its own position) -> o linear (+ all-reduce) -> add_rmsnorm -> gate/up linear ->
     silu_mul_pairs -> down linear (+ all-reduce)
 

@@ -7,6 +7,7 @@
 //
 //   pre-pass   one small kernel rescales the activations per token by an exact power of two and stores
 //              them as fp16 (the decode GEMV's staging) in the chunk-major order of the B operand;
+//   (threads below: one CTA an SM; the small form of the narrow tiles has eight producer warps)
 //   warps 0-15 producers: 128-bit loads of the tiled BC4 payload, decode in registers exactly like the decode GEMV
 //              (masked index fields + HFMA2 -> exact numerators n * 2^-16, n = 7*e0 + g*(e1-e0), as fp16) and
 //              tcgen05.st of the A stage into TMEM: the payload's lane order is the 16x256b fragment order, so

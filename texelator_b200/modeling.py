@@ -342,8 +342,8 @@ class BC4Decoder:
         return not dense and c.head_dim % 16 == 0 and c.head_dim <= 256 and c.hidden % 8 == 0 and c.hidden <= 16384 and self.i_loc % 8 == 0
 
     def _prompt_stack(self, h):
-        """All layers and the final norm over the prompt rows ``h [T, hidden]`` (overwritten): nine launches a layer with the
-        rounding points of ``_layer``.  Written with PyTorch ops the same layer is 58 launches that move the gate/up rows
+        """All layers and the final norm over the prompt rows ``h [T, hidden]`` (overwritten) with the rounding points of ``_layer``.  Norms and,
+        for few tokens, SwiGLU write the tile's staged form, so that only the other linears stage their rows in a launch of their own.  Written with PyTorch ops the same layer is 58 launches that move the gate/up rows
         (the widest of the layer) seven times in fp32; the host could not keep the GPU busy with them and they
         cost more than half of what the linears did."""
         c, ext = self.config, self.ext

@@ -452,7 +452,8 @@ class _Extension:
 
     def attention_step(self, qkv, cos, sin, position, k_cache, v_cache, scratch, out, q_heads: int, kv_heads: int,
                        head_dim: int) -> None:
-        """RoPE + cache append + single-query attention + split merge of one token in one launch."""
+        """RoPE + cache append + single-query attention of one token in one call; old cache rows and the position are read before the launch in
+        front has finished, so it must not be what writes them."""
         if scratch.numel() < self.attention_step_scratch_floats(q_heads, k_cache.shape[1]):
             raise ValueError("attention_step scratch is too small for this cache length")
         self._check(self._lib.tx_aux_attention_step(qkv.data_ptr(), cos.data_ptr(), sin.data_ptr(), position.data_ptr(),
@@ -462,7 +463,7 @@ class _Extension:
 
     def attention_step_batch(self, qkv, cos, sin, positions, k_cache, v_cache, scratch, out, q_heads: int, kv_heads: int,
                              head_dim: int) -> None:
-        """``attention_step`` for one token of each sequence of a batch in one launch: ``qkv [B, ...]``, ``positions``
+        """``attention_step`` for one token of each sequence of a batch: ``qkv [B, ...]``, ``positions``
         int64 ``[B]``, caches ``[B, kv_heads, max_len, head_dim]``, ``out [B, q_heads * head_dim]``."""
         sequences, max_len = k_cache.shape[0], k_cache.shape[2]
         if qkv.shape[0] != sequences or positions.numel() != sequences or not (k_cache.is_contiguous() and v_cache.is_contiguous()):
