@@ -596,6 +596,7 @@ prefill_umma_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap x
   if (merge) {
     // The ranges of this tile, in order, bias, one rounding: launch_combine's sums to the bit, without its launch and without [ranges][T][M] floats
     // through global memory.  A CTA takes every gridDim.z-th token, a warp a token, a lane four rows (a row of sums is one conflict-free read).
+    __syncwarp();                          // (the cluster barrier wants whole warps, and the roles end in single lanes)
     cluster_sync();
     const bool whole = !*abort_flag;       // (an abort is reported; what this CTA would add is not there)
     if (warp < kProducerWarps && whole) {
@@ -635,6 +636,7 @@ prefill_umma_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap x
         }
       }
     }
+    __syncwarp();
     cluster_sync();                        // no CTA leaves while another reads its sums
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
