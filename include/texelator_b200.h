@@ -231,7 +231,9 @@ int tx_kernel_status(int device, int clear);
  *                      (they overlap that launch's tail): they must be complete when that launch starts, as they
  *                      are in a decode loop, where earlier steps wrote them, and behind rope_append_prompt;
  *                      rope_append and attention_step itself let the launches behind them start early, so a
- *                      step over rows they wrote needs a launch that is not one of this library's in between
+ *                      step over rows they wrote needs a launch that is not one of this library's in between.
+ *                      That the writer lies several launches back is not enough where all between are early ones; a
+ *                      kernel of another library, or embed_rmsnorm, starts when everything in front of it has ended
  *   silu_mul         : out[t,i] = silu(gate_up[t,i]) * gate_up[t,intermediate+i]                     */
 int tx_aux_add_rmsnorm(void *h, const void *delta, const void *weight, void *y, int tokens, int hidden, float eps, void *stream);
 /* The same with rows of h taken from an embedding table [vocab, hidden] first: h[r] = table[row_tokens[r]]; a token outside the table records

@@ -9,8 +9,17 @@ class _KernelNode(ctypes.Structure):          # CUDA_KERNEL_NODE_PARAMS_v2
                 ("params", ctypes.c_void_p), ("extra", ctypes.c_void_p), ("kern", ctypes.c_void_p), ("context", ctypes.c_void_p)]
 
 
+class _EdgeData(ctypes.Structure):            # CUgraphEdgeData
+    _fields_ = [("from_port", ctypes.c_ubyte), ("to_port", ctypes.c_ubyte), ("type", ctypes.c_ubyte), ("reserved", ctypes.c_ubyte * 5)]
+
+
 def launched(call):
     """``[(mangled name, grid)]`` of one call, in launch order (``call`` runs once before it is recorded)."""
+    return [(name, grid) for name, grid, _ in recorded(call)]
+
+
+def recorded(call):
+    """``[(mangled name, grid, early)]``: ``early`` where the kernel may start before the launch in front of it has ended."""
     call()
     torch.cuda.synchronize()
     graph = torch.cuda.CUDAGraph(keep_graph=True)
@@ -25,6 +34,12 @@ def launched(call):
     check(driver.cuGraphGetNodes(handle, None, ctypes.byref(count)))
     nodes = (ctypes.c_void_p * count.value)()
     check(driver.cuGraphGetNodes(handle, nodes, ctypes.byref(count)))
+    edges = ctypes.c_size_t(0)
+    check(driver.cuGraphGetEdges_v2(handle, None, None, None, ctypes.byref(edges)))
+    sources, targets, data = (ctypes.c_void_p * edges.value)(), (ctypes.c_void_p * edges.value)(), (_EdgeData * edges.value)()
+    if edges.value:
+        check(driver.cuGraphGetEdges_v2(handle, sources, targets, data, ctypes.byref(edges)))
+    early = {target for target, edge in zip(targets, data) if edge.type == 1}      # CU_GRAPH_DEPENDENCY_TYPE_PROGRAMMATIC
     found = []
     for node in nodes:
         kind = ctypes.c_int(-1)
@@ -37,5 +52,5 @@ def launched(call):
             check(driver.cuKernelGetName(ctypes.byref(name), ctypes.c_void_p(params.kern)))
         else:
             check(driver.cuFuncGetName(ctypes.byref(name), ctypes.c_void_p(params.func)))
-        found.append((name.value.decode(), tuple(params.grid)))
+        found.append((name.value.decode(), tuple(params.grid), node in early))
     return found

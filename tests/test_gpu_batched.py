@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 import torch
 
+from graph_kernels import recorded
 from oracle import bc4_oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -208,5 +209,30 @@ def test_capture_on_the_last_cache_row(batch):
         model.decode_graph()
         model.check_status()
         assert model.pos.tolist() == [p + 1 for p in positions]
+    finally:
+        model.free()
+
+
+@pytest.mark.parametrize("batch", [1, 3, 16])
+def test_a_step_starts_behind_the_whole_step_before(batch):
+    """The attention kernel reads the position, which ends a step, before it waits for the launches in front of it; these may all start early,
+    so the first launch of a step must not: eager steps behind one another read a finished position."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    from texelator_b200.batched import BatchedBC4Decoder
+    from texelator_b200.modeling import BC4Decoder, CONFIGS
+    config = CONFIGS["toy128"]
+    model = BC4Decoder(config, "cuda:0", max_len=40, seed=2) if batch == 1 else BatchedBC4Decoder(config, "cuda:0", max_len=40, batch=batch, seed=2)
+    step = model._decode_step_fused if batch == 1 else model.decode_step
+    try:
+        with torch.no_grad():
+            kernels = recorded(lambda: (step(), step()))
+        attention = [i for i, (name, _, _) in enumerate(kernels) if "attention_step" in name]
+        assert len(attention) == 2 * config.layers and any(early for _, _, early in kernels)
+        first = attention[config.layers]                     # of the second step
+        between = [early for _, _, early in kernels[attention[config.layers - 1] + 1:first + 1]]
+        writer = max(i for i, (name, _, _) in enumerate(kernels[:first]) if "N2tx" not in name)    # the step before ends with the position
+        assert not all(early for _, _, early in kernels[writer + 1:first + 1]), (between, writer, first)
+        model.check_status()
     finally:
         model.free()

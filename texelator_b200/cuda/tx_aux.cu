@@ -1743,8 +1743,11 @@ int tx_aux_embed_rmsnorm(const void *table, int64_t vocab, const int64_t *row_to
   Workspace *ws = workspace_for(device);
   if (!ws) return TX_ECUDA;
   const EmbedRows embed{static_cast<const __nv_bfloat16 *>(table), reinterpret_cast<const long long *>(row_tokens), vocab, ws->status};
-  TX_CUDA(launch_pdl(add_rmsnorm_kernel<true, false>, dim3(tokens), dim3(kNormThreads), 0, static_cast<cudaStream_t>(stream), static_cast<__nv_bfloat16 *>(h),
-                     static_cast<const __nv_bfloat16 *>(nullptr), static_cast<const __nv_bfloat16 *>(weight), static_cast<__nv_bfloat16 *>(y), hidden, eps, embed));
+  // A plain launch: it opens a decode step, and attention_step reads the position (which the step before ended with) without waiting for the launches
+  // between them, all of which let the next one start early.
+  TX_CUDA(launch_cluster(add_rmsnorm_kernel<true, false>, false, 1, dim3(tokens), dim3(kNormThreads), 0, static_cast<cudaStream_t>(stream),
+                         static_cast<__nv_bfloat16 *>(h), static_cast<const __nv_bfloat16 *>(nullptr), static_cast<const __nv_bfloat16 *>(weight),
+                         static_cast<__nv_bfloat16 *>(y), hidden, eps, embed));
   count_launch();
   TX_CUDA(cudaGetLastError());
   return TX_OK;
