@@ -207,7 +207,8 @@ int tx_unpack_blocks(uint64_t handle, uint8_t *out_host);
 
 /* New: device status word.  Kernels never spin without a limit; when a bounded wait of the tensor-core
  * prefill kernel runs out it records a positive code here and returns early (1: a producer, 2: the TMA lane waiting
- * for a free stage; 3: a full stage; 5: the accumulators).  Synchronises the device; returns the code (0 = healthy)
+ * for a free stage; 3: a full stage; 5: the accumulators; 32: a peer that did not deliver).  33 is no wait: a token outside
+ * the vocabulary (tx_aux_embed_rmsnorm).  Synchronises the device; returns the code (0 = healthy)
  * or a negative TX_E* value; `clear` resets it. */
 int tx_kernel_status(int device, int clear);
 
@@ -237,9 +238,12 @@ int tx_kernel_status(int device, int clear);
  *   silu_mul         : out[t,i] = silu(gate_up[t,i]) * gate_up[t,intermediate+i]                     */
 int tx_aux_add_rmsnorm(void *h, const void *delta, const void *weight, void *y, int tokens, int hidden, float eps, void *stream);
 /* The same with rows of h taken from an embedding table [vocab, hidden] first: h[r] = table[row_tokens[r]]; a token outside the table records
- * code 33 in the device status word (tx_kernel_status) and takes row 0. */
+ * code 33 in the device status word (tx_kernel_status), takes row 0 and leaves a row of y that is not a number.  _watched: 1 is stored to *unknown
+ * too (mapped host memory: the host learns of it without a synchronisation). */
 int tx_aux_embed_rmsnorm(const void *table, int64_t vocab, const int64_t *row_tokens, void *h, const void *weight, void *y, int tokens, int hidden,
                          float eps, int device, void *stream);
+int tx_aux_embed_rmsnorm_watched(const void *table, int64_t vocab, const int64_t *row_tokens, void *h, const void *weight, void *y, int tokens, int hidden,
+                                 float eps, int *unknown, int device, void *stream);
 /* tx_aux_add_rmsnorm and tx_aux_silu_mul_pairs with the result in staged form (tx_linear_staged) instead of rows */
 int tx_aux_add_rmsnorm_staged(void *h, const void *delta, const void *weight, void *staged, int tokens, int hidden, float eps, void *stream);
 int tx_aux_silu_mul_pairs_staged(const void *gate_up, void *staged, int tokens, int intermediate, int accurate, void *stream);

@@ -236,3 +236,39 @@ def test_a_step_starts_behind_the_whole_step_before(batch):
         model.check_status()
     finally:
         model.free()
+
+
+@pytest.mark.parametrize("batch", [1, 3, 16])
+def test_a_token_outside_the_vocabulary_ends_the_decoder_s_next_call(batch):
+    """Steps are asynchronous: the step itself leaves a hidden state that is not a number, and the call behind it refuses; the other
+    sequences' states are those of a step without the token, and the decoder is usable again once the token is mended."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    from texelator_b200.batched import BatchedBC4Decoder
+    from texelator_b200.modeling import BC4Decoder, CONFIGS
+    config = CONFIGS["toy128"]
+    model = BC4Decoder(config, "cuda:0", max_len=40, seed=2) if batch == 1 else BatchedBC4Decoder(config, "cuda:0", max_len=40, batch=batch, seed=2)
+    eager = (lambda: model.decode_eager(fused=True)) if batch == 1 else model.decode_step
+    try:
+        model.capture()
+        for step in (eager, model.decode_graph):
+            start = (model.tok.clone(), model.pos.clone())
+            step()
+            want = model.last_hidden.clone()
+            model.tok.copy_(start[0]); model.pos.copy_(start[1])
+            model.tok[-1] = config.vocab
+            step()
+            torch.cuda.synchronize()
+            assert bool(model.last_hidden[-1].isnan().all()) and torch.equal(model.last_hidden[:-1], want[:-1])
+            with pytest.raises(RuntimeError, match="outside the vocabulary"):
+                step()
+            model.tok.copy_(start[0]); model.pos.copy_(start[1])
+            step()
+            assert torch.equal(model.last_hidden, want)
+            model.check_status()
+        model.tok[-1] = -1
+        with pytest.raises(RuntimeError, match="outside the vocabulary"):
+            model.capture()
+        assert model.ext.kernel_status() == 0
+    finally:
+        model.free()

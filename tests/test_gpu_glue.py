@@ -349,6 +349,23 @@ def test_embed_rmsnorm_is_a_gather_and_a_norm(ext, tokens, hidden):
     assert ext.kernel_status(clear=True) == 33 and torch.equal(h[-1], table[0])
 
 
+@pytest.mark.parametrize("tokens,hidden", [(1, 256), (5, 5120)])
+@pytest.mark.parametrize("bad", [-1, 50, 1 << 40])
+def test_embed_rmsnorm_of_an_unknown_token_is_not_a_number(ext, tokens, hidden, bad):
+    """The row of a token outside the table passes for no answer, the other rows are what they are, and the host sees the word without asking."""
+    gen = torch.Generator(device="cuda").manual_seed(hidden)
+    table, weight = torch.randn(50, hidden, device="cuda", generator=gen).bfloat16(), torch.randn(hidden, device="cuda", generator=gen).bfloat16()
+    ids = torch.randint(0, 50, (tokens,), device="cuda", generator=gen)
+    want_h, want_y = table[ids], torch.empty(tokens, hidden, dtype=torch.bfloat16, device="cuda")
+    ext.add_rmsnorm(want_h.clone(), None, weight, want_y, 1e-6)
+    ids[-1] = bad
+    h, y, unknown = torch.zeros_like(want_h), torch.zeros_like(want_y), torch.zeros(1, dtype=torch.int32).pin_memory()
+    ext.embed_rmsnorm(table, ids, h, weight, y, 1e-6, unknown)
+    torch.cuda.synchronize()
+    assert int(unknown[0]) == 1 and ext.kernel_status(clear=True) == 33
+    assert torch.equal(y[:-1], want_y[:-1]) and torch.equal(h[:-1], want_h[:-1]) and bool(y[-1].isnan().all())
+
+
 @pytest.mark.parametrize("sequences,q_heads,kv_heads,max_len,positions", [
     (16, 40, 8, 1040, [0, 1, 15, 16, 17, 63, 64, 65, 127, 128, 500, 640, 1000, 1023, 1024, 1039]),   # two splits: a cluster
     (3, 8, 8, 700, [699, 16, 448]),                          # a chunk a CTA, merged behind

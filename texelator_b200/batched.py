@@ -182,6 +182,7 @@ class BatchedBC4Decoder(BC4Decoder):
     @torch.no_grad()
     def decode_step(self) -> None:
         """One token for every sequence, library kernels only (this is what ``capture`` records)."""
+        self._refuse_unknown_token()
         c, ext = self.config, self.ext
         q_heads, kv_heads = c.q_heads // self.world, c.kv_heads // self.world
         staged = lambda handle: ext.takes_staged(handle, self.batch)     # the tile reads what the kernel in front leaves in its form
@@ -192,7 +193,7 @@ class BatchedBC4Decoder(BC4Decoder):
                 ext.linear_staged(self.h_qkv[layer], self.buf_staged, self.buf_qkv)
             else:
                 if layer == 0:
-                    ext.embed_rmsnorm(self.embed, self.tok, self.buf_h, self.norm1[layer], self.buf_x, c.rms_eps)
+                    ext.embed_rmsnorm(self.embed, self.tok, self.buf_h, self.norm1[layer], self.buf_x, c.rms_eps, self.unknown_token)
                 else:
                     ext.add_rmsnorm(self.buf_h, delta, self.norm1[layer], self.buf_x, c.rms_eps)
                 ext.linear_out(self.h_qkv[layer], self.buf_x, self.buf_qkv)
@@ -265,6 +266,7 @@ class BatchedBC4Decoder(BC4Decoder):
                     self.tok.copy_(saved[0]); self.pos.copy_(saved[1])
             self.tok.copy_(saved[0]); self.pos.copy_(saved[1])
             stream.synchronize()
+            self._refuse_unknown_token()
             before = self.ext.launch_count()
             graph = torch.cuda.CUDAGraph()
             with torch.cuda.graph(graph, stream=stream):
@@ -276,5 +278,6 @@ class BatchedBC4Decoder(BC4Decoder):
         self.graph, self.stream = graph, stream
 
     def decode_graph(self) -> None:
+        self._refuse_unknown_token()
         self.graph.replay()
 

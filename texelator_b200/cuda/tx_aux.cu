@@ -81,7 +81,8 @@ struct EmbedRows {
   const __nv_bfloat16 *table;   // [vocab, hidden]
   const long long *tokens;
   long long vocab;
-  int *status;                  // code 33: a token outside the table (row 0 is taken)
+  int *status;                  // code 33: a token outside the table.  h takes row 0 and y is not a number, so that nothing behind it passes for an answer
+  int *unknown;                 // 1 is stored here too (null: nowhere), where the host sees it without a synchronisation
 };
 // STAGED: y is the staged form of the rows (tx_decode.cuh) that the next linear's tile reads, instead of rows: no staging launch in between.
 template <bool EMBED, bool STAGED>
@@ -103,10 +104,15 @@ __global__ void __launch_bounds__(kNormThreads) add_rmsnorm_kernel(__nv_bfloat16
   uint4 *hr = reinterpret_cast<uint4 *>(h + size_t(row) * hidden);
   const uint4 *dr = delta ? reinterpret_cast<const uint4 *>(delta + size_t(row) * hidden) : nullptr;
   const uint4 *er = nullptr;
+  bool unknown = false;
   if (EMBED) {
     long long token = __ldcg(embed.tokens + row);
-    if (token < 0 || token >= embed.vocab) {
-      if (threadIdx.x == 0) atomicCAS(embed.status, 0, 33);
+    unknown = token < 0 || token >= embed.vocab;
+    if (unknown) {
+      if (threadIdx.x == 0) {
+        atomicCAS(embed.status, 0, 33);
+        if (embed.unknown) *static_cast<volatile int *>(embed.unknown) = 1;
+      }
       token = 0;
     }
     er = reinterpret_cast<const uint4 *>(embed.table + size_t(token) * hidden);
@@ -144,7 +150,7 @@ __global__ void __launch_bounds__(kNormThreads) add_rmsnorm_kernel(__nv_bfloat16
   float total = 0.f;
 #pragma unroll
   for (int w = 0; w < kNormThreads / 32; ++w) total += partial[w];
-  const float inv = rsqrtf(total / float(hidden) + eps);
+  const float inv = EMBED && unknown ? __int_as_float(0x7fffffff) : rsqrtf(total / float(hidden) + eps);
   uint4 *yr = reinterpret_cast<uint4 *>(y + size_t(row) * hidden);
   unsigned peak = 0;
 #pragma unroll
@@ -1738,11 +1744,16 @@ int tx_aux_add_rmsnorm_staged(void *h, const void *delta, const void *weight, vo
 
 int tx_aux_embed_rmsnorm(const void *table, int64_t vocab, const int64_t *row_tokens, void *h, const void *weight, void *y, int tokens, int hidden,
                          float eps, int device, void *stream) {
+  return tx_aux_embed_rmsnorm_watched(table, vocab, row_tokens, h, weight, y, tokens, hidden, eps, nullptr, device, stream);
+}
+
+int tx_aux_embed_rmsnorm_watched(const void *table, int64_t vocab, const int64_t *row_tokens, void *h, const void *weight, void *y, int tokens, int hidden,
+                                 float eps, int *unknown, int device, void *stream) {
   if (!table || !row_tokens || !h || !weight || !y || vocab < 1 || tokens < 1 || hidden < 8 || hidden % 8 || hidden > kNormThreads * 8 * kNormChunks)
     return fail(TX_EINVAL, "tx_aux_embed_rmsnorm: hidden must be a multiple of 8 and at most 16384");
   Workspace *ws = workspace_for(device);
   if (!ws) return TX_ECUDA;
-  const EmbedRows embed{static_cast<const __nv_bfloat16 *>(table), reinterpret_cast<const long long *>(row_tokens), vocab, ws->status};
+  const EmbedRows embed{static_cast<const __nv_bfloat16 *>(table), reinterpret_cast<const long long *>(row_tokens), vocab, ws->status, unknown};
   // A plain launch: it opens a decode step, and attention_step reads the position (which the step before ended with) without waiting for the launches
   // between them, all of which let the next one start early.
   TX_CUDA(launch_cluster(add_rmsnorm_kernel<true, false>, false, 1, dim3(tokens), dim3(kNormThreads), 0, static_cast<cudaStream_t>(stream),

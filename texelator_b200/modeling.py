@@ -233,6 +233,9 @@ class BC4Decoder:
             self.mask = torch.zeros(1, 1, 1, max_len, dtype=torch.bool, device=self.device)
             self.next_tok = torch.zeros(1, dtype=torch.int64, device=self.device)
             self.last_hidden = torch.zeros(1, c.hidden, dtype=torch.bfloat16, device=self.device)
+            # a step whose token is outside the vocabulary stores 1 here, where the host sees it without a synchronisation
+            self.unknown_token = torch.zeros(1, dtype=torch.int32).pin_memory()
+            self.unknown_seen = self.unknown_token.numpy()
             # static buffers of the fused decode step
             q_heads = c.q_heads // tp_world
             bf = dict(dtype=torch.bfloat16, device=self.device)
@@ -525,7 +528,7 @@ class BC4Decoder:
         for layer in range(c.layers):
             if not self.fuse_norm:
                 if layer == 0:
-                    ext.embed_rmsnorm(self.embed, self.tok, residual, self.norm1[layer], self.buf_x, c.rms_eps)
+                    ext.embed_rmsnorm(self.embed, self.tok, residual, self.norm1[layer], self.buf_x, c.rms_eps, self.unknown_token)
                 else:
                     self._add_norm(residual, delta, self.norm1[layer])
                 ext.linear_out(self.h_qkv[layer], self.buf_x, self.buf_qkv)
@@ -568,6 +571,7 @@ class BC4Decoder:
 
     @torch.no_grad()
     def decode_eager(self, dense: bool = False, fused: bool = False, single: bool = False) -> None:
+        self._refuse_unknown_token()
         if single:
             self._decode_step_single()
         elif fused:
@@ -596,6 +600,7 @@ class BC4Decoder:
                     self.tok.copy_(saved[0]); self.pos.copy_(saved[1]); self.mask.copy_(saved[2])
             self.tok.copy_(saved[0]); self.pos.copy_(saved[1]); self.mask.copy_(saved[2])
             stream.synchronize()
+            self._refuse_unknown_token()
             before = self.ext.launch_count()
             self.graph = torch.cuda.CUDAGraph()
             with torch.cuda.graph(self.graph, stream=stream):
@@ -607,14 +612,23 @@ class BC4Decoder:
         self.stream = stream
 
     def decode_graph(self) -> None:
+        self._refuse_unknown_token()
         self.graph.replay()
 
+    def _refuse_unknown_token(self) -> None:
+        """A step is asynchronous, so a token outside the vocabulary ends the decoder's next call (its own hidden state is not a number)."""
+        if self.unknown_seen[0]:
+            self.check_status()
+
     def check_status(self) -> None:
-        """Raise if any kernel of this rank gave up on a bounded wait (a peer that never delivered, a pipeline
-        barrier that never completed): whatever was decoded since the last check cannot be trusted then.
+        """Raise if a step met a token outside the vocabulary, or any kernel of this rank gave up on a bounded wait (a peer that never delivered, a
+        pipeline barrier that never completed): whatever was decoded since the last check cannot be trusted then.
         Synchronises the device; call it at host synchronisation points (every few tokens, or when a
         sequence ends), not per launch."""
         code = self.ext.kernel_status(clear=True, device=self.device.index)
+        unknown, self.unknown_seen[0] = self.unknown_seen[0] or code == 33, 0
+        if unknown:
+            raise RuntimeError("a decoded token lies outside the vocabulary; what was decoded from it since the last check is invalid")
         if code:
             raise RuntimeError(f"a device-side bounded wait ran out (status {code}); the tokens decoded since the last check are invalid")
 

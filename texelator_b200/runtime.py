@@ -68,6 +68,7 @@ C_API = {
     "tx_kernel_status": (_i32, [_i32, _i32]),
     "tx_aux_add_rmsnorm": (_i32, [_vp, _vp, _vp, _vp, _i32, _i32, ctypes.c_float, _vp]),
     "tx_aux_embed_rmsnorm": (_i32, [_vp, ctypes.c_int64, _vp, _vp, _vp, _vp, _i32, _i32, ctypes.c_float, _i32, _vp]),
+    "tx_aux_embed_rmsnorm_watched": (_i32, [_vp, ctypes.c_int64, _vp, _vp, _vp, _vp, _i32, _i32, ctypes.c_float, _vp, _i32, _vp]),
     "tx_staged_prompt_bytes": (_sz, [_i32, _i32]),
     "tx_linear_takes_staged": (_i32, [_u64, _i32]),
     "tx_linear_staged": (_i32, [_u64, _vp, _vp, _i32, _vp]),
@@ -413,11 +414,14 @@ class _Extension:
             raise RuntimeError("the staged buffer is too small")
         self._check(self._lib.tx_aux_silu_mul_pairs_staged(gate_up.data_ptr(), staged.data_ptr(), tokens, two_i // 2, int(accurate), self._stream(gate_up)))
 
-    def embed_rmsnorm(self, table: torch.Tensor, row_tokens: torch.Tensor, h: torch.Tensor, weight: torch.Tensor, y: torch.Tensor, eps: float) -> None:
-        """``h = table[row_tokens]`` (int64, one per row), ``y = rmsnorm(h) * weight``."""
+    def embed_rmsnorm(self, table: torch.Tensor, row_tokens: torch.Tensor, h: torch.Tensor, weight: torch.Tensor, y: torch.Tensor, eps: float,
+                      unknown: torch.Tensor | None = None) -> None:
+        """``h = table[row_tokens]`` (int64, one per row), ``y = rmsnorm(h) * weight``.  A token outside the table leaves status 33 and a row of ``y``
+        that is not a number, and stores 1 to ``unknown`` (one int32, pinned: the host then sees it without a synchronisation)."""
         tokens, hidden = h.shape
-        self._check(self._lib.tx_aux_embed_rmsnorm(table.data_ptr(), table.shape[0], row_tokens.data_ptr(), h.data_ptr(), weight.data_ptr(),
-                                                   y.data_ptr(), tokens, hidden, eps, h.device.index, self._stream(h)))
+        self._check(self._lib.tx_aux_embed_rmsnorm_watched(table.data_ptr(), table.shape[0], row_tokens.data_ptr(), h.data_ptr(), weight.data_ptr(),
+                                                           y.data_ptr(), tokens, hidden, eps, unknown.data_ptr() if unknown is not None else None,
+                                                           h.device.index, self._stream(h)))
 
     def rope_append(self, qkv, cos, sin, position, k_cache, v_cache, q_heads: int, kv_heads: int, head_dim: int) -> None:
         self._check(self._lib.tx_aux_rope_append(qkv.data_ptr(), cos.data_ptr(), sin.data_ptr(), position.data_ptr(),
