@@ -168,3 +168,17 @@ def test_large_matrices_get_the_bytes_of_their_slabs(ext, lut, kind, m, k, palet
     slabs = [ext.encode(w[i:i + rows], hdiag, table) for i in range(0, m, rows)]
     assert torch.equal(blocks, torch.cat([b for b, _ in slabs]))
     assert torch.equal(scales.view(torch.int32), torch.cat([s for _, s in slabs]).view(torch.int32))
+
+
+def test_blocks_of_tiny_moments_in_a_large_matrix_get_the_bytes_of_their_slabs(ext, lut):
+    """Sixteen moments so small that the reference's products underflow: which neighbour wins is then its rounding's choice."""
+    m, k = 1024, 4096
+    gen = torch.Generator(device="cuda").manual_seed(11)
+    w = torch.randn(m, k, device="cuda", generator=gen) * 0.02
+    levels = torch.tensor([1e-28, 1e-30, 1e-32, 1e-36, 1e-38, 1e-40, 1e-41, 1e-42, 1e-44, 0.0, 1.0], device="cuda")
+    hdiag = levels[torch.arange(k, device="cuda") // 16 % len(levels)].contiguous()
+    table = torch.from_numpy(lut).cuda()
+    blocks, _ = ext.encode(w, hdiag, table)
+    rows = ((1 << 21) - 1) // k
+    slabs = torch.cat([ext.encode(w[i:i + rows], hdiag, table)[0] for i in range(0, m, rows)])
+    assert torch.equal(blocks, slabs)

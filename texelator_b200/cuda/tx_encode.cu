@@ -421,12 +421,14 @@ __device__ __forceinline__ bool encode_block_spaced(const Block &b, const float 
   //   here       the five sums are ten deep and r is rounded once: 2 (154 + 70 + 14) u G and (1960 + 1960 + 490) u H, their combination
   //              140 u G + 980 u H;  a listed weight's x is off by 2 u D, the sums of gains are eighteen deep:
   //              2 (D + 2) (2 u D H_listed + 18 u gain)
-  // `slack` is their sum, rounded up.
+  // `slack` is their sum, rounded up.  All of it is relative: sums of moments that are not zero but below 2^-100 are left to the other way, as the
+  // reference's products, 889^2 times smaller than the ones here, would lose to underflow (2^-149 each, 2^-125 of sixteen in these units) what `slack`
+  // (2^-9 of the sum of moments or more) does not hold.
   constexpr float u = 0x1p-24f;
   const float spread = fmaf(sum_h, D, sum_s * (7.f * inverse));   // 2 G at most
   const float slack = u * (2100.f * spread + 32000.f * sum_h + 28.f * sum_s + (D + 2.f) * fmaf(5.f * D, listed_h, 40.f * most));
   const float limit = smallest + 2.f * slack;
-  if (int(signs) < 0 || !(limit < INFINITY)) return false;    // (a moment below zero, or sums that are not numbers)
+  if (int(signs) < 0 || !(limit < INFINITY) || (sum_h > 0.f && sum_h < 0x1p-100f)) return false;    // (a moment below zero, or sums that are not numbers)
   unsigned contenders = 0;
 #pragma unroll
   for (int n = 0; n < 9; ++n) contenders |= error[n] <= limit ? 1u << n : 0u;
