@@ -303,6 +303,29 @@ def test_staged_activations_give_the_linear_of_their_rows(ext, lut, tokens, k, m
         ext.free(h)
 
 
+@pytest.mark.parametrize("tokens", [3073, 3112, 6200])
+def test_staged_prompts_beyond_the_scratch_give_the_linear_of_their_rows(ext, lut, tokens):
+    """The scratch holds 3072 tokens of 16384 columns, and rows beyond them are a chunk of their own, summed in other K ranges; a staged prompt,
+    which needs no scratch, takes the same chunks."""
+    m, k = 200, 16384
+    blocks, scales, _ = _case(5, m, k, 1, lut)
+    h = _pack(ext, blocks, scales)
+    try:
+        gen = torch.Generator(device="cuda").manual_seed(tokens)
+        x, weight = torch.randn(tokens, k, device="cuda", generator=gen).bfloat16(), torch.randn(k, device="cuda", generator=gen).bfloat16()
+        ext.set_prefill(h, 1, 1024)
+        staged, rows = ext.staged_buffer(k, tokens, "cuda").fill_(0x7e), torch.empty_like(x)
+        ext.add_rmsnorm(x.clone(), None, weight, rows, 1e-6)
+        ext.add_rmsnorm_staged(x.clone(), None, weight, staged, 1e-6)
+        y = torch.empty(tokens, m, dtype=torch.bfloat16, device="cuda")
+        for backend in (5, 6, 7, 8, 9, 0):
+            ext.set_prefill_backend(h, backend)
+            assert torch.equal(ext.linear_staged(h, staged, y), ext.linear(h, rows)), backend
+        assert ext.kernel_status() == 0
+    finally:
+        ext.free(h)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("m,k,tokens", [(128, 1024, 16), (132, 1024, 33), (130, 1040, 64), (257, 2064, 65), (1024, 4096, 127), (3000, 1536, 1),
                                         (4250, 2896, 29), (5120, 1024, 17), (2304, 8192, 40), (9216, 1024, 31), (9344, 1024, 31)])

@@ -762,12 +762,12 @@ static int resident_clusters(Kernel kernel, int ranges, int sm_count) {
   return 0;
 }
 
-// One launch of the tile over `n` staged tokens, and where K is cut the sum of its ranges: inside the launch, by clusters, where all of them are
+// One launch of the tile over `n` staged tokens (of `padded_tokens` in the buffer), and where K is cut the sum of its ranges: inside the launch, by clusters, where all of them are
 // resident at once (a cluster waits for as many free SMs of one GPC as it has CTAs), else by a combine behind it.  By clusters / by a combine, us a
 // call from HBM with 16, 64 and 128 tokens on the 64-token tile: 256x2048 6.3, 6.9, 7.3 / 7.7, 7.9, 8.9; 5120x5120 10.2, 12.6, 21.7 / 12.1, 14.0,
 // 22.7; 5120x17408 19.8, 24.4, 42.5 / 22.7, 26.8, 46.5; 8192x28672 39.5, 44.5, 84.6 / 44.1, 48.4, 88.3.  No shape was slower.
 template <int CTAS, int BN, int GROUPS>
-static int launch_staged_groups(const Handle *h, const Workspace *ws, const __half *staged, const float *xmul, __nv_bfloat16 *y, int n, cudaStream_t stream, bool half_io) {
+static int launch_staged_groups(const Handle *h, const Workspace *ws, const __half *staged, int padded_tokens, const float *xmul, __nv_bfloat16 *y, int n, cudaStream_t stream, bool half_io) {
   using Cfg = TileConfig<CTAS, BN, GROUPS>;
   // the lean variant decodes high-mode blocks of the software palette and nothing else
   const bool generic = h->has_low_mode || h->palette == TX_PALETTE_HARDWARE;
@@ -790,11 +790,11 @@ static int launch_staged_groups(const Handle *h, const Workspace *ws, const __ha
       merge = int(grid.x * grid.y) <= clusters;
     }
   }
-  const int KP = h->KI * 128, padded_tokens = padded_prompt(n);
+  const int KP = h->KI * 128;
   // staged X viewed as [KP/8 chunks][padded_tokens/32][32 tokens x 8 elements]: a box is one run of
   // 512 contiguous bytes per 32 tokens and chunk and lands as core-matrix columns
   CUtensorMap map;
-  cuuint64_t dims[3] = {256, cuuint64_t(padded_tokens / 32), cuuint64_t(KP / 8)};
+  cuuint64_t dims[3] = {256, cuuint64_t(padded_prompt(n) / 32), cuuint64_t(KP / 8)};
   cuuint64_t strides[2] = {512, cuuint64_t(padded_tokens) * 16};
   cuuint32_t box[3] = {256, cuuint32_t(Cfg::tokens / 32), cuuint32_t(kChunks)};
   cuuint32_t elem[3] = {1, 1, 1};
@@ -825,11 +825,17 @@ static int launch_staged_groups(const Handle *h, const Workspace *ws, const __ha
 }
 
 template <int CTAS, int BN>
-static int launch_staged_tile(const Handle *h, const Workspace *ws, const __half *staged, const float *xmul, __nv_bfloat16 *y, int n, cudaStream_t stream, bool half_io) {
+static int launch_staged_tile(const Handle *h, const Workspace *ws, const __half *staged, int padded_tokens, const float *xmul, __nv_bfloat16 *y, int n, cudaStream_t stream, bool half_io) {
   constexpr bool small = CTAS == 1 && BN <= 128;
   if (small && two_an_sm(long(h->M + kMmaM - 1) / kMmaM * ((n + BN - 1) / BN), prefill_k_ranges(h, n, ws), h->KI, ws->sm_count))
-    return launch_staged_groups<CTAS, BN, small ? 1 : 2>(h, ws, staged, xmul, y, n, stream, half_io);
-  return launch_staged_groups<CTAS, BN, 2>(h, ws, staged, xmul, y, n, stream, half_io);
+    return launch_staged_groups<CTAS, BN, small ? 1 : 2>(h, ws, staged, padded_tokens, xmul, y, n, stream, half_io);
+  return launch_staged_groups<CTAS, BN, 2>(h, ws, staged, padded_tokens, xmul, y, n, stream, half_io);
+}
+
+// A call goes in chunks of as many tokens as the per-device scratch holds in staged form, also where the activations come staged and need no scratch:
+// the number of K ranges, and so the order of the sums, follows from a chunk's tokens.
+static int chunk_tokens(const Handle *h, const Workspace *ws) {
+  return int(std::min<size_t>(ws->xprep_halfs / (size_t(h->KI) * 128), 65536)) & ~31;   // staged tokens are padded to 32
 }
 
 template <int CTAS, int BN>
@@ -847,8 +853,7 @@ static int launch_tile(const Handle *h, const __nv_bfloat16 *x, __nv_bfloat16 *y
   }
   // Activations are staged once as fp16 after an exact per-token power-of-two rescale (the decode GEMV's
   // arithmetic), in chunks of tokens that fit the per-device scratch.
-  const int KP = h->KI * 128;
-  const int capacity = int(std::min<size_t>(ws->xprep_halfs / size_t(KP), 65536)) & ~31;   // staged tokens are padded to 32
+  const int KP = h->KI * 128, capacity = chunk_tokens(h, ws);
   if (capacity < 32) return fail(TX_EINVAL, "K is too large for the prefill activation scratch");
   for (int t0 = 0; t0 < tokens; t0 += capacity) {
     const int n = std::min(capacity, tokens - t0);
@@ -864,7 +869,7 @@ static int launch_tile(const Handle *h, const __nv_bfloat16 *x, __nv_bfloat16 *y
       TX_CUDA(launch_pdl(stage_activations_kernel, dim3(padded_tokens / per_cta), dim3(kStageThreads), rows_fit ? per_cta * stage_row_bytes(h->K) : 0,
                        stream, x + size_t(t0) * h->K, ws->xprep, ws->xmul, h->K, KP, n, padded_tokens, per_cta, rows_fit ? 1 : 0, half_io ? 1 : 0));
     count_launch();
-    const int rc = launch_staged_tile<CTAS, BN>(h, ws, ws->xprep, ws->xmul, y + size_t(t0) * h->M, n, stream, half_io);
+    const int rc = launch_staged_tile<CTAS, BN>(h, ws, ws->xprep, padded_tokens, ws->xmul, y + size_t(t0) * h->M, n, stream, half_io);
     if (rc != TX_OK) return rc;
   }
   TX_CUDA(cudaGetLastError());
@@ -889,18 +894,24 @@ int launch_prefill_tile(const Handle *h, int backend, const __nv_bfloat16 *x, __
 int launch_prefill_staged(const Handle *h, int backend, const uint8_t *staged, __nv_bfloat16 *y, int tokens, cudaStream_t stream) {
   Workspace *ws = workspace_for(h->device);
   if (!ws) return TX_ECUDA;
-  const __half *x = reinterpret_cast<const __half *>(staged);
-  const float *xmul = reinterpret_cast<const float *>(staged + staged_prompt_multipliers(h->K, tokens));
-  int rc;
-  switch (backend) {
-    case 5: rc = launch_staged_tile<1, 256>(h, ws, x, xmul, y, tokens, stream, false); break;
-    case 6: rc = launch_staged_tile<2, 256>(h, ws, x, xmul, y, tokens, stream, false); break;
-    case 7: rc = launch_staged_tile<1, 128>(h, ws, x, xmul, y, tokens, stream, false); break;
-    case 8: rc = launch_staged_tile<1, 64>(h, ws, x, xmul, y, tokens, stream, false); break;
-    case 9: rc = launch_staged_tile<1, 192>(h, ws, x, xmul, y, tokens, stream, false); break;
-    default: return fail(TX_EINVAL, "backend is not a tensor-core tile candidate");
+  const int capacity = chunk_tokens(h, ws), padded = padded_prompt(tokens);
+  if (capacity < 32) return fail(TX_EINVAL, "K is too large for the prefill activation scratch");
+  for (int t0 = 0; t0 < tokens; t0 += capacity) {
+    const int n = std::min(capacity, tokens - t0);
+    const __half *x = reinterpret_cast<const __half *>(staged) + size_t(t0) * 8;   // (a chunk of eight columns is a run of tokens)
+    const float *xmul = reinterpret_cast<const float *>(staged + staged_prompt_multipliers(h->K, tokens)) + t0;
+    __nv_bfloat16 *out = y + size_t(t0) * h->M;
+    int rc;
+    switch (backend) {
+      case 5: rc = launch_staged_tile<1, 256>(h, ws, x, padded, xmul, out, n, stream, false); break;
+      case 6: rc = launch_staged_tile<2, 256>(h, ws, x, padded, xmul, out, n, stream, false); break;
+      case 7: rc = launch_staged_tile<1, 128>(h, ws, x, padded, xmul, out, n, stream, false); break;
+      case 8: rc = launch_staged_tile<1, 64>(h, ws, x, padded, xmul, out, n, stream, false); break;
+      case 9: rc = launch_staged_tile<1, 192>(h, ws, x, padded, xmul, out, n, stream, false); break;
+      default: return fail(TX_EINVAL, "backend is not a tensor-core tile candidate");
+    }
+    if (rc != TX_OK) return rc;
   }
-  if (rc != TX_OK) return rc;
   TX_CUDA(cudaGetLastError());
   return TX_OK;
 }
