@@ -209,3 +209,32 @@ def test_model_with_weights_from_the_gpu_encoder():
         model.check_status()
     finally:
         model.free()
+
+
+@pytest.mark.parametrize("tokens", [40, 3000])
+def test_a_prompt_takes_no_memory_for_its_hand_over(tokens):
+    """What the norms hand over staged lies where SwiGLU's rows do: beyond the rows of the layer's steps, a prompt takes no memory
+    (but for 32 tokens' padding of the staged form and soft-max statistics)."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    from texelator_b200.modeling import CONFIGS, BC4Decoder
+    c = CONFIGS["toy128"]
+    model = BC4Decoder(c, "cuda:0", max_len=tokens, seed=3)
+    try:
+        ids = torch.randint(0, c.vocab, (tokens,), device="cuda")
+        for handle in model.handles:
+            model.ext.set_prefill_backend(handle, 8)
+        assert all(model.ext.takes_staged(handle, tokens) for handle in model.handles)
+        model.prefill(ids)
+        torch.cuda.synchronize()
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_stats()["requested_bytes.all.current"]
+        model.prefill(ids)
+        torch.cuda.synchronize()
+        taken = torch.cuda.memory_stats()["requested_bytes.all.peak"] - before
+        # residual, x, out; qkv; gate and up; SwiGLU; attention's output twice (as the kernel leaves it, and in rows)
+        rows = 2 * tokens * (3 * c.hidden + c.q_rows + 2 * c.kv_rows + 3 * c.intermediate + 2 * c.q_rows)
+        slack = 32 * 2 * max(c.hidden, c.intermediate) + 4 * tokens * c.q_heads + (64 << 10)
+        assert taken <= rows + slack, (taken, rows, slack)
+    finally:
+        model.free()

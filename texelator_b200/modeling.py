@@ -353,9 +353,12 @@ class BC4Decoder:
         tokens = h.shape[0]
         q_heads, kv_heads = c.q_heads // self.world, c.kv_heads // self.world
         make = lambda columns: torch.empty(tokens, columns, dtype=torch.bfloat16, device=self.device)
-        x, qkv, gate_up, act, out = make(c.hidden), make(self.q_loc + 2 * self.kv_loc), make(2 * self.i_loc), make(self.i_loc), make(c.hidden)
+        x, qkv, gate_up, out = make(c.hidden), make(self.q_loc + 2 * self.kv_loc), make(2 * self.i_loc), make(c.hidden)
+        # SwiGLU's rows and what the norms (or SwiGLU) hand over staged are never needed at the same time: one buffer, the rows at its start
+        staged_columns = max(c.hidden, self.i_loc if ext.stages_swiglu(tokens, self.i_loc) else 0)
+        staged = torch.empty(max(ext.staged_bytes(staged_columns, tokens), 2 * tokens * self.i_loc), dtype=torch.uint8, device=self.device)
+        act = staged[:2 * tokens * self.i_loc].view(torch.bfloat16).view(tokens, self.i_loc)
         q = qkv[:, :self.q_loc].view(tokens, q_heads, c.head_dim).transpose(0, 1).unsqueeze(0)
-        staged = ext.staged_buffer(max(c.hidden, self.i_loc), tokens, self.device)
 
         def normed(handle, delta, weight, out):
             if ext.takes_staged(handle, tokens):

@@ -381,7 +381,10 @@ class _Extension:
     # -- activations in the form the tiles read: from the kernel that makes them to the linear, without a staging launch --------
     def staged_buffer(self, columns: int, tokens: int, device) -> torch.Tensor:
         """A buffer for ``tokens`` rows of up to ``columns`` activations in staged form."""
-        return torch.empty(self._lib.tx_staged_prompt_bytes(columns, tokens), dtype=torch.uint8, device=device)
+        return torch.empty(self.staged_bytes(columns, tokens), dtype=torch.uint8, device=device)
+
+    def staged_bytes(self, columns: int, tokens: int) -> int:
+        return self._lib.tx_staged_prompt_bytes(columns, tokens)
 
     def takes_staged(self, handle: int, tokens: int) -> bool:
         """Whether ``linear_staged`` serves this many tokens (``linear`` would take a tile for them)."""
