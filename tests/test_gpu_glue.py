@@ -2,6 +2,8 @@
 import pytest
 import torch
 
+from graph_kernels import launched
+
 pytestmark = pytest.mark.gpu
 
 
@@ -397,3 +399,29 @@ def test_attention_step_batch_matches_64_bits(ext, sequences, q_heads, kv_heads,
         got = out[b].view(q_heads, 128).double()
         # (a rotated query may be rounded the other way where the product was contracted: 2^-8 of one element)
         assert float((got - want).norm() / want.norm()) <= 4e-3, (b, pos)
+
+
+@pytest.mark.parametrize("q_heads,kv_heads", [(40, 8), (8, 8), (64, 8)])
+@pytest.mark.parametrize("sequences,clusters", [(5, False), (6, False), (7, True), (8, True), (9, False), (10, True), (12, False), (16, True)])
+def test_splits_of_a_batch_are_clusters_where_all_of_them_fit(ext, sequences, clusters, q_heads, kv_heads):
+    """148 SMs hold 37 clusters of 7 splits, 45 of 6, 56 of 5, 71 of 4, 93 of 3 and 148 of 2, two CTAs an SM.  Beyond that the splits are merged by a launch
+    of their own, with the same sums: the outputs of a sequence alone (the same chunks in other splits) and of the batch agree either way."""
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the cluster counts are those of 148 SMs")
+    max_len = 1064
+    gen = torch.Generator(device="cuda").manual_seed(sequences)
+    bf = dict(device="cuda", dtype=torch.bfloat16)
+    k_cache, v_cache = (torch.randn(sequences, kv_heads, max_len, 128, generator=gen, **bf) for _ in range(2))
+    angles = torch.rand(max_len, 64, device="cuda", generator=gen) * 6.28
+    cos, sin = angles.cos().contiguous(), angles.sin().contiguous()
+    qkv = torch.randn(sequences, (q_heads + 2 * kv_heads) * 128, generator=gen, **bf)
+    positions = torch.tensor([1000 - 37 * i for i in range(sequences)], device="cuda")
+    scratch = torch.zeros(sequences * ext.attention_step_scratch_floats(q_heads, max_len), dtype=torch.float32, device="cuda")
+    out, alone = torch.zeros(sequences, q_heads * 128, **bf), torch.zeros(sequences, q_heads * 128, **bf)
+    names = [name for name, _ in launched(lambda: ext.attention_step_batch(qkv, cos, sin, positions, k_cache, v_cache, scratch, out, q_heads, kv_heads, 128))]
+    assert sum("attention_step_loop" in name for name in names) == 1
+    assert any("attention_merge" in name for name in names) != clusters, names
+    for b in range(sequences):
+        ext.attention_step(qkv[b:b + 1], cos, sin, positions[b:b + 1], k_cache[b], v_cache[b], scratch, alone[b:b + 1], q_heads, kv_heads, 128)
+    # both are the bf16 rounding of fp32 sums in two orders
+    assert float((out.float() - alone.float()).norm() / alone.float().norm()) <= 4e-3

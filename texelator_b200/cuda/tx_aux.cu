@@ -1196,7 +1196,7 @@ __global__ void __launch_bounds__(kStepThreads, 2) attention_step_kernel(const _
 // HBM busy across the chunk's barriers; the first chunks are requested before the wait for the launch in front, like the kernel above.  Products,
 // sums and their order are the kernel's above.
 //
-// DIRECT (a batch with up to eight splits, which are a cluster): the splits meet in distributed shared memory, with the arithmetic of
+// DIRECT (a batch with up to eight splits, which are a cluster; splits_meet_in_clusters): the splits meet in distributed shared memory, with the arithmetic of
 // attention_merge_kernel, and that launch falls away.
 //
 // What bounds it: HBM for long batches, else the chain of a chunk (three barriers).  us a call with the merge (a graph over caches larger than L2), 40 query
@@ -1673,23 +1673,60 @@ static bool merge_inline() {
   return value;
 }
 
+// The ring kernel's shared memory, set once a device
+template <int GROUP, bool DIRECT>
+static cudaError_t configure_ring(int device) {
+  static std::atomic<unsigned long long> configured;       // a bit a device
+  if (device < 64 && (configured.load(std::memory_order_relaxed) >> device & 1)) return cudaSuccess;
+  const auto kernel = attention_step_loop_kernel<GROUP, DIRECT>;
+  cudaError_t status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kRingSmem));
+  if (status == cudaSuccess) status = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+  if (status == cudaSuccess && device < 64) configured.fetch_or(1ull << device, std::memory_order_relaxed);
+  return status;
+}
+
+// Whether the splits of a batch are clusters (DIRECT): where all clusters are resident at once.  One cluster too many waits for a whole place in one GPC and
+// costs a second pass over a nearly idle chip: 5 sequences of 500 to 1000 positions, 40 query heads on 8 kv heads, 40 clusters of 7 with room for 37, 18.5 us
+// by clusters and 12.6 with the merge launch; 9 sequences (72 of 4, room for 71) 22.8 and 16.2; 12 (96 of 3, room for 93) 24.1 and 20.8.  Where they fit:
+// 10 sequences 19.2 and 19.9, 16 25.5 and 27.3, 32 42.8 and 48.9.
+template <int GROUP>
+static bool splits_meet_in_clusters(int splits, int clusters, int device) {
+  if (splits == 1) return true;                            // (no cluster at all)
+  static std::atomic<int> resident[64][9];                 // what fits the chip, and 1; 0: not asked yet
+  int found = device < 64 ? resident[device][splits].load(std::memory_order_relaxed) - 1 : -1;
+  if (found < 0) {
+    cudaLaunchConfig_t config{};
+    cudaLaunchAttribute attribute{};
+    config.gridDim = dim3(splits, clusters);
+    config.blockDim = dim3(kStepThreads);
+    config.dynamicSmemBytes = kRingSmem;
+    attribute.id = cudaLaunchAttributeClusterDimension;
+    attribute.val.clusterDim.x = unsigned(splits);
+    attribute.val.clusterDim.y = attribute.val.clusterDim.z = 1;
+    config.attrs = &attribute;
+    config.numAttrs = 1;
+    if (configure_ring<GROUP, true>(device) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&found, attention_step_loop_kernel<GROUP, true>, &config) != cudaSuccess) {
+      cudaGetLastError();
+      return false;                                        // (asked again by the next call)
+    }
+    if (device < 64) resident[device][splits].store(found + 1, std::memory_order_relaxed);
+  }
+  return clusters <= found;
+}
+
 template <int GROUP, bool LOOP>
 static cudaError_t launch_attention_step(int splits, int kv_heads, int sequences, cudaStream_t s, const __nv_bfloat16 *qkv, const float *cos_table,
                                          const float *sin_table, const long long *position, __nv_bfloat16 *k_cache,
                                          __nv_bfloat16 *v_cache, float *scratch, __nv_bfloat16 *out, int q_heads, int max_len, float scale, int device) {
   const int merge_here = merge_inline() ? 1 : 0;
   // (one sequence keeps the launch behind its splits: as a dependent it is resident and waiting when the last split ends)
-  const bool direct = LOOP && !merge_here && sequences > 1 && splits <= 8;
+  const bool direct = LOOP && !merge_here && sequences > 1 && splits <= 8 && splits_meet_in_clusters<GROUP>(splits, kv_heads * sequences, device);
   cudaError_t status;
   if (LOOP) {
     const auto kernel = direct ? attention_step_loop_kernel<GROUP, true> : attention_step_loop_kernel<GROUP, false>;
-    static std::atomic<unsigned long long> configured[2];       // a bit a device
-    if (device >= 64 || !(configured[direct].load(std::memory_order_relaxed) >> device & 1)) {
-      status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kRingSmem));
-      if (status == cudaSuccess) status = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-      if (status != cudaSuccess) return status;
-      if (device < 64) configured[direct].fetch_or(1ull << device, std::memory_order_relaxed);
-    }
+    status = direct ? configure_ring<GROUP, true>(device) : configure_ring<GROUP, false>(device);
+    if (status != cudaSuccess) return status;
     status = launch_pdl_cluster(kernel, direct ? splits : 1, dim3(splits, kv_heads, sequences), dim3(kStepThreads), kRingSmem, s, qkv, cos_table, sin_table,
                                 position, k_cache, v_cache, scratch, out, q_heads, kv_heads, max_len, splits, scale, merge_here);
   } else {
