@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 import torch
 
+from graph_kernels import recorded
 from oracle import bc4_oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -168,6 +169,21 @@ def test_large_matrices_get_the_bytes_of_their_slabs(ext, lut, kind, m, k, palet
     slabs = [ext.encode(w[i:i + rows], hdiag, table) for i in range(0, m, rows)]
     assert torch.equal(blocks, torch.cat([b for b, _ in slabs]))
     assert torch.equal(scales.view(torch.int32), torch.cat([s for _, s in slabs]).view(torch.int32))
+
+
+@pytest.mark.parametrize("m,k", [(2048, 1024), (9500, 1024), (10000, 2048), (44000, 48), (40000, 64)])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_the_search_for_magnitudes_runs_beside_the_verdict(ext, lut, m, k, offset):
+    """The kernel behind the verdict on the palette starts with it, the verdict itself behind everything in front; with few and many rows, rows
+    shorter than a verdict's bytes, and a palette off the boundary of wide loads.  The bytes are those of the slabs."""
+    gen = torch.Generator(device="cuda").manual_seed(m + k)
+    w, hdiag = torch.randn(m, k, device="cuda", generator=gen) * 0.02, torch.exp(torch.randn(k, device="cuda", generator=gen))
+    table = torch.zeros(255 * 255 * 8 + offset, device="cuda")[offset:].copy_(torch.from_numpy(lut).reshape(-1)).view(255, 255, 8)
+    rows, out = ((1 << 21) - 1) // k, []
+    kernels = [(name, early) for name, _, early in recorded(lambda: out.append(ext.encode(w, hdiag, table))) if "N2tx" in name]
+    assert ["verdict" in name for name, _ in kernels] == [True, False] and [early for _, early in kernels] == [False, True], kernels
+    slabs = torch.cat([ext.encode(w[i:i + rows], hdiag, table)[0] for i in range(0, m, rows)])
+    assert torch.equal(out[0][0], slabs)
 
 
 def test_blocks_of_tiny_moments_in_a_large_matrix_get_the_bytes_of_their_slabs(ext, lut):

@@ -466,35 +466,51 @@ __device__ __forceinline__ bool encode_block_spaced(const Block &b, const float 
   return true;
 }
 
-// Whether a table is the software palette where the endpoints are apart (the others are only ever read).  Each of the CTAS CTAs looks at its share and leaves a byte, 1 or 0, in the
+// Whether a table is the software palette where the endpoints are apart (the others are only ever read).  Each of CTAS CTAs looks at its share, a
+// row of the table a thread and step, and leaves a byte, 1 or 0, in the
 // first CTAS bytes that every CTA of the encode kernel behind it is going to write, which reads them before it writes there: the verdict
 // belongs to the call, without a word of its own that calls on two streams would share.
 //
-// 128 CTAs where a CTA has that many bytes to write, 16 where rows are short: 5 and 9 us with the launch.
-constexpr int kPaletteEntries = 255 * 255 * 8;
-template <int CTAS, int THREADS>
-__global__ void __launch_bounds__(THREADS) palette_verdict_kernel(const float *__restrict__ lut, uint8_t *__restrict__ blocks, int ctas, size_t cta_bytes,
-                                                                  int shares, int share_bytes) {
-  bool same = true;
-  constexpr int kEach = (kPaletteEntries + CTAS * THREADS - 1) / (CTAS * THREADS);
-  const int first = int(blockIdx.x) * kEach * THREADS + int(threadIdx.x);
-  float entry[kEach];
+// The encode kernel starts beside it and finds its first rows' largest magnitudes before it waits.  A call that cannot use the answer pays 1.0 us for the launch
+// and about two for what the wait is longer than that search: under the texture palette 2048 x 1024 takes 23.1 us without a verdict and
+// 26.1 with, 2048 x 2048 43.4 and 46.4, 4096 x 4096 155.9 and 156.5 (28.5, 49.4 and 160.8 with a verdict of 128 CTAs in front of the whole encode kernel).
+// 32 CTAs, 16 where a CTA's first step writes fewer bytes: 16, 32 and 64 take 26.3, 26.1 and 26.1 there.
+constexpr int kPaletteRows = 255 * 255, kVerdicts = 32, kFewVerdicts = 16, kVerdictThreads = 1024;
+template <int CTAS, bool WIDE>
+__global__ void __launch_bounds__(kVerdictThreads) palette_verdict_kernel(const float *__restrict__ lut, uint8_t *__restrict__ blocks, int ctas, size_t cta_bytes,
+                                                                          int shares, int share_bytes) {
+  grid_launch_dependents();      // the encode kernel finds its first rows' largest magnitudes meanwhile
+  constexpr int kEach = (kPaletteRows + CTAS * kVerdictThreads - 1) / (CTAS * kVerdictThreads);
+  float4 entries[kEach][2];
+  int left[kEach], right[kEach];
 #pragma unroll
   for (int i = 0; i < kEach; ++i) {                     // all loads in flight together
-    const int at = first + i * THREADS;
-    entry[i] = at < kPaletteEntries ? lut[at] : 0.f;
+    const int row = (i * CTAS + int(blockIdx.x)) * kVerdictThreads + int(threadIdx.x);
+    right[i] = row / 255 - 127;
+    left[i] = row < kPaletteRows ? row % 255 - 127 : -128;
+    if (left[i] - right[i] >= kApart - 2) {
+      entries[i][0] = palette_half<WIDE>(lut + size_t(row) * 8, 0);
+      entries[i][1] = palette_half<WIDE>(lut + size_t(row) * 8, 1);
+    }
   }
+  bool same = true;
 #pragma unroll
   for (int i = 0; i < kEach; ++i) {
-    const int at = first + i * THREADS, e1 = (at >> 3) / 255 - 127, e0 = (at >> 3) % 255 - 127, selector = at & 7;
-    const int g = selector == 0 ? 0 : (selector == 1 ? 7 : selector - 1);
-    const float off = __fmaf_rn(entry[i], 889.f, -float((7 - g) * e0 + g * e1));
-    same &= at >= kPaletteEntries || e0 - e1 < kApart - 2 || fabsf(off) <= 889.f * kEntryError;
+    if (left[i] - right[i] < kApart - 2) continue;
+    const float4 lo = entries[i][0], hi = entries[i][1];
+    const float entry[8] = {lo.x, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w, lo.y};   // by interpolation index
+    const float step = float(right[i] - left[i]);
+    float expected = float(7 * left[i]);                  // 889 times the entry, a whole number
+#pragma unroll
+    for (int g = 0; g < 8; ++g) {
+      same &= fabsf(__fmaf_rn(entry[g], 889.f, -expected)) <= 889.f * kEntryError;
+      expected += step;
+    }
   }
   same = __syncthreads_and(same);
-  for (int i = threadIdx.x; i < ctas * shares; i += THREADS) blocks[size_t(i / shares) * cta_bytes + size_t(i % shares) * share_bytes + blockIdx.x] = same ? 1 : 0;
+  for (int i = threadIdx.x; i < ctas * shares; i += kVerdictThreads)
+    blocks[size_t(i / shares) * cta_bytes + size_t(i % shares) * share_bytes + blockIdx.x] = same ? 1 : 0;
 }
-constexpr int kVerdicts = 128, kFewVerdicts = 16;
 
 // From here on the verdict pays: 2000 x 1040 takes 37.0 us without it and 28.2 with; 300 x 4096, half the size, 20.6 and 20.7.
 constexpr size_t kSpacedWeights = size_t(1) << 21;
@@ -541,8 +557,9 @@ __global__ void __launch_bounds__(kEncodeThreads, 4) encode_kernel(const float *
     }
     if (SPACED && row0 == int(blockIdx.x) * kGroups) {
       const unsigned long long *verdict = blocks + size_t(row0) * bpr + blockIdx.y * GROUP;
+      grid_dependency_wait();
       // (one barrier for all: read before one writes blocks there)
-      spaced = __syncthreads_and(int(threadIdx.x) >= verdicts / 8 || verdict[threadIdx.x] == 0x0101010101010101ull);
+      spaced = __syncthreads_and(int(threadIdx.x) >= verdicts / 8 || __ldcg(verdict + threadIdx.x) == 0x0101010101010101ull);
     }
     const float scale = fmaxf(m, 1e-12f), reciprocal = __frcp_rn(scale);
     const bool normal = scale >= 0x1p-40f && scale <= 0x1p60f;
@@ -585,13 +602,14 @@ __global__ void __launch_bounds__(kEncodeThreads, 4) encode_kernel(const float *
 }
 
 template <int GROUP>
-static void launch_encode_rows(const float *weight, const float *hdiag, const float *lut, int M, int K, uint8_t *blocks, float *scales, cudaStream_t stream) {
+static cudaError_t launch_encode_rows(const float *weight, const float *hdiag, const float *lut, int M, int K, uint8_t *blocks, float *scales, cudaStream_t stream) {
   const int per_cta = kEncodeThreads / GROUP, ctas = (M + per_cta - 1) / per_cta;
-  // Rows alone fill the chip from about 600 blocks of threads on (four to an SM); beyond three times that the blocks take several each (4096 x 4096 79.6,
-  // 80.4, 84.4 us with one wave of blocks, three and a block a row; under the texture palette 171, 162, 164).  Below that
-  // a row is shared, by as many groups as fit one wave and have a step each: 8 x 17408 84.6 -> 11.4 us, 100 x 11200 57.9 -> 16.6,
+  // Rows alone fill the chip from about 600 blocks of threads on (four to an SM).  Beyond three times that the blocks take several each, beyond sixteen times
+  // six times as many blocks share the rows.  One wave of blocks, three, six and a block a row, us -- 4096 x 4096 (6.9 waves) 75.8, 76.5, 78.3, 80.2, under the
+  // texture palette 164, 157, 158, 159; 20000 x 4000 (33) 384, 387, 384, 425 and 830, 789, 763, 773; 34816 x 5120 (29) 738, 731, 727, 740 and
+  // 1698, 1597, 1558, 1557.  Below one wave a row is shared, by as many groups as fit one wave and have a step each: 8 x 17408 84.6 -> 11.4 us, 100 x 11200 57.9 -> 16.6,
   // 300 x 11200 74.9 -> 44.3 (the kernel that spread single blocks over the chip took 29.2, 61.6 and 153.7).
-  const int grid = std::min(ctas, 3 * kEncodeWave);
+  const int grid = std::min(ctas, (ctas > 16 * kEncodeWave ? 6 : 3) * kEncodeWave);
   const int steps = (K / 16 + GROUP - 1) / GROUP, most = std::max(1, std::min(kEncodeWave / grid, steps));
   const int rounds = (steps + most - 1) / most;   // steps of a group
   const int shares = (steps + rounds - 1) / rounds;
@@ -602,23 +620,25 @@ static void launch_encode_rows(const float *weight, const float *hdiag, const fl
   const int verdicts = fewest >= kVerdicts ? kVerdicts : kFewVerdicts;
   if (spaced) {
     const size_t cta_bytes = size_t(per_cta) * K / 2;
-    if (verdicts == kVerdicts) palette_verdict_kernel<kVerdicts, 256><<<kVerdicts, 256, 0, stream>>>(lut, blocks, grid, cta_bytes, shares, GROUP * 8);
-    else palette_verdict_kernel<kFewVerdicts, 1024><<<kFewVerdicts, 1024, 0, stream>>>(lut, blocks, grid, cta_bytes, shares, GROUP * 8);
+    const auto verdict = verdicts == kVerdicts ? (wide ? palette_verdict_kernel<kVerdicts, true> : palette_verdict_kernel<kVerdicts, false>)
+                                               : (wide ? palette_verdict_kernel<kFewVerdicts, true> : palette_verdict_kernel<kFewVerdicts, false>);
+    verdict<<<verdicts, kVerdictThreads, 0, stream>>>(lut, blocks, grid, cta_bytes, shares, GROUP * 8);
     count_launch();
   }
   // four blocks of threads to an SM want 132 KB of its shared memory
   const auto kernel = spaced ? (wide ? encode_kernel<GROUP, true, true> : encode_kernel<GROUP, false, true>)
                              : (wide ? encode_kernel<GROUP, true, false> : encode_kernel<GROUP, false, false>);
-  kernel<<<dim3(grid, shares), kEncodeThreads, 0, stream>>>(weight, hdiag, lut, reinterpret_cast<unsigned long long *>(blocks), scales, M, K, verdicts);
+  // early only behind the verdict, which is a plain launch: what the caller left on the stream has ended before either starts
+  return launch_cluster(kernel, spaced, 1, dim3(grid, shares), dim3(kEncodeThreads), 0, stream, weight, hdiag, lut, reinterpret_cast<unsigned long long *>(blocks),
+                        scales, M, K, verdicts);
 }
 
 int launch_encode(const float *weight, const float *hdiag, const float *lut, int M, int K, uint8_t *blocks, float *scales, cudaStream_t stream) {
   // lanes per row: the size that leaves the fewest lanes without a block in the last step of a row, the larger one when
   // equal (a row of 198 blocks is 2 steps of 128 lanes with 58 idle, 4 of 64 with 58 idle, 7 of 32 with 26 idle)
   const auto idle = [&](int group) { return (K / 16 + group - 1) / group * group - K / 16; };
-  if (idle(128) <= idle(64) && idle(128) <= idle(32)) launch_encode_rows<128>(weight, hdiag, lut, M, K, blocks, scales, stream);
-  else if (idle(64) <= idle(32)) launch_encode_rows<64>(weight, hdiag, lut, M, K, blocks, scales, stream);
-  else launch_encode_rows<32>(weight, hdiag, lut, M, K, blocks, scales, stream);
+  const auto rows = idle(128) <= idle(64) && idle(128) <= idle(32) ? launch_encode_rows<128> : idle(64) <= idle(32) ? launch_encode_rows<64> : launch_encode_rows<32>;
+  TX_CUDA(rows(weight, hdiag, lut, M, K, blocks, scales, stream));
   count_launch();
   TX_CUDA(cudaGetLastError());
   return TX_OK;
