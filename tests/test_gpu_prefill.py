@@ -374,3 +374,37 @@ def test_two_tiles_an_sm_are_bitwise_the_tile_of_one(ext, lut, m, k, tokens):
         assert ext.kernel_status() == 0
     finally:
         ext.free(h)
+
+
+@pytest.mark.parametrize("hardware,m,k,tokens,backend,groups", [
+    (False, 19072, 4224, 64, 8, 1),        # 149 CTAs: two an SM fill one wave instead of two
+    (True, 19072, 4224, 64, 8, 2),         # ... but not where a unit takes longer to decode
+    (True, 19072, 2048, 64, 8, 1), (True, 19072, 2176, 64, 8, 2),
+    (True, 18560, 2176, 385, 7, 1),        # four waves of one, two of two
+    (True, 18560, 4224, 385, 7, 2),
+    (False, 38400, 2176, 64, 8, 2),        # three waves of one, two of two
+    (False, 18944, 2048, 64, 8, 2),        # 148 CTAs: one wave
+])
+def test_two_tiles_an_sm_where_they_fill_waves(ext, hardware, m, k, tokens, backend, groups):
+    """Which instance serves grids of more CTAs than the 148 SMs, and that both give the bits of the wide tile."""
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the waves are those of 148 SMs")
+    from texelator_b200 import modeling, runtime
+    gen = torch.Generator(device="cuda").manual_seed(m + k)
+    weight = torch.randn(m, k, device="cuda", generator=gen) * 0.02
+    h = ext.pack_encoded_device(*modeling.encode_minmax_cuda(weight, modeling.software_palette_table("cuda")), None)
+    try:
+        if hardware:
+            ext.set_palette(h, runtime.PALETTE_HARDWARE)
+        ext.set_prefill(h, 1, 1024)
+        x = torch.randn(tokens, k, device="cuda", generator=gen).bfloat16()
+        ext.set_prefill_backend(h, 5)
+        want = ext.linear(h, x)
+        ext.set_prefill_backend(h, backend)
+        out = []
+        names = [name for name, _ in launched(lambda: out.append(ext.linear(h, x)))]
+        expected = f"prefill_umma_kernelILi1ELi{ {8: 64, 7: 128}[backend] }ELb{int(hardware)}ELi{groups}E"
+        assert any(expected in name for name in names), names
+        assert torch.equal(out[0], want) and ext.kernel_status() == 0
+    finally:
+        ext.free(h)

@@ -691,10 +691,17 @@ static int prefill_k_ranges(const Handle *h, int tokens, const Workspace *ws) {
 // each other's gaps.  They lose where rounding the grid up to two an SM costs a wave and the rows are long enough to show it.  One / two an SM, us a
 // call from HBM, waves of one an SM before the figures -- 64 tokens: 24576x1024 2: 11.9 / 9.6; 22016x2048 2: 16.3 / 14.2; 34816x5120 2: 32.8 / 30.3;
 // 57344x8192 4: 85.9 / 79.6.  With the 128-token tile: 22016x2048 2: 20.1 / 17.5, 3: 29.1 / 27.1, 7: 65.0 / 59.8; 19200x4096 3: 43.0 / 44.9,
-// 7: 106.4 / 101.0; 28672x8192 4: 100.3 / 92.8, 5: 141.6 / 144.1; 24576x1024 8: 52.0 / 38.6.
-static bool two_an_sm(long ctas, int ranges, int units, int sm_count) {
+// 7: 106.4 / 101.0; 28672x8192 4: 100.3 / 92.8, 5: 141.6 / 144.1; 24576x1024 8: 52.0 / 38.6; 5120x17408 9: 492 / 563.
+//
+// The generic instance spends longer on a unit than the gaps last, so it gains on short rows and where there are many waves.  Under the texture palette, 64
+// tokens: 22016x2048 2: 21.1 / 21.4, 34816x5120 2: 44.8 / 47.3, 34816x8192 2: 66.6 / 71.6, 57344x3072 4: 53.7 / 52.7, 57344x8192 4: 123.7 / 127.0; with the
+// 128-token tile: 22016x2048 7: 77.7 / 73.1, 22016x3072 7: 107.9 / 106.3, 5120x17408 2: 147.8 / 158.0, 22016x17408 7: 557 / 581.
+static bool two_an_sm(long ctas, int ranges, int units, int sm_count, bool generic) {
   const long one = (ctas + sm_count - 1) / sm_count, two = (ctas + 2 * sm_count - 1) / (2 * sm_count);
-  return ranges == 1 && one > 1 && (2 * two <= one || one >= 7 || units <= 16);
+  if (ranges != 1 || one < 2) return false;
+  if (units <= 16) return true;
+  if (generic) return units <= 32 && one >= 4 && (2 * two <= one || one >= 7);
+  return 2 * two <= one || (one >= 7 && units <= 64);
 }
 
 // The tile of handles without a tuned backend (ids 0..4; 5..9 name one): all tiles give the same bits, so only time decides.
@@ -738,6 +745,9 @@ int prefill_choose_backend(const Handle *h, int tokens) {
   return pick;
 }
 
+// the lean instances decode high-mode blocks of the software palette and nothing else
+static bool takes_generic(const Handle *h) { return h->has_low_mode || h->palette == TX_PALETTE_HARDWARE; }
+
 // What a tile's instance is asked for once per device: its shared memory, and how many clusters of 2 to 8 K ranges are resident at once.
 struct TileSetup {
   bool ready = false;
@@ -769,8 +779,7 @@ static int resident_clusters(Kernel kernel, int ranges, int sm_count) {
 template <int CTAS, int BN, int GROUPS>
 static int launch_staged_groups(const Handle *h, const Workspace *ws, const __half *staged, int padded_tokens, const float *xmul, __nv_bfloat16 *y, int n, cudaStream_t stream, bool half_io) {
   using Cfg = TileConfig<CTAS, BN, GROUPS>;
-  // the lean variant decodes high-mode blocks of the software palette and nothing else
-  const bool generic = h->has_low_mode || h->palette == TX_PALETTE_HARDWARE;
+  const bool generic = takes_generic(h);
   const auto kernel = generic ? prefill_umma_kernel<CTAS, BN, true, GROUPS> : prefill_umma_kernel<CTAS, BN, false, GROUPS>;
   const int ranges = prefill_k_ranges(h, n, ws);
   dim3 grid((h->M + Cfg::rows - 1) / Cfg::rows * CTAS, (n + BN - 1) / BN, ranges);
@@ -827,7 +836,7 @@ static int launch_staged_groups(const Handle *h, const Workspace *ws, const __ha
 template <int CTAS, int BN>
 static int launch_staged_tile(const Handle *h, const Workspace *ws, const __half *staged, int padded_tokens, const float *xmul, __nv_bfloat16 *y, int n, cudaStream_t stream, bool half_io) {
   constexpr bool small = CTAS == 1 && BN <= 128;
-  if (small && two_an_sm(long(h->M + kMmaM - 1) / kMmaM * ((n + BN - 1) / BN), prefill_k_ranges(h, n, ws), h->KI, ws->sm_count))
+  if (small && two_an_sm(long(h->M + kMmaM - 1) / kMmaM * ((n + BN - 1) / BN), prefill_k_ranges(h, n, ws), h->KI, ws->sm_count, takes_generic(h)))
     return launch_staged_groups<CTAS, BN, small ? 1 : 2>(h, ws, staged, padded_tokens, xmul, y, n, stream, half_io);
   return launch_staged_groups<CTAS, BN, 2>(h, ws, staged, padded_tokens, xmul, y, n, stream, half_io);
 }
