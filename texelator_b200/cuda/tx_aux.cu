@@ -1205,7 +1205,10 @@ __global__ void __launch_bounds__(kStepThreads, 2) attention_step_kernel(const _
 // another order: with logits that tie, a decoder then picks other tokens than the one-sequence kernel above.)
 constexpr int kRingStages = 3, kChunkBytes = kStepKeys * kHeadDim * 2 * 2;   // keys, then values
 constexpr size_t kRingSmem = size_t(kRingStages) * kChunkBytes;
-__device__ __forceinline__ void cluster_barrier() { asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_barrier() {
+  __syncwarp();                  // the barrier wants whole warps, and what comes before it ends in branches
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 __device__ __forceinline__ float load_remote(const float *mine, int rank) {   // the float at this place in the shared memory of another CTA of the cluster
   float v;
   asm volatile("{\n\t.reg .b32 remote;\n\tmapa.shared::cluster.u32 remote, %1, %2;\n\tld.shared::cluster.f32 %0, [remote];\n\t}"

@@ -356,6 +356,7 @@ __device__ __forceinline__ void stage_split_row(uint4 *staged, float *multiplier
     for (int w = 0; w < kSplitThreads / 32; ++w) peak = max(peak, warp_peak[w]);
     if (shares > 1) {
       if (threadIdx.x == 0) peak_s = peak;
+      __syncwarp();              // (the cluster barriers want whole warps)
       asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
       for (int r = 0; r < shares; ++r) {
         unsigned other;
@@ -373,6 +374,7 @@ __device__ __forceinline__ void stage_split_row(uint4 *staged, float *multiplier
     if (first + c * kSplitThreads < last) store(first + int(threadIdx.x) + c * kSplitThreads, held[c]);
   for (int i0 = first + kSplitHeld * kSplitThreads; i0 < last; i0 += kSplitThreads) store(i0 + int(threadIdx.x), fetch(i0 + int(threadIdx.x)));
   if (share == 0 && threadIdx.x == 0) multipliers[tok] = inverse * kNumeratorScale;
+  __syncwarp();
   if (!half_in && shares > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // CTAs of a row: up to eight while two CTAs an SM are not exceeded and each has eight half units or more
