@@ -324,11 +324,11 @@ __device__ __forceinline__ unsigned long long selectors_of(unsigned long long g)
 
 constexpr int kEncodeThreads = 128;
 
+// `lanes`: those of the warp that have a block in this step, all of which call.
 // false: the block is one for encode_block (weights that are not numbers among them: their solution has no two endpoints apart)
 template <bool WIDE>
-__device__ __forceinline__ bool encode_block_spaced(const Block &b, const float *lut, const Coefficients &coef, float4 (*list)[kEncodeThreads], Encoded &e) {
+__device__ __forceinline__ bool encode_block_spaced(const Block &b, const float *lut, const Coefficients &coef, float4 (*list)[kEncodeThreads], unsigned lanes, Encoded &e) {
   // (a lane that goes to encode_block takes its warp's time anyway, so the whole warp goes)
-  const unsigned lanes = __activemask();
   if (__any_sync(lanes, b.e0 - b.e1 < kApart)) return false;
   int c0, c1;
   {
@@ -595,7 +595,9 @@ __global__ void __launch_bounds__(kEncodeThreads, 4) encode_kernel(const float *
       }
       b.find_extremes();
       Encoded e;
-      if (!SPACED || !spaced || !encode_block_spaced<WIDE>(b, lut, coef, list, e)) e = encode_block<WIDE>(b, lut, coef);
+      const int rest = bpr - (kb - int(threadIdx.x & 31));   // blocks from the warp's first lane on (a warp has one row)
+      const unsigned lanes = rest >= 32 ? 0xffffffffu : (1u << rest) - 1;
+      if (!SPACED || !spaced || !encode_block_spaced<WIDE>(b, lut, coef, list, lanes, e)) e = encode_block<WIDE>(b, lut, coef);
       blocks[size_t(row) * bpr + kb] = (unsigned long long)(unsigned(e.e0) & 0xffu) | ((unsigned long long)(unsigned(e.e1) & 0xffu) << 8) | (e.bits << 16);
     }
   }
