@@ -162,3 +162,53 @@ def test_no_product_code_imports_the_oracle():
     for path in list((ROOT / "texelator_b200").rglob("*.py")) + list((ROOT / "texelator_b200").rglob("*.cu")):
         text = path.read_text()
         assert "oracle" not in text.replace("oracle/bc4_oracle.py", ""), path
+
+
+def test_staged_calls_refuse_what_they_cannot_read():
+    """Buffers of another device or type, short ones and unknown handles are refused before anything is launched."""
+    import torch
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    from texelator_b200 import runtime
+    ext = runtime.extension()
+    handle = 1 << 40                                        # never dereferenced
+    ext._remember(handle, 32, 64, 0)
+    try:
+        with FakeTensorMode():
+            cuda = dict(device="cuda")
+            y, rows, gate_up = (torch.empty(4, n, dtype=torch.bfloat16, **cuda) for n in (32, 64, 128))
+            staged, weight = torch.empty(ext.staged_bytes(64, 4), dtype=torch.uint8, **cuda), torch.empty(64, dtype=torch.bfloat16, **cuda)
+            short, words, strided = staged[:-4], torch.empty(1 << 20, dtype=torch.int32, **cuda), torch.empty(1 << 20, dtype=torch.uint8, **cuda)[::2]
+        with pytest.raises(RuntimeError, match="null Texelator handle"):
+            ext.linear_staged(1234, staged, y)
+        with pytest.raises(RuntimeError, match="input shape/device mismatch"):
+            ext.linear_staged(handle, staged, torch.empty(4, 32, dtype=torch.bfloat16))
+        calls = (lambda s: ext.linear_staged(handle, s, y), lambda s: ext.add_rmsnorm_staged(rows, None, weight, s, 1e-6),
+                 lambda s: ext.silu_mul_pairs_staged(gate_up, s))
+        for call in calls:
+            with pytest.raises(RuntimeError, match="too small"):
+                call(short)
+            for wrong in (torch.empty(1 << 20, dtype=torch.uint8), words, strided):
+                with pytest.raises(RuntimeError, match="contiguous uint8 tensor on the CUDA device"):
+                    call(wrong)
+    finally:
+        ext._forget(handle)
+
+
+def test_embedding_norm_refuses_what_it_cannot_read():
+    import torch
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    from texelator_b200 import runtime
+    ext = runtime.extension()
+    with FakeTensorMode():
+        cuda, bf = dict(device="cuda"), dict(device="cuda", dtype=torch.bfloat16)
+        table, ids, h, weight, y = torch.empty(50, 64, **bf), torch.empty(3, dtype=torch.int64, **cuda), torch.empty(3, 64, **bf), torch.empty(64, **bf), torch.empty(3, 64, **bf)
+        short, narrow, few, wrong, flipped = ids[:2], torch.empty(3, dtype=torch.int32, **cuda), torch.empty(50, 32, **bf), table.float(), torch.empty(64, 50, **bf).t()
+    for tokens in (short, narrow):
+        with pytest.raises(RuntimeError, match="one int64 token a row"):
+            ext.embed_rmsnorm(table, tokens, h, weight, y, 1e-6)
+    for other in (few, wrong, flipped):
+        with pytest.raises(RuntimeError, match="the table is contiguous BF16"):
+            ext.embed_rmsnorm(other, ids, h, weight, y, 1e-6)
+    for other in ((table, torch.zeros(3, dtype=torch.int64), h), (torch.zeros(50, 64, dtype=torch.bfloat16), ids, h)):
+        with pytest.raises(RuntimeError, match="on one CUDA device"):
+            ext.embed_rmsnorm(other[0], other[1], other[2], weight, y, 1e-6)

@@ -386,23 +386,32 @@ class _Extension:
     def staged_bytes(self, columns: int, tokens: int) -> int:
         return self._lib.tx_staged_prompt_bytes(columns, tokens)
 
+    def _check_staged(self, staged: torch.Tensor, columns: int, tokens: int, device: int) -> None:
+        if device < 0 or staged.dtype != torch.uint8 or not staged.is_contiguous() or staged.get_device() != device:
+            raise RuntimeError("staged activations are a contiguous uint8 tensor on the CUDA device of the rows")
+        if staged.numel() < self.staged_bytes(columns, tokens):
+            raise RuntimeError("the staged buffer is too small")
+
     def takes_staged(self, handle: int, tokens: int) -> bool:
         """Whether ``linear_staged`` serves this many tokens (``linear`` would take a tile for them)."""
         return self._lib.tx_linear_takes_staged(handle, tokens) == 1
 
     def linear_staged(self, handle: int, staged: torch.Tensor, y: torch.Tensor) -> torch.Tensor:
         """``linear_out`` of rows in staged form: the same result bit for bit."""
-        m, k, _ = self._shapes[handle]
+        shape = self._shapes.get(handle)
+        if shape is None:
+            raise RuntimeError("null Texelator handle")
+        m, k, device = shape
         tokens = y.numel() // m
-        if y.numel() != tokens * m or y.dtype != torch.bfloat16 or not y.is_contiguous() or staged.numel() < self._lib.tx_staged_prompt_bytes(k, tokens):
+        if y.numel() != tokens * m or y.dtype != torch.bfloat16 or not y.is_contiguous() or y.get_device() != device:
             raise RuntimeError("input shape/device mismatch")
+        self._check_staged(staged, k, tokens, device)
         self._check(self._lib.tx_linear_staged(handle, staged.data_ptr(), y.data_ptr(), tokens, self._stream(y)))
         return y
 
     def add_rmsnorm_staged(self, h: torch.Tensor, delta: torch.Tensor | None, weight: torch.Tensor, staged: torch.Tensor, eps: float) -> None:
         tokens, hidden = h.shape
-        if staged.numel() < self._lib.tx_staged_prompt_bytes(hidden, tokens):
-            raise RuntimeError("the staged buffer is too small")
+        self._check_staged(staged, hidden, tokens, h.get_device())
         self._check(self._lib.tx_aux_add_rmsnorm_staged(h.data_ptr(), delta.data_ptr() if delta is not None else None, weight.data_ptr(),
                                                         staged.data_ptr(), tokens, hidden, eps, self._stream(h)))
 
@@ -413,8 +422,7 @@ class _Extension:
 
     def silu_mul_pairs_staged(self, gate_up: torch.Tensor, staged: torch.Tensor, accurate: bool = False) -> None:
         tokens, two_i = gate_up.shape
-        if staged.numel() < self._lib.tx_staged_prompt_bytes(two_i // 2, tokens):
-            raise RuntimeError("the staged buffer is too small")
+        self._check_staged(staged, two_i // 2, tokens, gate_up.get_device())
         self._check(self._lib.tx_aux_silu_mul_pairs_staged(gate_up.data_ptr(), staged.data_ptr(), tokens, two_i // 2, int(accurate), self._stream(gate_up)))
 
     def embed_rmsnorm(self, table: torch.Tensor, row_tokens: torch.Tensor, h: torch.Tensor, weight: torch.Tensor, y: torch.Tensor, eps: float,
@@ -422,6 +430,12 @@ class _Extension:
         """``h = table[row_tokens]`` (int64, one per row), ``y = rmsnorm(h) * weight``.  A token outside the table leaves status 33 and a row of ``y``
         that is not a number, and stores 1 to ``unknown`` (one int32, pinned: the host then sees it without a synchronisation)."""
         tokens, hidden = h.shape
+        if row_tokens.dtype != torch.int64 or row_tokens.numel() != tokens or not row_tokens.is_contiguous():
+            raise RuntimeError("embed_rmsnorm: one int64 token a row")
+        if table.dtype != torch.bfloat16 or table.dim() != 2 or table.shape[1] != hidden or not table.is_contiguous():
+            raise RuntimeError("embed_rmsnorm: the table is contiguous BF16 [vocab, hidden]")
+        if not h.is_cuda or not table.get_device() == row_tokens.get_device() == weight.get_device() == y.get_device() == h.get_device():
+            raise RuntimeError("embed_rmsnorm: tensors on one CUDA device")
         self._check(self._lib.tx_aux_embed_rmsnorm_watched(table.data_ptr(), table.shape[0], row_tokens.data_ptr(), h.data_ptr(), weight.data_ptr(),
                                                            y.data_ptr(), tokens, hidden, eps, unknown.data_ptr() if unknown is not None else None,
                                                            h.device.index, self._stream(h)))
