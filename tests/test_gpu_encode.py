@@ -198,3 +198,27 @@ def test_blocks_of_tiny_moments_in_a_large_matrix_get_the_bytes_of_their_slabs(e
     rows = ((1 << 21) - 1) // k
     slabs = torch.cat([ext.encode(w[i:i + rows], hdiag, table)[0] for i in range(0, m, rows)])
     assert torch.equal(blocks, slabs)
+
+
+def test_the_software_palette_takes_the_quadratic_form(ext, lut):
+    """Both ways through a block give the same bytes, so what shows which one ran is its time: half of the other's (75 and 157 us)."""
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    w, hdiag = torch.randn(4096, 4096, device="cuda", generator=gen) * 0.02, torch.exp(torch.randn(4096, device="cuda", generator=gen))
+    software = torch.from_numpy(lut).cuda()
+    other = software.clone()
+    other[60, 190, 4] += 1e-3
+    times = []
+    for table in (software, other):
+        call = lambda: ext.encode(w, hdiag, table)
+        assert [name for name, _, _ in recorded(call) if "encode_kernel" in name and "ELb1ELb1E" in name]
+        best = float("inf")
+        for _ in range(5):
+            begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            begin.record()
+            for _ in range(10):
+                call()
+            end.record()
+            end.synchronize()
+            best = min(best, begin.elapsed_time(end))
+        times.append(best)
+    assert times[0] < 0.75 * times[1], times

@@ -266,7 +266,7 @@ def test_hardware_palettes_and_texture_gate(ext, lut, tmp_path, monkeypatch):
 
 
 @pytest.mark.parametrize("tokens,k,m", [(16, 256, 200), (17, 1168, 300), (33, 2048, 128), (700, 5120, 640), (1, 144, 64), (40, 16384, 128),
-                                        (303, 2064, 64), (595, 4096, 64), (601, 8192, 64), (593, 8208, 64)])     # two and four rows a CTA
+                                        (303, 2064, 64), (595, 4096, 64), (601, 8192, 64), (593, 8208, 64)])     # two rows a CTA, and one
 def test_staged_activations_give_the_linear_of_their_rows(ext, lut, tokens, k, m):
     """A norm or a SwiGLU that writes the tile's form, then the tile: the bits of the rows' own linear, at edges of 128-column units and 32
     tokens, whichever tile; and refused where the linear would not take one."""
@@ -406,5 +406,29 @@ def test_two_tiles_an_sm_where_they_fill_waves(ext, hardware, m, k, tokens, back
         expected = f"prefill_umma_kernelILi1ELi{ {8: 64, 7: 128}[backend] }ELb{int(hardware)}ELi{groups}E"
         assert any(expected in name for name in names), names
         assert torch.equal(out[0], want) and ext.kernel_status() == 0
+    finally:
+        ext.free(h)
+
+
+@pytest.mark.parametrize("m,k,tokens,backend,inside", [
+    (256, 2048, 16, 5, True), (256, 2048, 16, 7, True), (256, 2048, 16, 8, True), (256, 2048, 16, 9, True), (256, 2048, 16, 6, False),
+    (3968, 2896, 29, 8, True), (1024, 4096, 127, 7, True),
+    (4250, 2896, 29, 8, False), (2304, 8192, 40, 8, False),      # 34 clusters of four and 18 of eight: more than are resident at once
+])
+def test_k_ranges_are_added_by_clusters_where_all_are_resident(ext, m, k, tokens, backend, inside):
+    """One launch behind the staging where the clusters fit, else a second one that adds."""
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the cluster counts are those of 148 SMs")
+    from texelator_b200 import modeling
+    weight = torch.randn(m, k, device="cuda", generator=torch.Generator(device="cuda").manual_seed(m)) * 0.02
+    h = ext.pack_encoded_device(*modeling.encode_minmax_cuda(weight, modeling.software_palette_table("cuda")), None)
+    try:
+        ext.set_prefill(h, 1, 1024)
+        ext.set_prefill_backend(h, backend)
+        x = torch.randn(tokens, k, device="cuda").bfloat16()
+        kernels = [(name, grid) for name, grid in launched(lambda: ext.linear(h, x)) if "N2tx" in name]
+        tiles = [grid for name, grid in kernels if "prefill_umma" in name]
+        assert len(tiles) == 1 and tiles[0][2] > 1, kernels                       # K is cut
+        assert any("combine" in name for name, _ in kernels) != inside, kernels
     finally:
         ext.free(h)
