@@ -549,7 +549,7 @@ prefill_umma_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap x
         tmem_load32(tmem_base + (unsigned(quarter * 32) << 16) + unsigned(c * 32), v);
         scale_to(sums + c * 32 * kMmaM + quarter * 32 + lane, kMmaM, v, row_scale, token_scale[i], 32);
       }
-    } else if (ready && gridDim.z > 1) {
+    } else if (GROUPS == 2 && ready && gridDim.z > 1) {                        // (two_an_sm: the small form has one range)
 #pragma unroll
       for (int i = 0; i < kMost; ++i) {
         const int c = (warp >> 2) + i * kParts;
