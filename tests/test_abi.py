@@ -164,6 +164,12 @@ def test_no_product_code_imports_the_oracle():
         assert "oracle" not in text.replace("oracle/bc4_oracle.py", ""), path
 
 
+def test_unknown_handles_take_no_staged_activations():
+    """The library reads what a handle number points to, so a number that names none must not reach it."""
+    from texelator_b200 import runtime
+    assert runtime.extension().takes_staged(1234, 16) is False
+
+
 def test_staged_calls_refuse_what_they_cannot_read():
     """Buffers of another device or type, short ones and unknown handles are refused before anything is launched."""
     import torch

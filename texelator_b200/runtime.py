@@ -394,7 +394,7 @@ class _Extension:
 
     def takes_staged(self, handle: int, tokens: int) -> bool:
         """Whether ``linear_staged`` serves this many tokens (``linear`` would take a tile for them)."""
-        return self._lib.tx_linear_takes_staged(handle, tokens) == 1
+        return handle in self._shapes and self._lib.tx_linear_takes_staged(handle, tokens) == 1
 
     def linear_staged(self, handle: int, staged: torch.Tensor, y: torch.Tensor) -> torch.Tensor:
         """``linear_out`` of rows in staged form: the same result bit for bit."""
