@@ -432,3 +432,28 @@ def test_k_ranges_are_added_by_clusters_where_all_are_resident(ext, m, k, tokens
         assert any("combine" in name for name, _ in kernels) != inside, kernels
     finally:
         ext.free(h)
+
+
+def test_staged_calls_without_the_binding_give_the_same_outputs(ext, lut):
+    """The methods in Python serve where the native calls cannot be had: the same answers, outputs and refusals."""
+    from texelator_b200 import runtime
+    blocks, scales, x = _case(3, 300, 528, 40, lut)
+    h = _pack(ext, blocks, scales)
+    plain = runtime._Extension(ext._lib)
+    plain._shapes[h] = ext._shapes[h]
+    try:
+        x, weight = x.cuda(), torch.ones(528, device="cuda", dtype=torch.bfloat16)
+        outs = []
+        for one in (plain, ext):
+            assert [one.takes_staged(h, tokens) for tokens in (15, 16, 40)] == [False, True, True] and one.takes_staged(1234, 40) is False
+            staged, y = one.staged_buffer(528, 40, "cuda"), torch.empty(40, 300, device="cuda", dtype=torch.bfloat16)
+            one.add_rmsnorm_staged(x.clone(), None, weight, staged, 1e-6)
+            assert one.linear_staged(handle=h, staged=staged, y=y) is y
+            outs.append(y)
+            with pytest.raises(RuntimeError, match="too small"):
+                one.linear_staged(h, staged[:-4], y)
+            with pytest.raises(RuntimeError, match="does not take staged"):
+                one.linear_staged(h, staged, y[:8])
+        assert torch.equal(outs[0], outs[1])
+    finally:
+        ext.free(h)

@@ -23,12 +23,18 @@ namespace {
 
 using LinearFn = int (*)(uint64_t, const void *, void *, int, int, void *);
 using ErrorFn = const char *(*)();
+using StagedFn = int (*)(uint64_t, const void *, void *, int, void *);
+using TakesFn = int (*)(uint64_t, int);
+using BytesFn = size_t (*)(int, int);
 
 struct Shape {
   int64_t m, k;
   int device;
   LinearFn linear;
   ErrorFn last_error;
+  StagedFn staged;   // null where the library has none
+  TakesFn takes;
+  BytesFn bytes;
 };
 
 std::unordered_map<uint64_t, Shape> g_shapes;   // every access holds the GIL
@@ -39,7 +45,7 @@ PyObject *raise(const char *message) {
 }
 
 // positional or keyword arguments called `names[0..count)`; false with an exception set when they do not fit
-bool take_arguments(PyObject *const *args, Py_ssize_t nargs, PyObject *kwnames, const char *const *names, int count, PyObject **out) {
+bool take_arguments(PyObject *const *args, Py_ssize_t nargs, PyObject *kwnames, const char *const *names, int count, PyObject **out, const char *usage) {
   for (int i = 0; i < count; ++i) out[i] = i < nargs ? args[i] : nullptr;
   bool fits = nargs <= count;
   if (kwnames && fits) {
@@ -52,7 +58,7 @@ bool take_arguments(PyObject *const *args, Py_ssize_t nargs, PyObject *kwnames, 
     }
   }
   for (int i = 0; i < count; ++i) fits = fits && out[i];
-  if (!fits) PyErr_SetString(PyExc_TypeError, count == 2 ? "linear(handle, x)" : "linear_out(handle, x, y)");
+  if (!fits) PyErr_SetString(PyExc_TypeError, usage);
   return fits;
 }
 
@@ -60,8 +66,8 @@ bool take_arguments(PyObject *const *args, Py_ssize_t nargs, PyObject *kwnames, 
 // a view of one has its offset for an address: nothing may be launched on it.
 bool has_memory(const at::Tensor &t) { return t.numel() == 0 || (t.has_storage() && t.storage().data() != nullptr); }
 
-// the checks of texelator_cuda.cu:1332-1337; null with an exception set when one fails
-const Shape *check_input(PyObject *handle_object, PyObject *x_object, uint64_t *handle, const at::Tensor **x) {
+// null where no handle of that number is known
+const Shape *find(PyObject *handle_object, uint64_t *handle) {
   // any integer (NumPy's too); what is none, or does not fit, names no handle
   PyObject *number = PyNumber_Index(handle_object);
   *handle = number ? PyLong_AsUnsignedLongLong(number) : 0;
@@ -71,7 +77,13 @@ const Shape *check_input(PyObject *handle_object, PyObject *x_object, uint64_t *
     *handle = 0;
   }
   auto found = g_shapes.find(*handle);
-  if (found == g_shapes.end()) {
+  return found == g_shapes.end() ? nullptr : &found->second;
+}
+
+// the checks of texelator_cuda.cu:1332-1337; null with an exception set when one fails
+const Shape *check_input(PyObject *handle_object, PyObject *x_object, uint64_t *handle, const at::Tensor **x) {
+  const Shape *found = find(handle_object, handle);
+  if (!found) {
     raise("null Texelator handle");
     return nullptr;
   }
@@ -89,11 +101,11 @@ const Shape *check_input(PyObject *handle_object, PyObject *x_object, uint64_t *
     raise("input must be contiguous CUDA FP16 or BF16");
     return nullptr;
   }
-  if (t.dim() < 1 || t.size(-1) != found->second.k || t.get_device() != found->second.device) {
+  if (t.dim() < 1 || t.size(-1) != found->k || t.get_device() != found->device) {
     raise("input shape/device mismatch");
     return nullptr;
   }
-  return &found->second;
+  return found;
 }
 
 bool launch(uint64_t handle, const at::Tensor &x, const at::TensorBase &y, const Shape &shape) {
@@ -123,7 +135,7 @@ PyObject *linear(PyObject *, PyObject *const *args, Py_ssize_t nargs, PyObject *
   HANDLE_TH_ERRORS
   static const char *const names[] = {"handle", "x"};
   PyObject *given[2];
-  if (!take_arguments(args, nargs, kwnames, names, 2, given)) return nullptr;
+  if (!take_arguments(args, nargs, kwnames, names, 2, given, "linear(handle, x)")) return nullptr;
   uint64_t handle;
   const at::Tensor *x;
   const Shape *found = check_input(given[0], given[1], &handle, &x);
@@ -141,7 +153,7 @@ PyObject *linear_out(PyObject *, PyObject *const *args, Py_ssize_t nargs, PyObje
   HANDLE_TH_ERRORS
   static const char *const names[] = {"handle", "x", "y"};
   PyObject *given[3];
-  if (!take_arguments(args, nargs, kwnames, names, 3, given)) return nullptr;
+  if (!take_arguments(args, nargs, kwnames, names, 3, given, "linear_out(handle, x, y)")) return nullptr;
   uint64_t handle;
   const at::Tensor *x;
   const Shape *found = check_input(given[0], given[1], &handle, &x);
@@ -161,13 +173,63 @@ PyObject *linear_out(PyObject *, PyObject *const *args, Py_ssize_t nargs, PyObje
   END_HANDLE_TH_ERRORS
 }
 
+// Short prompts wait for the host: with this call and the question below in Python a prompt of 58 tokens through five layers of the 2048-wide model took 605 us,
+// 520 with rows and their staging launches.
+PyObject *linear_staged(PyObject *, PyObject *const *args, Py_ssize_t nargs, PyObject *kwnames) {
+  HANDLE_TH_ERRORS
+  static const char *const names[] = {"handle", "staged", "y"};
+  PyObject *given[3];
+  if (!take_arguments(args, nargs, kwnames, names, 3, given, "linear_staged(handle, staged, y)")) return nullptr;
+  uint64_t handle;
+  const Shape *found = find(given[0], &handle);
+  if (!found || !found->staged || !found->bytes) return raise("null Texelator handle");
+  const Shape shape = *found;
+  if (!THPVariable_Check(given[1]) || !THPVariable_Check(given[2])) {
+    PyErr_SetString(PyExc_TypeError, "staged activations and output must be tensors");
+    return nullptr;
+  }
+  const at::Tensor &staged = THPVariable_Unpack(given[1]), &y = THPVariable_Unpack(given[2]);
+  const int64_t tokens = y.numel() / shape.m;
+  if (!y.is_cuda() || y.scalar_type() != at::kBFloat16 || !y.is_contiguous() || y.get_device() != shape.device || y.numel() != tokens * shape.m || tokens > INT32_MAX)
+    return raise("input shape/device mismatch");
+  if (!staged.is_cuda() || staged.scalar_type() != at::kByte || !staged.is_contiguous() || staged.get_device() != shape.device)
+    return raise("staged activations are a contiguous uint8 tensor on the CUDA device of the rows");
+  if (size_t(staged.numel()) < shape.bytes(int(shape.k), int(tokens))) return raise("the staged buffer is too small");
+  if (!has_memory(staged) || !has_memory(y)) return raise("input shape/device mismatch");
+  void *stream = c10::cuda::getCurrentCUDAStream(c10::DeviceIndex(shape.device)).stream();
+  const void *in = staged.const_data_ptr();
+  void *out = y.mutable_data_ptr();
+  int status;
+  Py_BEGIN_ALLOW_THREADS
+  status = shape.staged(handle, in, out, int(tokens), stream);
+  Py_END_ALLOW_THREADS
+  if (status != 0) {
+    const char *message = shape.last_error();
+    return raise(message && message[0] ? message : "texelator_b200 call failed");
+  }
+  return Py_NewRef(given[2]);
+  END_HANDLE_TH_ERRORS
+}
+
+PyObject *takes_staged(PyObject *, PyObject *const *args, Py_ssize_t nargs, PyObject *kwnames) {
+  static const char *const names[] = {"handle", "tokens"};
+  PyObject *given[2];
+  if (!take_arguments(args, nargs, kwnames, names, 2, given, "takes_staged(handle, tokens)")) return nullptr;
+  const long tokens = PyLong_AsLong(given[1]);
+  if (tokens == -1 && PyErr_Occurred()) return nullptr;
+  uint64_t handle;
+  const Shape *found = find(given[0], &handle);
+  return PyBool_FromLong(found && tokens > 0 && tokens <= INT32_MAX && found->takes && found->takes(handle, int(tokens)) == 1);
+}
+
 PyObject *remember(PyObject *, PyObject *args) {
-  unsigned long long handle, linear_address, error_address;
+  unsigned long long handle, linear_address, error_address, staged_address, takes_address, bytes_address;
   long long m, k;
   int device;
-  if (!PyArg_ParseTuple(args, "KLLiKK", &handle, &m, &k, &device, &linear_address, &error_address)) return nullptr;
+  if (!PyArg_ParseTuple(args, "KLLiKKKKK", &handle, &m, &k, &device, &linear_address, &error_address, &staged_address, &takes_address, &bytes_address)) return nullptr;
   HANDLE_TH_ERRORS
-  g_shapes[handle] = Shape{m, k, device, reinterpret_cast<LinearFn>(linear_address), reinterpret_cast<ErrorFn>(error_address)};
+  g_shapes[handle] = Shape{m, k, device, reinterpret_cast<LinearFn>(linear_address), reinterpret_cast<ErrorFn>(error_address),
+                           reinterpret_cast<StagedFn>(staged_address), reinterpret_cast<TakesFn>(takes_address), reinterpret_cast<BytesFn>(bytes_address)};
   Py_RETURN_NONE;
   END_HANDLE_TH_ERRORS
 }
@@ -183,7 +245,10 @@ PyObject *forget(PyObject *, PyObject *args) {
 PyMethodDef methods[] = {
     {"linear", TX_FAST(linear), "linear(handle, x) -> tensor [..., M]"},
     {"linear_out", TX_FAST(linear_out), "linear_out(handle, x, y) -> y, for outputs the caller keeps (CUDA graphs)"},
-    {"remember", remember, METH_VARARGS, "remember(handle, m, k, device, address of tx_linear, address of tx_last_error)"},
+    {"linear_staged", TX_FAST(linear_staged), "linear_staged(handle, staged, y) -> y, rows that the kernel in front left in staged form"},
+    {"takes_staged", TX_FAST(takes_staged), "takes_staged(handle, tokens) -> bool"},
+    {"remember", remember, METH_VARARGS,
+     "remember(handle, m, k, device, addresses of tx_linear, tx_last_error, tx_linear_staged, tx_linear_takes_staged and tx_staged_prompt_bytes)"},
     {"forget", forget, METH_VARARGS, "forget(handle)"},
     {nullptr, nullptr, 0, nullptr}};
 

@@ -15,6 +15,7 @@ There is no CPU fallback: if the CUDA library is missing and cannot be built,
 from __future__ import annotations
 
 import ctypes
+import functools
 import gc
 import json
 import os
@@ -131,10 +132,13 @@ class _Extension:
     def __init__(self, library: ctypes.CDLL, binding=None):
         self._lib, self._binding = library, binding
         self._shapes: dict[int, tuple[int, int, int]] = {}   # handle -> (M, K, device)
+        # bytes of (columns, tokens) in staged form; every staged call of a prompt asks, and a short prompt's launches wait for the host
+        self.staged_bytes = functools.lru_cache(maxsize=256)(lambda columns, tokens: library.tx_staged_prompt_bytes(columns, tokens))
         if binding is not None:
-            address = lambda function: ctypes.cast(function, ctypes.c_void_p).value
-            self._entry = address(library.tx_linear), address(library.tx_last_error)
+            address = lambda name: ctypes.cast(getattr(library, name, None), ctypes.c_void_p).value or 0     # (0: not in this library)
+            self._entry = tuple(map(address, ("tx_linear", "tx_last_error", "tx_linear_staged", "tx_linear_takes_staged", "tx_staged_prompt_bytes")))
             self.linear, self.linear_out = binding.linear, binding.linear_out
+            self.linear_staged, self.takes_staged = binding.linear_staged, binding.takes_staged
 
     def _remember(self, handle: int, m: int, k: int, device: int) -> int:
         self._shapes[handle] = (m, k, device)
@@ -382,9 +386,6 @@ class _Extension:
     def staged_buffer(self, columns: int, tokens: int, device) -> torch.Tensor:
         """A buffer for ``tokens`` rows of up to ``columns`` activations in staged form."""
         return torch.empty(self.staged_bytes(columns, tokens), dtype=torch.uint8, device=device)
-
-    def staged_bytes(self, columns: int, tokens: int) -> int:
-        return self._lib.tx_staged_prompt_bytes(columns, tokens)
 
     def _check_staged(self, staged: torch.Tensor, columns: int, tokens: int, device: int) -> None:
         if device < 0 or staged.dtype != torch.uint8 or not staged.is_contiguous() or staged.get_device() != device:
