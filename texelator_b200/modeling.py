@@ -355,9 +355,10 @@ class BC4Decoder:
         make = lambda columns: torch.empty(tokens, columns, dtype=torch.bfloat16, device=self.device)
         x, qkv, gate_up, out = make(c.hidden), make(self.q_loc + 2 * self.kv_loc), make(2 * self.i_loc), make(c.hidden)
         # SwiGLU's rows and what the norms (or SwiGLU) hand over staged are never needed at the same time: one buffer, the rows at its start
-        staged_columns = max(c.hidden, self.i_loc if ext.stages_swiglu(tokens, self.i_loc) else 0)
-        staged = torch.empty(max(ext.staged_bytes(staged_columns, tokens), 2 * tokens * self.i_loc), dtype=torch.uint8, device=self.device)
-        act = staged[:2 * tokens * self.i_loc].view(torch.bfloat16).view(tokens, self.i_loc)
+        stages_swiglu = ext.stages_swiglu(tokens, self.i_loc)
+        needed = ext.staged_bytes(max(c.hidden, self.i_loc) if stages_swiglu else c.hidden, tokens)
+        space = torch.empty(max(tokens, -(-needed // (2 * self.i_loc))), self.i_loc, dtype=torch.bfloat16, device=self.device)
+        act, staged = space[:tokens], space.view(torch.uint8)
         q = qkv[:, :self.q_loc].view(tokens, q_heads, c.head_dim).transpose(0, 1).unsqueeze(0)
 
         def normed(handle, delta, weight, out):
@@ -378,7 +379,7 @@ class BC4Decoder:
             attended = attended.squeeze(0).transpose(0, 1).reshape(tokens, self.q_loc).contiguous()
             delta = self._reduce(ext.linear_out(self.h_o[layer], attended, out))
             normed(self.h_gu[layer], delta, self.norm2[layer], gate_up)
-            if ext.stages_swiglu(tokens, self.i_loc) and ext.takes_staged(self.h_down[layer], tokens):
+            if stages_swiglu and ext.takes_staged(self.h_down[layer], tokens):
                 ext.silu_mul_pairs_staged(gate_up, staged, accurate=True)
                 ext.linear_staged(self.h_down[layer], staged, out)
             else:
