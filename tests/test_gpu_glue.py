@@ -371,7 +371,7 @@ def test_embed_rmsnorm_of_an_unknown_token_is_not_a_number(ext, tokens, hidden, 
 @pytest.mark.parametrize("sequences,q_heads,kv_heads,max_len,positions", [
     (16, 40, 8, 1040, [0, 1, 15, 16, 17, 63, 64, 65, 127, 128, 500, 640, 1000, 1023, 1024, 1039]),   # two splits: a cluster
     (3, 8, 8, 700, [699, 16, 448]),                          # a chunk a CTA, merged behind
-    (5, 64, 8, 1000, [999, 0, 64, 300, 15]),                 # eight heads a kv head, a cluster of seven
+    (5, 64, 8, 1000, [999, 0, 64, 300, 15]),                 # eight heads a kv head, seven splits, merged behind
     (2, 24, 8, 2900, [2899, 1300]),                          # eighteen splits of several chunks: merged behind
     (40, 16, 8, 400, [(37 * i) % 400 for i in range(40)]),   # one split: written directly
 ])

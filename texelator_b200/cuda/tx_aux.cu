@@ -76,7 +76,8 @@ __device__ __forceinline__ void stage_rows(uint8_t *staged, const uint8_t *rows_
   }
 }
 // EMBED: the first norm of a decode step.  A row of h is the embedding of the row's token, fetched here and stored for the residual
-// (a launch of its own before: 16 rows of 5120 14.2 us, of which the wait for one more kernel in the chain is most; one row 2.0).
+// (a launch of its own before: 16 rows of 5120 14.2 us, of which the wait for one more kernel in the chain is most; one row 2.0).  A row is gathered without
+// the library call's assertion on the token, which ended the program: EmbedRows says what takes its place.
 struct EmbedRows {
   const __nv_bfloat16 *table;   // [vocab, hidden]
   const long long *tokens;
@@ -1193,16 +1194,19 @@ __global__ void __launch_bounds__(kStepThreads, 2) attention_step_kernel(const _
 
 // The same step for long caches and batches: the grid is capped at two resident CTAs per SM and every CTA walks several
 // 64-key chunks (chunk = split, split + gridDim.x, ...) with running soft-max statistics.  A ring of chunks in shared memory, filled by cp.async, keeps
-// HBM busy across the chunk's barriers; the first chunks are requested before the wait for the launch in front, like the kernel above.  Products,
-// sums and their order are the kernel's above.
+// HBM busy across the chunk's barriers; the first chunks are requested before the wait for the launch in front, like the kernel above.  A chunk's products
+// and sums are the kernel's above; several chunks of a CTA are added in one set of sums that is rescaled when the maximum moves, where that
+// kernel leaves a record a chunk, so the two agree to rounding.
 //
 // DIRECT (a batch with up to eight splits, which are a cluster; splits_meet_in_clusters): the splits meet in distributed shared memory, with the arithmetic of
 // attention_merge_kernel, and that launch falls away.
 //
 // What bounds it: HBM for long batches, else the chain of a chunk (three barriers).  us a call with the merge (a graph over caches larger than L2), 40 query
-// heads on 8 kv heads, rows in registers requested when the ones before were used up / this: 16 sequences of 500 to 1000 positions 31.7 / 26.1, 32 of 2000
-// to 4000 193 / 152; 64 heads on 8, 8 of 1000 to 2000 42.7 / 33.9.  (Tensor cores, a warp to sixteen keys and no barriers, take 14.0, 73 and 15.2, but add in
-// another order: with logits that tie, a decoder then picks other tokens than the one-sequence kernel above.)
+// heads on 8 kv heads, rows in registers requested when the ones before were used up / this: 16 sequences of 500 to 1000 positions 31.7 / 25.5, 32 of 2000
+// to 4000 193 / 152; one of 5000 14.9 / 12.6, 8300 18.7 / 15.4, 32768 49.6 / 39.7; 64 heads on 8, 8 of 1000 to 2000 42.7 / 33.3, one of 8300 24.2 / 19.7 (16 to 44
+// bytes a thread spill with five heads and more where the splits are merged by a launch).
+// (Tensor cores, a warp to sixteen keys and no barriers, take 14.0, 73 and 15.2, but round otherwise: with logits that tie, a decoder then
+// picks other tokens than before.)
 constexpr int kRingStages = 3, kChunkBytes = kStepKeys * kHeadDim * 2 * 2;   // keys, then values
 constexpr size_t kRingSmem = size_t(kRingStages) * kChunkBytes;
 __device__ __forceinline__ void cluster_barrier() {

@@ -331,8 +331,9 @@ __device__ __forceinline__ void stage_piece(uint4 *staged, int padded_tokens, in
 // One row by the CTAs of a cluster (blockIdx.x the share, blockIdx.y the token): every CTA takes a run of half units, the largest magnitudes meet
 // through distributed shared memory.  For few tokens: a CTA a row leaves most SMs idle and a long row is a long chain (16 rows of 17408 columns
 // took 9.8 us that way).  From kSplitColumns columns on: a linear of 5120 x 17408 with 16 and 64 tokens
-// 26.8 -> 23.5 and 28.4 -> 24.3 us, 8192 x 28672 49.0 -> 41.4 and 51.3 -> 46.9, but 2048 x 11008 with 29 13.4 -> 14.1 and 5120 x 5120 with 16 12.0 -> 13.6 (a cluster's
-// launch).  piece(i): eight columns as bf16 (or, half_in, fp16), asked for once where a thread has up to kSplitHeld of them.
+// 21.7 -> 19.6 and 26.4 -> 24.1 us, 8192 x 28672 45.0 -> 38.6 and 49.5 -> 43.5, but 2048 x 11008 with 29 13.4 -> 14.1 and 5120 x 5120 with 16 12.0 -> 13.6 (a cluster's
+// launch).  At the line, 2048 x 12288 with 16, 32, 64, 96, 128 and 148 tokens: 13.6 -> 11.6, 13.7 -> 14.2, 13.6 -> 13.5, 21.4 -> 22.5, 23.5 -> 23.5, 28.4 -> 26.3; 5120 x 17408
+// with 96, 128 and 148: 43.9 -> 42.4, 44.5 -> 41.9, 46.8 -> 47.4.  piece(i): eight columns as bf16 (or, half_in, fp16), asked for once where a thread has up to kSplitHeld of them.
 constexpr int kSplitThreads = 256, kSplitHeld = 4, kSplitColumns = 12288;
 template <typename Piece>
 __device__ __forceinline__ void stage_split_row(uint4 *staged, float *multipliers, int K, int padded_tokens, bool half_in, Piece piece) {

@@ -18,10 +18,10 @@
 //                        entry it is: packed subtractions (two weights per instruction) and three-input minima, ten instructions per
 //                        weight and neighbour.  Selectors are found twice (start and winner).  About 2900 instructions.
 //   encode_block_spaced  the software palette: weights are assigned by rounding, the nine errors come from a quadratic form and what is
-//                        too close to call is evaluated the first way.  About 1600 instructions, 64 % of the issue slots.
+//                        too close to call is evaluated the first way.  About 1600 instructions, 69 % of the issue slots.
 //
-// us a call, all blocks the first way / as launched: 4096 x 4096 156.8 / 80.4, 11000 x 11008 1097 / 505, 9000 x 2000 182.6 / 99.0;
-// 4096 x 4096 with nine weights of ten zero 166 / 171, under the texture palette 156 / 162 (the verdict).
+// us a call, all blocks the first way / as launched: 4096 x 4096 156.2 / 75.7, 12000 x 4096 453 / 209, 34816 x 5120 1548 / 723, 2048 x 1024 23.2 / 16.6;
+// 4096 x 4096 with nine weights of ten zero 164.7 / 166.8, under the texture palette 156.0 / 157.2 (the verdict).
 #include "tx_common.cuh"
 
 namespace tx {
@@ -512,7 +512,7 @@ __global__ void __launch_bounds__(kVerdictThreads) palette_verdict_kernel(const 
     blocks[size_t(i / shares) * cta_bytes + size_t(i % shares) * share_bytes + blockIdx.x] = same ? 1 : 0;
 }
 
-// From here on the verdict pays: 2000 x 1040 takes 37.0 us without it and 28.2 with; 300 x 4096, half the size, 20.6 and 20.7.
+// From here on the verdict pays: 2048 x 1024 takes 23.2 us without it and 16.6 with; 300 x 4096, half the size, 20.6 and 20.7.
 constexpr size_t kSpacedWeights = size_t(1) << 21;
 constexpr int kEncodeWave = 148 * 4;   // blocks of threads resident at once (registers)
 

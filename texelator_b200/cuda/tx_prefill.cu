@@ -710,15 +710,14 @@ static bool two_an_sm(long ctas, int ranges, int units, int sm_count, bool gener
 // (136 stages): 0.30, 0.35, 0.50 and 0.67 us a stage for 64, 128, 192 and 256 tokens and about 4 us a CTA; the tile with
 // the smallest sum over the waves wins, the wider one on a tie (it reads the activations less often).  The sums are those of one CTA an SM also where
 // two_an_sm would take two: the line then lies a little late for short rows (24576x1024 with 700 tokens: 128-token tile 38.6, 192 tokens 42.5 us).
-// The pair tile (id 6)
-// is left out: against the 256-token tile it measured between 6 % less and 13 % more for 512 to 4096 tokens, by the
+// The pair tile (id 6) is left out: against the 256-token tile it measured between 6 % less and 13 % more for 512 to 4096 tokens, by the
 // GPU's power state more than by shape, and never less below that.
 //
 // Up to eight tokens (a threshold below the default of 16) the decode kernel keeps the call: it pays one group of MMA columns
-// there, and two from nine on.  Decode kernel against the 64-token tile, us a call from HBM with one, eight, ten and fifteen
-// tokens: 256x2048 2.7 / 6.9, 3.8 / 7.3, 4.6 / 7.4, 4.9 / 7.5; 5120x5120 6.3 / 11.4, 9.4 / 11.9, 11.3 / 12.1, 11.8 / 12.6;
-// 34816x5120 22.4 / 31.6, 29.3 / 31.9, 35.5 / 32.1, 38.3 / 32.0.  From nine tokens on the tile is the faster one on the widest
-// matrices alone; the line was drawn for a decode kernel that took 11.2, 20.0 and 51.5 us for ten.
+// there, and two from nine on.  Decode kernel against the 64-token tile, us a call from HBM with one, eight, nine and fifteen
+// tokens: 256x2048 2.7 / 5.9, 3.8 / 6.0, 4.5 / 6.0, 5.0 / 6.3; 2560x2048 3.4 / 6.1, 4.5 / 6.1, 5.3 / 6.2, 5.7 / 6.4; 5120x5120 6.2 / 9.3, 9.3 / 9.6,
+// 11.1 / 9.6, 11.8 / 10.2; 22016x2048 8.1 / 13.4, 12.7 / 13.4, 14.8 / 13.5, 17.0 / 13.5; 34816x5120 22.6 / 28.6, 29.0 / 28.7, 35.1 / 28.9, 38.7 / 29.4.
+// From nine tokens on the tile is the faster one but on matrices of few rows.
 //
 // Distance from 64 bits, tile against decode kernel, which adds a row in sixteen shorter chains: on Gaussian activations
 // both end at the output's rounding (fp16, 11008x2048, 160 tokens: 2.0759e-4 and 2.0757e-4 of the result; bf16 equal to

@@ -56,7 +56,7 @@ class DecoderConfig:
 
 
 CONFIGS = {
-    # BASELINE.json configs[1], [3], [4] and a toy model for tests
+    # the shapes of the benchmark and of its batched and tensor-parallel runs, and toy models for tests
     "qwen2.5-3b-shaped": DecoderConfig("qwen2.5-3b-shaped", 2048, 36, 16, 2, 128, 11008, 151936, qkv_bias=True),
     "27b-class": DecoderConfig("27b-class", 5120, 64, 40, 8, 128, 17408, 151936),
     "70b-class": DecoderConfig("70b-class", 8192, 80, 64, 8, 128, 28672, 128256, rope_theta=5e5),
